@@ -46,17 +46,18 @@ def listed():
         # the cube on which transforms are compared, in both precision forms
         dict(_case("transform", "plain", (256, 256, 256)), name="transform_256"),
         dict(_case("transform", "mixed", (256, 256, 256)), name="transform_256_mixed"),
-        # the default grid: physical fields of a state, as written out or fed to diagnostics
-        dict(_case("fields", "plain", (256, 128, 128)), name="fields_256x128x128"),
+        # the default grid: one nonlinear term
+        dict(_case("advect", "plain", (256, 128, 128)), name="advect_256x128x128"),
         # a small ragged vortex run in the mixed form
         dict(_case("run", "mixed", (96, 120, 90), (96, 41, 31), steps=10, dt=2.0e-4, is_svv=1), name="run_ragged_mixed"),
         # the vortex run that the library is quoted on, in both precision forms
         dict(_case("run", "mixed", (192, 128, 128), steps=10, dt=2.0e-4, visc=1.0e-4, is_svv=1), name="run_192_mixed"),
         dict(_case("run", "plain", (192, 128, 128), steps=4, dt=2.0e-4, visc=1.0e-4, is_svv=1), name="run_192"),
-        # gradient of the perturbation energy on the sensitivity study's grid
-        dict(_case("adjoint", "plain", (128, 64, 64), steps=10, dt=2.0e-3, visc=2.0e-4, ckpt=5), name="adjoint_128"),
-        # the large grid: one nonlinear term in the plain form, steps in the mixed form
-        dict(_case("advect", "plain", (512, 512, 256), ell=6.0, visc=5.0e-5), name="advect_512"),
+        # gradient of the perturbation energy over a horizon
+        dict(_case("adjoint", "plain", (40, 64, 64), steps=10, dt=2.0e-3, ckpt=5), name="adjoint_40"),
+        # the large grid: physical fields of a state, as written out or fed to diagnostics, in the plain form, and
+        # steps in the mixed form
+        dict(_case("fields", "plain", (512, 512, 256), ell=6.0, visc=5.0e-5), name="fields_512"),
         dict(_case("run", "mixed", (512, 512, 256), ell=6.0, steps=2, dt=2.0e-4, visc=5.0e-5, is_svv=1), name="run_512_mixed"),
     ]
 
@@ -79,21 +80,25 @@ def _fft_size(v):
 
 # points of the grid times steps that keep a drawn case within the largest listed one, by operation and form
 MOST = {("transform", "plain"): 67e6, ("transform", "mixed"): 67e6, ("diffuse", "plain"): 67e6, ("diffuse", "mixed"): 67e6,
-        ("fields", "plain"): 33e6, ("fields", "mixed"): 67e6, ("advect", "plain"): 20e6, ("advect", "mixed"): 33e6,
+        ("fields", "plain"): 33e6, ("fields", "mixed"): 67e6, ("advect", "plain"): 17e6, ("advect", "mixed"): 33e6,
         ("run", "plain"): 20e6, ("run", "mixed"): 60e6, ("adjoint", "plain"): 5e6, ("adjoint", "mixed"): 5e6}
+# radial points up to which nonlinear terms and gradients are drawn: beyond, the inverse Laplacian of the (m, k) =
+# (0, 0) column (and its transpose, in the gradient) magnifies the last bit of 64-bit arithmetic a millionfold and
+# more, and two right answers differ visibly there; gradients in the plain form for the same reason
+MOST_NR = {"advect": 256, "run": 256, "adjoint": 48}
 
 
 def draw(rng):
-    """One more case of the listed ranges: grids of 24 to 512 radial points, powers of two and products of 2, 3
+    """One more case of the listed ranges: grids of 24 to 512 radial points (see MOST_NR), powers of two and products of 2, 3
     and 5 along the periodic directions, full and short truncations, both forms."""
     op = rng.choice(("transform", "transform", "diffuse", "fields", "advect", "run", "run", "adjoint"))
-    precision = rng.choice(("plain", "mixed"))
+    precision = rng.choice(("plain", "mixed")) if op != "adjoint" else "plain"
     steps = {"run": rng.randint(2, 10), "diffuse": rng.randint(1, 4), "adjoint": rng.choice((4, 8))}.get(op, 1)
     flat = op in ("transform", "diffuse") and rng.random() < 0.2
     pow2 = rng.random() < 0.5
     fft_ok = (lambda v: v >= 4 and v & (v - 1) == 0) if pow2 else _fft_size
     while True:
-        nr = _size(rng, 24, 512, lambda v: v % 2 == 0)
+        nr = _size(rng, 24, MOST_NR.get(op, 512), lambda v: v % 2 == 0)
         np_ = _size(rng, 16, 512, fft_ok)
         nz = 1 if flat else _size(rng, 12, 256, fft_ok)
         if nr * np_ * nz * steps <= MOST[op, precision]:
@@ -191,7 +196,7 @@ def _vortex(c, seed):
     out = []
     for i, f in enumerate((2.0, 0.25)):
         col, ln = _axis_column(c, -f * np.exp(-r ** 2) / (1.0 - x) ** 2)
-        e = _noise(c, 2 * seed + i, 1.0e-4, 0.3, 4, 8)
+        e = _noise(c, 2 * seed + i, 1.0e-2, 1.0, 4, 8)
         e[0, 0, : len(col)] += torch.from_numpy(col).to(e.device)
         out.append((e, ln))
     return out
@@ -208,7 +213,7 @@ def _inputs(c, seed):
     d = {"psi": psi, "chi": chi}
     if c["op"] == "run":
         for i, n in enumerate(("nlpsi", "nlchi", "nlpsi_p", "nlchi_p")):
-            d[n] = (_noise(c, 7 * seed + 3 + i, 1.0e-4, 0.3, 4, 8), 0.0)
+            d[n] = (_noise(c, 7 * seed + 3 + i, 1.0e-2, 1.0, 4, 8), 0.0)
         d["psi_p"], d["chi_p"] = psi, chi
     return d
 
