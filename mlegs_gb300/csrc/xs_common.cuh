@@ -7,6 +7,13 @@
 //   d_s in [0, 2^w) for s > 0.
 // Every digit is an exact BF16 and every digit product an exact FP32 integer of magnitude <= 2^(2w), so
 // a K-term sum of the products of one digit order stays exact while K (pairs of the order) 2^(2w) < 2^24.
+// Balanced digits (nb = 63): the digits after the first lie in [-2^(w-1), 2^(w-1)) and the first, of
+// eight bits, in [-128, 128), so a digit product is at most 2^(2w-2) (2^(w+6) with one first digit, 2^14 with two) and
+// the order sums stay exact for 8 digits of 8 bits up to K = 128 and for 9 of 7 bits up to K = 372 (unsigned digits
+// need 9 of 7 bits up to K = 113 and 10 of 6, 60 bits, beyond).
+// The first digit needs |X| < 2^63 - 2^56, so that the carry of the digits below it does not leave its eight bits: the
+// scale E of a row or column whose largest magnitude has its upper six fraction bits set is one larger
+// (xs_ebound_bal).
 // All conversions run on the integer and FP32 pipes: GB300 issues FP64 at about 2 operations per clock
 // per SM.
 #pragma once
@@ -34,6 +41,61 @@ __device__ __forceinline__ long long xs_fix(double x, int E, int nb) {
   if (sh >= 0) X = (sh <= 10) ? (M << sh) : 0ull;  // sh < nb - 52 <= 11 when |x| < 2^E
   else X = (sh > -63) ? ((M + (1ull << (-sh - 1))) >> (-sh)) : 0ull;
   return (b >> 63) ? -(long long)X : (long long)X;
+}
+
+// exponent bound for balanced digits from a magnitude's high word: |v| < 2^E (1 - 2^-7)
+__device__ __forceinline__ int xs_ebound_bal(unsigned abshi) { return (int)((abshi + 0x4000u) >> 20) - 1022; }
+
+// the shift base of xs_fixs for a scale E; `ok` false (no column, or an all-zero one): every value gives 0
+__device__ __forceinline__ int xs_fix_base(int E, int nb, bool ok) { return ok && E > -2000 ? 1085 - nb + E : (1 << 20); }
+// xs_fix with the shift base worked out once per column.  The significand starts at bit 63 and is shifted right only
+// (by base - exponent >= 0, clamped to 64 by the instruction) with one bit to spare, which the rounding consumes:
+// halves go away from zero, as in xs_fix.
+__device__ __forceinline__ long long xs_fixs(double x, int base) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const int e = (int)((hi >> 20) & 0x7FFu);
+  int r = base - e;
+  if ((unsigned)(e - 1) >= 0x7FEu) r = 64;   // zero, subnormal, non-finite
+  const unsigned mh = __funnelshift_l(lo, hi, 11) | 0x80000000u, ml = lo << 11;
+  unsigned long long M = ((unsigned long long)mh << 32) | ml, X;
+  asm("shr.u64 %0, %1, %2;" : "=l"(X) : "l"(M), "r"(r));
+  X = (X + 1) >> 1;
+  const long long sg = (long long)((int)hi >> 31);
+  return (long long)(X ^ (unsigned long long)sg) - sg;
+}
+
+// the offset that makes every balanced digit non-negative: 2^(w-1) in the place of each digit, 128 in the first one's
+template <int NS, int W> __host__ __device__ constexpr unsigned long long xs_bias() {
+  unsigned long long b = 128ull << (W * (NS - 1));
+  for (int s = 0; s < NS - 1; ++s) b += (1ull << (W - 1)) << (W * s);
+  return b;
+}
+// a.x - c, a.y - c for the two FP32 bit patterns a0, a1, in one instruction; returned as a packed BF16 pair (the
+// results are small integers, so their BF16 patterns are their upper halves)
+__device__ __forceinline__ uint32_t xs_sub2_pack(uint32_t a0, uint32_t a1, float c) {
+  unsigned long long v, d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(a0), "r"(a1));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(-c), "f"(-c));
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(v), "l"(d));
+  return __byte_perm((uint32_t)v, (uint32_t)(v >> 32), 0x7632);
+}
+// digit S of the values X0, X1 (balanced: X + xs_bias) as a packed BF16 pair (X0 low): the digit's bits are put into
+// the fraction of 2^23, and one packed FP32 subtraction takes 2^23 (and the balanced digit's offset) away again
+template <int NS, int W, bool BAL, int S> __device__ __forceinline__ uint32_t xs_digit2(unsigned long long X0, unsigned long long X1) {
+  constexpr int SH = W * (NS - 1 - S);
+  static_assert(!BAL || W * (NS - 1) == 56, "the first balanced digit is the upper byte");
+  if constexpr (BAL && (W == 8 || S == 0)) {   // digits that are bytes
+    constexpr unsigned sel = 0x7440u + (SH & 31) / 8;
+    const unsigned a = SH >= 32 ? (unsigned)(X0 >> 32) : (unsigned)X0, b = SH >= 32 ? (unsigned)(X1 >> 32) : (unsigned)X1;
+    return xs_sub2_pack(__byte_perm(a, 0x4B000000u, sel), __byte_perm(b, 0x4B000000u, sel), 8388608.0f + 128.0f);
+  } else if constexpr (BAL || S > 0) {
+    constexpr unsigned mask = (1u << W) - 1u;
+    return xs_sub2_pack(((unsigned)(X0 >> SH) & mask) | 0x4B000000u, ((unsigned)(X1 >> SH) & mask) | 0x4B000000u,
+                        8388608.0f + (BAL ? (float)(1 << (W - 1)) : 0.0f));
+  } else {   // the signed first digit
+    return xs_sub2_pack(0x4B400000u + (unsigned)(int)((long long)X0 >> SH), 0x4B400000u + (unsigned)(int)((long long)X1 >> SH),
+                        12582912.0f);
+  }
 }
 
 // the FP32 value of a small integer (|d| < 2^22), exactly, on the FP32 pipe

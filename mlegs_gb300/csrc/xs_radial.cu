@@ -9,16 +9,14 @@
 // an exact BF16 and every digit product an exact FP32 integer.  The products of one digit order
 // d = t + s are summed over K in their own FP32 accumulator in tensor memory,
 //   G_d = sum_{t+s=d} sum_k a_t(row, k) b_s(k, n),
-// which stays exact while K * (d+1) * 2^(2w) < 2^24 (w = 7 up to K ~ 113 with nine orders, w = 6
-// beyond).  Orders d < NO = NS are kept; the epilogue forms the exact integer
-//   T = sum_d G_d 2^(w (NO-1-d))
-// in 64-bit integer arithmetic (the lowest orders shifted right when T would pass 2^62: a loss below
-// 2^-60 of the largest term) and rounds T 2^(EA + EB - w (NO+1)) once to FP64, on the integer pipe.
-// The result differs from the exact product of the FP64 operands by about 2^-(w NS - 1) of
-// max|A(row,:)| max|B(:,n)| per term: NS = 9, w = 7 (63 bits) is an FP64-grade product (the plain
-// form), NS = 6 (42 bits) the mixed form's.  No floating-point rounding happens anywhere else: the
-// forward fold f(i) +- f(nr-1-i) is an exact integer sum of the two rounded samples, and the
-// quadrature weights are folded into the table (A = pf w, one FP64 rounding at kit init).
+// which stays exact while K (d+1) (largest digit product) <= 2^24.  Orders d < NO = NS are kept; the epilogue forms the
+// integer T = sum_d G_d 2^(w (NO-1-d)) in 64 bits (its lowest bits shifted out where it would not fit) and rounds
+// T 2^(EA + EB + const) once to FP64, on the integer pipe.
+// The result differs from the exact product of the FP64 operands by what the dropped orders hold, about 2^-(nb - 2) of
+// max|A(row,:)| max|B(:,n)|: 63 bits, in eight or nine balanced digits, is an FP64-grade product (the plain form), 42
+// bits the mixed form's.  No floating-point rounding happens anywhere else: the forward fold f(i) +- f(nr-1-i) is an exact
+// integer sum of the two rounded samples, and the quadrature weights are folded into the table (A = pf w, one FP64
+// rounding at kit init).
 //
 // Forward: per m and row parity par, C_par(t, n) = sum_{i < nr/2} A_par(t, i) B_par(i, n) with
 //   A_par(t, i) = pf(i, 2t+par, m) w(i),  B_par(i, n) = f(i) + (-1)^par f(nr-1-i)  (n: re/im of z),
@@ -29,22 +27,17 @@
 //   integers, so both parities share one row scale per i and one column scale per n; the log term
 //   ln * lnx(i) is added at m = 0 (trans, :194).
 //
-// Engine: a persistent grid of one CTA per SM (512 threads).  A work item is one (m, tile of NZ complex
-// z columns); the CTA
+// Engine: a persistent grid of one CTA per SM.  A work item is one (m, tile of NZ complex z columns); the CTA
 //  * bulk-copies the item's FP64 field columns (NZ runs of consecutive r, each contiguous in HBM) into
-//    shared memory on the TMA engine, completing on an mbarrier;
-//  * takes the item's column scales, which the epilogue warps computed two items ahead from global memory;
-//  * per row tile and K chunk of 16: the table digits of both parities arrive by one bulk copy (pre-split
-//    at kit init in the UMMA canonical no-swizzle K-major layout), the threads cut the field digits
-//    from shared memory into the same layout (each warp's 32 stores in 32 banks), and one thread issues
-//    the chunk's tcgen05.mma, commits, and as soon as the other stage is free starts the next chunk's
-//    table copy into it; the stages are double-buffered, so the digits and the table copy of chunk
-//    k + 1 overlap the MMAs of chunk k.  The field digits of a parity lie side by side (digit s at
-//    rows s N .. s N + N-1 of the B operand) and so do the accumulators of the orders, so table digit
-//    t meets all field digits s <= NO-1-t in one MMA of M = 128, N = (NO - t) 2 NZ, K = 16 whose
-//    column block s lands on order t + s: NO MMAs per parity and chunk instead of NO (NO+1)/2, and
-//    each table tile is read from shared memory once;
-//  * reads the 2 NO accumulators back with tcgen05.ld and writes FP64 results.
+//    shared memory on the TMA engine, completing on an mbarrier, and scans them for the column scales;
+//  * per row tile, parity and K chunk of 16: the table digits arrive by one bulk copy (pre-split at kit init in the
+//    UMMA canonical no-swizzle K-major layout), the digit warps cut the field digits from shared memory into the same
+//    layout (each warp's 32 stores in 32 banks), and one thread issues the chunk's tcgen05.mma and commits.  The field
+//    digits lie side by side (digit s at rows s N .. s N + N-1 of the B operand) and so do the accumulators of the
+//    orders, so table digit t meets all field digits s <= NO-1-t in one MMA of M = 128, N = (NO - t) 2 NZ, K = 16 whose
+//    column block s lands on order t + s: NO MMAs per stage instead of NO (NO+1)/2, and each table tile is read
+//    from shared memory once;
+//  * reads the NO accumulators of a parity back with tcgen05.ld and, after the second parity, writes FP64 results.
 // Every wait is bounded (about a second of SM clock): a timeout sets the library's timeout word and the
 // CTA stops issuing work, waits (bounded) for what it issued, frees its tensor memory and returns.
 #include "common.cuh"
@@ -55,7 +48,7 @@
 namespace mlg {
 
 constexpr int XS_KC = 16;                         // K per chunk: one MMA K step
-constexpr int XS_THREADS = 512;
+constexpr int XS_THREADS = 896;
 constexpr int XS_ATILE = 128 * XS_KC * 2;         // 4 KiB: 128 rows x 16 K of BF16
 constexpr int XS_SBO = XS_KC * 16;                // between 8-row core-matrix groups
 constexpr int XS_LBO = 128;                       // between the two 8-K core matrices of a row group
@@ -76,7 +69,7 @@ __device__ __forceinline__ double xs_a(const double* __restrict__ pf, const doub
 
 // row scales: fwd aexp[(m * 2 + par) * nrp + t], bwd aexp[m * nrp + i] (both parities); -2000: all zero
 __global__ void k_xs_aexp(const double* __restrict__ pf, const double* __restrict__ w, int* __restrict__ aexp, int mode,
-                          int nrh, int ne, int nrc, int nrp, int nk) {
+                          int nrh, int ne, int nrc, int nrp, int nk, int bal) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   const int m = blockIdx.y, nn = max(min(nrc, nrc - m), 0);
   if (row >= nrp) return;
@@ -88,19 +81,26 @@ __global__ void k_xs_aexp(const double* __restrict__ pf, const double* __restric
                                0x7FFFFFFFFFFFFFFFull;
         mx = v > mx ? v : mx;
       }
-    aexp[(size_t)(mode == 0 ? m * 2 + p : m) * nrp + row] = mx ? xs_ebound(mx) : -2000;
+    aexp[(size_t)(mode == 0 ? m * 2 + p : m) * nrp + row] = !mx ? -2000 : bal ? xs_ebound_bal((unsigned)(mx >> 32)) : xs_ebound(mx);
   }
 }
 
-// digit tiles per (m, row tile mt, chunk kc): [par][digit t] of 128 rows x 16 K
+// the digit configuration of a digit count: 6 or 9 digits of 7 bits, 7 or 10 of 6, 8 of 8; eight and nine digits are
+// balanced
+template <int NS> __host__ __device__ constexpr int xs_w() { return NS == 8 ? 8 : NS == 7 || NS == 10 ? 6 : 7; }
+template <int NS> __host__ __device__ constexpr bool xs_bal() { return NS == 8 || NS == 9; }
+template <int NS> __host__ __device__ constexpr int xs_nb() { return xs_bal<NS>() ? 63 : xs_w<NS>() * NS; }
+
+// digit tiles of 128 rows x 16 K: [m][row tile mt][par][chunk kc][digit t]
 template <int NS>
 __global__ void k_xs_table(const double* __restrict__ pf, const double* __restrict__ w, const int* __restrict__ aexp,
-                           uint16_t* __restrict__ img, int mode, int nrh, int ne, int nrc, int nmt, int nkc, int nrp,
-                           int wbits) {
+                           uint16_t* __restrict__ img, int mode, int nrh, int ne, int nrc, int nmt, int nkc, int nrp) {
+  constexpr int W = xs_w<NS>();
   const size_t blk = blockIdx.x;   // (m * nmt + mt) * nkc + kc
   const int kc = (int)(blk % nkc), mt = (int)((blk / nkc) % nmt), m = (int)(blk / ((size_t)nkc * nmt));
   const int nn = max(min(nrc, nrc - m), 0);
-  uint8_t* base = (uint8_t*)img + blk * (size_t)(2 * NS * XS_ATILE);
+  uint8_t* base = (uint8_t*)img + ((blk / nkc) * 2 * nkc + kc) * (size_t)(NS * XS_ATILE);
+  const size_t pstep = (size_t)nkc * NS * XS_ATILE;   // from the even to the odd parity
   for (int idx = threadIdx.x; idx < 2 * 128 * XS_KC; idx += blockDim.x) {
     const int k = idx % XS_KC, r = (idx / XS_KC) % 128, par = idx / (XS_KC * 128);
     const int row = mt * 128 + r, kk = kc * XS_KC + k;
@@ -110,10 +110,11 @@ __global__ void k_xs_table(const double* __restrict__ pf, const double* __restri
       E = aexp[(size_t)(mode == 0 ? m * 2 + par : m) * nrp + row];
       a = xs_a(pf, w, mode, row, kk, par, m, nn, nrh, ne);
     }
-    float f[NS];
-    xs_digits_f<NS>(xs_fix(a, E, wbits * NS), wbits, f);
-#pragma unroll
-    for (int t = 0; t < NS; ++t) *(uint16_t*)(base + (par * NS + t) * XS_ATILE + xs_off(r, k)) = (uint16_t)(__float_as_uint(f[t]) >> 16);
+    const unsigned long long X = (unsigned long long)xs_fix(a, E, xs_nb<NS>()) + (xs_bal<NS>() ? xs_bias<NS, W>() : 0ull);
+    xs_static_for<NS>([&](auto tc) {
+      constexpr int t = decltype(tc)::value;
+      *(uint16_t*)(base + par * pstep + t * XS_ATILE + xs_off(r, k)) = (uint16_t)xs_digit2<NS, W, xs_bal<NS>(), t>(X, X);
+    });
   }
 }
 
@@ -129,7 +130,7 @@ struct XsArgs {
   const double* lnx;
   int* status;
   int add_ln, nf, nr, nrh, nrdim, npdim, nzdim, nrc, m0, npc, nmt, nkc, nrp, rawk;
-  int astages;   // table-chunk stages (2 or 3, as shared memory allows)
+  int aent, bst, nraw;   // ring sizes: table entries and field-digit stages (one parity of a chunk), field-column buffers
 };
 // field f's pointer without an indexed access to the kernel parameters (which would copy them to local
 // memory)
@@ -145,16 +146,23 @@ __device__ __forceinline__ bool xs_wait(uint64_t* bar, uint32_t phase, bool& ok)
 
 
 
-// Warp roles of the contraction kernel (512 threads, one CTA per SM):
-//   warp 0      producer: the item's field columns and the table chunks, by bulk copy
-//   warp 1      MMA issue (one thread) and the tensor-memory allocation
-//   warps 2..7  field digits
-//   warps 8..15 epilogue: tensor memory -> 64-bit order sums -> FP64 results; the column scales of
-//               the item two ahead
-// Every hand-off is an mbarrier: the table chunks and the field-digit stages are rings (2 and XS_SB
-// stages), the field columns are one buffer (the next item's columns land while the MMAs and the
-// epilogue of this one run), the accumulators are released by the epilogue as soon as it has read
-// them, so the MMAs of the next work unit overlap the FP64 conversion and the stores of this one.
+// Warp roles of the contraction kernel (896 threads, one CTA per SM):
+//   warp 0        the table entries, by bulk copy (one thread)
+//   warp 1        MMA issue (one thread) and the tensor-memory allocation
+//   warps 2, 3    the items' field columns, by bulk copy (one thread), and their scales
+//   warps 4..11   field digits, in two groups that take the stages in turn
+//   warps 12..27  epilogue: tensor memory -> 64-bit order sums -> FP64 results
+// A work unit is one parity of a row tile of an item: its accumulators are NO N columns, so that two sets fit tensor
+// memory (one with nine digits and 32 columns) and the MMAs of a unit run while the epilogue reads the one before.
+// Every hand-off is an mbarrier: the table entries and the field-digit stages (one parity of a chunk each) are rings,
+// the field columns are one buffer (the next item's columns land while the MMAs and the epilogue of this one run).  The
+// epilogue keeps the even parity's sums in registers and writes both parities' results after the odd unit.
+// What bounds it (clock64 traces, 192 points, six digits, 14 000 cycles an item): the integer pipe, on which the digits,
+// the order sums and the conversions take about 8 000 of them; the MMAs need 7 400 (shared-memory bandwidth: per stage a
+// 24 KiB table entry is written and read once, the digits are written once and read by the MMAs).  A cluster of two CTAs
+// sharing the table entries by multicast measured the same.  Ten steps' radial transforms at 192 x 128 x 128, mixed:
+// 4.27 -> 3.70 ms against eight-warp epilogues that released both parities together and reduced the scales themselves
+// (20 700 cycles an item); 512 x 512 x 256, two mixed steps: 22.4 -> 16.5 ms; plain: 2.48 -> 1.85 ms for four steps.
 // a bounded wait whose outcome every lane of the warp shares (the warp-collective operations that
 // follow need the whole warp)
 __device__ __forceinline__ bool xs_wait_w(uint64_t* bar, uint32_t phase, bool& ok) {
@@ -163,18 +171,34 @@ __device__ __forceinline__ bool xs_wait_w(uint64_t* bar, uint32_t phase, bool& o
   return ok;
 }
 
-constexpr int XS_SB = 3;                 // field-digit stages
-constexpr int XS_NDW = 6, XS_NEW = 8;    // digit warps (2..7), epilogue warps (8..15)
-constexpr int XS_NDIG = XS_NDW * 32, XS_NEPI = XS_NEW * 32;
-static_assert(2 + XS_NDW + XS_NEW == XS_THREADS / 32, "warp roles");
+constexpr int XS_SBMAX = 4, XS_AEMAX = 8;   // ring sizes (at most)
+constexpr int XS_CXS = 4;                   // column-scale slots (items)
+constexpr int XS_NSW = 2, XS_NDW = 8, XS_NEW = 16;   // scale warps (2, 3), digit warps (4..11), epilogue warps (12..27)
+constexpr int XS_NG = 2;                    // groups of digit warps (at most the digit stages: a group waits at most one phase ahead)
+constexpr int XS_NEPI = XS_NEW * 32;
+constexpr int XS_NBAR = 4 + 2 * XS_AEMAX + 2 * XS_SBMAX + 4 + 2 * XS_CXS;
+static_assert(2 + XS_NSW + XS_NDW + XS_NEW == XS_THREADS / 32, "warp roles");
 
 // MODE 0 forward, 1 backward; NS digits (and orders), NZ complex z columns per item
-// digit width of a digit count (xs_cfg): 7 bits for 6 and 9 digits, 6 bits for 7 and 10
-template <int NS> __host__ __device__ constexpr int xs_w() { return (NS == 6 || NS == 9) ? 7 : 6; }
-// right shift of the 64-bit order sums: |G_d| < 2^24 / (pairs) keeps sum_d G_d 2^(w (NS-1-d) - ESH)
+// right shift of the unsigned digits' 64-bit order sums: |G_d| < 2^24 / (pairs) keeps sum_d G_d 2^(w (NS-1-d) - ESH)
 // below 2^62
 template <int NS> __host__ __device__ constexpr int xs_esh() {
   return 24 + xs_w<NS>() * (NS - 1) - 62 > 0 ? 24 + xs_w<NS>() * (NS - 1) - 62 : 0;
+}
+// The plain form's order sums.  A fixed shift that keeps K max|A| max|B| within 64 bits would cut the sums at 2^-52 of
+// max|A| max|B|, far above what the digits hold (2^-61, the dropped orders), and rows whose largest table entries meet
+// small coefficients (the innermost points, where the Legendre functions grow like a power of the degree) would lose
+// bits that FP64 keeps.  So the sum of the orders from 2 on, L = sum_{d>=2} G_d 2^(w (NO-1-d) - low), is formed exactly
+// (but for the last order's `low` bits), and added to C = G_0 2^w + G_1 with the smallest shift that fits:
+// T = C 2^(cb - esh) + (L >> esh), cb = w (NO-2) - low.
+// low: |G_2| <= K (2^(2w-2) + 2 2^(w+6)) and the orders below it keep |L| < 2^63 (8 digits: 3 2^21 2^40) or, with K <=
+// 372 and nine digits, 2^22.9 2^(42 - 3)
+template <int NS> __host__ __device__ constexpr int xs_low() { return NS == 9 ? 3 : 0; }
+template <int NS> __host__ __device__ constexpr int xs_cb() { return xs_w<NS>() * (NS - 2) - xs_low<NS>(); }
+// the shift for sums with |C| <= mx: |T| <= (mx + 2^16) 2^(cb - esh) < 2^62 (|L| 2^-cb <= 2^16), so that the sum of two
+// fits 64 bits too
+template <int NS> __device__ __forceinline__ int xs_order_shift(int mx) {
+  return max(32 - __clz(mx + 65536) + xs_cb<NS>() - 62, 0);
 }
 // T += v 2^SH (floor for SH < 0), SH a compile-time constant: one wide multiply-add for 0 <= SH <= 30
 template <int SH> __device__ __forceinline__ void xs_acc(long long& T, int v) {
@@ -186,64 +210,64 @@ template <int NO, int W, int ESH, int D> __device__ __forceinline__ void xs_acc_
   xs_acc<W * (NO - 1 - D) - ESH>(T, xs_f2i(__uint_as_float(g)));
 }
 
+// CW consecutive columns of tensor memory into each lane (no wait)
+template <int CW> __device__ __forceinline__ void xs_tmem_ld(uint32_t taddr, uint32_t* r) {
+  static_assert(CW == 4 || CW == 8, "columns of an epilogue warp");
+  if constexpr (CW == 8) tmem_ld8_nw(taddr, r);
+  else tmem_ld4_nw(taddr, r);
+}
+
 template <int MODE, int NS, int NZ>
 __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   constexpr int NO = NS;
-  constexpr int W = xs_w<NS>(), ESH = xs_esh<NS>();
+  constexpr int W = xs_w<NS>(), ESH = xs_esh<NS>(), nb = xs_nb<NS>();
+  constexpr bool BAL = xs_bal<NS>();
   constexpr int N = 2 * NZ;                       // real columns (MMA N per digit)
   constexpr int BT = N * XS_KC * 2;               // B digit tile bytes
-  constexpr int ASTAGE = 2 * NS * XS_ATILE;
-  constexpr int BSTAGE = 2 * NS * BT;
-  // the accumulators of one work unit, and two sets of them where tensor memory holds both: the MMAs of
-  // the next unit then run while the epilogue reads this one's
-  constexpr int ACC = 2 * NO * N;
-  constexpr int TB = 2 * ACC <= 512 ? 2 : 1;
+  constexpr int AENT = NS * XS_ATILE;             // a table entry: the digits of one parity of a chunk
+  constexpr int BSTAGE = NS * BT;
+  constexpr int ACC = NO * N;                     // accumulator columns of a unit
+  constexpr int TB = 2 * ACC <= 512 ? 2 : 1;      // sets of them
   constexpr int TUSE = TB * ACC;
-  constexpr int TCOLS = TUSE <= 32 ? 32 : TUSE <= 64 ? 64 : TUSE <= 128 ? 128 : TUSE <= 256 ? 256 : 512;
-  constexpr int NBLK = (MODE == 0 ? 1 : 2) * (N / 8) * 2;   // digit blocks per chunk
-  constexpr int CPW = N / 16;                     // 8-column groups of an epilogue warp
+  constexpr int TCOLS = TUSE <= 128 ? 128 : TUSE <= 256 ? 256 : 512;
+  constexpr int NBLK = (N / 8) * 2;               // digit blocks per stage
+  constexpr int NG = XS_NG, GW = XS_NDW / NG;     // digit groups, warps of a group
+  constexpr int CW = N / 4;                       // columns of an epilogue warp
   static_assert(ACC <= 512, "accumulators exceed tensor memory");
   static_assert(N == 16 || N == 32, "MMA N per digit");
-  static_assert((NO - 1) * N + N <= 256, "MMA N of the widest digit product");
+  static_assert(NBLK % GW == 0, "digit blocks per warp");
   extern __shared__ __align__(1024) uint8_t xs_smem_raw[];
   uint8_t* sbase = (uint8_t*)(((uintptr_t)xs_smem_raw + 1023) & ~(uintptr_t)1023);
-  const int AS = a.astages;
-  uint8_t* sA = sbase;                                   // [AS][ASTAGE]
-  uint8_t* sB = sA + AS * ASTAGE;                        // [XS_SB][BSTAGE]
-  double* raw = (double*)(sB + XS_SB * BSTAGE);          // [NZ][rawk] complex (re, im)
-  int* colexp = (int*)(raw + (size_t)2 * NZ * a.rawk);   // [2][N]: by item parity
-  uint64_t* bars = (uint64_t*)(colexp + 2 * N);
-  uint64_t* bar_rf = bars;                 // field columns landed
-  uint64_t* bar_re = bars + 1;             // field columns consumed (digit threads)
-  uint64_t* bar_af = bars + 2;             // [AS] table chunk landed
-  uint64_t* bar_ae = bars + 5;             // [AS] table chunk consumed (MMA commit)
-  uint64_t* bar_bf = bars + 8;             // [XS_SB] digit stage written (digit threads)
-  uint64_t* bar_be = bar_bf + XS_SB;       // [XS_SB] digit stage consumed (MMA commit)
-  uint64_t* bar_tf = bar_be + XS_SB;       // [TB] accumulators complete (MMA commit)
+  const uint32_t AE = (uint32_t)a.aent, SB = (uint32_t)a.bst;
+  const int RB = a.nraw;
+  uint8_t* sA = sbase;                                   // [AE][AENT]
+  uint8_t* sB = sA + AE * AENT;                          // [SB][BSTAGE]
+  double* raw0 = (double*)(sB + SB * BSTAGE);            // [RB][NZ][rawk] complex (re, im)
+  const size_t rawsz = (size_t)2 * NZ * a.rawk;
+  int* colexp = (int*)(raw0 + RB * rawsz);               // [XS_CXS][N], by item
+  uint64_t* bars = (uint64_t*)(colexp + XS_CXS * N);
+  uint64_t* bar_rf = bars;                 // [RB] field columns landed
+  uint64_t* bar_re = bars + 2;             // [RB] field columns consumed (digit threads)
+  uint64_t* bar_af = bars + 4;             // [AE] table entry landed
+  uint64_t* bar_ae = bar_af + XS_AEMAX;    // [AE] table entry consumed (MMA commit)
+  uint64_t* bar_bf = bar_ae + XS_AEMAX;    // [SB] digit stage written (the group's digit threads)
+  uint64_t* bar_be = bar_bf + XS_SBMAX;    // [SB] digit stage consumed (MMA commit)
+  uint64_t* bar_tf = bar_be + XS_SBMAX;    // [TB] accumulators complete (MMA commit)
   uint64_t* bar_te = bar_tf + 2;           // [TB] accumulators read (epilogue threads)
-  uint64_t* bar_cx = bar_te + 2;           // [2] column scales written (epilogue threads), by item parity
-  uint64_t* bar_ce = bar_cx + 2;           // [2] column scales read (epilogue threads), by item parity
-  uint32_t* tslot = (uint32_t*)(bar_ce + 2);
+  uint64_t* bar_cx = bar_te + 2;           // [XS_CXS] column scales written (scale threads)
+  uint64_t* bar_ce = bar_cx + XS_CXS;      // [XS_CXS] column scales read (epilogue threads: the item's last readers)
+  uint32_t* tslot = (uint32_t*)(bar_ce + XS_CXS);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  constexpr int w = W, nb = W * NS;
-  if (tid == 0) {
-    mbar_init(bar_rf, 1);
-    mbar_init(bar_re, XS_NDIG);
-    for (int i = 0; i < 3; ++i) {
-      mbar_init(bar_af + i, 1);
-      mbar_init(bar_ae + i, 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_cx + i, XS_NEPI);
-      mbar_init(bar_ce + i, XS_NEPI);
-      mbar_init(bar_tf + i, 1);
-      mbar_init(bar_te + i, XS_NEPI);
-    }
-    for (int i = 0; i < XS_SB; ++i) {
-      mbar_init(bar_bf + i, XS_NDIG);
-      mbar_init(bar_be + i, 1);
-    }
+  if (tid < XS_NBAR) {   // a barrier per thread
+    const int i = tid;
+    const uint64_t* q = bars + i;
+    mbar_init(bars + i, q == bar_re || q == bar_re + 1 ? XS_NDW * 32
+                        : q >= bar_bf && q < bar_be    ? GW * 32
+                        : q >= bar_te && q < bar_cx    ? XS_NEPI
+                        : q >= bar_cx && q < bar_ce    ? XS_NSW * 32
+                        : q >= bar_ce                  ? XS_NEPI
+                                                       : 1);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -262,6 +286,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   const int nitems = (a.npc - a.m0) * nzt * a.nf;
   auto item_m = [&](int item) { return a.m0 + item / (nzt * a.nf); };
   auto item_z0 = [&](int item) { return ((item / a.nf) % nzt) * NZ; };
+  auto item_f = [&](int item) { return item % a.nf; };
   auto item_nn = [&](int item) { const int m = item_m(item); return max(min(a.nrc, a.nrc - m), 0); };
   auto next_item = [&](int item) {
     for (item += gridDim.x; item < nitems && item_nn(item) == 0; item += gridDim.x) {}
@@ -280,316 +305,338 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   if (warp == 0) {
     // ---- producer
     if (lane == 0) {
-      uint32_t c = 0, nraw = 0;   // table chunks and field-column copies issued
-      int ii = 0;
-      for (int item = first; item < nitems && ok; item = next_item(item), ++ii) {
-        const int m = item_m(item), z0 = item_z0(item), nn = item_nn(item);
-        const double2* fin = xs_sel(a.in, item % a.nf);
+      uint32_t c = 0, s = 0, ph = 0;   // table entries issued, ring slot and phase
+      for (int item = first; item < nitems && ok; item = next_item(item)) {
+        const int m = item_m(item);
         int nkc_m, nrows, nmt_m;
-        geom(nn, nkc_m, nrows, nmt_m);
-        // the item's field columns, once the digit threads are done with the previous item's
-        if (ii > 0 && !xs_wait(bar_re, (ii - 1) & 1, ok)) break;
-        const int kraw = MODE == 0 ? a.nr : nn;
-        fence_async_smem();
-        uint32_t bytes = 0;
-        for (int zz = 0; zz < NZ; ++zz)
-          if (z0 + zz < a.nzdim) bytes += (uint32_t)kraw * 16u;
-        mbar_expect_tx(bar_rf, bytes);
-        for (int zz = 0; zz < NZ; ++zz)
-          if (z0 + zz < a.nzdim)
-            bulk_g2s(raw + (size_t)2 * zz * a.rawk, fin + (size_t)a.nrdim * (m + (size_t)a.npdim * (z0 + zz)),
-                     (uint32_t)kraw * 16u, bar_rf);
-        ++nraw;
-        for (int mt = 0; mt < nmt_m && ok; ++mt) {
-          const uint8_t* img_m = (const uint8_t*)a.img + ((size_t)m * a.nmt + mt) * a.nkc * (size_t)ASTAGE;
-          for (int kc = 0; kc < nkc_m; ++kc, ++c) {
-            const uint32_t s = c % (uint32_t)AS;
-            if (c >= (uint32_t)AS && !xs_wait(&bar_ae[s], ((c - AS) / AS) & 1, ok)) break;
-            mbar_expect_tx(&bar_af[s], ASTAGE);
-            bulk_g2s(sA + s * ASTAGE, img_m + (size_t)kc * ASTAGE, ASTAGE, &bar_af[s]);
+        geom(item_nn(item), nkc_m, nrows, nmt_m);
+        for (int mt = 0; mt < nmt_m && ok; ++mt)
+          for (int par = 0; par < 2 && ok; ++par) {
+            const uint8_t* img_u = (const uint8_t*)a.img + (((size_t)m * a.nmt + mt) * 2 + par) * a.nkc * (size_t)AENT;
+            for (int kc = 0; kc < nkc_m; ++kc, ++c) {
+              if (c >= AE && !xs_wait(&bar_ae[s], ph ^ 1u, ok)) break;
+              mbar_expect_tx(&bar_af[s], AENT);
+              bulk_g2s(sA + s * AENT, img_u + (size_t)kc * AENT, AENT, &bar_af[s]);
+              if (++s == AE) { s = 0; ph ^= 1u; }
+            }
           }
-        }
       }
       // the copies issued complete on their own: wait (bounded) for the last of them, so that no copy
       // is in flight when the CTA's shared memory goes away (at once in a run without a timeout)
-      for (uint32_t j = c > (uint32_t)AS ? c - AS : 0; j < c; ++j) {
+      for (uint32_t j = c > AE ? c - AE : 0; j < c; ++j) {
         bool ok2 = true;
-        xs_wait(&bar_af[j % AS], (j / AS) & 1, ok2);
+        xs_wait(&bar_af[j % AE], (j / AE) & 1, ok2);
       }
-      bool ok2 = true;
-      if (nraw >= 1) xs_wait(bar_rf, (nraw - 1) & 1, ok2);
     }
   } else if (warp == 1) {
     // ---- MMA issue
     if (lane == 0) {
-      uint32_t c = 0, u = 0;
+      uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
+      bool any = false;
       for (int item = first; item < nitems && ok; item = next_item(item)) {
         int nkc_m, nrows, nmt_m;
         geom(item_nn(item), nkc_m, nrows, nmt_m);
-        for (int mt = 0; mt < nmt_m && ok; ++mt, ++u) {
-          // the accumulator set of this unit, once the epilogue has read what it held TB units before
+        for (int v = 0; v < 2 * nmt_m && ok; ++v, ++u) {   // units: row tile v / 2, parity v % 2
+          // the unit's accumulators, once the epilogue has read what they held TB units before
           const uint32_t tb = u % TB;
           if (u >= (uint32_t)TB && !xs_wait(&bar_te[tb], ((u - TB) / TB) & 1, ok)) break;
-          tc_fence_after();
           const uint32_t tacc = tmem + tb * (uint32_t)ACC;
-          for (int kc = 0; kc < nkc_m; ++kc, ++c) {
-            const uint32_t sa = c % (uint32_t)AS, sb = c % XS_SB;
-            if (!xs_wait(&bar_af[sa], (c / AS) & 1, ok)) break;
-            if (!xs_wait(&bar_bf[sb], (c / XS_SB) & 1, ok)) break;
+          for (int kc = 0; kc < nkc_m; ++kc) {
+            if (!xs_wait(&bar_bf[sb], pb, ok)) break;
+            if (!xs_wait(&bar_af[sa], pa, ok)) break;
             tc_fence_after();
-            const uint32_t a0 = smem_u32(sA + sa * ASTAGE), b0 = smem_u32(sB + sb * BSTAGE);
-            // table digit t times the field digits s = 0 .. NO-1-t in one MMA of N (NO - t) columns: the
-            // field digits lie side by side in shared memory and the orders d = t + s side by side in
-            // tensor memory, so the product of digit s lands on order t + s
+            const uint32_t a0 = smem_u32(sA + sa * AENT), b0 = smem_u32(sB + sb * BSTAGE);
+            // table digit t times the field digits s = 0 .. NO-1-t in one MMA of N (NO - t) columns (two where that
+            // passes the 256 columns of an MMA): the field digits lie side by side in shared memory and the orders
+            // d = t + s side by side in tensor memory, so the product of digit s lands on order t + s
 #pragma unroll
-            for (int par = 0; par < 2; ++par)
-#pragma unroll
-              for (int t = 0; t < NO; ++t) {
-                const uint64_t ad = sdesc(a0 + (par * NS + t) * XS_ATILE, XS_LBO, XS_SBO);
-                const uint64_t bd = sdesc(b0 + (par * NS) * BT, XS_LBO, XS_SBO);
-                umma_bf16(tacc + (uint32_t)((par * NO + t) * N), ad, bd, idesc_bf16(128, (NO - t) * N),
-                          (kc > 0 || t > 0) ? 1u : 0u);
-              }
+            for (int t = 0; t < NO; ++t) {
+              const uint64_t ad = sdesc(a0 + t * XS_ATILE, XS_LBO, XS_SBO);
+              constexpr int NB1 = 256 / N;   // digits of one MMA
+              const int n1 = NO - t < NB1 ? NO - t : NB1;
+              umma_bf16(tacc + (uint32_t)(t * N), ad, sdesc(b0, XS_LBO, XS_SBO), idesc_bf16(128, n1 * N),
+                        (kc > 0 || t > 0) ? 1u : 0u);
+              if (NO - t > NB1)
+                umma_bf16(tacc + (uint32_t)((t + NB1) * N), ad, sdesc(b0 + NB1 * BT, XS_LBO, XS_SBO),
+                          idesc_bf16(128, (NO - t - NB1) * N), (kc > 0 || t > 0) ? 1u : 0u);
+            }
             umma_commit(&bar_ae[sa]);
             umma_commit(&bar_be[sb]);
+            last = sa; plast = pa; any = true;
+            if (++sa == AE) { sa = 0; pa ^= 1u; }
+            if (++sb == SB) { sb = 0; pb ^= 1u; }
           }
           if (ok) umma_commit(&bar_tf[tb]);
         }
       }
-      if (c > 0) {   // the MMAs issued have finished (bounded) before tensor memory is freed
+      if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
         bool ok2 = true;
-        xs_wait(&bar_ae[(c - 1) % AS], ((c - 1) / AS) & 1, ok2);
+        xs_wait(&bar_ae[last], plast, ok2);
       }
     }
-  } else if (warp < 2 + XS_NDW) {
+  } else if (warp < 2 + XS_NSW) {
+    // ---- column scales from the largest magnitudes' high words of the re and im parts: |x| < 2^(exponent field - 1022),
+    // and the forward folds may double.  Lane 0 of the first of the two warps also copies the field columns: with two
+    // buffers the next item's as soon as this item's scales are out, so that they land while its digits are cut (issued
+    // behind the item's table entries they came late: 20 500 cycles an item)
+    int nraw = 0;   // copies issued
+    auto copy_columns = [&](int item, int ii) {
+      if (warp != 2 || lane != 0 || item >= nitems) return;
+      const int rb = ii % RB, m = item_m(item), z0 = item_z0(item), kraw = MODE == 0 ? a.nr : item_nn(item);
+      const double2* fin = xs_sel(a.in, item_f(item)) + (size_t)a.nrdim * (m + (size_t)a.npdim * z0);
+      // once the digit threads are done with the item that had the buffer before
+      if (ii >= RB && !xs_wait(&bar_re[rb], (ii / RB - 1) & 1, ok)) return;
+      fence_async_smem();
+      const int nzc = max(min(NZ, a.nzdim - z0), 0);
+      mbar_expect_tx(&bar_rf[rb], (uint32_t)(nzc * kraw) * 16u);
+      for (int zz = 0; zz < nzc; ++zz)
+        bulk_g2s(raw0 + rb * rawsz + (size_t)2 * zz * a.rawk, fin + (size_t)a.nrdim * a.npdim * zz, (uint32_t)kraw * 16u,
+                 &bar_rf[rb]);
+      ++nraw;
+    };
+    int ii = 0;
+    if (RB > 1) copy_columns(first, 0);
+    for (int item = first; item < nitems && ok; item = next_item(item), ++ii) {
+      const int slot = ii % XS_CXS, rb = ii % RB;
+      if (ii >= XS_CXS && !xs_wait_w(&bar_ce[slot], (ii / XS_CXS - 1) & 1, ok)) break;
+      if (RB > 1 && !xs_wait_w(&bar_rf[rb], (ii / RB) & 1, ok)) break;
+      const int z0 = item_z0(item);
+      const int kraw = MODE == 0 ? a.nr : item_nn(item);
+      int* cxw = colexp + slot * N;
+      // eight columns per warp, four lanes per column, their loads independent (a column after the other, reduced over the
+      // whole warp, took 4 600 cycles an item alone and 12 000 beside the other warps)
+      const int zz = (warp - 2) * 8 + (lane >> 2);
+      unsigned mr = 0, mi = 0;
+      if (zz < NZ && z0 + zz < a.nzdim) {
+        // (re lo, re hi, im lo, im hi); with one column buffer read from global memory, ahead of the copy, so that the scan
+        // does not stand between the copy and the digits
+        auto scan = [&](const int4* col) {
+#pragma unroll 8
+          for (int i = lane & 3; i < kraw; i += 4) {
+            const int4 v = col[i];
+            mr = max(mr, (unsigned)v.y & 0x7FFFFFFFu);
+            mi = max(mi, (unsigned)v.w & 0x7FFFFFFFu);
+          }
+        };
+        if (RB > 1) scan((const int4*)(raw0 + rb * rawsz + (size_t)2 * zz * a.rawk));
+        else scan((const int4*)(xs_sel(a.in, item_f(item)) + (size_t)a.nrdim * (item_m(item) + (size_t)a.npdim * (z0 + zz))));
+      }
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        mr = max(mr, __shfl_xor_sync(0xFFFFFFFFu, mr, o));
+        mi = max(mi, __shfl_xor_sync(0xFFFFFFFFu, mi, o));
+      }
+      if ((lane & 3) == 0 && zz < NZ) {
+        constexpr int fold = MODE == 0 ? 1 : 0;
+        // an all-subnormal column counts as zero
+        cxw[2 * zz] = (mr >> 20) ? (BAL ? xs_ebound_bal(mr) : (int)(mr >> 20) - 1022) + fold : -2000;
+        cxw[2 * zz + 1] = (mi >> 20) ? (BAL ? xs_ebound_bal(mi) : (int)(mi >> 20) - 1022) + fold : -2000;
+      }
+      mbar_arrive(&bar_cx[slot]);
+      if (RB > 1) copy_columns(next_item(item), ii + 1);
+      else copy_columns(item, ii);
+      ok = __all_sync(0xFFFFFFFFu, ok);
+    }
+    // no copy is in flight when the CTA's shared memory goes away (bounded; at once in a run without a timeout)
+    for (int j = max(nraw - RB, 0); j < nraw; ++j) {
+      bool ok2 = true;
+      xs_wait(&bar_rf[j % RB], (j / RB) & 1, ok2);
+    }
+  } else if (warp < 2 + XS_NSW + XS_NDW) {
     // ---- field digits
-    const int dw = warp - 2;
-    uint32_t c = 0;
+    const int dw = (warp - 2 - XS_NSW) % GW, grp = (warp - 2 - XS_NSW) / GW;
+    uint32_t c = 0, s = 0, ph = 0;
     int ii = 0;
     for (int item = first; item < nitems && ok; item = next_item(item), ++ii) {
       const int z0 = item_z0(item), nn = item_nn(item);
       int nkc_m, nrows, nmt_m;
       geom(nn, nkc_m, nrows, nmt_m);
-      const int* cx = colexp + (ii & 1) * N;
-      if (!xs_wait_w(bar_rf, ii & 1, ok)) break;
-      // the item's column scales, written by the epilogue warps two items ahead
-      if (!xs_wait_w(&bar_cx[ii & 1], (ii >> 1) & 1, ok)) break;
-      for (int mt = 0; mt < nmt_m && ok; ++mt) {
+      const int* cx = colexp + (ii % XS_CXS) * N;
+      if (!xs_wait_w(&bar_cx[ii % XS_CXS], (ii / XS_CXS) & 1, ok)) break;
+      const int rb = ii % RB;
+      const double* raw = raw0 + rb * rawsz;
+      if (!xs_wait_w(&bar_rf[rb], (ii / RB) & 1, ok)) break;
+      // a warp writes (8 columns, 4 K pairs) blocks, each its 32 four-byte stores in 32 banks; the warp's blocks
+      // unrolled, so that their independent chains interleave.  The columns' shift bases once per item.
+      int base[NBLK / GW];
+#pragma unroll
+      for (int bi = 0; bi < NBLK / GW; ++bi) {
+        const int n = ((dw + bi * GW) % (N / 8)) * 8 + (lane & 7);
+        base[bi] = xs_fix_base(cx[n], nb, z0 + (n >> 1) < a.nzdim);
+      }
+      for (int v = 0; v < 2 * nmt_m && ok; ++v) {
+        const int par = v & 1;
         for (int kc = 0; kc < nkc_m; ++kc, ++c) {
-          const uint32_t s = c % XS_SB;
-          if (c >= XS_SB && !xs_wait_w(&bar_be[s], ((c - XS_SB) / XS_SB) & 1, ok)) break;
-          uint8_t* bst = sB + s * BSTAGE;
-          // a warp writes (parity, 8 columns, 4 K pairs) blocks, each its 32 four-byte stores in 32 banks;
-          // the warp's blocks unrolled, so that their independent chains interleave
+          if ((int)(c % NG) == grp) {   // the group's stage
+            if (c >= SB && !xs_wait_w(&bar_be[s], ph ^ 1u, ok)) break;
+            uint8_t* bst = sB + s * BSTAGE;
 #pragma unroll
-          for (int bi = 0; bi < (NBLK + XS_NDW - 1) / XS_NDW; ++bi) {
-            const int blk = dw + bi * XS_NDW;
-            if (blk >= NBLK) break;
-            const int par = MODE == 0 ? 0 : (blk & 1), bb = MODE == 0 ? blk : (blk >> 1);
-            const int ng = bb % (N / 8), kh = bb / (N / 8);
-            const int n = ng * 8 + (lane & 7), kp = kh * 4 + (lane >> 3), zz = n >> 1;
-            const int E = cx[n];
-            const bool zok = (z0 + zz < a.nzdim) && E > -2000;
-            const double* col = raw + (size_t)2 * zz * a.rawk + (n & 1);
-            const int off = xs_off(n, 2 * kp);
-            if (MODE == 0) {
-              // B_par(i) = f(i) + (-1)^par f(nr-1-i) for both parities, exact in the integers
-              float he[2][NS], ho[2][NS];
+            for (int bi = 0; bi < NBLK / GW; ++bi) {
+              const int blk = dw + bi * GW, ng = blk % (N / 8), kh = blk / (N / 8);
+              const int n = ng * 8 + (lane & 7), kp = kh * 4 + (lane >> 3), zz = n >> 1;
+              const double* col = raw + (size_t)2 * zz * a.rawk + (n & 1);
+              const int off = xs_off(n, 2 * kp);
+              unsigned long long x[2];
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const int i = kc * XS_KC + 2 * kp + u;
-                long long x1 = 0, x2 = 0;
-                if (zok && i < a.nrh) { x1 = xs_fix(col[2 * i], E, nb); x2 = xs_fix(col[2 * (a.nr - 1 - i)], E, nb); }
-                xs_digits_f<NS>(x1 + x2, w, he[u]);
-                xs_digits_f<NS>(x1 - x2, w, ho[u]);
+              for (int h = 0; h < 2; ++h) {
+                const int k = kc * XS_KC + 2 * kp + h;
+                long long X = 0;
+                if (MODE == 0) {
+                  // B_par(i) = f(i) + (-1)^par f(nr-1-i), exact in the integers
+                  if (k < a.nrh) {
+                    const long long x2 = xs_fixs(col[2 * (a.nr - 1 - k)], base[bi]);
+                    X = xs_fixs(col[2 * k], base[bi]) + (par ? -x2 : x2);
+                  }
+                } else {
+                  // B_par(t) = c(2t + par)
+                  const int j = 2 * k + par;
+                  if (j < nn) X = xs_fixs(col[2 * j], base[bi]);
+                }
+                x[h] = (unsigned long long)X + (BAL ? xs_bias<NS, W>() : 0ull);
               }
-#pragma unroll
-              for (int t = 0; t < NS; ++t) {
-                *(uint32_t*)(bst + t * BT + off) = xs_pack(he[0][t], he[1][t]);
-                *(uint32_t*)(bst + (NS + t) * BT + off) = xs_pack(ho[0][t], ho[1][t]);
-              }
-            } else {
-              // B_par(t) = c(2t + par)
-              float h[2][NS];
-#pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const int j = 2 * (kc * XS_KC + 2 * kp + u) + par;
-                xs_digits_f<NS>((zok && j < nn) ? xs_fix(col[2 * j], E, nb) : 0ll, w, h[u]);
-              }
-#pragma unroll
-              for (int t = 0; t < NS; ++t) *(uint32_t*)(bst + (par * NS + t) * BT + off) = xs_pack(h[0][t], h[1][t]);
+              xs_static_for<NS>([&](auto tc) {
+                constexpr int t = decltype(tc)::value;
+                *(uint32_t*)(bst + t * BT + off) = xs_digit2<NS, W, BAL, t>(x[0], x[1]);
+              });
             }
+            fence_async_smem();
+            mbar_arrive(&bar_bf[s]);
           }
-          fence_async_smem();
-          mbar_arrive(&bar_bf[s]);
+          if (++s == SB) { s = 0; ph ^= 1u; }
         }
       }
-      mbar_arrive(bar_re);   // done with the item's field columns
+      mbar_arrive(&bar_re[rb]);   // done with the item's field columns
     }
   } else {
-    // ---- epilogue: warp e reads TMEM lanes 32 (e % 4) .. +31 (rows of the tile) and the column half
-    // e / 4; the orders are combined exactly in 64-bit integers, T = sum_d G_d 2^(w (NO-1-d) - esh), on the
-    // integer pipe, and T 2^(EA + EB + esh - w (NO+1)) is then rounded once to FP64
-    const int ew = warp - 2 - XS_NDW, lq = warp & 3, ch = ew >> 2;
+    // ---- epilogue: warp e reads TMEM lanes 32 (e % 4) .. +31 (rows of the tile) and the column group e / 4; the
+    // orders are combined exactly in 64-bit integers on the integer pipe, and the sums rounded once to FP64
+    const int ew = warp - 2 - XS_NSW - XS_NDW, lq = warp & 3, cg = ew >> 2;
     const uint32_t lrow = (uint32_t)(lq * 32) << 16;
-    // The column scales of an item, into its slot of colexp: a warp per complex column z, its lanes over
-    // the column's samples (read from global memory through L2, before the item's own bulk copy), the
-    // largest exponent fields of the re and im parts (the high words without their sign bits order like
-    // the magnitudes' exponent fields) reduced by warp shuffles; |x| < 2^(field - 1022), and the
-    // forward folds may double.  The epilogue warps compute them two items ahead, in the time between
-    // their last stores of one item and the accumulators of the next, so that the digit warps find them
-    // ready when the item's columns land.
-    auto col_scales = [&](int item, int slot) {
-      const int m = item_m(item), z0 = item_z0(item);
-      const int kraw = MODE == 0 ? a.nr : item_nn(item);
-      const double2* fin = xs_sel(a.in, item % a.nf);
-      int* cxw = colexp + slot * N;
-      for (int zz = ew; zz < NZ; zz += XS_NEW) {
-        unsigned mr = 0, mi = 0;
-        if (z0 + zz < a.nzdim) {
-          const double2* col = fin + (size_t)a.nrdim * (m + (size_t)a.npdim * (z0 + zz));
-#pragma unroll 4
-          for (int i = lane; i < kraw; i += 32) {
-            const double2 v = __ldcg(col + i);
-            mr = max(mr, (unsigned)__double2hiint(v.x) & 0x7FFFFFFFu);
-            mi = max(mi, (unsigned)__double2hiint(v.y) & 0x7FFFFFFFu);
-          }
-        }
-        mr = __reduce_max_sync(0xFFFFFFFFu, mr >> 20);
-        mi = __reduce_max_sync(0xFFFFFFFFu, mi >> 20);
-        if (lane == 0) {
-          cxw[2 * zz] = mr ? (int)mr - 1022 + (MODE == 0 ? 1 : 0) : -2000;
-          cxw[2 * zz + 1] = mi ? (int)mi - 1022 + (MODE == 0 ? 1 : 0) : -2000;
-        }
-      }
-      mbar_arrive(&bar_cx[slot]);
-    };
-    if (first < nitems) {
-      col_scales(first, 0);
-      const int second = next_item(first);
-      if (second < nitems) col_scales(second, 1);
-    }
     uint32_t u = 0;
     int ii = 0;
     for (int item = first; item < nitems && ok; item = next_item(item), ++ii) {
       const int m = item_m(item), z0 = item_z0(item), nn = item_nn(item);
-      double2* fout = xs_sel(a.out, item % a.nf);
-      const double* flnp = xs_sel(a.lnp, item % a.nf);
+      double2* fout = xs_sel(a.out, item_f(item));
       int nkc_m, nrows, nmt_m;
       geom(nn, nkc_m, nrows, nmt_m);
-      const int* cx = colexp + (ii & 1) * N;
-      // the item's column scales (written into this slot by all epilogue warps)
-      if (!xs_wait_w(&bar_cx[ii & 1], (ii >> 1) & 1, ok)) break;
-      for (int mt = 0; mt < nmt_m && ok; ++mt, ++u) {
+      for (int mt = 0; mt < nmt_m && ok; ++mt) {
         const int row = mt * 128 + lq * 32 + lane;
         const bool live = mt * 128 + lq * 32 < nrows;   // a warp of rows past the tile's rows reads nothing
         // the row exponents, loaded before the wait so that their latency hides behind it
-        int EA0 = -2000, EA1 = -2000;
+        int EA[2] = {-2000, -2000};
         if (MODE == 0) {
           if (row < nrows) {
-            EA0 = a.aexp[(size_t)(m * 2) * a.nrp + row];
-            EA1 = a.aexp[(size_t)(m * 2 + 1) * a.nrp + row];
+            EA[0] = a.aexp[(size_t)(m * 2) * a.nrp + row];
+            EA[1] = a.aexp[(size_t)(m * 2 + 1) * a.nrp + row];
           }
         } else if (row < a.nrh) {
-          EA0 = a.aexp[(size_t)m * a.nrp + row];
+          EA[0] = a.aexp[(size_t)m * a.nrp + row];
         }
-        const uint32_t tb = u % TB;
-        if (!xs_wait_w(&bar_tf[tb], (u / TB) & 1, ok)) break;
-        tc_fence_after();
-        const uint32_t tacc = tmem + tb * (uint32_t)ACC;
-        constexpr int eo = ESH - W * (NO + 1);
-        // the warp's columns eight at a time; after the last group's loads the accumulators are free for
-        // the next unit's MMAs (and, after the item's last unit, this thread is done with the item's
-        // column scales), so the last group's conversions and stores overlap them
-#pragma unroll 1
-        for (int q = 0; q < CPW; ++q) {
-          const int cb = ch * (N / 2) + q * 8;
-          int E[8];
+        // T 2^(row exp + column exp + eo + esh): the products carry 2^(-2 nb), the orders' unit is
+        // 2^(2 w (NS-1) - w (NO-1)).  The mixed form's sums fit 64 bits with a fixed shift; the plain form's take the
+        // shift esh that the unit's own sums allow (xs_order_shift), one for the warp's columns
+        constexpr int eo = (BAL ? xs_low<NS>() : ESH) + W * (2 * (NS - 1) - (NO - 1)) - 2 * nb;
+        long long T[2][CW];
+        int esh[2] = {0, 0};
 #pragma unroll
-          for (int c = 0; c < 8; ++c) E[c] = cx[cb + c];
-          long long T[2][8];
+        for (int par = 0; par < 2; ++par, ++u) {
+          const uint32_t tb = u % TB;
+          if (!xs_wait_w(&bar_tf[tb], (u / TB) & 1, ok)) break;
+          tc_fence_after();
+          const uint32_t tcol = tmem + tb * (uint32_t)ACC + lrow + (uint32_t)(cg * CW);
 #pragma unroll
-          for (int par = 0; par < 2; ++par)
-#pragma unroll
-            for (int c = 0; c < 8; ++c) T[par][c] = 0;
+          for (int c = 0; c < CW; ++c) T[par][c] = 0;
           if (live) {
-            // two orders per load batch (one wait for four 8-column loads)
-            auto order2 = [&](auto dc) {
-              constexpr int D = 2 * decltype(dc)::value, D2 = D + 1 < NO ? D + 1 : D;
-              uint32_t g[2][8], h[2][8];
-#pragma unroll
-              for (int par = 0; par < 2; ++par) {
-                tmem_ld8_nw(tacc + lrow + (uint32_t)((par * NO + D) * N + cb), g[par]);
-                if constexpr (D2 != D) tmem_ld8_nw(tacc + lrow + (uint32_t)((par * NO + D2) * N + cb), h[par]);
-              }
+            // two orders per load batch
+            xs_static_for<(NO + 1 - (BAL ? 2 : 0)) / 2>([&](auto dc) {
+              constexpr int D = 2 * decltype(dc)::value + (BAL ? 2 : 0), D2 = D + 1 < NO ? D + 1 : D;
+              uint32_t g[CW], h[CW];
+              xs_tmem_ld<CW>(tcol + (uint32_t)(D * N), g);
+              if constexpr (D2 != D) xs_tmem_ld<CW>(tcol + (uint32_t)(D2 * N), h);
               tmem_wait_ld();
 #pragma unroll
-              for (int par = 0; par < 2; ++par)
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                  xs_acc_order<NO, W, ESH, D>(T[par][c], g[par][c]);
-                  if constexpr (D2 != D) xs_acc_order<NO, W, ESH, D2>(T[par][c], h[par][c]);
-                }
-            };
-            xs_static_for<(NO + 1) / 2>(order2);
-          }
-          if (q == CPW - 1) {
-            tc_fence_before();
-            mbar_arrive(&bar_te[tb]);
-            if (mt == nmt_m - 1) mbar_arrive(&bar_ce[ii & 1]);
-          }
-          if (!live) continue;
-          if (MODE == 0) {
-#pragma unroll
-            for (int par = 0; par < 2; ++par) {
-              const int j = 2 * row + par;
-              if (row >= nrows || j >= nn) continue;
-              const int EA = par ? EA1 : EA0;
-#pragma unroll
-              for (int c = 0; c < 8; c += 2) {
-                const int zo = z0 + ((cb + c) >> 1);
-                if (zo >= a.nzdim) continue;
-                const double re = EA > -2000 && E[c] > -2000 ? xs_i64_to_double(T[par][c], EA + E[c] + eo) : 0.0;
-                const double im = EA > -2000 && E[c + 1] > -2000 ? xs_i64_to_double(T[par][c + 1], EA + E[c + 1] + eo) : 0.0;
-                fout[j + (size_t)a.nrdim * (m + (size_t)a.npdim * zo)] = make_double2(re, im);
+              for (int c = 0; c < CW; ++c) {
+                xs_acc_order<NO, W, BAL ? xs_low<NS>() : ESH, D>(T[par][c], g[c]);
+                if constexpr (D2 != D) xs_acc_order<NO, W, BAL ? xs_low<NS>() : ESH, D2>(T[par][c], h[c]);
               }
+            });
+            if constexpr (BAL) {
+              // C = G_0 2^w + G_1, then T = C 2^(cb - esh) + (L >> esh)
+              uint32_t g[CW], h[CW];
+              xs_tmem_ld<CW>(tcol, g);
+              xs_tmem_ld<CW>(tcol + (uint32_t)N, h);
+              tmem_wait_ld();
+              int mx = 0;
+#pragma unroll
+              for (int c = 0; c < CW; ++c) {
+                const int C = xs_f2i(__uint_as_float(g[c])) * (1 << W) + xs_f2i(__uint_as_float(h[c]));
+                mx = max(mx, abs(C));
+                g[c] = (uint32_t)C;
+              }
+              const int es = xs_order_shift<NS>(mx);
+              esh[par] = es;
+#pragma unroll
+              for (int c = 0; c < CW; ++c) T[par][c] = ((long long)(int)g[c] << (xs_cb<NS>() - es)) + (T[par][c] >> es);
             }
-          } else {
-            const int i = row;
-            if (i < a.nrh) {
-              const int EA = EA0;
-              // the log term is added at m = 0 only: an integer test per item, so that the other items
-              // issue no FP64 compares or (predicated) FP64 additions on GB300's narrow FP64 pipe
-              const bool ln_here = a.add_ln && m == 0;
+          }
+          tc_fence_before();
+          mbar_arrive(&bar_te[tb]);
+        }
+        if (!ok) break;
+        // the item's column scales: written before its digits were cut, and so before its accumulators were complete
+        const int* cx = colexp + (ii % XS_CXS) * N + cg * CW;
+        if (!xs_wait_w(&bar_cx[ii % XS_CXS], (ii / XS_CXS) & 1, ok)) break;
+        if (MODE == 0 ? row < nrows : row < a.nrh) {
+          if (MODE == 1 && BAL) {   // the two parities are added: the same shift for both
+            const int es = max(esh[0], esh[1]);
 #pragma unroll
-              for (int c = 0; c < 8; c += 2) {
-                const int zo = z0 + ((cb + c) >> 1);
-                if (zo >= a.nzdim) continue;
-                double v[4] = {0.0, 0.0, 0.0, 0.0};   // f(i) re, im; f(nr-1-i) re, im
+            for (int c = 0; c < CW; ++c) {
+              T[0][c] >>= es - esh[0];
+              T[1][c] >>= es - esh[1];
+            }
+            esh[0] = es;
+          }
+          // the log term is added at m = 0 only: an integer test per item, so that the other items
+          // issue no FP64 compares or (predicated) FP64 additions on GB300's narrow FP64 pipe
+          const bool ln_here = MODE == 1 && a.add_ln && m == 0;
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                  if (EA > -2000 && E[c + h] > -2000) {
-                    // f(i) = D_0 + D_1, f(nr-1-i) = D_0 - D_1: both parities share the scales
-                    v[h] = xs_i64_to_double(T[0][c + h] + T[1][c + h], EA + E[c + h] + eo);
-                    v[2 + h] = xs_i64_to_double(T[0][c + h] - T[1][c + h], EA + E[c + h] + eo);
-                  }
-                }
-                if (ln_here) {
-                  const double lnv = *flnp;
-                  v[0] += lnv * a.lnx[i];
-                  v[2] += lnv * a.lnx[a.nr - 1 - i];
-                }
-                const size_t b0 = (size_t)a.nrdim * (m + (size_t)a.npdim * zo);
-                fout[b0 + i] = make_double2(v[0], v[1]);
-                fout[b0 + a.nr - 1 - i] = make_double2(v[2], v[3]);
+          for (int c = 0; c < CW; c += 2) {
+            const int zo = z0 + ((cg * CW + c) >> 1);
+            if (zo >= a.nzdim) continue;
+            const int E0 = cx[c], E1 = cx[c + 1];
+            double2* o = fout + (size_t)a.nrdim * (m + (size_t)a.npdim * zo);
+            if (MODE == 0) {
+#pragma unroll
+              for (int par = 0; par < 2; ++par) {
+                if (2 * row + par >= nn) continue;
+                const int e = EA[par] + esh[par] + eo;
+                const double re = EA[par] > -2000 && E0 > -2000 ? xs_i64_to_double(T[par][c], e + E0) : 0.0;
+                const double im = EA[par] > -2000 && E1 > -2000 ? xs_i64_to_double(T[par][c + 1], e + E1) : 0.0;
+                o[2 * row + par] = make_double2(re, im);
               }
+            } else {
+              double v[4] = {0.0, 0.0, 0.0, 0.0};   // f(i) re, im; f(nr-1-i) re, im
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                const int E = h ? E1 : E0;
+                if (EA[0] > -2000 && E > -2000) {
+                  // f(i) = D_0 + D_1, f(nr-1-i) = D_0 - D_1: both parities share the scales
+                  v[h] = xs_i64_to_double(T[0][c + h] + T[1][c + h], EA[0] + E + esh[0] + eo);
+                  v[2 + h] = xs_i64_to_double(T[0][c + h] - T[1][c + h], EA[0] + E + esh[0] + eo);
+                }
+              }
+              if (ln_here) {
+                const double lnv = *xs_sel(a.lnp, item_f(item));
+                v[0] += lnv * a.lnx[row];
+                v[2] += lnv * a.lnx[a.nr - 1 - row];
+              }
+              o[row] = make_double2(v[0], v[1]);
+              o[a.nr - 1 - row] = make_double2(v[2], v[3]);
             }
           }
         }
       }
-      // the scales of item ii+2 into this item's slot, once every epilogue thread has read it
-      const int ahead = next_item(next_item(item));
-      if (ok && ahead < nitems && xs_wait_w(&bar_ce[ii & 1], (ii >> 1) & 1, ok)) col_scales(ahead, ii & 1);
+      if (ok) mbar_arrive(&bar_ce[ii % XS_CXS]);   // this thread is done with the item's column scales
     }
   }
   if (!ok) atomicExch(a.status, 2);
@@ -603,7 +650,7 @@ struct XsImg {
   uint16_t* p = nullptr;
   int* aexp = nullptr;
   size_t bytes = 0, abytes = 0;
-  int nrc = -1, npc = -1, ns = 0, w = 0, nmt = 0, nkc = 0, nrp = 0;
+  int nrc = -1, npc = -1, ns = 0, nmt = 0, nkc = 0, nrp = 0;
 };
 static XsImg g_xs[2][2];   // [mode][plain/mixed]
 
@@ -616,8 +663,8 @@ void xs_free() {
     }
 }
 
-// the digit configuration: FP64-grade (plain: 63 or 60 bits) or the mixed form's 42 bits; w = 7 while
-// the orders stay exact (K (pairs) 2^14 < 2^24), else w = 6 with one digit more.  The mixed form
+// the digit configuration: FP64-grade (plain: 63 bits) or the mixed form's 42 bits, with the widest digits whose
+// orders stay exact.  The mixed form
 // needs 42 bits: its transform errors are deterministic, so a slowly changing flow meets the same
 // error step after step and they add up along a run; with 35-bit slices the backward transforms alone
 // left the vortex step's nonlinear term 9.6e-7 from the FP64 form after 1000 steps at 192 x 128 x 128,
@@ -625,47 +672,60 @@ void xs_free() {
 // needs more than 53 bits: the rounding is relative to the column maximum, and the nonlinear term's
 // curl cancellation magnifies what that loses on small entries (at 192 x 128 x 128 the vortex step's
 // nonlinear term differed from the FP64 reference by 5e-10 with 49-bit and 2.4e-11 with 56-bit digits).
-struct XsCfg { int ns, w; };
-static bool xs_cfg(int kmax, bool plain, XsCfg& c) {
+// The plain form takes balanced digits, eight (K <= 113) or nine.  Between 114 and 142 terms on grids of up to 284 points
+// it keeps ten unsigned digits of 6 bits with a fixed 64-bit shift, as it always had there: its sums are cut at 2^-52 of
+// max|A| max|B|, and the inverse Laplacian of the projection's (0, 0) column magnifies that cut to 4e-8 of single
+// coefficients of the nonlinear term, so that other digits would visibly move the results of a kit of 256 points.
+// returns the digit count (its width is xs_w's), 0 where no configuration is exact
+static int xs_rawk(int nrc) { return std::max(G.nr, nrc) | 1; }   // odd: the staged columns start in different banks
+static int xs_cfg(int kmax, int nrc, bool plain) {
   const double lim = 16777216.0;
   if (plain) {
-    if (9.0 * kmax * 128 * 128 < lim) { c = {9, 7}; return true; }
-    if (10.0 * kmax * 64 * 64 < lim) { c = {10, 6}; return true; }
+    if (kmax <= 113) return 8;                         // 8 128 128 K <= 2^24 up to 128
+    if (kmax <= 142 && xs_rawk(nrc) <= 285) return 10;
+    if (11.0 * kmax * 64 * 64 <= lim) return 9;        // order 8: seven pairs of 64 x 64 and two of 64 x 128
   } else {
-    if (6.0 * kmax * 128 * 128 < lim) { c = {6, 7}; return true; }
-    if (7.0 * kmax * 64 * 64 < lim) { c = {7, 6}; return true; }
+    if (6.0 * kmax * 128 * 128 < lim) return 6;
+    if (7.0 * kmax * 64 * 64 < lim) return 7;
   }
+  return 0;
+}
+
+static size_t xs_smem(int ns, int nz, int rawk, int aent, int bst, int nraw) {
+  const int n = 2 * nz;
+  return 1024 + aent * (size_t)(ns * XS_ATILE) + bst * (size_t)(ns * n * XS_KC * 2) +
+         nraw * (size_t)2 * nz * rawk * sizeof(double) + XS_CXS * n * sizeof(int) + 512;
+}
+constexpr size_t XS_SMEM_MAX = 227 * 1024;
+// The work items and rings of a digit count: 16 complex z columns per item where shared memory holds one buffer of field
+// columns beside two digit stages and two table entries (up to 512 points in the plain form), else 8: half the columns
+// per table entry means twice the table traffic, through L2 and shared memory, for the same result (512 points, seven
+// digits: 19.1 ms for two steps' backward transforms with 8 columns, 13.8 ms with 16).  Two column buffers where they fit
+// (up to 256 points), so that an item's columns land and are scanned while the one before is cut; then digit stages, at
+// most four (six measured the same), and table entries in what is left.
+struct XsPlan { int nz, aent, bst, nraw; };
+static bool xs_plan(int ns, int rawk, XsPlan& p) {
+  for (int nz = G.nzdim > 8 ? 16 : 8; nz >= 8; nz /= 2)
+    for (int nraw = 2; nraw >= 1; --nraw)
+      for (int sb = XS_SBMAX; sb >= 2; --sb)
+        for (int ae = XS_AEMAX; ae >= 2; --ae)
+          if (xs_smem(ns, nz, rawk, ae, sb, nraw) <= XS_SMEM_MAX) { p = {nz, ae, sb, nraw}; return true; }
   return false;
 }
-
-static size_t xs_smem(int ns, int nz, int rawk, int astages) {
-  const int n = 2 * nz;
-  return 1024 + astages * (size_t)(2 * ns * XS_ATILE) + XS_SB * (size_t)(2 * ns * n * XS_KC * 2) +
-         (size_t)2 * nz * rawk * sizeof(double) + 2 * n * sizeof(int) + 256;
-}
-// table-chunk stages: three where shared memory holds them, else two
-static int xs_astages(int ns, int nz, int rawk) { return xs_smem(ns, nz, rawk, 3) <= 227 * 1024 ? 3 : 2; }
-// complex z columns per work item: 16 while the accumulators (2 NS orders x 2 NZ columns) fit the 512
-// columns of tensor memory and the field columns fit shared memory, else 8.  (With 8 columns two sets of
-// accumulators fit for up to eight digits and the kernel double-buffers them, but at 192 x 128 x 128
-// the halved items doubled the per-item costs: backward 102 -> 124 us per three-field launch.)
-static int xs_nz(int ns) { return (G.nr <= 256 && ns <= 8) ? 16 : 8; }
-
-// whether the exact-slice contraction covers this kit: the orders stay exact and the stages fit
+// whether the exact-slice contraction covers this kit: the orders stay exact and the rings fit
 bool xs_supported(int mode, int nrc, bool plain) {
-  XsCfg c;
-  const int kmax = mode == 0 ? G.nrh : (nrc + 1) / 2;
-  return xs_cfg(kmax, plain, c) && xs_smem(c.ns, xs_nz(c.ns), std::max(G.nr, nrc) | 1, 2) <= 227 * 1024;
+  const int ns = xs_cfg(mode == 0 ? G.nrh : (nrc + 1) / 2, nrc, plain);
+  XsPlan p;
+  return ns > 0 && xs_plan(ns, xs_rawk(nrc), p);
 }
 
 template <int MODE, int NS, int NZ>
 static int xs_launch(const XsArgs& args, int nitems) {
-  const size_t sm = xs_smem(NS, NZ, args.rawk, args.astages);
-  if (sm > 227 * 1024) return set_error(MLG_ESIZE, "radial contraction: shared-memory stage too large");
+  const size_t sm = xs_smem(NS, NZ, args.rawk, args.aent, args.bst, args.nraw);
+  if (sm > XS_SMEM_MAX) return set_error(MLG_ESIZE, "radial contraction: shared-memory stage too large");
   auto kern = k_xs_rtrans<MODE, NS, NZ>;
   MLG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  int grid = std::min(nitems, 152);
-  kern<<<grid, XS_THREADS, sm, G.stream>>>(args);
+  kern<<<std::min(nitems, 152), XS_THREADS, sm, G.stream>>>(args);
   MLG_LAUNCH();
   return 0;
 }
@@ -677,29 +737,32 @@ int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int n
   if (nf > XS_NF) return set_error(MLG_EPARAM, "radial contraction: at most three fields per launch");
   const int nrows = mode == 0 ? (nrc + 1) / 2 : G.nrh;
   const int kmax = mode == 0 ? G.nrh : (nrc + 1) / 2;
-  XsCfg cfg;
-  if (!xs_cfg(kmax, plain, cfg)) return set_error(MLG_ESIZE, "radial contraction: too many radial points for exact slices");
+  const int ns = xs_cfg(kmax, nrc, plain);
+  XsPlan plan;
+  if (!ns || !xs_plan(ns, xs_rawk(nrc), plan)) return set_error(MLG_ESIZE, "radial contraction: too many radial points for exact slices");
   const int nmt = cdiv(nrows, 128), nkc = cdiv(kmax, XS_KC), nrp = nmt * 128;
   XsImg& im = g_xs[mode][plain ? 0 : 1];
-  if (im.nrc != nrc || im.npc != npc || !im.p || im.ns != cfg.ns || im.w != cfg.w) {
+  if (im.nrc != nrc || im.npc != npc || !im.p || im.ns != ns) {
     if (im.p) dfree(im.p, im.bytes);
     if (im.aexp) dfree(im.aexp, im.abytes);
     im = XsImg();
-    im.bytes = (size_t)npc * nmt * nkc * 2 * cfg.ns * XS_ATILE;
+    im.bytes = (size_t)npc * nmt * nkc * 2 * ns * XS_ATILE;
     im.abytes = (size_t)npc * (mode == 0 ? 2 : 1) * nrp * sizeof(int);
     MLG_TRY(dmalloc((void**)&im.p, im.bytes));
     MLG_TRY(dmalloc((void**)&im.aexp, im.abytes));
-    k_xs_aexp<<<dim3(cdiv(nrp, 128), npc), 128, 0, G.stream>>>(G.pf, G.w, im.aexp, mode, G.nrh, G.ne, nrc, nrp, kmax);
+    k_xs_aexp<<<dim3(cdiv(nrp, 128), npc), 128, 0, G.stream>>>(G.pf, G.w, im.aexp, mode, G.nrh, G.ne, nrc, nrp, kmax,
+                                                                   ns == 8 || ns == 9 ? 1 : 0);
     MLG_LAUNCH();
     const int nblk_t = npc * nmt * nkc;
-    switch (cfg.ns) {
-      case 6: k_xs_table<6><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp, cfg.w); break;
-      case 7: k_xs_table<7><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp, cfg.w); break;
-      case 9: k_xs_table<9><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp, cfg.w); break;
-      default: k_xs_table<10><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp, cfg.w); break;
+    switch (ns) {
+      case 6: k_xs_table<6><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+      case 7: k_xs_table<7><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+      case 8: k_xs_table<8><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+      case 10: k_xs_table<10><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+      default: k_xs_table<9><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
     }
     MLG_LAUNCH();
-    im.nrc = nrc; im.npc = npc; im.ns = cfg.ns; im.w = cfg.w; im.nmt = nmt; im.nkc = nkc; im.nrp = nrp;
+    im.nrc = nrc; im.npc = npc; im.ns = ns; im.nmt = nmt; im.nkc = nkc; im.nrp = nrp;
   }
   XsArgs args;
   for (int f = 0; f < XS_NF; ++f) {
@@ -711,22 +774,22 @@ int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int n
   args.status = (int*)(G.dscal + DS_FLAG + 1) + 1;
   args.add_ln = add_ln ? 1 : 0; args.nr = G.nr; args.nrh = G.nrh; args.nrdim = G.nrdim; args.npdim = G.npdim;
   args.nzdim = G.nzdim; args.nrc = nrc; args.m0 = m0; args.npc = npc; args.nmt = nmt; args.nkc = nkc; args.nrp = nrp;
-  // odd, so that the columns of the staged field start in different shared-memory banks
-  args.rawk = std::max(G.nr, nrc) | 1;
-  args.astages = xs_astages(cfg.ns, xs_nz(cfg.ns), args.rawk);
-  // the kernels' compile-time digit widths (xs_w) are those of xs_cfg
-  if (cfg.w != (cfg.ns == 6 || cfg.ns == 9 ? 7 : 6)) return set_error(MLG_EPARAM, "radial contraction: digit configuration");
-  const int nz16 = xs_nz(cfg.ns) == 16;
-  const int nitems = (npc - m0) * cdiv(G.nzdim, nz16 ? 16 : 8) * nf;
+  args.rawk = xs_rawk(nrc);
+  args.aent = plan.aent;
+  args.bst = plan.bst;
+  args.nraw = plan.nraw;
+  const bool nz16 = plan.nz == 16;
+  const int nitems = (npc - m0) * cdiv(G.nzdim, plan.nz) * nf;
 #define XS_CASE(NSV)                                                                                   \
   case NSV:                                                                                            \
     if (mode == 0) return nz16 ? xs_launch<0, NSV, 16>(args, nitems) : xs_launch<0, NSV, 8>(args, nitems); \
     return nz16 ? xs_launch<1, NSV, 16>(args, nitems) : xs_launch<1, NSV, 8>(args, nitems);
-  switch (cfg.ns) {
+  switch (ns) {
     XS_CASE(6)
     XS_CASE(7)
-    case 9: return mode == 0 ? xs_launch<0, 9, 8>(args, nitems) : xs_launch<1, 9, 8>(args, nitems);
-    case 10: return mode == 0 ? xs_launch<0, 10, 8>(args, nitems) : xs_launch<1, 10, 8>(args, nitems);
+    XS_CASE(8)
+    XS_CASE(9)
+    XS_CASE(10)
   }
 #undef XS_CASE
   return set_error(MLG_EPARAM, "radial contraction: digit configuration");
