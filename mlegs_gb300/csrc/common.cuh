@@ -162,10 +162,10 @@ int xs_rtrans(int mode, const cd* in, cd* out, int nrc, int npc, int m0, const d
 int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int nrc, int npc, int m0,
                     const double* const* lnp, bool add_ln, bool plain);
 void xs_free();
-// the mixed form's projection contraction as exact slices (xs_vec2tp.cu): psi, chi rows of
-// m0 <= m < npc written
-bool xv_supported();
-int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0);
+// the projection contraction as exact slices (xs_vec2tp.cu): psi, chi rows of m0 <= m < npc written; plain: FP64-grade
+// digits, else the mixed form's
+bool xv_supported(bool plain);
+int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain);
 void xv_free();
 int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc_off);
 // zeros to the rows of a mixed-form contraction's output that its kernels leave unwritten (radial.cu)

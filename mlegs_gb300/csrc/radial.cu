@@ -429,7 +429,7 @@ k_vec2tp(const double2* __restrict__ ur, const double2* __restrict__ up, const d
   }
 }
 
-// the m = 0 plane of vec2tp (mixed form, double-float): the m V terms vanish at m = 0, so
+// the m = 0 plane of vec2tp (double-float in the mixed form, FP64 in the plain one): the m V terms vanish at m = 0, so
 //   psi = -D.F_o(up),   chi = i k D.F_o(ur) - T.F_s(uz),
 // three contractions instead of five.  One output (j, z) per thread of a slice; KS slices of the K
 // range (radial points, chunks of KC dealt round-robin) in the block's z dimension give the plane
@@ -561,6 +561,16 @@ static int plane_rtrans_bwd(const cd* const* in, cd* const* out, const double* c
   dim3 grid(cdiv(G.nzdim, ZT), cdiv(G.nrh, IT), n), blk(ZT, IT, KS);
   k_rtrans_bwd_plane<T, IT, ZT, KC, KS><<<grid, blk, 0, st>>>(ps, G.pf, G.lnx, add_ln ? 1 : 0, G.nr, G.nrh, G.ne, G.nrdim,
                                                               G.npdim, G.nzdim, nrc);
+  MLG_LAUNCH();
+  return 0;
+}
+// the projection's m = 0 plane
+template <typename T>
+static int plane_vec2tp(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int nzc, int nzcu, cudaStream_t st) {
+  constexpr int MT = 16, ZT = 8, KC = 8, KS = 4;
+  dim3 grid(cdiv(G.nzdim, ZT), 2 * cdiv((nrc + 1) / 2, MT), 1), blk(ZT, MT, KS);
+  k_vec2tp_plane<T, MT, ZT, KC, KS><<<grid, blk, 0, st>>>(ur, up, uz, psi, chi, G.tD, G.tT, G.ak, G.nr, G.nrh, G.ne, G.nrdim,
+                                                          G.npdim, G.nzdim, nrc, nzc, nzcu);
   MLG_LAUNCH();
   return 0;
 }
@@ -800,11 +810,7 @@ int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd
   int nzc = G.chopzl, nzcu = G.chopzu;
   if (nrc > G.ne || nrc > G.nrdim) return set_error(MLG_ECHOP, "vec2tp: chopping in r too large");
   const bool mixed = G.precision == MLG_MIXED;
-  // the exact-slice tensor-core contraction (xs_vec2tp.cu) in the mixed form; the plain form keeps the
-  // FP64 contraction: chi = k X - Y cancels, and the slices' truncation relative to the column maxima
-  // (54-bit digits) left chi 7e-9 from the FP64 reference on the 32^3 kit (sliced radial transforms
-  // hold 1e-12 there)
-  const bool xv = mixed && xv_supported();
+  const bool xv = xv_supported(!mixed);   // the exact-slice tensor-core contraction (xs_vec2tp.cu)
   // the tensor-core contractions write rows < nn(m) of the kept columns: only the rest needs zeros
   // (beside them, below)
   if (!xv) {
@@ -816,20 +822,17 @@ int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd
   int tt = cdiv((nrc + 1) / 2, MT);
   dim3 grid(cdiv(G.nzdim, ZT), 2 * tt, npc), blk(ZT / ZPT, MT);
   if (xv) {
-    // m >= 1 on the tensor cores as exact slices, m = 0 in double-float beside it (after the zeros)
+    // m >= 1 on the tensor cores as exact slices, m = 0 beside it (after the zeros) in double-float (mixed) or FP64
     MLG_TRY(side_fork());
     cd* pc[2] = {psi, chi};
     MLG_TRY(launch_zero_tails_n(pc, 2, 0, nrc, npc, nzc, nzcu, G.side));
-    constexpr int DMT = 16, DZT = 8, DKC = 8, DKS = 4;
-    dim3 dgrid(cdiv(G.nzdim, DZT), 2 * cdiv((nrc + 1) / 2, DMT), 1), dblk(DZT, DMT, DKS);
-    k_vec2tp_plane<dfl, DMT, DZT, DKC, DKS><<<dgrid, dblk, 0, G.side>>>(ur, up, uz, psi, chi, G.tD, G.tT, G.ak, G.nr, G.nrh,
-                                                                         G.ne, G.nrdim, G.npdim, G.nzdim, nrc, nzc, nzcu);
-    MLG_LAUNCH();
-    MLG_TRY(xv_contract(ur, up, uz, psi, chi, nrc, npc, 1));   // m >= 1: 35/49-bit slices
+    MLG_TRY(mixed ? plane_vec2tp<dfl>(ur, up, uz, psi, chi, nrc, nzc, nzcu, G.side)
+                  : plane_vec2tp<double>(ur, up, uz, psi, chi, nrc, nzc, nzcu, G.side));
+    MLG_TRY(xv_contract(ur, up, uz, psi, chi, nrc, npc, 1, !mixed));
     MLG_TRY(side_join());
     kt_end(KT_V2TP, 5.0 * fwd_flops(nrc, npc));
     return 0;
-  } else   // the plain form, and the mixed form beyond the slices' range: FP64 DFMA over every m
+  } else   // beyond the slices' range: FP64 DFMA over every m, in both forms
     k_vec2tp<double, MT, ZT, KC, ZPT><<<grid, blk, 0, G.stream>>>(ur, up, uz, psi, chi, G.tV, G.tD, G.tT, G.ak, G.nr,
                                                                    G.nrh, G.ne, G.nrdim, G.npdim, G.nzdim, nrc, nzc, nzcu, 0);
   MLG_LAUNCH();

@@ -16,23 +16,33 @@
 // multiply-add.  The row parity of a work item fixes the folds, so each item is one (m, parity,
 // 128-row tile, NZ complex z columns).
 //
-// Digits: NS for psi and X, NT for Y, of w bits: the mixed form's NS = 5 (35 bits) and NT = 7 (49
-// bits; 6 and 8 of 6 bits beyond about 100 radial points); w and the digit counts keep every order's
-// accumulator exact: (pairs of the order) x (nr/2) x 2^(2w) < 2^24, where psi's and X's orders hold two
-// products per digit pair.  Y needs the extra digits: at k = 0 chi is -Y alone, and the inverse
+// Digits: NS for psi and X, NT for Y, of w bits.
+// Mixed form: NS = 5 (35 bits) and NT = 7 (49 bits; 6 and 8 of 6 bits beyond about 200 radial points); w and the digit
+// counts keep every order's accumulator exact: (pairs of the order) x (nr/2) x 2^(2w) < 2^24, where psi's and X's orders
+// hold two products per digit pair.  Y needs the extra digits: at k = 0 chi is -Y alone, and the inverse
 // Laplacian that ends the projection magnifies its error in the weak low modes; with 42-bit Y the
 // (m = 1, k = 0) column left the step's nonlinear term chi 9e-6 from FP64 at 192 x 128 x 128, with
-// 49 bits 2e-7.  (The plain form keeps its FP64 contraction: chi = k X - Y cancels, and even 54-bit
-// slices, cut relative to the column maxima, left chi 7e-9 from the FP64 reference.)
+// 49 bits 2e-7.
+// Plain form: nine balanced digits of 7 bits (63 bits) for all three, up to 744 radial points.  With up to 372 points
+// every order is exact; beyond, the orders from 6 on could pass 2^24 if all their digits were extreme and would then
+// lose units of 2^-56 of max|A| max|B|.  The order sums are shifted by what they need (xs_radial.cu): cut at a fixed
+// 2^-52, as 54-bit slices once were, chi = k X - Y is left 7e-9 from FP64.
 //
-// Engine: a persistent grid of one 256-thread CTA per SM over work items (m, parity, 128-row tile, 8
-// complex z columns).  Per K chunk of 16 radial points the table digits (m V, D and T, laid out at kit
-// init in the UMMA canonical K-major layout) arrive by one bulk copy into a two-stage ring, six warps
-// cut the field digits (ur, up and uz at i and nr-1-i, fetched in FP64 a chunk ahead) into the same
-// layout and arrive on the stage's mbarrier, and one thread issues the chunk's tcgen05.mma as soon as
-// both halves of a stage are in: a table digit t meets every field digit s <= n-1-t of its operands in
-// a single MMA (M = 128, K = 16; the field digits side by side in shared memory, the orders side by
-// side in tensor memory, psi's and X's alternating), 2 NS + NT MMAs per chunk.  Every wait is bounded.
+// Engine: a persistent grid of one CTA per SM over work items (m, 8 complex z columns, 128-row tile, parity).
+//   warp 0        the table entries (the digits of m V, D or T for a chunk of 16 radial points), by bulk copy
+//   warp 1        MMA issue (one thread): a table digit t meets every field digit s <= n-1-t of its operands in
+//                 one MMA (M = 128, K = 16; the field digits side by side in shared memory, the orders side by
+//                 side in tensor memory, psi's and X's alternating), two where that passes 256 columns
+//   warps 2, 3    the items' column scales, up to four items ahead
+//   warps 4..15   field digits, in two groups of six warps that take the chunks in turn (ur, up and uz at i and nr-1-i,
+//                 fetched in FP64 a chunk ahead; one staging item per thread: field, z column, K pair)
+//   warps 16..23  epilogue
+// Every hand-off is an mbarrier and every wait is bounded.  psi's and X's accumulators are released before Y's are
+// read.
+// What bounds it: the table entries' way through L2 (plain: 108 KiB per chunk for 8 columns, 1.3 GB per launch at
+// 192 x 128 x 128) and shared memory, and the integer pipe for the digits.
+// Per launch at 192 x 128 x 128: plain 302 us (FP64 DFMA 2 602), mixed 234 us (264 when one CTA of 256 threads walked scales,
+// chunks and epilogue in turn); 512 x 512 x 256 mixed 6.7 ms (7.3).
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "xs_common.cuh"
@@ -53,11 +63,17 @@ __device__ __forceinline__ bool xs_wait(uint64_t* bar, uint32_t phase, bool& ok)
   ok = mbar_wait(bar, phase);
   return ok;
 }
+// the same for a whole warp, whose lanes share the outcome
+__device__ __forceinline__ bool xs_wait_w(uint64_t* bar, uint32_t phase, bool& ok) {
+  xs_wait(bar, phase, ok);
+  ok = __all_sync(0xFFFFFFFFu, ok);
+  return ok;
+}
 
 // ------------------------------------------------------------------------------------------------
 // kit-time: row scales rexp[(m * 2 + par) * ntr + t] over (m V, D) and texp over T (-2000: zero row)
 __global__ void k_xv_rexp(const double* __restrict__ tV, const double* __restrict__ tD, const double* __restrict__ tT,
-                          int* __restrict__ rexp, int* __restrict__ texp, int nrh, int ne, int nrc, int ntr) {
+                          int* __restrict__ rexp, int* __restrict__ texp, int nrh, int ne, int nrc, int ntr, int bal) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int mp = blockIdx.y, m = mp >> 1, par = mp & 1;
   if (t >= ntr) return;
@@ -73,15 +89,21 @@ __global__ void k_xv_rexp(const double* __restrict__ tV, const double* __restric
       mv = b > mv ? b : mv;
       mt = c > mt ? c : mt;
     }
-  rexp[(size_t)mp * ntr + t] = mv ? xs_ebound(mv) : -2000;
-  texp[(size_t)mp * ntr + t] = mt ? xs_ebound(mt) : -2000;
+  auto bound = [&](unsigned long long v) { return !v ? -2000 : bal ? xs_ebound_bal((unsigned)(v >> 32)) : xs_ebound(v); };
+  rexp[(size_t)mp * ntr + t] = bound(mv);
+  texp[(size_t)mp * ntr + t] = bound(mt);
 }
 
+// digit configurations: the plain form's nine balanced digits, else two's complement
+template <int NS> __host__ __device__ constexpr bool xv_bal() { return NS == 9; }
+template <int NS, int W> __host__ __device__ constexpr int xv_nb(int n) { return xv_bal<NS>() ? 63 : W * n; }
+
 // tiles per (m, par, row tile mt, chunk kc): [m V digits NS | D digits NS | T digits NT]
-template <int NS, int NT>
+template <int NS, int NT, int W>
 __global__ void k_xv_table(const double* __restrict__ tV, const double* __restrict__ tD, const double* __restrict__ tT,
                            const int* __restrict__ rexp, const int* __restrict__ texp, uint16_t* __restrict__ img,
-                           int nrh, int ne, int nrc, int nmt, int nkc, int ntr, int w) {
+                           int nrh, int ne, int nrc, int nmt, int nkc, int ntr) {
+  constexpr bool BAL = xv_bal<NS>();
   const size_t blk = blockIdx.x;   // ((m * 2 + par) * nmt + mt) * nkc + kc
   const int kc = (int)(blk % nkc), mt = (int)((blk / nkc) % nmt), mp = (int)(blk / ((size_t)nkc * nmt));
   const int m = mp >> 1, par = mp & 1;
@@ -98,16 +120,19 @@ __global__ void k_xv_table(const double* __restrict__ tV, const double* __restri
       er = rexp[(size_t)mp * ntr + t]; et = texp[(size_t)mp * ntr + t];
     }
     const int off = xv_off(r, k);
-    float h[NS > NT ? NS : NT];
-    xs_digits_f<NS>(xs_fix(v, er, w * NS), w, h);
-#pragma unroll
-    for (int s = 0; s < NS; ++s) *(uint16_t*)(base + s * XV_ATILE + off) = (uint16_t)(__float_as_uint(h[s]) >> 16);
-    xs_digits_f<NS>(xs_fix(d, er, w * NS), w, h);
-#pragma unroll
-    for (int s = 0; s < NS; ++s) *(uint16_t*)(base + (NS + s) * XV_ATILE + off) = (uint16_t)(__float_as_uint(h[s]) >> 16);
-    xs_digits_f<NT>(xs_fix(tt, et, w * NT), w, h);
-#pragma unroll
-    for (int s = 0; s < NT; ++s) *(uint16_t*)(base + (2 * NS + s) * XV_ATILE + off) = (uint16_t)(__float_as_uint(h[s]) >> 16);
+    constexpr unsigned long long bs = BAL ? xs_bias<NS, W>() : 0ull, bt = BAL ? xs_bias<NT, W>() : 0ull;
+    const unsigned long long xv = (unsigned long long)xs_fix(v, er, xv_nb<NS, W>(NS)) + bs;
+    const unsigned long long xd = (unsigned long long)xs_fix(d, er, xv_nb<NS, W>(NS)) + bs;
+    const unsigned long long xt = (unsigned long long)xs_fix(tt, et, xv_nb<NS, W>(NT)) + bt;
+    xs_static_for<NS>([&](auto sc) {
+      constexpr int q = decltype(sc)::value;
+      *(uint16_t*)(base + q * XV_ATILE + off) = (uint16_t)xs_digit2<NS, W, BAL, q>(xv, xv);
+      *(uint16_t*)(base + (NS + q) * XV_ATILE + off) = (uint16_t)xs_digit2<NS, W, BAL, q>(xd, xd);
+    });
+    xs_static_for<NT>([&](auto sc) {
+      constexpr int q = decltype(sc)::value;
+      *(uint16_t*)(base + (2 * NS + q) * XV_ATILE + off) = (uint16_t)xs_digit2<NT, W, BAL, q>(xt, xt);
+    });
   }
 }
 
@@ -119,52 +144,129 @@ struct XvArgs {
   const int *rexp, *texp;
   const double* ak;
   int* status;
-  int nr, nrh, nrdim, npdim, nzdim, nrc, nzc, nzcu, nmt, nkc, ntr, w, m0, npc;
-  int esh_s, esh_t;   // right shifts that keep the 64-bit order sums of psi / X and of Y below 2^62
+  int nr, nrh, nrdim, npdim, nzdim, nrc, nzc, nzcu, nmt, nkc, ntr, m0, npc;
+  int aent;           // table entries of the ring
+  int esh_s, esh_t;   // two's complement digits: right shifts that keep the 64-bit order sums of psi / X and of Y below 2^62
 };
 
-// NS digits for psi and X, NT for Y; 8 complex z columns per work item (N = 16).  Persistent: one CTA of
-// 256 threads per SM walks the items (m, parity, row tile, z tile); warp 0 (one thread) copies the table
-// chunks into a two-stage ring, warp 1 (one thread) issues the MMAs, warps 2..7 cut the field digits
-// (one staging item each: field, z column, K pair), all eight warps run the epilogue.
-constexpr int XV_NZ = 8;
-constexpr int XV_THREADS = 256;
-template <int NS, int NT>
+constexpr int XV_NZ = 8, XV_N = 2 * XV_NZ;   // complex z columns per item, real columns
+constexpr int XV_NSW = 2, XV_GW = 6, XV_NEW = 8;   // scale warps, warps of a digit group (two groups), epilogue warps
+constexpr int XV_THREADS = (2 + XV_NSW + 2 * XV_GW + XV_NEW) * 32;
+constexpr int XV_CXS = 4, XV_AEMAX = 6, XV_SB = 2;   // column-scale slots, table entries (at most), digit stages
+constexpr int XV_BTILE = XV_N * XV_KC * 2;
+static_assert(3 * XV_NZ * 8 == XV_GW * 32, "one staging item per digit thread");
+__host__ __device__ constexpr int xv_aent_bytes(int ns, int nt) { return (ns > nt ? ns : nt) * XV_ATILE; }
+__host__ __device__ constexpr int xv_bstage_bytes(int ns, int nt) { return (4 * ns + nt) * XV_BTILE; }
+
+// order sums of eight columns: T[c] = sum_d G_d 2^(w (n-1-d)) (shifted; see xs_radial.cu), order d at tcol + d step;
+// returns the shift of a balanced sum
+template <int NO, int W, bool BAL> __device__ __forceinline__ int xv_sums(uint32_t tcol, uint32_t step, int esh, long long* T) {
+  if constexpr (!BAL) {
+#pragma unroll
+    for (int c = 0; c < 8; ++c) T[c] = 0;
+    xs_static_for<(NO + 1) / 2>([&](auto dc) {
+      constexpr int D = 2 * decltype(dc)::value, D2 = D + 1 < NO ? D + 1 : D;
+      uint32_t g[8], h[8];
+      tmem_ld8_nw(tcol + D * step, g);
+      if constexpr (D2 != D) tmem_ld8_nw(tcol + D2 * step, h);
+      tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        T[c] += xs_shl((long long)xs_f2i(__uint_as_float(g[c])), W * (NO - 1 - D) - esh);
+        if constexpr (D2 != D) T[c] += xs_shl((long long)xs_f2i(__uint_as_float(h[c])), W * (NO - 1 - D2) - esh);
+      }
+    });
+    return esh;
+  } else {
+    // L = sum_{d>=2} G_d 2^(w (NO-1-d) - 3): |G_2| <= 2 K (2^(2w-2) + 2 2^(w+6)) with K <= 372, so |L| < 2^62.9 and
+    // |L| 2^-cb < 2^17; then C = G_0 2^w + G_1 (|C| < 2^31) and T = C 2^(cb - es) + (L >> es) below 2^62
+    constexpr int LOW = 3, CB = W * (NO - 2) - LOW;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) T[c] = 0;
+    auto acc = [&](auto dc, uint32_t g, int c) {
+      constexpr int SH = W * (NO - 1 - decltype(dc)::value) - LOW;
+      const int v = xs_f2i(__uint_as_float(g));
+      if constexpr (SH > 30) T[c] += (long long)v << SH;
+      else if constexpr (SH >= 0) T[c] += (long long)v * (long long)(1 << SH);
+      else T[c] += (long long)(v >> -SH);
+    };
+    xs_static_for<(NO - 1) / 2>([&](auto dc) {
+      constexpr int D = 2 * decltype(dc)::value + 2, D2 = D + 1 < NO ? D + 1 : D;
+      uint32_t g[8], h[8];
+      tmem_ld8_nw(tcol + D * step, g);
+      if constexpr (D2 != D) tmem_ld8_nw(tcol + D2 * step, h);
+      tmem_wait_ld();
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        acc(std::integral_constant<int, D>(), g[c], c);
+        if constexpr (D2 != D) acc(std::integral_constant<int, D2>(), h[c], c);
+      }
+    });
+    uint32_t g[8], h[8];
+    tmem_ld8_nw(tcol, g);
+    tmem_ld8_nw(tcol + step, h);
+    tmem_wait_ld();
+    int mx = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int C = xs_f2i(__uint_as_float(g[c])) * (1 << W) + xs_f2i(__uint_as_float(h[c]));
+      mx = max(mx, abs(C));
+      g[c] = (uint32_t)C;
+    }
+    const int es = max(32 - __clz(mx + 131072) + CB - 62, 0);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) T[c] = ((long long)(int)g[c] << (CB - es)) + (T[c] >> es);
+    return es + LOW;
+  }
+}
+
+template <int NS, int NT, int W>
 __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
-  constexpr int NZ = XV_NZ;
-  constexpr int N = 2 * NZ;
-  constexpr int BTILE = N * XV_KC * 2;
-  constexpr int NA = 2 * NS + NT;                 // A tiles per chunk
-  constexpr int NB = 4 * NS + NT;                 // B tiles: [psi_ur, X_up] and [psi_up, X_ur] by digit, uz (NT)
-  constexpr int ASTAGE = NA * XV_ATILE, BSTAGE = NB * BTILE;
+  constexpr bool BAL = xv_bal<NS>();
+  constexpr int NZ = XV_NZ, N = XV_N;
+  constexpr int nbs = xv_nb<NS, W>(NS), nbt = xv_nb<NS, W>(NT);
+  constexpr int AENT = xv_aent_bytes(NS, NT), BSTAGE = xv_bstage_bytes(NS, NT);
   constexpr int COLS = (2 * NS + NT) * N;
-  constexpr int TCOLS = COLS <= 128 ? 128 : COLS <= 256 ? 256 : 512;
-  constexpr int NDIG = 3 * NZ * 8;                // staging items = digit threads (warps 2..7)
+  constexpr int TCOLS = COLS <= 256 ? 256 : 512;
+  constexpr uint32_t TY = 2 * NS * N;             // Y's accumulators, after psi's and X's
   static_assert(COLS <= 512, "accumulators exceed tensor memory");
-  static_assert(NDIG == XV_THREADS - 64, "one staging item per digit thread");
   extern __shared__ __align__(1024) uint8_t xv_smem_raw[];
   uint8_t* sbase = (uint8_t*)(((uintptr_t)xv_smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* sA = sbase;                            // [2][ASTAGE]
-  uint8_t* sB = sA + 2 * ASTAGE;                  // [2][BSTAGE]
-  int* cexp = (int*)(sB + 2 * BSTAGE);            // [N]: ur/up columns
-  int* fexp = cexp + N;                           // [N]: uz columns
-  uint64_t* bars = (uint64_t*)(fexp + 2 * N);     // a[2], b[2], mma[2]
-  uint32_t* tslot = (uint32_t*)(bars + 6);
-  uint64_t* bar_a = bars;
-  uint64_t* bar_b = bars + 2;
-  uint64_t* bar_mma = bars + 4;
+  const uint32_t AE = (uint32_t)a.aent;
+  uint8_t* sA = sbase;                            // [AE][AENT]
+  uint8_t* sB = sA + AE * AENT;                   // [XV_SB][BSTAGE]
+  int* cxs = (int*)(sB + XV_SB * BSTAGE);         // [XV_CXS][2 N]: by item, ur/up columns then uz columns
+  uint64_t* bars = (uint64_t*)(cxs + XV_CXS * 2 * N);
+  uint64_t* bar_af = bars;                        // [AE] table entry landed
+  uint64_t* bar_ae = bar_af + XV_AEMAX;           // [AE] table entry consumed (MMA commit)
+  uint64_t* bar_bf = bar_ae + XV_AEMAX;           // [XV_SB] digit stage written (the group's digit threads)
+  uint64_t* bar_be = bar_bf + XV_SB;              // [XV_SB] digit stage consumed (MMA commit)
+  uint64_t* bar_tf = bar_be + XV_SB;              // accumulators complete (MMA commit)
+  uint64_t* bar_te = bar_tf + 1;                  // [2] psi's and X's, Y's accumulators read (epilogue threads)
+  uint64_t* bar_cx = bar_te + 2;                  // [XV_CXS] column scales written (scale threads)
+  uint64_t* bar_ce = bar_cx + XV_CXS;             // [XV_CXS] column scales read (epilogue threads: the item's last readers)
+  uint32_t* tslot = (uint32_t*)(bar_ce + XV_CXS);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int w = a.w, nbs = w * NS, nbt = w * NT;
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_a + i, 1);
-      mbar_init(bar_b + i, NDIG);
-      mbar_init(bar_mma + i, 1);
+    for (int i = 0; i < XV_AEMAX; ++i) {
+      mbar_init(bar_af + i, 1);
+      mbar_init(bar_ae + i, 1);
+    }
+    for (int i = 0; i < XV_SB; ++i) {
+      mbar_init(bar_bf + i, XV_GW * 32);
+      mbar_init(bar_be + i, 1);
+    }
+    mbar_init(bar_tf, 1);
+    mbar_init(bar_te, XV_NEW * 32);
+    mbar_init(bar_te + 1, XV_NEW * 32);
+    for (int i = 0; i < XV_CXS; ++i) {
+      mbar_init(bar_cx + i, XV_NSW * 32);
+      mbar_init(bar_ce + i, XV_NEW * 32);
     }
     fence_mbar_init();
   }
-  if (warp == 0) {
+  if (warp == 1) {
     tmem_alloc(tslot, TCOLS);
     tmem_relinquish();
   }
@@ -173,263 +275,284 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
   tc_fence_after();
   const uint32_t tmem = *tslot;
   bool ok = true;
-  uint32_t it = 0;   // chunk counter (stage and phase), the same in every thread
-  const int nzt = (a.nzdim + NZ - 1) / NZ;
-  const int nmp = a.npc - a.m0;
-  const int nitems = nmp * 2 * a.nmt * nzt;   // item = ((mi * 2 + par) * nmt + mt) * nzt + zt
-  // staging item of a digit thread: field f (0 ur, 1 up, 2 uz), z column zz, K pair kp (the eight K
-  // pairs of a column in consecutive lanes, so that a warp's loads are runs of consecutive r)
-  const int dt = tid - 64;
-  const int f = dt / (NZ * 8), kp = dt % 8, zz = (dt / 8) % NZ;
 
-  for (int item = blockIdx.x; item < nitems && ok; item += gridDim.x) {
-    const int zt = item % nzt, mt = (item / nzt) % a.nmt, par = (item / (nzt * a.nmt)) & 1;
-    const int m = a.m0 + item / (nzt * a.nmt * 2);
-    const int nn = max(min(a.nrc, a.nrc - m), 0);
-    if (2 * (mt * 128) + par >= nn) continue;   // no rows of this parity in the tile (every thread agrees)
-    const int z0 = zt * NZ;
-    const int ss = par ? -1 : 1;   // own-parity fold sign
-    // ---- column scales: cexp(2zz) over (Im ur, Re up), cexp(2zz+1) over (Re ur, Im up); fexp over uz.
-    // Warp cz scans column z0 + cz (runs of consecutive r) for the largest exponent fields and reduces
-    // them by warp shuffles; |x| < 2^(field - 1022) for every sample, +1 because the folds may double.
-    {
-      static_assert(XV_THREADS / 32 == NZ, "one warp per z column");
-      const int cz = warp, z = z0 + cz;
+  // the CTA's items ((m, z tile), row tile, parity), those without rows skipped; every role walks the same sequence
+  const int nzt = (a.nzdim + NZ - 1) / NZ, nv = 2 * a.nmt;
+  const int nitems = (a.npc - a.m0) * nzt * nv;
+  auto item_m = [&](int it) { return a.m0 + it / (nzt * nv); };
+  auto item_z0 = [&](int it) { return (it / nv) % nzt * NZ; };
+  auto item_mt = [&](int it) { return (it % nv) >> 1; };
+  auto item_par = [&](int it) { return it & 1; };
+  auto live = [&](int it) {
+    const int m = item_m(it), nn = max(min(a.nrc, a.nrc - m), 0);
+    return 2 * (item_mt(it) * 128) + item_par(it) < nn;
+  };
+  auto next_item = [&](int it) {
+    for (it += gridDim.x; it < nitems && !live(it); it += gridDim.x) {}
+    return it;
+  };
+  int first = blockIdx.x;
+  if (first < nitems && !live(first)) first = next_item(first);
+  const int nkc = a.nkc;
+
+  if (warp == 0) {
+    // ---- the table entries
+    if (lane == 0) {
+      uint32_t c = 0, s = 0, ph = 0;
+      for (int it = first; it < nitems && ok; it = next_item(it)) {
+        const uint8_t* img = (const uint8_t*)a.img +
+                             (((size_t)(item_m(it) * 2 + item_par(it)) * a.nmt + item_mt(it)) * nkc) * (size_t)((2 * NS + NT) * XV_ATILE);
+        for (int kc = 0; kc < nkc && ok; ++kc)
+          for (int q = 0; q < 3; ++q, ++c) {
+            if (c >= AE && !xs_wait(&bar_ae[s], ph ^ 1u, ok)) break;
+            const uint32_t bytes = (uint32_t)(q < 2 ? NS : NT) * XV_ATILE;
+            mbar_expect_tx(&bar_af[s], bytes);
+            bulk_g2s(sA + s * AENT, img, bytes, &bar_af[s]);
+            img += bytes;
+            if (++s == AE) { s = 0; ph ^= 1u; }
+          }
+      }
+      // the copies issued complete on their own: wait (bounded) for the last of them, so that no copy
+      // is in flight when the CTA's shared memory goes away (at once in a run without a timeout)
+      for (uint32_t j = c > AE ? c - AE : 0; j < c; ++j) {
+        bool ok2 = true;
+        xs_wait(&bar_af[j % AE], (j / AE) & 1, ok2);
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issue
+    if (lane == 0) {
+      uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
+      bool any = false;
+      // the MMAs of one table entry: digit t against the B tiles [b, b + (n - t) cols), cols tiles per digit, onto the
+      // accumulators from tc on
+      auto entry = [&](auto nc, auto colsc, uint32_t b, uint32_t tc, bool add) {
+        constexpr int n = decltype(nc)::value, cols = decltype(colsc)::value;
+        if (!xs_wait(&bar_af[sa], pa, ok)) return;
+        tc_fence_after();
+        const uint32_t a0 = smem_u32(sA + sa * AENT);
+#pragma unroll
+        for (int t = 0; t < n; ++t) {
+          const uint64_t ad = sdesc(a0 + t * XV_ATILE, XV_LBO, XV_SBO);
+          const int tiles = (n - t) * cols, t1 = tiles * N > 256 ? 256 / N : tiles;
+          umma_bf16(tmem + tc + (uint32_t)(t * cols * N), ad, sdesc(b, XV_LBO, XV_SBO), idesc_bf16(128, t1 * N),
+                    (add || t > 0) ? 1u : 0u);
+          if (tiles > t1)
+            umma_bf16(tmem + tc + (uint32_t)((t * cols + t1) * N), ad, sdesc(b + t1 * XV_BTILE, XV_LBO, XV_SBO),
+                      idesc_bf16(128, (tiles - t1) * N), (add || t > 0) ? 1u : 0u);
+        }
+        umma_commit(&bar_ae[sa]);
+        last = sa; plast = pa; any = true;
+        if (++sa == AE) { sa = 0; pa ^= 1u; }
+      };
+      for (int it = first; it < nitems && ok; it = next_item(it), ++u) {
+        // psi's and X's accumulators, once the epilogue has read the item before
+        if (u > 0 && !xs_wait(&bar_te[0], (u - 1) & 1, ok)) break;
+        for (int kc = 0; kc < nkc && ok; ++kc) {
+          if (!xs_wait(&bar_bf[sb], pb, ok)) break;
+          const uint32_t b0 = smem_u32(sB + sb * BSTAGE);
+          // psi and X alternate by order (psi_d at 2d N, X_d at (2d+1) N) and their field digits alternate the same way
+          // ([psi_ur_s, X_up_s] against m V, [psi_up_s, X_ur_s] against D), so one MMA covers both sums
+          entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, kc > 0);
+          if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, true);
+          if (kc == 0 && u > 0) xs_wait(&bar_te[1], (u - 1) & 1, ok);
+          if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, kc > 0);
+          if (!ok) break;
+          umma_commit(&bar_be[sb]);
+          if (++sb == XV_SB) { sb = 0; pb ^= 1u; }
+        }
+        if (ok) umma_commit(bar_tf);
+      }
+      if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
+        bool ok2 = true;
+        xs_wait(&bar_ae[last], plast, ok2);
+      }
+    }
+  } else if (warp < 2 + XV_NSW) {
+    // ---- column scales: cexp(2zz) over (Im ur, Re up), cexp(2zz+1) over (Re ur, Im up); fexp over uz.  Four z columns
+    // per warp, eight lanes each, over the magnitudes' high words; |x| < 2^(exponent field - 1022), +1 because the folds
+    // may double.
+    int ii = 0;
+    for (int it = first; it < nitems && ok; it = next_item(it), ++ii) {
+      const int slot = ii % XV_CXS;
+      if (ii >= XV_CXS && !xs_wait_w(&bar_ce[slot], (ii / XV_CXS - 1) & 1, ok)) break;
+      const int zz = (warp - 2) * 4 + (lane >> 3), z = item_z0(it) + zz;
       unsigned e0 = 0, e1 = 0, u0 = 0, u1 = 0;
       if (z < a.nzdim) {
-        const size_t cb = (size_t)a.nrdim * (m + (size_t)a.npdim * z);
-        auto ex = [](double v) { return ((unsigned)__double2hiint(v) >> 20) & 0x7FFu; };
-        // unrolled, so that the loads of several rows are in flight at once (the scan waits on them)
-#pragma unroll 6
-        for (int i = lane; i < a.nr; i += 32) {
-          const double2 r = a.ur[cb + i], pq = a.up[cb + i], q = a.uz[cb + i];
-          e0 = max(e0, max(ex(r.y), ex(pq.x)));
-          e1 = max(e1, max(ex(r.x), ex(pq.y)));
-          u0 = max(u0, ex(q.x));
-          u1 = max(u1, ex(q.y));
+        const size_t cb = (size_t)a.nrdim * (item_m(it) + (size_t)a.npdim * z);
+        const unsigned* pr = (const unsigned*)(a.ur + cb);   // (re lo, re hi, im lo, im hi)
+        const unsigned* pp = (const unsigned*)(a.up + cb);
+        const unsigned* pz = (const unsigned*)(a.uz + cb);
+#pragma unroll 4
+        for (int i = lane & 7; i < a.nr; i += 8) {
+          const unsigned rr = __ldcg(pr + 4 * i + 1), ri = __ldcg(pr + 4 * i + 3), qr = __ldcg(pp + 4 * i + 1),
+                         qi = __ldcg(pp + 4 * i + 3), wr = __ldcg(pz + 4 * i + 1), wi = __ldcg(pz + 4 * i + 3);
+          e0 = max(e0, max(ri & 0x7FFFFFFFu, qr & 0x7FFFFFFFu));
+          e1 = max(e1, max(rr & 0x7FFFFFFFu, qi & 0x7FFFFFFFu));
+          u0 = max(u0, wr & 0x7FFFFFFFu);
+          u1 = max(u1, wi & 0x7FFFFFFFu);
         }
       }
-      e0 = __reduce_max_sync(0xFFFFFFFFu, e0);
-      e1 = __reduce_max_sync(0xFFFFFFFFu, e1);
-      u0 = __reduce_max_sync(0xFFFFFFFFu, u0);
-      u1 = __reduce_max_sync(0xFFFFFFFFu, u1);
-      if (lane == 0) {
-        cexp[2 * cz] = e0 ? (int)e0 - 1021 : -2000;
-        cexp[2 * cz + 1] = e1 ? (int)e1 - 1021 : -2000;
-        fexp[2 * cz] = u0 ? (int)u0 - 1021 : -2000;
-        fexp[2 * cz + 1] = u1 ? (int)u1 - 1021 : -2000;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        e0 = max(e0, __shfl_xor_sync(0xFFFFFFFFu, e0, o));
+        e1 = max(e1, __shfl_xor_sync(0xFFFFFFFFu, e1, o));
+        u0 = max(u0, __shfl_xor_sync(0xFFFFFFFFu, u0, o));
+        u1 = max(u1, __shfl_xor_sync(0xFFFFFFFFu, u1, o));
       }
+      if ((lane & 7) == 0) {
+        // an all-subnormal column counts as zero
+        auto bound = [](unsigned h) { return !(h >> 20) ? -2000 : (BAL ? xs_ebound_bal(h) : (int)(h >> 20) - 1022) + 1; };
+        int* cx = cxs + slot * 2 * N;
+        cx[2 * zz] = bound(e0);
+        cx[2 * zz + 1] = bound(e1);
+        cx[N + 2 * zz] = bound(u0);
+        cx[N + 2 * zz + 1] = bound(u1);
+      }
+      mbar_arrive(&bar_cx[slot]);
     }
-    __syncthreads();
-    const uint8_t* img_b = (const uint8_t*)a.img + (((size_t)(m * 2 + par) * a.nmt + mt) * a.nkc) * (size_t)ASTAGE;
-    const int nkc = a.nkc;
-    const uint32_t it0 = it;
-    if (warp == 0) {
-      // ---- producer: each table chunk into its stage once the MMAs that read the stage before are done
-      if (lane == 0)
-        for (int kc = 0; kc < nkc && ok; ++kc) {
-          const uint32_t c = it0 + kc, s = c & 1;
-          if (c >= 2) xs_wait(&bar_mma[s], ((c - 2) >> 1) & 1, ok);
-          if (!ok) break;
-          mbar_expect_tx(&bar_a[s], ASTAGE);
-          bulk_g2s(sA + s * ASTAGE, img_b + (size_t)kc * ASTAGE, ASTAGE, &bar_a[s]);
-        }
-      __syncwarp();
-    } else if (warp == 1) {
-      // ---- MMA issue
-      if (lane == 0)
-        for (int kc = 0; kc < nkc && ok; ++kc) {
-          const uint32_t c = it0 + kc, s = c & 1;
-          xs_wait(&bar_a[s], (c >> 1) & 1, ok);
-          xs_wait(&bar_b[s], (c >> 1) & 1, ok);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t a0 = smem_u32(sA + s * ASTAGE), b0 = smem_u32(sB + s * BSTAGE);
-          auto A = [&](int t) { return sdesc(a0 + t * XV_ATILE, XV_LBO, XV_SBO); };
-          auto B = [&](int t) { return sdesc(b0 + t * BTILE, XV_LBO, XV_SBO); };
-          // table digit t against the field digits 0 .. n-1-t in one MMA: the field digits lie side by
-          // side in shared memory and the accumulators of the orders side by side in tensor memory, so
-          // the product of field digit s lands on order t + s.  psi and X alternate by order (psi_d at
-          // 2d N, X_d at (2d+1) N) and their field digits alternate the same way ([psi_ur_s, X_up_s]
-          // against m V, [psi_up_s, X_ur_s] against D), so one MMA of 2 N (NS - t) columns covers
-          // both sums
-#pragma unroll
-          for (int t = 0; t < NS; ++t) {
-            const uint32_t id = idesc_bf16(128, 2 * (NS - t) * N);
-            umma_bf16(tmem + 2 * t * N, A(t), B(0), id, (kc > 0 || t > 0) ? 1u : 0u);   // m V . [psi_ur | X_up]
-            umma_bf16(tmem + 2 * t * N, A(NS + t), B(2 * NS), id, 1u);                 // D . [psi_up | X_ur]
-          }
-#pragma unroll
-          for (int t = 0; t < NT; ++t)
-            umma_bf16(tmem + (2 * NS + t) * N, A(2 * NS + t), B(4 * NS), idesc_bf16(128, (NT - t) * N),
-                      (kc > 0 || t > 0) ? 1u : 0u);
-          umma_commit(&bar_mma[s]);
-        }
-      __syncwarp();
-    } else {
-      // ---- field digits: this thread's two K of its field at i and nr-1-i, fetched a chunk ahead
-      const int z = z0 + zz;
+  } else if (warp < 2 + XV_NSW + 2 * XV_GW) {
+    // ---- field digits: the group's chunks c = grp, grp + 2, ... of the CTA's sequence (item c / nkc, chunk c % nkc), a
+    // thread's two K of its field at i and nr-1-i fetched a chunk ahead
+    const int dt0 = tid - (2 + XV_NSW) * 32, grp = dt0 / (XV_GW * 32), dt = dt0 % (XV_GW * 32);
+    const int f = dt / (NZ * 8), kp = dt % 8, zz = (dt / 8) % NZ;   // eight K pairs of a column in consecutive lanes
+    const double2* src = f == 0 ? a.ur : (f == 1 ? a.up : a.uz);
+    const int off = xv_off(2 * zz, 2 * kp), off1 = xv_off(2 * zz + 1, 2 * kp);
+    double2 va[2], vb[2];
+    auto fetch = [&](int it, int kc) {
+      const int z = item_z0(it) + zz;
       const bool zok = z < a.nzdim;
-      const size_t cbase = (size_t)a.nrdim * (m + (size_t)a.npdim * (zok ? z : 0));
-      const double2* src = f == 0 ? a.ur : (f == 1 ? a.up : a.uz);
-      double2 va[2], vb[2];
-      auto fetch = [&](int kc) {
+      const size_t cbase = (size_t)a.nrdim * (item_m(it) + (size_t)a.npdim * (zok ? z : 0));
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int i = kc * XV_KC + 2 * kp + u;
-          const bool okk = zok && i < a.nrh;
-          va[u] = okk ? src[cbase + i] : make_double2(0.0, 0.0);
-          vb[u] = okk ? src[cbase + a.nr - 1 - i] : make_double2(0.0, 0.0);
-        }
-      };
-      fetch(0);
-      const int off = xv_off(2 * zz, 2 * kp), off1 = xv_off(2 * zz + 1, 2 * kp);
-      for (int kc = 0; kc < nkc && ok; ++kc) {
-        const uint32_t c = it0 + kc, s = c & 1;
-        if (c >= 2) xs_wait(&bar_mma[s], ((c - 2) >> 1) & 1, ok);
-        if (!ok) break;
-        uint8_t* bst = sB + s * BSTAGE;
-        if (f < 2) {
-          // integer folds of the two components with the column scales of the columns they land in
-          const int Ere = f == 0 ? cexp[2 * zz + 1] : cexp[2 * zz];       // Re ur -> col 2zz+1, Re up -> col 2zz
-          const int Eim = f == 0 ? cexp[2 * zz] : cexp[2 * zz + 1];
-          float h0[2][NS], h1[2][NS], g0[2][NS], g1[2][NS];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const long long ar = xs_fix(va[u].x, Ere, nbs), br = xs_fix(vb[u].x, Ere, nbs);
-            const long long ai = xs_fix(va[u].y, Eim, nbs), bi = xs_fix(vb[u].y, Eim, nbs);
-            const long long fs_re = ar + ss * br, fs_im = ai + ss * bi;
-            const long long fo_re = ar - ss * br, fo_im = ai - ss * bi;
-            if (f == 0) {   // psi_ur = -i F_s(ur): (Im, -Re); X_ur = i F_o(ur): (-Im, Re)
-              xs_digits_f<NS>(fs_im, w, h0[u]); xs_digits_f<NS>(-fs_re, w, h1[u]);
-              xs_digits_f<NS>(-fo_im, w, g0[u]); xs_digits_f<NS>(fo_re, w, g1[u]);
-            } else {        // psi_up = -F_o(up): (-Re, -Im); X_up = F_s(up): (Re, Im)
-              xs_digits_f<NS>(-fo_re, w, h0[u]); xs_digits_f<NS>(-fo_im, w, h1[u]);
-              xs_digits_f<NS>(fs_re, w, g0[u]); xs_digits_f<NS>(fs_im, w, g1[u]);
-            }
-          }
-          // B tiles: [psi_ur_s, X_up_s] at 2s, 2s+1; [psi_up_s, X_ur_s] at 2 NS + 2s, 2 NS + 2s + 1
-          const int tp = f == 0 ? 0 : 2 * NS, tx = f == 0 ? 2 * NS + 1 : 1;
-#pragma unroll
-          for (int q = 0; q < NS; ++q) {
-            *(uint32_t*)(bst + (tp + 2 * q) * BTILE + off) = xs_pack(h0[0][q], h0[1][q]);
-            *(uint32_t*)(bst + (tp + 2 * q) * BTILE + off1) = xs_pack(h1[0][q], h1[1][q]);
-            *(uint32_t*)(bst + (tx + 2 * q) * BTILE + off) = xs_pack(g0[0][q], g0[1][q]);
-            *(uint32_t*)(bst + (tx + 2 * q) * BTILE + off1) = xs_pack(g1[0][q], g1[1][q]);
-          }
-        } else {
-          // Y: F_s(uz) with the uz column scales
-          float h0[2][NT], h1[2][NT];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const long long re = xs_fix(va[u].x, fexp[2 * zz], nbt) + ss * xs_fix(vb[u].x, fexp[2 * zz], nbt);
-            const long long im = xs_fix(va[u].y, fexp[2 * zz + 1], nbt) + ss * xs_fix(vb[u].y, fexp[2 * zz + 1], nbt);
-            xs_digits_f<NT>(re, w, h0[u]);
-            xs_digits_f<NT>(im, w, h1[u]);
-          }
-#pragma unroll
-          for (int q = 0; q < NT; ++q) {
-            *(uint32_t*)(bst + (4 * NS + q) * BTILE + off) = xs_pack(h0[0][q], h0[1][q]);
-            *(uint32_t*)(bst + (4 * NS + q) * BTILE + off1) = xs_pack(h1[0][q], h1[1][q]);
-          }
-        }
-        fence_async_smem();
-        mbar_arrive(&bar_b[s]);
-        if (kc + 1 < nkc) fetch(kc + 1);
+      for (int u = 0; u < 2; ++u) {
+        const int i = kc * XV_KC + 2 * kp + u;
+        const bool okk = zok && i < a.nrh;
+        va[u] = okk ? src[cbase + i] : make_double2(0.0, 0.0);
+        vb[u] = okk ? src[cbase + a.nr - 1 - i] : make_double2(0.0, 0.0);
       }
+    };
+    int it = first, kc = grp, ii = 0;
+    auto settle = [&]() {   // chunk counts past an item's end run into the next items
+      while (it < nitems && kc >= nkc) { kc -= nkc; it = next_item(it); ++ii; }
+    };
+    settle();
+    if (it < nitems) fetch(it, kc);
+    int seen = -1, base0 = 0, base1 = 0;   // the item whose column scales are in base0 (re) and base1 (im)
+    for (uint32_t c = grp; it < nitems; c += 2) {
+      if (ii != seen) {
+        if (!xs_wait_w(&bar_cx[ii % XV_CXS], (ii / XV_CXS) & 1, ok)) break;
+        const int* cx = cxs + (ii % XV_CXS) * 2 * N + (f == 2 ? N : 0);
+        // Re ur lands in column 2zz+1 and Im ur in 2zz; Re up (and Re uz) in 2zz and Im up in 2zz+1
+        const int er = cx[2 * zz + (f == 0 ? 1 : 0)], ei = cx[2 * zz + (f == 0 ? 0 : 1)];
+        base0 = xs_fix_base(er, f == 2 ? nbt : nbs, true);
+        base1 = xs_fix_base(ei, f == 2 ? nbt : nbs, true);
+        seen = ii;
+      }
+      const uint32_t s = c % XV_SB;
+      if (c >= XV_SB && !xs_wait_w(&bar_be[s], (c / XV_SB - 1) & 1, ok)) break;
+      uint8_t* bst = sB + s * BSTAGE;
+      const bool odd = item_par(it);   // own-parity fold sign
+      // integer folds of the two components with the column scales of the columns they land in
+      long long sre[2], sim[2], ore[2], oim[2];   // F_s and F_o
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const long long ar = xs_fixs(va[u].x, base0), br0 = xs_fixs(vb[u].x, base0), br = odd ? -br0 : br0;
+        const long long ai = xs_fixs(va[u].y, base1), bi0 = xs_fixs(vb[u].y, base1), bi = odd ? -bi0 : bi0;
+        sre[u] = ar + br; sim[u] = ai + bi;
+        ore[u] = ar - br; oim[u] = ai - bi;
+      }
+      if (f < 2) {
+        // f = 0: psi_ur = -i F_s(ur) = (Im, -Re), X_ur = i F_o(ur) = (-Im, Re)
+        // f = 1: psi_up = -F_o(up) = (-Re, -Im),  X_up = F_s(up) = (Re, Im)
+        // B tiles: [psi_ur_s, X_up_s] at 2s, 2s+1; [psi_up_s, X_ur_s] at 2 NS + 2s, 2 NS + 2s + 1
+        constexpr unsigned long long bias = BAL ? xs_bias<NS, W>() : 0ull;
+        const int tp = f == 0 ? 0 : 2 * NS, tx = f == 0 ? 2 * NS + 1 : 1;
+        auto put = [&](int tile, int o, long long p, long long q) {
+          const unsigned long long x0 = (unsigned long long)p + bias, x1 = (unsigned long long)q + bias;
+          xs_static_for<NS>([&](auto sc) {
+            constexpr int g = decltype(sc)::value;
+            *(uint32_t*)(bst + (tile + 2 * g) * XV_BTILE + o) = xs_digit2<NS, W, BAL, g>(x0, x1);
+          });
+        };
+        put(tp, off, f == 0 ? sim[0] : -ore[0], f == 0 ? sim[1] : -ore[1]);
+        put(tp, off1, f == 0 ? -sre[0] : -oim[0], f == 0 ? -sre[1] : -oim[1]);
+        put(tx, off, f == 0 ? -oim[0] : sre[0], f == 0 ? -oim[1] : sre[1]);
+        put(tx, off1, f == 0 ? ore[0] : sim[0], f == 0 ? ore[1] : sim[1]);
+      } else {
+        // Y: F_s(uz) with the uz column scales
+        constexpr unsigned long long bias = BAL ? xs_bias<NT, W>() : 0ull;
+        xs_static_for<NT>([&](auto sc) {
+          constexpr int g = decltype(sc)::value;
+          *(uint32_t*)(bst + (4 * NS + g) * XV_BTILE + off) =
+              xs_digit2<NT, W, BAL, g>((unsigned long long)sre[0] + bias, (unsigned long long)sre[1] + bias);
+          *(uint32_t*)(bst + (4 * NS + g) * XV_BTILE + off1) =
+              xs_digit2<NT, W, BAL, g>((unsigned long long)sim[0] + bias, (unsigned long long)sim[1] + bias);
+        });
+      }
+      fence_async_smem();
+      mbar_arrive(&bar_bf[s]);
+      kc += 2;
+      settle();
+      if (it < nitems) fetch(it, kc);
     }
-    it = it0 + nkc;
-    // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. (rows t) and the 8-column block w / 4
-    const int t = mt * 128 + (warp & 3) * 32 + lane;
-    const int j = 2 * t + par;
-    const bool rok = j < nn && t < a.ntr;
-    // the row exponents, loaded before the wait so that their latency hides behind it
-    const int er = rok ? a.rexp[(size_t)(m * 2 + par) * a.ntr + t] : -2000;
-    const int et = rok ? a.texp[(size_t)(m * 2 + par) * a.ntr + t] : -2000;
-    {
-      const uint32_t lst = it - 1;
-      xs_wait(&bar_mma[lst & 1], (lst >> 1) & 1, ok);
-    }
-    ok = __syncthreads_and(ok);
-    if (!ok) break;
-    tc_fence_after();
-    if (mt * 128 + (warp & 3) * 32 < a.ntr) {   // a warp of rows past the tile's rows has nothing to write
-      const uint32_t lrow = (uint32_t)((warp & 3) * 32) << 16;
-      const int cb = warp >> 2;
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {   // four columns (two complex z) at a time
-        const int c0 = cb * 8 + half * 4;
-        // the orders combined exactly in 64-bit integers, T = sum_d G_d 2^(w (n-1-d) - esh), then
-        // T 2^(row exp + column exp + esh - w (n+1)) rounded once to FP64
-        long long tp[4] = {0, 0, 0, 0}, tx[4] = {0, 0, 0, 0}, ty[4] = {0, 0, 0, 0};
-        {
-          uint32_t gp[NS][4], gx[NS][4];
+  } else {
+    // ---- epilogue: warp e reads TMEM lanes 32 (e % 4) .. (rows t) and the 8-column block e / 4
+    const int lq = warp & 3, cb = (warp - 2 - XV_NSW - 2 * XV_GW) >> 2;
+    const uint32_t tcol = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(cb * 8);
+    uint32_t u = 0;
+    for (int it = first; it < nitems; it = next_item(it), ++u) {
+      const int m = item_m(it), mt = item_mt(it), par = item_par(it), z0 = item_z0(it);
+      const int nn = max(min(a.nrc, a.nrc - m), 0);
+      const int t = mt * 128 + lq * 32 + lane, j = 2 * t + par;
+      const bool rok = j < nn && t < a.ntr, wlive = mt * 128 + lq * 32 < a.ntr;
+      // the row exponents, loaded before the wait so that their latency hides behind it
+      const int er = rok ? a.rexp[(size_t)(m * 2 + par) * a.ntr + t] : -2000;
+      const int et = rok ? a.texp[(size_t)(m * 2 + par) * a.ntr + t] : -2000;
+      if (!xs_wait_w(bar_tf, u & 1, ok)) break;
+      tc_fence_after();
+      long long tp[8], tx[8], ty[8];
+      int ep = 0, ex = 0, ey = 0;
+      if (wlive) {
+        ep = xv_sums<NS, W, BAL>(tcol, 2 * N, a.esh_s, tp);
+        ex = xv_sums<NS, W, BAL>(tcol + N, 2 * N, a.esh_s, tx);
+      }
+      tc_fence_before();
+      mbar_arrive(&bar_te[0]);
+      if (wlive) ey = xv_sums<NT, W, BAL>(tcol + TY, N, a.esh_t, ty);
+      tc_fence_before();
+      mbar_arrive(&bar_te[1]);
+      const uint32_t slot = u % XV_CXS;
+      if (!xs_wait_w(&bar_cx[slot], (u / XV_CXS) & 1, ok)) break;   // long since complete
+      const int* cx = cxs + slot * 2 * N + cb * 8;
+      if (rok && wlive) {
+        // the products carry 2^(-2 nb), the orders' unit is 2^(w (n-1))
+        constexpr int os = W * (NS - 1) - 2 * nbs, ot = W * (NT - 1) - 2 * nbt;
 #pragma unroll
-          for (int d = 0; d < NS; ++d) {
-            tmem_ld4_nw(tmem + lrow + 2 * d * N + c0, gp[d]);
-            tmem_ld4_nw(tmem + lrow + (2 * d + 1) * N + c0, gx[d]);
+        for (int c = 0; c < 8; c += 2) {
+          const int zc = z0 + (cb * 8 + c) / 2, kk = zc + 1;
+          if (zc >= a.nzdim || !(kk <= a.nzc || kk >= a.nzcu)) continue;
+          double pv[2], xv[2], yv[2];
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int E = cx[c + h], F = cx[N + c + h];
+            const bool ox = er > -2000 && E > -2000, oy = et > -2000 && F > -2000;
+            pv[h] = ox ? xs_i64_to_double(tp[c + h], er + E + ep + os) : 0.0;
+            xv[h] = ox ? xs_i64_to_double(tx[c + h], er + E + ex + os) : 0.0;
+            yv[h] = oy ? xs_i64_to_double(ty[c + h], et + F + ey + ot) : 0.0;
           }
-          tmem_wait_ld();
-#pragma unroll
-          for (int d = 0; d < NS; ++d) {
-            const int sh = w * (NS - 1 - d) - a.esh_s;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              tp[c] += xs_shl((long long)xs_f2i(__uint_as_float(gp[d][c])), sh);
-              tx[c] += xs_shl((long long)xs_f2i(__uint_as_float(gx[d][c])), sh);
-            }
-          }
-        }
-        {
-          uint32_t gy[NT][4];
-#pragma unroll
-          for (int d = 0; d < NT; ++d) tmem_ld4_nw(tmem + lrow + (2 * NS + d) * N + c0, gy[d]);
-          tmem_wait_ld();
-#pragma unroll
-          for (int d = 0; d < NT; ++d) {
-            const int sh = w * (NT - 1 - d) - a.esh_t;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) ty[c] += xs_shl((long long)xs_f2i(__uint_as_float(gy[d][c])), sh);
-          }
-        }
-        double pv[4], xv[4], yv[4];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int E = cexp[c0 + c], F = fexp[c0 + c];
-          const bool ox = er > -2000 && E > -2000, oy = et > -2000 && F > -2000;
-          pv[c] = ox ? xs_i64_to_double(tp[c], er + E + a.esh_s - w * (NS + 1)) : 0.0;
-          xv[c] = ox ? xs_i64_to_double(tx[c], er + E + a.esh_s - w * (NS + 1)) : 0.0;
-          yv[c] = oy ? xs_i64_to_double(ty[c], et + F + a.esh_t - w * (NT + 1)) : 0.0;
-        }
-        if (rok) {
-#pragma unroll
-          for (int c = 0; c < 4; c += 2) {
-            const int n = c0 + c, zc = z0 + n / 2;
-            if (zc >= a.nzdim) continue;
-            const int kk = zc + 1;
-            if (!(kk <= a.nzc || kk >= a.nzcu)) continue;
-            const double kz = a.ak[zc];
-            const size_t o = j + (size_t)a.nrdim * (m + (size_t)a.npdim * zc);
-            a.psi[o] = make_double2(pv[c], pv[c + 1]);
-            a.chi[o] = make_double2(fma(kz, xv[c], -yv[c]), fma(kz, xv[c + 1], -yv[c + 1]));
-          }
+          const double kz = a.ak[zc];
+          const size_t o = j + (size_t)a.nrdim * (m + (size_t)a.npdim * zc);
+          a.psi[o] = make_double2(pv[0], pv[1]);
+          a.chi[o] = make_double2(fma(kz, xv[0], -yv[0]), fma(kz, xv[1], -yv[1]));
         }
       }
-    }
-    tc_fence_before();
-    __syncthreads();   // TMEM read out (and cexp / fexp read) before the next item
-  }
-  if (!ok) {
-    if (tid == 0) atomicExch(a.status, 2);
-    if (tid == 0 && it > 0) {   // let what was issued finish (bounded) before the memory goes away
-      bool ok2 = true;
-      const uint32_t lst = it - 1;
-      xs_wait(&bar_mma[lst & 1], (lst >> 1) & 1, ok2);
+      mbar_arrive(&bar_ce[slot]);
     }
   }
+  if (!ok) atomicExch(a.status, 2);
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, TCOLS);
+  if (warp == 1) tmem_dealloc(tmem, TCOLS);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -437,40 +560,60 @@ struct XvImg {
   uint16_t* p = nullptr;
   int *rexp = nullptr, *texp = nullptr;
   size_t bytes = 0, ebytes = 0;
-  int nrc = -1, npc = -1, ns = 0, nt = 0, w = 0;
+  int nrc = -1, npc = -1, ns = 0;
 };
-static XvImg g_xv;
+static XvImg g_xvs[2];   // plain, mixed
 
 void xv_free() {
-  if (g_xv.p) dfree(g_xv.p, g_xv.bytes);
-  if (g_xv.rexp) dfree(g_xv.rexp, g_xv.ebytes);
-  if (g_xv.texp) dfree(g_xv.texp, g_xv.ebytes);
-  g_xv = XvImg();
+  for (XvImg& im : g_xvs) {
+    if (im.p) dfree(im.p, im.bytes);
+    if (im.rexp) dfree(im.rexp, im.ebytes);
+    if (im.texp) dfree(im.texp, im.ebytes);
+    im = XvImg();
+  }
 }
 
+// digit counts of psi / X and of Y and their width; ns = 0 where no configuration is exact
 struct XvCfg { int ns, nt, w; };
-static bool xv_cfg(int k, XvCfg& c) {
+static XvCfg xv_cfg(int k, bool plain) {
+  if (plain) return k <= 372 ? XvCfg{9, 9, 7} : XvCfg{0, 0, 0};
   const double lim = 16777216.0;
   auto fits = [&](int ns, int nt, int w) {
     const double d = (double)(1 << w) * (1 << w);   // largest digit product (two's-complement digits)
     return 2.0 * ns * k * d < lim && (double)nt * k * d < lim;
   };
-  if (fits(5, 7, 7)) { c = {5, 7, 7}; return true; }
-  if (fits(6, 8, 6)) { c = {6, 8, 6}; return true; }
-  return false;
+  if (fits(5, 7, 7)) return {5, 7, 7};
+  if (fits(6, 8, 6)) return {6, 8, 6};
+  return {0, 0, 0};
 }
 
-bool xv_supported() {
-  XvCfg c;
-  return xv_cfg(G.nrh, c);
-}
+bool xv_supported(bool plain) { return xv_cfg(G.nrh, plain).ns > 0; }
 
-template <int NS, int NT>
-static int xv_launch(const XvArgs& args, int npc) {
-  constexpr int N = 2 * XV_NZ;
-  const size_t sm = 1024 + 2 * (size_t)(2 * NS + NT) * XV_ATILE + 2 * (size_t)(4 * NS + NT) * N * XV_KC * 2 +
-                    4 * N * sizeof(int) + 64;
-  auto kern = k_xv_contract<NS, NT>;
+template <int NS, int NT, int W>
+static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
+  if (im.nrc != args.nrc || im.npc != npc || !im.p || im.ns != NS) {
+    if (im.p) dfree(im.p, im.bytes);
+    if (im.rexp) dfree(im.rexp, im.ebytes);
+    if (im.texp) dfree(im.texp, im.ebytes);
+    im = XvImg();
+    im.bytes = (size_t)npc * 2 * args.nmt * args.nkc * (2 * NS + NT) * XV_ATILE;
+    im.ebytes = (size_t)npc * 2 * args.ntr * sizeof(int);
+    MLG_TRY(dmalloc((void**)&im.p, im.bytes));
+    MLG_TRY(dmalloc((void**)&im.rexp, im.ebytes));
+    MLG_TRY(dmalloc((void**)&im.texp, im.ebytes));
+    k_xv_rexp<<<dim3(cdiv(args.ntr, 128), npc * 2), 128, 0, G.stream>>>(G.tV, G.tD, G.tT, im.rexp, im.texp, G.nrh, G.ne, args.nrc,
+                                                                        args.ntr, plain ? 1 : 0);
+    MLG_LAUNCH();
+    k_xv_table<NS, NT, W><<<npc * 2 * args.nmt * args.nkc, 256, 0, G.stream>>>(
+        G.tV, G.tD, G.tT, im.rexp, im.texp, im.p, G.nrh, G.ne, args.nrc, args.nmt, args.nkc, args.ntr);
+    MLG_LAUNCH();
+    im.nrc = args.nrc; im.npc = npc; im.ns = NS;
+  }
+  args.img = im.p; args.rexp = im.rexp; args.texp = im.texp;
+  const size_t fixed = 1024 + XV_SB * (size_t)xv_bstage_bytes(NS, NT) + XV_CXS * 2 * XV_N * sizeof(int) + 512;
+  args.aent = (int)std::min<size_t>(XV_AEMAX, (227 * 1024 - fixed) / xv_aent_bytes(NS, NT));
+  const size_t sm = fixed + (size_t)args.aent * xv_aent_bytes(NS, NT);
+  auto kern = k_xv_contract<NS, NT, W>;
   MLG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int nitems = (npc - args.m0) * 2 * args.nmt * cdiv(G.nzdim, XV_NZ);
   kern<<<std::min(nitems, 152), XV_THREADS, sm, G.stream>>>(args);
@@ -479,39 +622,17 @@ static int xv_launch(const XvArgs& args, int npc) {
 }
 
 // psi, chi: the rows of m0 <= m < npc written (zeroed elsewhere by the caller)
-int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0) {
+int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain) {
   if (npc <= m0) return 0;
-  XvCfg cfg;
-  if (!xv_cfg(G.nrh, cfg)) return set_error(MLG_ESIZE, "vec2tp: too many radial points for exact slices");
-  const int ntr = (nrc + 1) / 2;
-  const int nmt = cdiv(ntr, 128), nkc = cdiv(G.nrh, XV_KC);
-  XvImg& im = g_xv;
-  if (im.nrc != nrc || im.npc != npc || !im.p || im.ns != cfg.ns || im.nt != cfg.nt || im.w != cfg.w) {
-    if (im.p) dfree(im.p, im.bytes);
-    if (im.rexp) dfree(im.rexp, im.ebytes);
-    if (im.texp) dfree(im.texp, im.ebytes);
-    im = XvImg();
-    im.bytes = (size_t)npc * 2 * nmt * nkc * (2 * cfg.ns + cfg.nt) * XV_ATILE;
-    im.ebytes = (size_t)npc * 2 * ntr * sizeof(int);
-    MLG_TRY(dmalloc((void**)&im.p, im.bytes));
-    MLG_TRY(dmalloc((void**)&im.rexp, im.ebytes));
-    MLG_TRY(dmalloc((void**)&im.texp, im.ebytes));
-    k_xv_rexp<<<dim3(cdiv(ntr, 128), npc * 2), 128, 0, G.stream>>>(G.tV, G.tD, G.tT, im.rexp, im.texp, G.nrh, G.ne, nrc, ntr);
-    MLG_LAUNCH();
-    const int nb = npc * 2 * nmt * nkc;
-    if (cfg.ns == 5)
-      k_xv_table<5, 7><<<nb, 256, 0, G.stream>>>(G.tV, G.tD, G.tT, im.rexp, im.texp, im.p, G.nrh, G.ne, nrc, nmt, nkc, ntr, cfg.w);
-    else
-      k_xv_table<6, 8><<<nb, 256, 0, G.stream>>>(G.tV, G.tD, G.tT, im.rexp, im.texp, im.p, G.nrh, G.ne, nrc, nmt, nkc, ntr, cfg.w);
-    MLG_LAUNCH();
-    im.nrc = nrc; im.npc = npc; im.ns = cfg.ns; im.nt = cfg.nt; im.w = cfg.w;
-  }
-  XvArgs args;
-  args.ur = ur; args.up = up; args.uz = uz; args.psi = psi; args.chi = chi; args.img = im.p; args.rexp = im.rexp;
-  args.texp = im.texp; args.ak = G.ak; args.status = (int*)(G.dscal + DS_FLAG + 1) + 1;
+  const XvCfg cfg = xv_cfg(G.nrh, plain);
+  if (!cfg.ns) return set_error(MLG_ESIZE, "vec2tp: too many radial points for exact slices");
+  XvArgs args{};
+  args.ur = ur; args.up = up; args.uz = uz; args.psi = psi; args.chi = chi;
+  args.ak = G.ak; args.status = (int*)(G.dscal + DS_FLAG + 1) + 1;
   args.nr = G.nr; args.nrh = G.nrh; args.nrdim = G.nrdim; args.npdim = G.npdim; args.nzdim = G.nzdim; args.nrc = nrc;
-  args.nzc = G.chopzl; args.nzcu = G.chopzu; args.nmt = nmt; args.nkc = nkc; args.ntr = ntr; args.w = cfg.w; args.m0 = m0;
-  args.npc = npc;
+  args.nzc = G.chopzl; args.nzcu = G.chopzu; args.m0 = m0; args.npc = npc;
+  args.ntr = (nrc + 1) / 2;
+  args.nmt = cdiv(args.ntr, 128); args.nkc = cdiv(G.nrh, XV_KC);
   {
     // the 64-bit order sums stay below 2^62: |G_d| <= K (pairs of order d) 2^(2w), with two products
     // per digit pair for psi and X
@@ -522,10 +643,10 @@ int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int 
     args.esh_s = esh(cfg.ns, 2 * cfg.ns);
     args.esh_t = esh(cfg.nt, cfg.nt);
   }
-  // 8 complex z columns per work item: the (2 NS + NT) orders of 2 x 8 columns fit the 512
-  // tensor-memory columns
-  if (cfg.ns == 5) return xv_launch<5, 7>(args, npc);
-  return xv_launch<6, 8>(args, npc);
+  XvImg& im = g_xvs[plain ? 0 : 1];
+  if (cfg.ns == 9) return xv_run<9, 9, 7>(args, im, npc, plain);
+  if (cfg.ns == 5) return xv_run<5, 7, 7>(args, im, npc, plain);
+  return xv_run<6, 8, 6>(args, im, npc, plain);
 }
 
 }  // namespace mlg
