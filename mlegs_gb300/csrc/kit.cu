@@ -263,6 +263,46 @@ static bool factors235(int n) {
   return n == 1;
 }
 
+// exp(-2 pi i k / L), k < count, for L a power of two, in units of 2^-61: (re, im) upper parts and (re, im) lower 31 bits of
+// the nearest integers.  The roots exp(2 pi i / 2^j) come from the half-angle formulas in double-double arithmetic and
+// every k is the product of the roots of its bits, so the entries do not depend on the machine's sin and cos.
+static std::vector<int4> twid_q(int L, int count) {
+  struct D2 { double h, l; };
+  auto two_s = [](double a, double b) { const double s = a + b, v = s - a; return D2{s, (a - (s - v)) + (b - v)}; };
+  auto quick = [](double a, double b) { const double s = a + b; return D2{s, b - (s - a)}; };
+  auto add = [&](D2 a, D2 b) { const D2 s = two_s(a.h, b.h); return quick(s.h, s.l + (a.l + b.l)); };
+  auto mul = [&](D2 a, D2 b) {
+    const double q = a.h * b.h, e = std::fma(a.h, b.h, -q);
+    return quick(q, e + (a.h * b.l + a.l * b.h));
+  };
+  auto neg = [](D2 a) { return D2{-a.h, -a.l}; };
+  auto root = [&](D2 a) {   // square root: a Newton step on the FP64 one
+    if (a.h <= 0.0) return D2{0.0, 0.0};
+    const double x = std::sqrt(a.h);
+    const D2 r = add(a, neg(mul({x, 0.0}, {x, 0.0})));
+    return quick(x, r.h / (2.0 * x));
+  };
+  std::vector<D2> c{{1.0, 0.0}, {-1.0, 0.0}, {0.0, 0.0}}, sn{{0.0, 0.0}, {0.0, 0.0}, {1.0, 0.0}};   // angles 2 pi, pi, pi / 2
+  while ((1 << (c.size() - 1)) < L) {
+    const D2 q = c.back();
+    c.push_back(root(mul(add({1.0, 0.0}, q), {0.5, 0.0})));
+    sn.push_back(root(mul(add({1.0, 0.0}, neg(q)), {0.5, 0.0})));
+  }
+  auto fixed = [](D2 v) { return (long long)std::ldexp(v.h, 61) + std::llrint(std::ldexp(v.l, 61)); };
+  std::vector<int4> t(std::max(count, 1));
+  for (int k = 0; k < count; ++k) {
+    D2 x{1.0, 0.0}, y{0.0, 0.0};
+    for (int j = 1, bit = L / 2; bit >= 1; ++j, bit /= 2)   // bit: an angle of 2 pi / 2^j
+      if (k & bit) {
+        const D2 nx = add(mul(x, c[j]), neg(mul(y, sn[j]))), ny = add(mul(x, sn[j]), mul(y, c[j]));
+        x = nx; y = ny;
+      }
+    const long long re = fixed(x), im = fixed(neg(y));
+    t[k] = make_int4((int)(re >> 31), (int)(im >> 31), (int)(re & 0x7FFFFFFF), (int)(im & 0x7FFFFFFF));
+  }
+  return t;
+}
+
 template <class T>
 static int upload(T** d, const std::vector<T>& h) {
   MLG_TRY(dmalloc((void**)d, h.size() * sizeof(T)));
@@ -403,6 +443,13 @@ int kit_build(const mlg_params* P) {
   MLG_TRY(upload(&G.tw_pdf, todf(tp)));
   MLG_TRY(upload(&G.tw_prdf, todf(tpr)));
   MLG_TRY(upload(&G.tw_zdf, todf(tz)));
+
+  // fixed-point twiddles of the plain form's power-of-two transforms
+  if (fftq_length(nz)) MLG_TRY(upload(&G.tw_zq, twid_q(nz, nz)));
+  if (fftq_length(G.nph)) {
+    MLG_TRY(upload(&G.tw_pq, twid_q(G.nph, G.nph)));
+    MLG_TRY(upload(&G.tw_prq, twid_q(np, G.nph + 1)));
+  }
 
   MLG_CUDA(cudaStreamSynchronize(G.stream));
   dfree(d_logfact, logfact.size() * sizeof(double));
