@@ -148,7 +148,7 @@ __device__ __forceinline__ bool xs_wait(uint64_t* bar, uint32_t phase, bool& ok)
 
 // Warp roles of the contraction kernel (896 threads, one CTA per SM):
 //   warp 0        the table entries, by bulk copy (one thread)
-//   warp 1        MMA issue (one thread) and the tensor-memory allocation
+//   warp 1        MMA issue and the tensor-memory allocation
 //   warps 2, 3    the items' field columns, by bulk copy (one thread), and their scales
 //   warps 4..11   field digits, in two groups that take the stages in turn
 //   warps 12..27  epilogue: tensor memory -> 64-bit order sums -> FP64 results
@@ -157,12 +157,12 @@ __device__ __forceinline__ bool xs_wait(uint64_t* bar, uint32_t phase, bool& ok)
 // Every hand-off is an mbarrier: the table entries and the field-digit stages (one parity of a chunk each) are rings,
 // the field columns are one buffer (the next item's columns land while the MMAs and the epilogue of this one run).  The
 // epilogue keeps the even parity's sums in registers and writes both parities' results after the odd unit.
-// What bounds it (clock64 traces, 192 points, six digits, 14 000 cycles an item): the integer pipe, on which the digits,
-// the order sums and the conversions take about 8 000 of them; the MMAs need 7 400 (shared-memory bandwidth: per stage a
-// 24 KiB table entry is written and read once, the digits are written once and read by the MMAs).  A cluster of two CTAs
-// sharing the table entries by multicast measured the same.  Ten steps' radial transforms at 192 x 128 x 128, mixed:
-// 4.27 -> 3.70 ms against eight-warp epilogues that released both parities together and reduced the scales themselves
-// (20 700 cycles an item); 512 x 512 x 256, two mixed steps: 22.4 -> 16.5 ms; plain: 2.48 -> 1.85 ms for four steps.
+// What bounds it (clock64 traces, 192 points, six digits, about 13 000 cycles an item): the integer pipe, on which the
+// digits, the order sums and the conversions take about 8 000 of them; the MMAs need 4 000 (7 400 while one lane issued
+// them from a branch: 3.70 ms below).  A cluster of two CTAs sharing the table entries by multicast measured the same.
+// Ten steps' radial transforms at 192 x 128 x 128, mixed: 4.27 -> 3.49 ms against eight-warp epilogues that released both
+// parities together and reduced the scales themselves (20 700 cycles an item); 512 x 512 x 256, two mixed steps:
+// 22.4 -> 15.1 ms; plain: 2.48 -> 1.70 ms for four steps.
 // a bounded wait whose outcome every lane of the warp shares (the warp-collective operations that
 // follow need the whole warp)
 __device__ __forceinline__ bool xs_wait_w(uint64_t* bar, uint32_t phase, bool& ok) {
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   uint64_t* bar_ce = bar_cx + XS_CXS;      // [XS_CXS] column scales read (epilogue threads: the item's last readers)
   uint32_t* tslot = (uint32_t*)(bar_ce + XS_CXS);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform
   if (tid < XS_NBAR) {   // a barrier per thread
     const int i = tid;
     const uint64_t* q = bars + i;
@@ -329,50 +329,49 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issue
-    if (lane == 0) {
-      uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
-      bool any = false;
-      for (int item = first; item < nitems && ok; item = next_item(item)) {
-        int nkc_m, nrows, nmt_m;
-        geom(item_nn(item), nkc_m, nrows, nmt_m);
-        for (int v = 0; v < 2 * nmt_m && ok; ++v, ++u) {   // units: row tile v / 2, parity v % 2
-          // the unit's accumulators, once the epilogue has read what they held TB units before
-          const uint32_t tb = u % TB;
-          if (u >= (uint32_t)TB && !xs_wait(&bar_te[tb], ((u - TB) / TB) & 1, ok)) break;
-          const uint32_t tacc = tmem + tb * (uint32_t)ACC;
-          for (int kc = 0; kc < nkc_m; ++kc) {
-            if (!xs_wait(&bar_bf[sb], pb, ok)) break;
-            if (!xs_wait(&bar_af[sa], pa, ok)) break;
-            tc_fence_after();
-            const uint32_t a0 = smem_u32(sA + sa * AENT), b0 = smem_u32(sB + sb * BSTAGE);
-            // table digit t times the field digits s = 0 .. NO-1-t in one MMA of N (NO - t) columns (two where that
-            // passes the 256 columns of an MMA): the field digits lie side by side in shared memory and the orders
-            // d = t + s side by side in tensor memory, so the product of digit s lands on order t + s
+    // ---- MMA issue (the whole warp, one elected lane issuing)
+    const uint32_t el = elect_lane();
+    uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
+    bool any = false;
+    for (int item = first; item < nitems && ok; item = next_item(item)) {
+      int nkc_m, nrows, nmt_m;
+      geom(item_nn(item), nkc_m, nrows, nmt_m);
+      for (int v = 0; v < 2 * nmt_m && ok; ++v, ++u) {   // units: row tile v / 2, parity v % 2
+        // the unit's accumulators, once the epilogue has read what they held TB units before
+        const uint32_t tb = u % TB;
+        if (u >= (uint32_t)TB && !xs_wait_w(&bar_te[tb], ((u - TB) / TB) & 1, ok)) break;
+        const uint32_t tacc = tmem + tb * (uint32_t)ACC;
+        for (int kc = 0; kc < nkc_m; ++kc) {
+          if (!xs_wait_w(&bar_bf[sb], pb, ok)) break;
+          if (!xs_wait_w(&bar_af[sa], pa, ok)) break;
+          tc_fence_after();
+          const uint32_t a0 = smem_u32(sA) + sa * AENT, b0 = smem_u32(sB) + sb * BSTAGE;
+          // table digit t times the field digits s = 0 .. NO-1-t in one MMA of N (NO - t) columns (two where that
+          // passes the 256 columns of an MMA): the field digits lie side by side in shared memory and the orders
+          // d = t + s side by side in tensor memory, so the product of digit s lands on order t + s
 #pragma unroll
-            for (int t = 0; t < NO; ++t) {
-              const uint64_t ad = sdesc(a0 + t * XS_ATILE, XS_LBO, XS_SBO);
-              constexpr int NB1 = 256 / N;   // digits of one MMA
-              const int n1 = NO - t < NB1 ? NO - t : NB1;
-              umma_bf16(tacc + (uint32_t)(t * N), ad, sdesc(b0, XS_LBO, XS_SBO), idesc_bf16(128, n1 * N),
-                        (kc > 0 || t > 0) ? 1u : 0u);
-              if (NO - t > NB1)
-                umma_bf16(tacc + (uint32_t)((t + NB1) * N), ad, sdesc(b0 + NB1 * BT, XS_LBO, XS_SBO),
-                          idesc_bf16(128, (NO - t - NB1) * N), (kc > 0 || t > 0) ? 1u : 0u);
-            }
-            umma_commit(&bar_ae[sa]);
-            umma_commit(&bar_be[sb]);
-            last = sa; plast = pa; any = true;
-            if (++sa == AE) { sa = 0; pa ^= 1u; }
-            if (++sb == SB) { sb = 0; pb ^= 1u; }
+          for (int t = 0; t < NO; ++t) {
+            const uint64_t ad = sdesc(a0 + t * XS_ATILE, XS_LBO, XS_SBO);
+            constexpr int NB1 = 256 / N;   // digits of one MMA
+            const int n1 = NO - t < NB1 ? NO - t : NB1;
+            umma_bf16(tacc + (uint32_t)(t * N), ad, sdesc(b0, XS_LBO, XS_SBO), idesc_bf16(128, n1 * N),
+                      (kc > 0 || t > 0) ? 1u : 0u, el);
+            if (NO - t > NB1)
+              umma_bf16(tacc + (uint32_t)((t + NB1) * N), ad, sdesc(b0 + NB1 * BT, XS_LBO, XS_SBO),
+                        idesc_bf16(128, (NO - t - NB1) * N), (kc > 0 || t > 0) ? 1u : 0u, el);
           }
-          if (ok) umma_commit(&bar_tf[tb]);
+          umma_commit(&bar_ae[sa], el);
+          umma_commit(&bar_be[sb], el);
+          last = sa; plast = pa; any = true;
+          if (++sa == AE) { sa = 0; pa ^= 1u; }
+          if (++sb == SB) { sb = 0; pb ^= 1u; }
         }
+        if (ok) umma_commit(&bar_tf[tb], el);
       }
-      if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
-        bool ok2 = true;
-        xs_wait(&bar_ae[last], plast, ok2);
-      }
+    }
+    if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
+      bool ok2 = true;
+      xs_wait_w(&bar_ae[last], plast, ok2);
     }
   } else if (warp < 2 + XS_NSW) {
     // ---- column scales from the largest magnitudes' high words of the re and im parts: |x| < 2^(exponent field - 1022),

@@ -30,7 +30,7 @@
 //
 // Engine: a persistent grid of one CTA per SM over work items (m, 8 complex z columns, 128-row tile, parity).
 //   warp 0        the table entries (the digits of m V, D or T for a chunk of 16 radial points), by bulk copy
-//   warp 1        MMA issue (one thread): a table digit t meets every field digit s <= n-1-t of its operands in
+//   warp 1        MMA issue: a table digit t meets every field digit s <= n-1-t of its operands in
 //                 one MMA (M = 128, K = 16; the field digits side by side in shared memory, the orders side by
 //                 side in tensor memory, psi's and X's alternating), two where that passes 256 columns
 //   warps 2, 3    the items' column scales, up to four items ahead
@@ -39,10 +39,12 @@
 //   warps 16..23  epilogue
 // Every hand-off is an mbarrier and every wait is bounded.  psi's and X's accumulators are released before Y's are
 // read.
-// What bounds it: the table entries' way through L2 (plain: 108 KiB per chunk for 8 columns, 1.3 GB per launch at
-// 192 x 128 x 128) and shared memory, and the integer pipe for the digits.
-// Per launch at 192 x 128 x 128: plain 302 us (FP64 DFMA 2 602), mixed 234 us (264 when one CTA of 256 threads walked scales,
-// chunks and epilogue in turn); 512 x 512 x 256 mixed 6.7 ms (7.3).
+// What bounds it (clock64 traces, 192 points): plain, the MMAs, 1 200 cycles an entry, three entries a chunk, and 4 000
+// cycles more a unit while the epilogue drains tensor memory (its three sets of order sums fill it, so that units do
+// not overlap there).  Mixed: the MMAs (600 an entry) and the digits (2 300 a chunk for each of two groups) alike.
+// Per launch at 192 x 128 x 128: plain 259 us (FP64 DFMA 2 602; 302 while one lane issued the MMAs from a branch), mixed
+// 199 us (234; 264 when one CTA of 256 threads walked scales, chunks and epilogue in turn); 512 x 512 x 256 mixed 5.4 ms
+// (6.7; 7.3).
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "xs_common.cuh"
@@ -247,7 +249,7 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
   uint64_t* bar_ce = bar_cx + XV_CXS;             // [XV_CXS] column scales read (epilogue threads: the item's last readers)
   uint32_t* tslot = (uint32_t*)(bar_ce + XV_CXS);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xFFFFFFFFu, tid >> 5, 0), lane = tid & 31;   // warp: uniform
   if (tid == 0) {
     for (int i = 0; i < XV_AEMAX; ++i) {
       mbar_init(bar_af + i, 1);
@@ -320,53 +322,52 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       }
     }
   } else if (warp == 1) {
-    // ---- MMA issue
-    if (lane == 0) {
-      uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
-      bool any = false;
-      // the MMAs of one table entry: digit t against the B tiles [b, b + (n - t) cols), cols tiles per digit, onto the
-      // accumulators from tc on
-      auto entry = [&](auto nc, auto colsc, uint32_t b, uint32_t tc, bool add) {
-        constexpr int n = decltype(nc)::value, cols = decltype(colsc)::value;
-        if (!xs_wait(&bar_af[sa], pa, ok)) return;
-        tc_fence_after();
-        const uint32_t a0 = smem_u32(sA + sa * AENT);
+    // ---- MMA issue (the whole warp, one elected lane issuing)
+    const uint32_t el = elect_lane();
+    uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
+    bool any = false;
+    // the MMAs of one table entry: digit t against the B tiles [b, b + (n - t) cols), cols tiles per digit, onto the
+    // accumulators from tc on
+    auto entry = [&](auto nc, auto colsc, uint32_t b, uint32_t tc, bool add) {
+      constexpr int n = decltype(nc)::value, cols = decltype(colsc)::value;
+      if (!xs_wait_w(&bar_af[sa], pa, ok)) return;
+      tc_fence_after();
+      const uint32_t a0 = smem_u32(sA) + sa * AENT;
 #pragma unroll
-        for (int t = 0; t < n; ++t) {
-          const uint64_t ad = sdesc(a0 + t * XV_ATILE, XV_LBO, XV_SBO);
-          const int tiles = (n - t) * cols, t1 = tiles * N > 256 ? 256 / N : tiles;
-          umma_bf16(tmem + tc + (uint32_t)(t * cols * N), ad, sdesc(b, XV_LBO, XV_SBO), idesc_bf16(128, t1 * N),
-                    (add || t > 0) ? 1u : 0u);
-          if (tiles > t1)
-            umma_bf16(tmem + tc + (uint32_t)((t * cols + t1) * N), ad, sdesc(b + t1 * XV_BTILE, XV_LBO, XV_SBO),
-                      idesc_bf16(128, (tiles - t1) * N), (add || t > 0) ? 1u : 0u);
-        }
-        umma_commit(&bar_ae[sa]);
-        last = sa; plast = pa; any = true;
-        if (++sa == AE) { sa = 0; pa ^= 1u; }
-      };
-      for (int it = first; it < nitems && ok; it = next_item(it), ++u) {
-        // psi's and X's accumulators, once the epilogue has read the item before
-        if (u > 0 && !xs_wait(&bar_te[0], (u - 1) & 1, ok)) break;
-        for (int kc = 0; kc < nkc && ok; ++kc) {
-          if (!xs_wait(&bar_bf[sb], pb, ok)) break;
-          const uint32_t b0 = smem_u32(sB + sb * BSTAGE);
-          // psi and X alternate by order (psi_d at 2d N, X_d at (2d+1) N) and their field digits alternate the same way
-          // ([psi_ur_s, X_up_s] against m V, [psi_up_s, X_ur_s] against D), so one MMA covers both sums
-          entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, kc > 0);
-          if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, true);
-          if (kc == 0 && u > 0) xs_wait(&bar_te[1], (u - 1) & 1, ok);
-          if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, kc > 0);
-          if (!ok) break;
-          umma_commit(&bar_be[sb]);
-          if (++sb == XV_SB) { sb = 0; pb ^= 1u; }
-        }
-        if (ok) umma_commit(bar_tf);
+      for (int t = 0; t < n; ++t) {
+        const uint64_t ad = sdesc(a0 + t * XV_ATILE, XV_LBO, XV_SBO);
+        const int tiles = (n - t) * cols, t1 = tiles * N > 256 ? 256 / N : tiles;
+        umma_bf16(tmem + tc + (uint32_t)(t * cols * N), ad, sdesc(b, XV_LBO, XV_SBO), idesc_bf16(128, t1 * N),
+                  (add || t > 0) ? 1u : 0u, el);
+        if (tiles > t1)
+          umma_bf16(tmem + tc + (uint32_t)((t * cols + t1) * N), ad, sdesc(b + t1 * XV_BTILE, XV_LBO, XV_SBO),
+                    idesc_bf16(128, (tiles - t1) * N), (add || t > 0) ? 1u : 0u, el);
       }
-      if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
-        bool ok2 = true;
-        xs_wait(&bar_ae[last], plast, ok2);
+      umma_commit(&bar_ae[sa], el);
+      last = sa; plast = pa; any = true;
+      if (++sa == AE) { sa = 0; pa ^= 1u; }
+    };
+    for (int it = first; it < nitems && ok; it = next_item(it), ++u) {
+      // psi's and X's accumulators, once the epilogue has read the item before
+      if (u > 0 && !xs_wait_w(&bar_te[0], (u - 1) & 1, ok)) break;
+      for (int kc = 0; kc < nkc && ok; ++kc) {
+        if (!xs_wait_w(&bar_bf[sb], pb, ok)) break;
+        const uint32_t b0 = smem_u32(sB) + sb * BSTAGE;
+        // psi and X alternate by order (psi_d at 2d N, X_d at (2d+1) N) and their field digits alternate the same way
+        // ([psi_ur_s, X_up_s] against m V, [psi_up_s, X_ur_s] against D), so one MMA covers both sums
+        entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, kc > 0);
+        if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, true);
+        if (kc == 0 && u > 0) xs_wait_w(&bar_te[1], (u - 1) & 1, ok);
+        if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, kc > 0);
+        if (!ok) break;
+        umma_commit(&bar_be[sb], el);
+        if (++sb == XV_SB) { sb = 0; pb ^= 1u; }
       }
+      if (ok) umma_commit(bar_tf, el);
+    }
+    if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
+      bool ok2 = true;
+      xs_wait_w(&bar_ae[last], plast, ok2);
     }
   } else if (warp < 2 + XV_NSW) {
     // ---- column scales: cexp(2zz) over (Im ur, Re up), cexp(2zz+1) over (Re ur, Im up); fexp over uz.  Four z columns
