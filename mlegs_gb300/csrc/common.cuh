@@ -284,29 +284,21 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
 // per SM, and cvt.f32.f64 / cvt.f64.f32 execute there; the mixed form converts every field element
 // it touches, so doing it with integer ops keeps those kernels off the FP64 pipe.
 // Round to nearest even; magnitudes below 2^-126 become signed zero; inf and NaN are kept.
+// Without branches on the common path: both words' fields move by one funnel shift, and the rounding is one comparison (the
+// dropped bits as a 32-bit fraction, plus the last kept bit, against one half).
 __device__ __forceinline__ float d2f_fast(double x) {
-  unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
-  unsigned sign = hi & 0x80000000u;
-  int e = (int)((hi >> 20) & 0x7FFu);
-  unsigned m = ((hi & 0xFFFFFu) << 3) | (lo >> 29);
-  unsigned rest = lo & 0x1FFFFFFFu;
-  int e32 = e - 1023 + 127;
-  if (e == 0x7FF) return __uint_as_float(sign | 0x7F800000u | (((hi & 0xFFFFFu) | lo) ? 0x400000u : 0u));
-  if (e32 <= 0) return __uint_as_float(sign);
-  if (e32 >= 255) return __uint_as_float(sign | 0x7F800000u);
-  unsigned r = sign | ((unsigned)e32 << 23) | m;
-  if (rest > 0x10000000u || (rest == 0x10000000u && (m & 1u))) r += 1u;   // carries into the exponent
-  return __uint_as_float(r);
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x), a = hi & 0x7FFFFFFFu;
+  unsigned r = __funnelshift_l(lo, a - 0x38000000u, 3);   // exponent rebased by 896
+  r += ((lo << 3) + (r & 1u) > 0x80000000u) ? 1u : 0u;    // may carry into the exponent
+  if (a < 0x38100000u) r = 0u;
+  if (a >= 0x47F00000u) r = 0x7F800000u | ((a > 0x7FF00000u || (a == 0x7FF00000u && lo != 0u)) ? 0x400000u : 0u);
+  return __uint_as_float(r | (hi & 0x80000000u));
 }
 __device__ __forceinline__ double f2d_fast(float y) {   // exact (FP32 subnormals become zero)
-  unsigned f = __float_as_uint(y);
-  unsigned sign = f & 0x80000000u;
-  unsigned e = (f >> 23) & 0xFFu;
-  unsigned m = f & 0x7FFFFFu;
-  if (e == 0u) return __hiloint2double((int)sign, 0);
-  unsigned hi = (e == 255u) ? (sign | 0x7FF00000u | (m >> 3)) : (sign | ((e + 896u) << 20) | (m >> 3));
-  return __hiloint2double((int)hi, (int)(m << 29));
+  const unsigned f = __float_as_uint(y), a = f & 0x7FFFFFFFu;
+  unsigned hi = (a >> 3) + (a >= 0x7F800000u ? 0x70000000u : 0x38000000u), lo = f << 29;
+  if (a < 0x800000u) hi = lo = 0u;
+  return __hiloint2double((int)(hi | (f & 0x80000000u)), (int)lo);
 }
 __device__ __forceinline__ float2 ld_c32(const double2* p) { double2 v = *p; return make_float2(d2f_fast(v.x), d2f_fast(v.y)); }
 __device__ __forceinline__ void st_c32(double2* p, float2 v) { *p = make_double2(f2d_fast(v.x), f2d_fast(v.y)); }
