@@ -16,9 +16,9 @@
 // φ lines all get it (their DC is the m = 0 coefficient).  The z lines of the m = 0 plane run in FP64.
 //
 // Layout: a field is (nrdim, npdim, nzdim) with r fastest.  Both transforms run along a strided
-// dimension; a CTA takes TR consecutive r (the contiguous batch, so every global access is a run of
-// TR*16 bytes) and TT threads per transform, keeps the TR transforms in shared memory as
-// [point][TR] and runs a Stockham autosort FFT (radix 4, 2, 3, 5) between two shared buffers.
+// dimension; a CTA takes TRL consecutive lines (the contiguous batch, so every global access is a run of
+// TRL*16 bytes) and several threads per line, which exchange through shared memory as [point][TRL].
+// Lengths: powers of two from 16 to 256 here (FP32 and FP64) and in fftq.cu (the plain form), others in fftr.cu.
 #include "common.cuh"
 #include "fft_common.cuh"
 #include <cmath>
@@ -30,177 +30,6 @@ namespace mlg {
 #define MLG_MIXED_FFT_DF 0
 #endif
 typedef std::conditional<MLG_MIXED_FFT_DF != 0, dfl, float>::type MixFT;
-
-// Stockham FFT over the TR transforms held in s0 ([L][TR]); result left in *res.
-template <typename T>
-__device__ void stockham(typename CT<T>::t* s0, typename CT<T>::t* s1, typename CT<T>::t** res, int L, int TR,
-                         int tr, int tt, int TT, const typename TW<T>::t* tw, int sgn) {
-  typedef typename CT<T>::t C;
-  C* src = s0;
-  C* dst = s1;
-  int rem = L;
-  for (int ns = 1; ns < L;) {
-    int p = (rem % 4 == 0) ? 4 : (rem % 2 == 0) ? 2 : (rem % 3 == 0) ? 3 : 5;
-    int m = L / p;
-    int span = ns * p, twstep = L / span;
-    for (int j = tt; j < m; j += TT) {
-      int k = j % ns;
-      C a[5];
-#pragma unroll
-      for (int r = 0; r < 5; ++r)
-        if (r < p) a[r] = src[(j + r * m) * TR + tr];
-      if (k) {
-#pragma unroll
-        for (int r = 1; r < 5; ++r)
-          if (r < p) a[r] = c_mul(a[r], load_tw<T>(tw, (k * r * twstep) % L, sgn));
-      }
-      dft_small<T>(a, p, sgn);
-      int base = (j / ns) * span + k;
-#pragma unroll
-      for (int r = 0; r < 5; ++r)
-        if (r < p) dst[(base + r * ns) * TR + tr] = a[r];
-    }
-    __syncthreads();
-    C* t = src; src = dst; dst = t;
-    ns = span;
-    rem /= p;
-  }
-  *res = src;
-}
-
-// z FFT of columns (r, m): points at stride nrdim*npdim; the grid covers m = m0, m0+1, ...
-template <typename T>
-__global__ void k_vfft(double2* __restrict__ e, int nrdim, int npdim, int L, int TR,
-                       const typename TW<T>::t* __restrict__ tw, int sgn, T scale, int m0) {
-  typedef typename CT<T>::t C;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* s0 = (C*)smem_raw;
-  C* s1 = s0 + (size_t)L * TR;
-  int tr = threadIdx.x, tt = threadIdx.y, TT = blockDim.y;
-  int r = blockIdx.x * TR + tr;
-  int m = blockIdx.y + m0;
-  bool ok = r < nrdim;
-  size_t pstride = (size_t)nrdim * npdim;
-  double2* base = e + r + (size_t)nrdim * m;
-  for (int pt = tt; pt < L; pt += TT) s0[pt * TR + tr] = ok ? ld<T>(base + pt * pstride) : mk<T>(0, 0);
-  __syncthreads();
-  C* res;
-  stockham<T>(s0, s1, &res, L, TR, tr, tt, TT, tw, sgn);
-  if (ok)
-    for (int pt = tt; pt < L; pt += TT) st<T>(base + pt * pstride, c_scale(res[pt * TR + tr], (T)scale));
-}
-
-// φ forward: packed reals -> X_0..X_{L} (L = np/2) scaled 1/np, in place.  Mixed form: X_0 from the
-// FP64 sum of the row, the FP32 FFT on the samples minus their FP64 mean.
-template <typename T>
-__global__ void k_hfft_fwd(double2* __restrict__ e, int nrdim, int npdim, int L, int TR,
-                           const typename TW<T>::t* __restrict__ tw, const typename TW<T>::t* __restrict__ twr, T scale,
-                           double scale_d, double inv_np, const double* __restrict__ rs, int nrs) {
-  typedef typename CT<T>::t C;
-  constexpr bool DC = std::is_same<T, float>::value;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* s0 = (C*)smem_raw;
-  C* s1 = s0 + (size_t)L * TR;
-  int tr = threadIdx.x, tt = threadIdx.y, TT = blockDim.y;
-  int r = blockIdx.x * TR + tr;
-  int z = blockIdx.y;
-  bool ok = r < nrdim;
-  double2* base = e + r + (size_t)nrdim * npdim * z;
-  const double rv = (rs != nullptr && ok && r < nrs) ? rs[r] : 1.0;   // scale_r of the input row
-  double sum = 0.0, mu = 0.0;
-  if (DC) {
-    double* red = (double*)(s1 + (size_t)L * TR);
-    double part = 0.0;
-    if (ok)
-      for (int pt = tt; pt < L; pt += TT) { double2 v = base[(size_t)pt * nrdim]; part += v.x * rv + v.y * rv; }
-    red[tt * TR + tr] = part;
-    __syncthreads();
-    for (int q = 0; q < TT; ++q) sum += red[q * TR + tr];
-    mu = sum * inv_np;
-  }
-  for (int pt = tt; pt < L; pt += TT) {
-    C v = mk<T>(0, 0);
-    if (ok) {
-      if (DC) {
-        double2 d = base[(size_t)pt * nrdim];
-        v = mk<T>((T)d2f_fast(d.x * rv - mu), (T)d2f_fast(d.y * rv - mu));
-      } else {
-        double2 d = base[(size_t)pt * nrdim];
-        v = mk<T>((T)(d.x * rv), (T)(d.y * rv));
-      }
-    }
-    s0[pt * TR + tr] = v;
-  }
-  __syncthreads();
-  C* res;
-  stockham<T>(s0, s1, &res, L, TR, tr, tt, TT, tw, -1);
-  if (!ok) return;
-  for (int k = tt; k <= L; k += TT) {
-    C zk = res[(k % L) * TR + tr];
-    C zc = res[((L - k) % L) * TR + tr];
-    zc.y = -zc.y;
-    C fe = c_scale(c_add(zk, zc), (T)0.5);
-    C fo = c_muli(c_scale(c_sub(zk, zc), (T)0.5), -1);   // (zk - zc)/(2i)
-    typename TW<T>::t wd = twr[k];
-    C w = mk<T>(wd.x, wd.y);
-    C x = c_scale(c_add(fe, c_mul(w, fo)), (T)scale);
-    if (DC && k == 0) {
-      base[0] = make_double2(f2d_fast((float)x.x) + sum * scale_d, f2d_fast((float)x.y));
-    } else {
-      st<T>(base + (size_t)k * nrdim, x);
-    }
-  }
-}
-
-// φ backward: X_0..X_L -> packed reals (unnormalised); slot L <- np * X_L (input), in place.  Mixed
-// form: Re X_0 is left out of the FP32 FFT and added to every sample in FP64.
-template <typename T>
-__global__ void k_hfft_bwd(double2* __restrict__ e, int nrdim, int npdim, int L, int TR,
-                           const typename TW<T>::t* __restrict__ tw, const typename TW<T>::t* __restrict__ twr, double np_d,
-                           const double* __restrict__ rs, int nrs) {
-  typedef typename CT<T>::t C;
-  constexpr bool DC = std::is_same<T, float>::value;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  C* s0 = (C*)smem_raw;
-  C* s1 = s0 + (size_t)L * TR;
-  int tr = threadIdx.x, tt = threadIdx.y, TT = blockDim.y;
-  int r = blockIdx.x * TR + tr;
-  int z = blockIdx.y;
-  bool ok = r < nrdim;
-  double2* base = e + r + (size_t)nrdim * npdim * z;
-  double2 nyq = make_double2(0, 0);
-  double dc = 0.0;
-  if (ok && tt == 0) nyq = base[(size_t)L * nrdim];
-  if (DC && ok) dc = base[0].x;
-  for (int k = tt; k < L; k += TT) {
-    C v = mk<T>(0, 0);
-    if (ok) {
-      C xk = ld<T>(base + (size_t)k * nrdim);
-      C xc = ld<T>(base + (size_t)(L - k) * nrdim);
-      if (k == 0) { xk.y = 0; xc.y = 0; if (DC) xk.x = 0; }
-      xc.y = -xc.y;
-      C g = c_add(xk, xc);
-      typename TW<T>::t wd = twr[k];
-      C w = mk<T>(wd.x, -wd.y);   // exp(+2 pi i k / np)
-      C h = c_mul(c_sub(xk, xc), w);
-      v = c_add(g, c_muli(h, 1));
-    }
-    s0[k * TR + tr] = v;
-  }
-  __syncthreads();
-  C* res;
-  stockham<T>(s0, s1, &res, L, TR, tr, tt, TT, tw, +1);
-  if (!ok) return;
-  const double rv = (rs != nullptr && r < nrs) ? rs[r] : 1.0;   // scale_r of the output row
-  for (int pt = tt; pt < L; pt += TT) {
-    C y = res[pt * TR + tr];
-    double2 v;
-    if (DC) v = make_double2(f2d_fast((float)y.x) + dc, f2d_fast((float)y.y) + dc);
-    else v = make_double2((double)y.x, (double)y.y);
-    base[(size_t)pt * nrdim] = make_double2(v.x * rv, v.y * rv);
-  }
-  if (tt == 0) base[(size_t)L * nrdim] = make_double2(nyq.x * np_d * rv, nyq.y * np_d * rv);
-}
 
 template <typename T, int L, int SGN, int TRL>
 __global__ void __launch_bounds__(TRL * Split<L>::R2) k_zfft2(FSet fs, int nrdim, int npdim,
@@ -248,13 +77,6 @@ template <> struct TwTab<dfl> {
   static const float4* pr() { return G.tw_prdf; }
   static const float4* z() { return G.tw_zdf; }
 };
-
-static int pick_tr(int L, size_t elem) {
-  // two shared buffers of L*TR complex values, at most 96 KB
-  int tr = 32;
-  while (tr > 1 && 2ull * L * tr * elem > 96 * 1024) tr /= 2;
-  return tr;
-}
 
 template <typename T>
 static int set_smem(const void* fn, size_t bytes) {
@@ -306,18 +128,9 @@ static int vfft_t(const FSet& fs, int dir, double scale, int m0, int nm, int tr_
     return tr_max >= 8 ? zfft2_any<T, 8>(fs, dir, scale, m0, nm, stream) : zfft2_any<T, 4>(fs, dir, scale, m0, nm, stream);
   }
   if constexpr (std::is_same<T, dfl>::value) {
-    return vfft_t<double>(fs, dir, scale, m0, nm, tr_max, stream);   // other lengths: the FP64 Stockham kernel
+    return vfft_t<double>(fs, dir, scale, m0, nm, tr_max, stream);   // other lengths: FP64
   } else {
-  int TR = std::min(pick_tr(L, sizeof(typename CT<T>::t)), tr_max);
-  int TT = std::max(1, std::min(256 / TR, L / 2));
-  size_t sm = 2ull * L * TR * sizeof(typename CT<T>::t);
-  MLG_TRY(set_smem<T>((const void*)k_vfft<T>, sm));
-  dim3 grid(cdiv(G.nrdim, TR), nm), blk(TR, TT);
-  for (int f = 0; f < fs.n; ++f) {   // other lengths: the Stockham kernel, field by field
-    k_vfft<T><<<grid, blk, sm, stream>>>(fs.e[f], G.nrdim, G.npdim, L, TR, TwTab<T>::z(), dir, (T)scale, m0);
-    MLG_LAUNCH();
-  }
-  return 0;
+    return launch_zfft_r<T>(fs, TwTab<T>::z(), dir, scale, m0, nm, stream);
   }
 }
 
@@ -397,28 +210,11 @@ static int hfft_t(const FSet& fs, int dir, double scale) {
   }
   if constexpr (std::is_same<T, dfl>::value) {
     kt_end(1, 0.0);
-    return hfft_t<double>(fs, dir, scale);   // other lengths: the FP64 Stockham kernels
+    return hfft_t<double>(fs, dir, scale);   // other lengths: FP64
   } else {
-  int TR = pick_tr(L, sizeof(typename CT<T>::t));
-  int TT = std::max(1, std::min(256 / TR, std::max(L / 2, 1)));
-  constexpr bool DC = std::is_same<T, float>::value;
-  size_t sm = 2ull * L * TR * sizeof(typename CT<T>::t) + (DC ? (size_t)TT * TR * sizeof(double) : 0);
-  dim3 grid(cdiv(G.nrdim, TR), G.nzdim), blk(TR, TT);
-  if (dir < 0) MLG_TRY(set_smem<T>((const void*)k_hfft_fwd<T>, sm));
-  else MLG_TRY(set_smem<T>((const void*)k_hfft_bwd<T>, sm));
-  for (int f = 0; f < fs.n; ++f) {   // other lengths: the Stockham kernels, field by field
-    if (dir < 0) {
-      k_hfft_fwd<T><<<grid, blk, sm, G.stream>>>(fs.e[f], G.nrdim, G.npdim, L, TR, TwTab<T>::p(),
-                                                  TwTab<T>::pr(), (T)scale,
-                                                  scale, 1.0 / G.np, fs.rs[f], G.nr);
-    } else {
-      k_hfft_bwd<T><<<grid, blk, sm, G.stream>>>(fs.e[f], G.nrdim, G.npdim, L, TR, TwTab<T>::p(),
-                                                  TwTab<T>::pr(), (double)G.np, fs.rs[f], G.nr);
-    }
-    MLG_LAUNCH();
-  }
-  kt_end(1, 2.0 * fs.n * G.fsize * 16);
-  return 0;
+    MLG_TRY(launch_pfft_r<T>(fs, TwTab<T>::p(), TwTab<T>::pr(), dir, scale));
+    kt_end(1, 2.0 * fs.n * G.fsize * 16);
+    return 0;
   }
 }
 

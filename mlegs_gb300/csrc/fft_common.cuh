@@ -419,5 +419,12 @@ __device__ __forceinline__ void pfft_bwd2_body(const FSet& fs, int nrdim, int np
 // backward
 int launch_zfft_q(const FSet& fs, int dir, int sexp);
 int launch_pfft_q(const FSet& fs, int dir, int sexp);
+// transforms of other lengths (fftr.cu), FP32 and FP64: z on the planes m0 .. m0 + nm - 1, phi
+// forward (scaled) and backward
+template <typename T>
+int launch_zfft_r(const FSet& fs, const typename TW<T>::t* tw, int dir, double scale, int m0, int nm,
+                  cudaStream_t stream);
+template <typename T>
+int launch_pfft_r(const FSet& fs, const typename TW<T>::t* tw, const typename TW<T>::t* twr, int dir, double scale);
 
 }  // namespace mlg
