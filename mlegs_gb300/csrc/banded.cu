@@ -551,7 +551,8 @@ struct SolveArgs {
   int* status;
   int nrdim, npdim, ne, nrc, npc, nzc, nzcu, nzdim;
   int nsys;             // npc * nzdim (the cached-factor paths: the positions of sys_mk)
-  int nsp = 0;          // the factor image's system stride: nsys rounded up to 32
+  int nsp = 0;          // the factor image's systems: nsys rounded up to 32
+  int frows = 0;        // and rows
   double alpha, beta, ell, preln;
   int kind;             // 0 ihelm, 1 idel2_proln, 2 idel2_preln, 3 ihelmp
   int power;
@@ -844,12 +845,19 @@ __device__ void window_solve(const SolveArgs& a, int sys, int kind, bool special
 // Factor cache.  The matrix of system (m, k) depends only on (kind, alpha, m, k), and the steppers
 // call ihelm with the same alpha every step (and vec2tp calls idel2), so the LU factors are computed
 // once per key and every later call is a forward and a back substitution.  Per row j the cache
-// holds, [row][slot][system] so that a warp reads consecutive addresses:
+// holds, [16 systems][row][slot][system], so that a warp of the substitution (16 systems) reads consecutive addresses at
+// compile-time offsets from one pointer, with FPAD rows of zeros before and behind each 16 systems' rows (the substitution
+// walks whole batches of rows):
 //   slot 0..KL-1     multipliers l(j+1..j+KL) (0 beyond the matrix)
 //   slot KL          pivot row offset p in 0..KL (gbtrf's ipiv(j) - j)
 //   slot KL+1        1 / U(j, j)
 //   slot KL+2 ..     U(j, j+1 .. j+KL+KU)
-constexpr int FKL = 2, FKU = 2, FSL = 2 * FKL + FKU + 2;
+constexpr int FKL = 2, FKU = 2, FSL = 2 * FKL + FKU + 2, FPAD = 16;
+// the doubles of one row (its slots are 16 apart), and of 16 systems with n rows each
+constexpr int FROW = FSL * 16;
+__host__ __device__ __forceinline__ size_t fac_group(int n) { return (size_t)(n + 2 * FPAD) * FROW; }
+// row 0 of the system at position sys
+__device__ __forceinline__ size_t fac_at(int sys, int n) { return (size_t)(sys >> 4) * fac_group(n) + (size_t)FPAD * FROW + (sys & 15); }
 
 __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restrict__ fac) {
   int sys = blockIdx.x * blockDim.x + threadIdx.x;   // position in the system order (sys_mk)
@@ -862,8 +870,8 @@ __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restr
   double akv = a.ak[k];
   double alpha = (a.kind == 0) ? a.alpha : 0.0;
   double e2 = a.ell * a.ell;
-  constexpr int WC = FKL + FKU + 1;
-  const size_t ns = a.nsp;
+  constexpr int WC = FKL + FKU + 1, ns = 16;
+  double* const f0 = fac + fac_at(sys, a.frows);
   double W[FKL + 1][WC];
 #pragma unroll
   for (int t = 0; t <= FKL; ++t)
@@ -885,7 +893,7 @@ __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restr
         for (int c = 0; c < WC; ++c) { double q = W[0][c]; W[0][c] = W[t][c]; W[t][c] = q; }
       }
     double rp = 1.0 / W[0][0];
-    double* f = fac + (size_t)j * FSL * ns + sys;
+    double* f = f0 + (size_t)j * FROW;
 #pragma unroll
     for (int t = 1; t <= FKL; ++t) {
       double l = 0.0;
@@ -913,29 +921,9 @@ __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restr
   }
 }
 
-// cp.async helpers: 16 bytes through L2 only (the staged rows include rows that other threads of the
-// block have just stored; a zero source size fills the destination with zeros)
-__device__ __forceinline__ void cpa16cg(void* sdst, const void* gsrc, bool pred) {
-  unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
-  int sz = pred ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(gsrc), "r"(sz));
-}
-__device__ __forceinline__ void cpa_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-template <int N> __device__ __forceinline__ void cpa_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
-
-// forward and back substitution with the cached factors (gbtrs 'N', one or two right-hand sides), in
-// place on the column.  One warp = 32 systems; factor rows and right-hand-side values are staged into shared
-// memory SST groups ahead of use by cp.async, so DRAM latency overlaps the recurrences.
-constexpr int SGR = 8, SST = 4, SNU = FKL + FKU, SFS = SNU + 1;
+// forward and back substitution with the cached factors (gbtrs 'N', one or two right-hand sides), in place on the column
+constexpr int SNU = FKL + FKU;
 static_assert(FKL == 2, "the substitution compares the pivot index by the high words of 1.0 and 2.0");
-template <int NR>
-struct SubstSmem {
-  double f[SST][SFS][SGR][32];   // factor rows by group: [slot][row in group][system]
-  double2 v[NR][SST][SGR][32];   // field rows by group: fwd the entering rows, bwd y(j)
-  double2 o[NR][2][SGR][32];     // outgoing rows by group parity: fwd y(j), bwd x(j)
-  long long off[32];             // the block's systems: column offset, active rows, passes
-  int nn[32], cnt[32];
-};
 
 // ihelm's pre-solve log-term handling of one field (:818-824): so%ln = s%ln/alpha, the log terms on
 // e(1..3, 1, 1)
@@ -948,195 +936,175 @@ __device__ __forceinline__ void subst_root_pre(const SolveArgs& a, double2* g, d
   g[2].x -= 2.0 / 3.0 / e2 / exp(a.lognorm[2]) * lno;
 }
 
+// accesses that stay where they are written: operands are read a batch of rows ahead of their use
+__device__ __forceinline__ double ld_here(const double* p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];\n" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ double ld_here(const double* p, bool in) {
+  double v;
+  asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n mov.f64 %0, 0d0000000000000000;\n @q ld.global.f64 %0, [%1];\n}\n"
+               : "=d"(v) : "l"(p), "r"((int)in) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_here(double* p, double v, bool in) {
+  asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %2, 0;\n @q st.global.f64 [%0], %1;\n}\n" ::"l"(p), "d"(v), "r"((int)in) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
+
+// A pass of the substitution over the rows of a thread's real system (factors f0, row 0; right-hand side x, stride 2): step
+// i = 0, 1, ... works on row j = i (forward) or nnw - 1 - i (backward).  Two batches of SB rows alternate: one is read while
+// the other is computed.
+template <bool BWD, bool NX>
+__device__ __forceinline__ void subst_pass(const double* __restrict__ f0, double* x, int nn, int nnw, int nrdim, bool act,
+                                           double (&r)[FKL + 1]) {
+  // without row exchanges: the multipliers, or 1 / U(j,j) and the FKU entries of U's own band only
+  constexpr int NF = BWD ? (NX ? FKU + 1 : SNU + 1) : (NX ? FKL : FKL + 1), S0 = BWD ? FKL + 1 : 0, SB = NX ? 8 : 4, AHEAD = 32;
+  constexpr int D = BWD ? -1 : 1, J0 = BWD ? 0 : 1 + FKL;   // direction; the row entering at a step is J0 further
+  static_assert(2 * SB <= FPAD && SB * NF <= 32, "whole batches of factor rows; one prefetch per batch");
+  const int rows = act ? nn : 0, jb = BWD ? nnw - 1 : 0, lane = threadIdx.x & 31;
+  const double* const fb = f0 + (ptrdiff_t)jb * FROW + S0 * 16;
+  double* const xb = x + 2 * jb;
+  // this lane's share of a batch's factor rows, a 128-byte line each
+  const ptrdiff_t pf = D * (min(lane, SB * NF - 1) / NF) * FROW + min(lane, SB * NF - 1) % NF * 16 + (ptrdiff_t)D * AHEAD * FROW;
+  double xs[SNU], late = 0.0;
+#pragma unroll
+  for (int c = 0; c < SNU; ++c) xs[c] = 0.0;
+  auto take = [&](double (&v)[SB][NF + 1], int i0) {
+    const double* f = fb + (ptrdiff_t)D * i0 * FROW;
+    const double* xv = xb + 2 * D * i0;
+#pragma unroll
+    for (int u = 0; u < SB; ++u)
+#pragma unroll
+      for (int t = 0; t < NF; ++t) v[u][t] = ld_here(f + D * u * FROW + t * 16);
+    // (rows past a system's own count reach no row of its own: a whole batch inside the column is read as it stands)
+    const int jn = BWD ? jb - (i0 + SB - 1) : i0 + J0 + SB - 1;   // the batch's last row
+    if (BWD ? jn >= 0 : jn < nrdim) {
+#pragma unroll
+      for (int u = 0; u < SB; ++u) v[u][NF] = ld_here(xv + 2 * (D * u + J0));
+    } else {
+#pragma unroll
+      for (int u = 0; u < SB; ++u) v[u][NF] = ld_here(xv + 2 * (D * u + J0), BWD ? jb - i0 - u >= 0 : i0 + J0 + u < rows);
+    }
+    if (i0 + AHEAD < nnw) {
+      prefetch_l2(f + pf);
+      prefetch_l2(xv + 2 * D * AHEAD);
+    }
+  };
+  auto work = [&](const double (&v)[SB][NF + 1], int i0) {
+    double* xo = xb + 2 * D * i0;
+#pragma unroll
+    for (int u = 0; u < SB; ++u) {
+      if constexpr (!BWD) {
+        if constexpr (!NX) {
+          // the pivot row index p (0..FKL), stored as a double: compared by its high word, off the FP64 pipe
+          const int ph = __double2hiint(v[u][FKL]);
+#pragma unroll
+          for (int t = 1; t <= FKL; ++t)
+            if (ph == (t == 1 ? 0x3FF00000 : 0x40000000)) { double w = r[0]; r[0] = r[t]; r[t] = w; }
+        }
+        st_here(xo + 2 * u, r[0], rows - i0 > u);
+#pragma unroll
+        for (int t = 1; t <= FKL; ++t) r[t] = fma(-v[u][t - 1], r[0], r[t]);
+#pragma unroll
+        for (int t = 0; t < FKL; ++t) r[t] = r[t + 1];
+        r[FKL] = v[u][NF];
+      } else {
+        constexpr int NU = NX ? FKU : SNU;
+        // x(j) = y(j)/U(j,j) - sum_c (U(j,j+c)/U(j,j)) x(j+c): only the last FMA waits on x(j+1)
+        double t = v[u][NF] * v[u][0];
+#pragma unroll
+        for (int c = 2; c <= NU; ++c) t = fma(-v[u][c], xs[c - 1], t);
+        double xj = fma(-v[u][1], xs[0], t);
+        if (jb - i0 - u >= nn) xj = 0.0;
+        // the row before is stored behind this one's operations, which would wait behind a store waiting for its own
+        st_here(xo - 2 * (u - 1), late, (unsigned)(nnw - i0 - u) < (unsigned)rows);
+        late = xj;
+#pragma unroll
+        for (int c = SNU - 1; c >= 1; --c) xs[c] = xs[c - 1];
+        xs[0] = xj;
+      }
+    }
+  };
+  double va[SB][NF + 1], vb[SB][NF + 1];
+  take(va, 0);
+  int i = 0;
+  for (; i < nnw; i += 2 * SB) {
+    take(vb, i + SB);
+    work(va, i);
+    if (i + 2 * SB < nnw) take(va, i + 2 * SB);
+    work(vb, i + SB);
+  }
+  if (BWD) st_here(xb - 2 * (i - 1), late, (unsigned)(nnw - i) < (unsigned)rows);   // row 0, if the last step was its
+}
+
 // The matrices are real, so the real and imaginary parts of a right-hand side are two independent
-// real systems with the same factors.  A block takes 32 consecutive systems (m, k) and has 64*NR
-// threads: one per system, part (real / imaginary) and field (NR = 2 solves the psi and chi fields of
-// a vortex step with the same matrices).  The systems' serial recurrences are all the parallelism
-// there is (a few warps per SM), so the kernel is built to issue few instructions per row: the
-// factors and field rows are staged by groups of SGR rows with 16-byte copies shared by the whole
-// block (the factors laid out [row][slot][system], a field's rows 128-byte runs per system), the
-// outgoing rows go back the same way, and the rows are walked by absolute index with no early exit
-// (rows past a system's own count are computed on whatever was staged and never stored; in the
-// backward pass they keep the recurrence at zero until the system's last row).  Only the real-part
-// thread of system (0,0) touches ln and the log terms, which all act on real parts.
+// real systems with the same factors.  A warp takes both parts of 16 consecutive systems (m, k) of one field (the parts in
+// neighbouring lanes, so that a row is read and written 16 bytes at a time); a CTA of four warps, one on each of the SM's
+// partitions, takes 32 systems of the psi and chi fields of a vortex step, solved with the same matrices (NR = 2), or 64
+// systems of one field.  Rows are walked by absolute index with no early exit (rows past a system's own count are computed
+// on what is there and never stored; in the backward pass they keep the recurrence at zero until the system's last row).
+// Only the real-part thread of system (0,0) touches ln and the log terms, which all act on real parts.
+// What bounds it: an FP64 instruction of a warp takes 64 cycles of its partition however many lanes are active, two a row
+// forward and three backward, and with one or two warps per partition what else a warp issues per row adds to that (it
+// measures 230 and 310 cycles a row alone on a partition).  So the loop holds little else: every operand is one load at a
+// compile-time offset from a pointer of the batch, in batches (loads spread between the rows shared scoreboards with them:
+// 10 % slower), with no shared memory and no barriers.  The systems solved twice in a row make a chain of 768 rows at 192
+// points.  Staged through shared memory by the same threads with a CTA barrier per 8 rows, a row took 330 to 460 cycles;
+// with staging warps beside the computing ones and mbarriers, 270 to 330 (each wait cost 200).  Per call at 192 x 128 x
+// 128, one and two fields' mean: 157 -> 106 us; two fields at 512 x 512 x 256: 1.24 -> 0.84 ms; the FP64 instructions alone,
+// spread evenly, 27 and 46 us at 192.
 template <int NR>
-__global__ void __launch_bounds__(64 * NR) k_band_subst(SolveArgs a, const double* __restrict__ fac) {
-  typedef double R;
-  constexpr int NT = 64 * NR;
-  extern __shared__ __align__(16) unsigned char subst_smem[];
-  SubstSmem<NR>& sm = *reinterpret_cast<SubstSmem<NR>*>(subst_smem);
-  const int th = threadIdx.x, q = th >> 6, comp = (th >> 5) & 1, lane = th & 31;
-  const size_t nsp = a.nsp;
-  const int sys0 = blockIdx.x * 32, sys = sys0 + lane;
+__global__ void __launch_bounds__(128, 2) k_band_subst(SolveArgs a, const double* __restrict__ fac) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = NR == 2 ? warp >> 1 : 0, comp = lane & 1;
+  // The systems that are solved twice (the first positions) make the longest chains.  Where two CTAs per SM hold the whole
+  // grid, their CTAs start last of the first one on every SM, so that those which come second join others (two fields at
+  // 192 x 128 x 128: 113 -> 106 us); in larger grids they start first.
+  const int nl = (a.lead + (NR == 2 ? 31 : 63)) / (NR == 2 ? 32 : 64), last = min(gridDim.x, 152);
+  int b = blockIdx.x;
+  if (gridDim.x <= 304 && nl < last && b < last) b = b < last - nl ? b + nl : b - (last - nl);
+  const int sys = NR == 2 ? b * 32 + (warp & 1) * 16 + (lane >> 1) : b * 64 + warp * 16 + (lane >> 1);
   double2* ev = q == 0 ? a.e : a.e2;
   double* lv = q == 0 ? a.lnp : a.lnp2;
-  auto sys_info = [&](int s, int& nn, int& cnt, size_t& off) {
-    bool valid = s < a.nsys;
-    int m = 0, k = 0;
-    if (valid) valid = sys_mk(a, s, m, k);
-    cnt = valid ? k_count(k, a.nzc, a.nzcu, a.nzdim) : 0;
-    nn = max(min(a.nrc, a.nrc - m), 0);
-    if (valid && m == 0 && k == 0 && a.skip_root) cnt = 0;
-    if (!valid || m >= a.npc || nn < 1) cnt = 0;
-    off = (size_t)a.nrdim * (m + (size_t)a.npdim * k);
-  };
-  int nn, cnt;
-  size_t off;
-  sys_info(sys, nn, cnt, off);
-  if (th < 32) { sm.nn[th] = nn; sm.cnt[th] = cnt; sm.off[th] = (long long)off; }
+  bool valid = sys < a.nsys;
+  int m = 0, k = 0;
+  if (valid) valid = sys_mk(a, sys, m, k);
+  int cnt = valid ? k_count(k, a.nzc, a.nzcu, a.nzdim) : 0;
+  const int nn = max(min(a.nrc, a.nrc - m), 0);
+  if (valid && m == 0 && k == 0 && a.skip_root) cnt = 0;
+  if (!valid || m >= a.npc || nn < 1) cnt = 0;
+  const size_t off = (size_t)a.nrdim * (m + (size_t)a.npdim * k);
   const bool root = sys < a.nsys && off == 0;
   if (root && comp == 0 && a.kind == 0 && !a.skip_root && !a.no_ln) subst_root_pre(a, ev, lv);
-  double* x = reinterpret_cast<double*>(ev + off) + comp;   // stride 2
-  // every warp holds the same 32 systems: warp-wide maxima are block-wide
-  int nnw = (cnt > 0) ? nn : 0;
-  for (int o = 16; o; o >>= 1) nnw = max(nnw, __shfl_xor_sync(0xffffffffu, nnw, o));
-  int cntw = cnt;
-  for (int o = 16; o; o >>= 1) cntw = max(cntw, __shfl_xor_sync(0xffffffffu, cntw, o));
-  const int ng = (nnw + SGR - 1) / SGR;
-  const double* dummy = fac;   // a 256-byte aligned address for the zero-size copies
-  __syncthreads();             // the system table
-  // the block's field rows of a group: chunk c = th + i*NT -> field c/256, system (c%256)/8, row in
-  // group c%8 (eight consecutive threads copy one system's 128-byte run); each thread's four chunks
-  // keep their system for the whole kernel
-  constexpr int NCH = NR * 256 / NT;   // 4
-  double2* cbase[NCH];
-  int cnn[NCH], ccnt[NCH];
-  const int cu = th & 7;
-#pragma unroll
-  for (int i = 0; i < NCH; ++i) {
-    const int c = th + i * NT, qq = c >> 8, sl = (c >> 3) & 31;
-    cbase[i] = (qq == 0 ? a.e : a.e2) + sm.off[sl];
-    cnn[i] = sm.nn[sl];
-    ccnt[i] = sm.cnt[sl];
+  double* x = reinterpret_cast<double*>(ev + (cnt > 0 ? off : 0)) + comp;   // stride 2 (an idle lane reads column 0)
+  int nnw = (cnt > 0) ? nn : 0, cntw = cnt;
+  for (int o = 16; o; o >>= 1) {
+    nnw = max(nnw, __shfl_xor_sync(0xffffffffu, nnw, o));
+    cntw = max(cntw, __shfl_xor_sync(0xffffffffu, cntw, o));
   }
-  auto stage_rows = [&](int g, int rep, bool bwd) {
-    const int st = g % SST;
-#pragma unroll
-    for (int i = 0; i < NCH; ++i) {
-      const int c = th + i * NT, qq = c >> 8, sl = (c >> 3) & 31;
-      const int j = bwd ? nnw - 1 - (g * SGR + cu) : g * SGR + cu + 1 + FKL;
-      const bool ok = rep < ccnt[i] && j >= 0 && j < cnn[i];
-      cpa16cg(&sm.v[qq][st][cu][sl], ok ? (const void*)(cbase[i] + j) : (const void*)dummy, ok);
-    }
-  };
-  auto write_out = [&](int g, int rep, bool bwd) {
-#pragma unroll
-    for (int i = 0; i < NCH; ++i) {
-      const int c = th + i * NT, qq = c >> 8, sl = (c >> 3) & 31;
-      const int j = bwd ? nnw - 1 - (g * SGR + cu) : g * SGR + cu;
-      if (rep < ccnt[i] && j >= 0 && j < cnn[i]) cbase[i][j] = sm.o[qq][g & 1][cu][sl];
-    }
-  };
-  // the factor rows of group g: NSL slots from S0 of rows j(u), 256 bytes per (row, slot), 16 per copy
-  // (backward without row exchanges: 1/U(j,j) and the FKU entries of U's own band only)
-  const double* fbase = fac + sys0 + 2 * (th & 15);
-  auto stage_fac_t = [&](auto bwdc, auto npc, int g) {
-    constexpr bool BWD = decltype(bwdc)::value, NP = decltype(npc)::value;
-    constexpr int NSL = BWD ? (NP ? FKU + 1 : SNU + 1) : (NP ? FKL : FKL + 1), S0 = BWD ? FKL + 1 : 0;
-    const int st = g % SST;
-#pragma unroll
-    for (int c = th; c < SGR * NSL * 16; c += NT) {
-      const int pr = c >> 4;
-      const int u = pr / NSL, t = pr - u * NSL;
-      const int j = BWD ? nnw - 1 - (g * SGR + u) : g * SGR + u;
-      const bool ok = j >= 0 && j < nnw;
-      cpa16cg(&sm.f[st][t][u][2 * (th & 15)], ok ? (const void*)(fbase + ((size_t)j * FSL + S0 + t) * nsp) : (const void*)dummy, ok);
-    }
-  };
-  // the factorisation records, per 32 systems, whether any of them exchanges rows; a block whose systems
-  // never do runs the forward pass without the pivot slot and the exchanges (the same result bit for bit)
-  const bool blk_nopiv = a.pivflag != nullptr && __ldcg(&a.pivflag[blockIdx.x]) == 0;
+  if (cntw == 0) return;
+  const double* fc = fac + fac_at(sys, a.frows);
+  // the factorisation records, per 32 systems, whether any of them exchanges rows; where none does the forward pass runs
+  // without the pivot slot and the exchanges, and U keeps the matrix's own FKU superdiagonals (its fill-in entries are exact
+  // zeros), so that the backward pass reads and applies only those, with the same result bit for bit, since
+  // fma(-0, x, t) = t for finite x
+  const bool nopiv = a.pivflag != nullptr && __ldcg(&a.pivflag[sys >> 5]) == 0;
   for (int rep = 0; rep < cntw; ++rep) {
-    // ---- forward: L y = P b, y(j) into the field's slot of row j ----
-    R r[FKL + 1];
-    bool piv = false;   // a row exchange in one of this thread's staged rows
+    const bool act = rep < cnt;
+    double r[FKL + 1];
 #pragma unroll
-    for (int t = 0; t <= FKL; ++t) r[t] = ((rep < cnt && t < nn) ? __ldcg(x + 2 * t) : 0.0);
-    auto forward = [&](auto npc) {
-      constexpr bool NP = decltype(npc)::value;
-      auto stage_f = [&](int g) { stage_fac_t(std::integral_constant<bool, false>(), npc, g); };
-      for (int g = 0; g < SST - 1; ++g) { if (g < ng) { stage_f(g); stage_rows(g, rep, false); } cpa_commit(); }
-      for (int g = 0; g < ng; ++g) {
-        cpa_wait<SST - 2>();
-        __syncthreads();   // group g staged; group g-1 computed; stage (g-1)%SST free
-        if (g + SST - 1 < ng) { stage_f(g + SST - 1); stage_rows(g + SST - 1, rep, false); }
-        cpa_commit();
-        if (g > 0) write_out(g - 1, rep, false);
-        const int st = g % SST;
-#pragma unroll
-        for (int u = 0; u < SGR; ++u) {
-          if constexpr (!NP) {
-            // the pivot row index p (0..FKL), stored as a double: compared by its high word, off the FP64 pipe
-            const int ph = __double2hiint(sm.f[st][FKL][u][lane]);
-            piv = piv || ph != 0;
-#pragma unroll
-            for (int t = 1; t <= FKL; ++t)
-              if (ph == (t == 1 ? 0x3FF00000 : 0x40000000)) { R w = r[0]; r[0] = r[t]; r[t] = w; }
-          }
-#pragma unroll
-          for (int t = 1; t <= FKL; ++t) r[t] = fma(-sm.f[st][t - 1][u][lane], r[0], r[t]);
-          reinterpret_cast<double*>(&sm.o[q][g & 1][u][lane])[comp] = r[0];
-#pragma unroll
-          for (int t = 0; t < FKL; ++t) r[t] = r[t + 1];
-          r[FKL] = reinterpret_cast<const double*>(&sm.v[q][st][u][lane])[comp];
-        }
-      }
-    };
-    if (blk_nopiv) forward(std::integral_constant<bool, true>());
-    else forward(std::integral_constant<bool, false>());
-    cpa_wait<0>();
-    __syncthreads();
-    if (ng > 0) write_out(ng - 1, rep, false);
-    __threadfence_block();
-    __syncthreads();   // y(j) in the fields, read back below by other threads' copies
-    // ---- backward: U x = y from row nnw-1 down; a system joins at its own last row.  Without a row
-    // exchange in any of the block's systems (every forward pass saw pivot offset 0), U keeps the
-    // matrix's own FKU superdiagonals and its fill-in entries are exact zeros: the pass then stages and
-    // applies only those (1 / U(j,j) and FKU ratios), with the same result bit for bit, since
-    // fma(-0, x, t) = t for finite x.
-    const bool nopiv = !__syncthreads_or(piv);
-    auto backward = [&](auto npc) {
-      constexpr bool NP = decltype(npc)::value;
-      constexpr int NU = NP ? FKU : SNU;
-      auto stage_b = [&](int g) { stage_fac_t(std::integral_constant<bool, true>(), npc, g); };
-      R xs[SNU];
-#pragma unroll
-      for (int c = 0; c < SNU; ++c) xs[c] = 0.0;
-      for (int g = 0; g < SST - 1; ++g) { if (g < ng) { stage_b(g); stage_rows(g, rep, true); } cpa_commit(); }
-      for (int g = 0; g < ng; ++g) {
-        cpa_wait<SST - 2>();
-        __syncthreads();
-        if (g + SST - 1 < ng) { stage_b(g + SST - 1); stage_rows(g + SST - 1, rep, true); }
-        cpa_commit();
-        if (g > 0) write_out(g - 1, rep, true);
-        const int st = g % SST;
-#pragma unroll
-        for (int u = 0; u < SGR; ++u) {
-          const int j = nnw - 1 - (g * SGR + u);
-          const R f0 = sm.f[st][0][u][lane];
-          // x(j) = y(j)/U(j,j) - sum_c (U(j,j+c)/U(j,j)) x(j+c): only the last FMA waits on x(j+1)
-          const R yj = reinterpret_cast<const double*>(&sm.v[q][st][u][lane])[comp];
-          R t = yj * f0;
-#pragma unroll
-          for (int c = 2; c <= NU; ++c) t = fma(-sm.f[st][c][u][lane], xs[c - 1], t);
-          R xj = fma(-sm.f[st][1][u][lane], xs[0], t);
-          if (j >= nn) xj = 0.0;
-          reinterpret_cast<double*>(&sm.o[q][g & 1][u][lane])[comp] = xj;
-#pragma unroll
-          for (int c = SNU - 1; c >= 1; --c) xs[c] = xs[c - 1];
-          xs[0] = xj;
-        }
-      }
-    };
-    if (nopiv) backward(std::integral_constant<bool, true>());
-    else backward(std::integral_constant<bool, false>());
-    cpa_wait<0>();
-    __syncthreads();
-    if (ng > 0) write_out(ng - 1, rep, true);
-    __threadfence_block();
-    __syncthreads();   // x complete before the next pass (or the log-term read below)
+    for (int t = 0; t <= FKL; ++t) r[t] = ld_here(x + 2 * t, act && t < nn);
+    // L y = P b, y(j) into the field's slot of row j; then U x = y from row nnw-1 down, a system joining at its own last row
+    if (nopiv) {
+      subst_pass<false, true>(fc, x, nn, nnw, a.nrdim, act, r);
+      subst_pass<true, true>(fc, x, nn, nnw, a.nrdim, act, r);
+    } else {
+      subst_pass<false, false>(fc, x, nn, nnw, a.nrdim, act, r);
+      subst_pass<true, false>(fc, x, nn, nnw, a.nrdim, act, r);
+    }
   }
-  if (root && comp == 0 && a.kind == 1 && !a.skip_root && !a.no_ln && cnt > 0) *lv = __ldcg(x) * exp(a.lognorm[0]);
+  if (root && comp == 0 && a.kind == 1 && !a.skip_root && !a.no_ln && cnt > 0) *lv = x[0] * exp(a.lognorm[0]);
 }
 
 // the bordered (0,0) system of idel2_preln (KL = 3), single thread, after the batch
@@ -1277,7 +1245,10 @@ int ihelm_noalloc(void* e_dev, double* ln, double alpha) {
   return 0;
 }
 
-// the positions of the cached-factor system order (sys_mk) for a's chop window: sets lead, nsys and nsp
+// rows per system in the factor cache
+static int lu_rows(int nrc) { return std::max(std::min(nrc, G.nrdim), 1); }
+
+// the positions of the cached-factor system order (sys_mk) for a's chop window: sets lead, nsys, nsp and frows
 static size_t set_positions(SolveArgs& a) {
   const int klo = std::max(a.nzcu, 1) - 1, khi = std::min(a.nzdim, a.nzc) - 1;
   const size_t nd = (size_t)std::max(khi - klo + 1, 0);
@@ -1285,6 +1256,7 @@ static size_t set_positions(SolveArgs& a) {
   const size_t n = (size_t)a.lead + (size_t)std::max(a.npc, 1) * a.nzdim;
   a.nsys = (int)n;
   a.nsp = (int)((n + 31) / 32 * 32);
+  a.frows = lu_rows(a.nrc);
   return n;
 }
 
@@ -1302,14 +1274,11 @@ void lu_cache_clear() {
 }
 
 // the factors' per-32-system row-exchange flags follow the factor rows in the cache entry
-static size_t lu_flag_offset(int nrc, size_t nsp) {
-  const int nnmax = std::max(std::min(nrc, G.nrdim), 1);
-  return (size_t)nnmax * FSL * nsp;
-}
+static size_t lu_flag_offset(int nrc, size_t nsp) { return nsp / 16 * fac_group(lu_rows(nrc)); }
 static int* lu_flags(double* buf, int nrc, size_t nsp) { return (int*)(buf + lu_flag_offset(nrc, nsp)); }
 
-// the cached factors of (kind, alpha, chop window), laid out [row][slot][system] with system stride
-// nsp, then nsp/32 row-exchange flags; made by factor() on a miss
+// the cached factors of (kind, alpha, chop window) for nsp positions, then nsp/32 row-exchange flags; made by factor() on a
+// miss
 template <class F>
 static int lu_cache_get(int kind, double alpha, const ChopIdx& c, size_t nsp, double** out, F factor) {
   for (auto& e : g_lu)
@@ -1335,12 +1304,10 @@ static int lu_cache_get(int kind, double alpha, const ChopIdx& c, size_t nsp, do
   return 0;
 }
 
-// the substitution launch: 64*NR threads per 32 systems
+// the substitution launch: 32 systems of two fields or 64 of one per CTA
 template <int NR>
 static int launch_subst(const SolveArgs& a, const double* fac, size_t nsys) {
-  size_t smb = sizeof(SubstSmem<NR>);
-  MLG_CUDA(cudaFuncSetAttribute(k_band_subst<NR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smb));
-  k_band_subst<NR><<<cdiv(nsys, 32), 64 * NR, smb, G.stream>>>(a, fac);
+  k_band_subst<NR><<<cdiv(nsys, NR == 2 ? 32 : 64), 128, 0, G.stream>>>(a, fac);
   MLG_LAUNCH();
   return 0;
 }
