@@ -278,9 +278,10 @@ static int r_spread(long long lines) {
   while (tr > 2 && lines / tr < 152) tr /= 2;
   return tr;
 }
-// With less than four lines per CTA most of the chip's issue slots are idle and a line's chain of operations is the time: a
-// thread then takes one radix at a time (288 lines of 90 points in FP64: 28 -> 14 us)
-static bool r_narrow(int most) { return most < 4; }
+// With fewer lines than a CTA of 32 for every SM, issue slots are idle and a line's chain of operations is the time: a
+// thread then takes one radix at a time (288 lines of 90 points in FP64: 28 -> 14 us; transforms at 40 x 400 x 20, plain:
+// 204 -> 133 us)
+static bool r_narrow(int most) { return most < 32; }
 // threads per line: the fewest thread steps over the passes, or (narrow) the shortest chain of steps
 static int r_threads(const RPlan& pl, int lines, bool narrow = false) {
   int best = 1;
