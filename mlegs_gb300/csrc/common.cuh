@@ -86,7 +86,8 @@ struct Ctx {
   float2 *tw_p32 = nullptr, *tw_z32 = nullptr, *tw_pr32 = nullptr;   // FP32 copies for the mixed form
   float4 *tw_pdf = nullptr, *tw_zdf = nullptr, *tw_prdf = nullptr;   // double-float copies (re hi, re lo, im hi, im lo)
 
-  int4 *tw_zq = nullptr, *tw_pq = nullptr, *tw_prq = nullptr;   // fixed-point copies (power-of-two lengths; fftq.cu)
+  double2 *tw_zqd = nullptr, *tw_pqd = nullptr, *tw_prqd = nullptr;   // those copies rounded to FP64 (fftqr.cu)
+  int4 *tw_zq = nullptr, *tw_pq = nullptr, *tw_prq = nullptr;   // fixed-point copies (fftq.cu, fftqr.cu)
 
   // ln slots of all scalars (device), and per-step scalars (svv gains, flags, scratch reductions)
   double* ln_slots = nullptr;  int n_slots = 0;  std::vector<int> free_slots;
@@ -136,7 +137,9 @@ int chop_index(const Scalar& s, ChopIdx& c);
 // kernels (host launchers), defined in the .cu files
 int kit_build(const mlg_params* p);
 int kit_free();
-bool fftq_length(int L);   // lengths of the fixed-point transforms (fftq.cu)
+bool fftq_length(int L);    // lengths of the fixed-point transforms: powers of two (fftq.cu)
+bool fftqr_length(int L);   // and others (fftqr.cu), used for so many lines
+bool fftqr_pays(int L, long long lines);
 int launch_hfft(Scalar& s, int dir);             // dir -1 forward (1/np), +1 backward
 int launch_hfft_rs(Scalar& s, int dir, const double* rs);   // with the rows times rs (before fwd / after bwd)
 int launch_vfft(Scalar& s, int dir);             // dir -1 forward (1/nz), +1 backward

@@ -18,7 +18,8 @@
 // Layout: a field is (nrdim, npdim, nzdim) with r fastest.  Both transforms run along a strided
 // dimension; a CTA takes TRL consecutive lines (the contiguous batch, so every global access is a run of
 // TRL*16 bytes) and several threads per line, which exchange through shared memory as [point][TRL].
-// Lengths: powers of two from 16 to 256 here (FP32 and FP64) and in fftq.cu (the plain form), others in fftr.cu.
+// Lengths: powers of two from 16 to 256 here (FP32 and FP64) and, for the plain form, in fftq.cu; others in fftr.cu and, for the
+// plain form where they split into two passes, in fftqr.cu.
 #include "common.cuh"
 #include "fft_common.cuh"
 #include <cmath>
@@ -146,6 +147,7 @@ static int vfft_any(const FSet& fs, int dir, double scale) {
   } else {
     int sexp;
     if (fftq_length(G.nz) && std::frexp(scale, &sexp) == 0.5) MLG_TRY(launch_zfft_q(fs, dir, sexp - 1));
+    else if (fftqr_pays(G.nz, (long long)G.nrdim * G.npdim * fs.n)) MLG_TRY(launch_zfft_qr(fs, dir, scale));
     else MLG_TRY(vfft_t<double>(fs, dir, scale, 0, G.npdim, 32, G.stream));
   }
   kt_end(1, 2.0 * fs.n * G.fsize * 16);
@@ -193,6 +195,11 @@ static int hfft_t(const FSet& fs, int dir, double scale) {
     int sexp = 1;
     if (fftq_length(L) && (dir > 0 || std::frexp(scale, &sexp) == 0.5)) {
       MLG_TRY(launch_pfft_q(fs, dir, dir > 0 ? 0 : sexp - 1));
+      kt_end(1, 2.0 * fs.n * G.fsize * 16);
+      return 0;
+    }
+    if (fftqr_pays(L, (long long)G.nrdim * G.nzdim * fs.n)) {
+      MLG_TRY(launch_pfft_qr(fs, dir, scale));
       kt_end(1, 2.0 * fs.n * G.fsize * 16);
       return 0;
     }

@@ -415,10 +415,66 @@ __device__ __forceinline__ void pfft_bwd2_body(const FSet& fs, int nrdim, int np
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// Other lengths: one or two Stockham stages in registers
+struct RPass { unsigned char p1, p2; unsigned short ns, m; unsigned magic; };   // radices, points combined before it, butterfly pairs, ceil(2^32 / ns)
+// a b with the roundings fixed (one product of each component is rounded, the other is added to it unrounded), so that it does
+// not depend on how a compiler contracts the sums: an FP32 transform's last bits reach the spectrum of a mixed run
+template <typename C> __device__ __forceinline__ C r_mul(C a, C b) {
+  C r;
+  r.x = fma(a.x, b.x, -(a.y * b.y));
+  r.y = fma(a.y, b.x, a.x * b.y);
+  return r;
+}
+// one pass over a line's L points: butterfly pair j takes the points j + m i, i < p1 p2, as p2 transforms of radix p1 over
+// groups combined ns at a time, then p1 of radix p2
+template <typename T, int P1, int P2, class LD, class ST>
+__device__ __forceinline__ void r_pass(const RPass& ps, int L, const typename TW<T>::t* __restrict__ tw, int sgn, int tt,
+                                       int TT, LD ld, ST st) {
+  typedef typename CT<T>::t C;
+  constexpr int R = P1 * P2;
+  const int m = ps.m, ns = ps.ns;
+  const int st2 = ns == 1 ? m : (int)__umulhi((unsigned)m, ps.magic), st1 = st2 * P2;   // L / (ns p1 p2), L / (ns p1)
+  for (int j = tt; j < m; j += TT) {
+    const int q = ns == 1 ? j : (int)__umulhi((unsigned)j, ps.magic), k = j - q * ns;
+    C a[P2][P1];
+#pragma unroll
+    for (int i = 0; i < R; ++i) a[i % P2][i / P2] = ld(j + m * i);
+    if (k) {
+#pragma unroll
+      for (int r1 = 1; r1 < P1; ++r1) {
+        const C w = load_tw<T>(tw, k * r1 * st1, sgn);
+#pragma unroll
+        for (int r2 = 0; r2 < P2; ++r2) a[r2][r1] = r_mul(a[r2][r1], w);
+      }
+    }
+#pragma unroll
+    for (int r2 = 0; r2 < P2; ++r2) dft_small<T>(a[r2], P1, sgn);
+    const int base = q * ns * R + k;
+#pragma unroll
+    for (int r1 = 0; r1 < P1; ++r1) {
+      C b[P2];
+#pragma unroll
+      for (int r2 = 0; r2 < P2; ++r2) b[r2] = a[r2][r1];
+      const int kb = k + r1 * ns;
+      if (P2 > 1 && kb) {
+#pragma unroll
+        for (int r2 = 1; r2 < P2; ++r2) b[r2] = r_mul(b[r2], load_tw<T>(tw, kb * r2 * st2, sgn));
+      }
+      dft_small<T>(b, P2, sgn);
+#pragma unroll
+      for (int r2 = 0; r2 < P2; ++r2) st(base + ns * (r1 + r2 * P1), b[r2]);
+    }
+  }
+}
+
 // fixed-point transforms of power-of-two lengths (fftq.cu), the plain form's: z (scale 2^sexp), phi forward (2^sexp) and
 // backward
 int launch_zfft_q(const FSet& fs, int dir, int sexp);
 int launch_pfft_q(const FSet& fs, int dir, int sexp);
+// and of products of two of 2..6, 8, 9, 10, 12, 15 and 16 (fftqr.cu), with any FP64 scale
+int launch_zfft_qr(const FSet& fs, int dir, double scale);
+int launch_pfft_qr(const FSet& fs, int dir, double scale);
 // transforms of other lengths (fftr.cu), FP32 and FP64: z on the planes m0 .. m0 + nm - 1, phi
 // forward (scaled) and backward
 template <typename T>

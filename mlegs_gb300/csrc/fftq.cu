@@ -18,40 +18,9 @@
 //
 // Shape: as the FP64 transforms (fft_common.cuh): TRL lines per CTA, R2 threads per line, L = R1 R2 in two register
 // passes through shared memory.
-#include "fft_common.cuh"
+#include "fft_fixed.cuh"
 
 namespace mlg {
-
-struct qc { long long x, y; };   // a complex fixed-point value
-__device__ __forceinline__ qc q_add(qc a, qc b) { return {a.x + b.x, a.y + b.y}; }
-__device__ __forceinline__ qc q_sub(qc a, qc b) { return {a.x - b.x, a.y - b.y}; }
-__device__ __forceinline__ qc q_conj(qc a) { return {a.x, -a.y}; }
-__device__ __forceinline__ qc q_muli(qc a, int sgn) { return sgn > 0 ? qc{-a.y, a.x} : qc{a.y, -a.x}; }   // a (sgn i)
-
-// x w for |x| <= 2^62 and a real constant w = (WH 2^31 + WL) 2^-61 below 1: with x = xh 2^31 + xl the products xh WH, xh WL
-// and xl WH are summed in their places and xl WL, less than one unit, is replaced by its mean WL / 2 (it spreads by 0.29
-// units at most); the middle terms are rounded at the unit
-template <int WH, int WL> __device__ __forceinline__ long long q_mulc(long long x) {
-  const int xh = (int)(x >> 31), xl = (int)((unsigned)x & 0x7FFFFFFFu);
-  const long long m = (long long)xh * WL + (long long)xl * WH + ((1ll << 29) + (WL >> 1));
-  return (((long long)xh * WH) << 1) + (m >> 30);
-}
-// v w for a twiddle w = ((wx + i wy) 2^31 + (wz + i ww)) 2^-61 (low parts in [0, 2^31), or both parts of a component
-// negated); |v| <= 2^61.5, so that the four middle products stay below 2^63
-__device__ __forceinline__ qc q_mul(qc v, int4 w) {
-  const int xh = (int)(v.x >> 31), xl = (int)((unsigned)v.x & 0x7FFFFFFFu);
-  const int yh = (int)(v.y >> 31), yl = (int)((unsigned)v.y & 0x7FFFFFFFu);
-  long long a = (long long)((w.z - w.w) >> 1) + (1ll << 29), b = (long long)((w.z >> 1) + (w.w >> 1)) + (1ll << 29);
-  a += (long long)xh * w.z; a += (long long)xl * w.x; a -= (long long)yh * w.w; a -= (long long)yl * w.y;
-  b += (long long)xh * w.w; b += (long long)xl * w.y; b += (long long)yh * w.z; b += (long long)yl * w.x;
-  return {(((long long)xh * w.x - (long long)yh * w.y) << 1) + (a >> 30),
-          (((long long)xh * w.y + (long long)yh * w.x) << 1) + (b >> 30)};
-}
-__device__ __forceinline__ int4 q_tw(const int4* __restrict__ tw, int idx, int sgn) {   // tables hold exp(-2 pi i k / L)
-  int4 w = __ldg(tw + idx);
-  if (sgn > 0) { w.y = -w.y; w.w = -w.w; }
-  return w;
-}
 
 // cos(pi/4), cos(pi/8), sin(pi/8) in units of 2^-61: upper and lower 31 bits
 constexpr int Q_C4H = 759250124, Q_C4L = 2134625425, Q_C8H = 992008094, Q_C8L = 848119337, Q_S8H = 410903206, Q_S8L = 1465168233;
@@ -86,9 +55,6 @@ template <int N, int SGN> __device__ __forceinline__ void q_dft(qc* a) {
     }
   }
 }
-// a line's scale: samples x_n become x_n 2^(NB - e1) for the first pass and are shifted right by sh after it, so that a
-// result of 2^(NB - e) is 1
-struct QScale { int e1, sh; };
 // from 128 points on (q_scale)
 template <int L> __host__ __device__ constexpr bool q_two_units() { return L >= 128; }
 
@@ -117,22 +83,6 @@ __device__ __forceinline__ void q_fft2pass(qc* a, qc (*b)[Split<L>::R2], qc* S, 
   }
 }
 
-// a thread's share of its line's statistics: the largest magnitude's high word, and the sum of the magnitudes in units of
-// the largest one's power of two, in FP32 (the double's upper bits moved into place; what is 2^126 smaller counts as 0)
-struct QStat { unsigned mx; float s; };
-template <int N> __device__ __forceinline__ QStat q_stat(const double2* d) {
-  QStat q{0u, 0.f};
-#pragma unroll
-  for (int i = 0; i < N; ++i)
-    q.mx = max(q.mx, max((unsigned)__double2hiint(d[i].x) & 0x7FFFFFFFu, (unsigned)__double2hiint(d[i].y) & 0x7FFFFFFFu));
-  const int sub = (int)(q.mx & 0x7FF00000u) - (126 << 20);
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    q.s += __int_as_float(max((__double2hiint(d[i].x) & 0x7FFFFFFF) - sub, 0) << 3);
-    q.s += __int_as_float(max((__double2hiint(d[i].y) & 0x7FFFFFFF) - sub, 0) << 3);
-  }
-  return q;
-}
 // the line's scale from its R2 threads' shares: sum |x| < 2^e over the line, and < 2^e1 over any one thread's samples
 // (HALF: over those of threads w and R2 - w together), sh = e - e1; false where the line needs FP64.  A thread's samples
 // are what the first pass sums: its own, finer unit keeps the rounding of the first pass' twiddles, which all later

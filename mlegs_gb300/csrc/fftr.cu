@@ -19,59 +19,9 @@
 
 namespace mlg {
 
-constexpr int RP_MAX = 16;
-struct RPass { int p1, p2, ns, m; unsigned magic; };   // radices, points combined before it, butterfly pairs, ceil(2^32 / ns)
+constexpr int RP_MAX = 10;
 struct RPlan { int L, n; RPass s[RP_MAX]; };
 
-// a b with the roundings fixed (one product of each component is rounded, the other is added to it unrounded), so that it does
-// not depend on how a compiler contracts the sums: an FP32 transform's last bits reach the spectrum of a mixed run
-template <typename C> __device__ __forceinline__ C r_mul(C a, C b) {
-  C r;
-  r.x = fma(a.x, b.x, -(a.y * b.y));
-  r.y = fma(a.y, b.x, a.x * b.y);
-  return r;
-}
-// one pass over a line's L points: butterfly pair j takes the points j + m i, i < p1 p2, as p2 transforms of radix p1 over
-// groups combined ns at a time, then p1 of radix p2
-template <typename T, int P1, int P2, class LD, class ST>
-__device__ __forceinline__ void r_pass(const RPass& ps, int L, const typename TW<T>::t* __restrict__ tw, int sgn, int tt,
-                                       int TT, LD ld, ST st) {
-  typedef typename CT<T>::t C;
-  constexpr int R = P1 * P2;
-  const int m = ps.m, ns = ps.ns;
-  const int st2 = ns == 1 ? m : (int)__umulhi((unsigned)m, ps.magic), st1 = st2 * P2;   // L / (ns p1 p2), L / (ns p1)
-  for (int j = tt; j < m; j += TT) {
-    const int q = ns == 1 ? j : (int)__umulhi((unsigned)j, ps.magic), k = j - q * ns;
-    C a[P2][P1];
-#pragma unroll
-    for (int i = 0; i < R; ++i) a[i % P2][i / P2] = ld(j + m * i);
-    if (k) {
-#pragma unroll
-      for (int r1 = 1; r1 < P1; ++r1) {
-        const C w = load_tw<T>(tw, k * r1 * st1, sgn);
-#pragma unroll
-        for (int r2 = 0; r2 < P2; ++r2) a[r2][r1] = r_mul(a[r2][r1], w);
-      }
-    }
-#pragma unroll
-    for (int r2 = 0; r2 < P2; ++r2) dft_small<T>(a[r2], P1, sgn);
-    const int base = q * ns * R + k;
-#pragma unroll
-    for (int r1 = 0; r1 < P1; ++r1) {
-      C b[P2];
-#pragma unroll
-      for (int r2 = 0; r2 < P2; ++r2) b[r2] = a[r2][r1];
-      const int kb = k + r1 * ns;
-      if (P2 > 1 && kb) {
-#pragma unroll
-        for (int r2 = 1; r2 < P2; ++r2) b[r2] = r_mul(b[r2], load_tw<T>(tw, kb * r2 * st2, sgn));
-      }
-      dft_small<T>(b, P2, sgn);
-#pragma unroll
-      for (int r2 = 0; r2 < P2; ++r2) st(base + ns * (r1 + r2 * P1), b[r2]);
-    }
-  }
-}
 template <typename T, class LD, class ST>
 __device__ __forceinline__ void r_pass_any(const RPass& ps, int L, const typename TW<T>::t* __restrict__ tw, int sgn, int tt,
                                            int TT, LD ld, ST st) {
@@ -251,7 +201,8 @@ static int r_plan(int L, RPlan& pl, bool single = false) {
   int ns = 1;
   auto add = [&](int p1, int p2) {
     if (pl.n < RP_MAX)
-      pl.s[pl.n] = {p1, p2, ns, L / (p1 * p2), ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0u};
+      pl.s[pl.n] = {(unsigned char)p1, (unsigned char)p2, (unsigned short)ns, (unsigned short)(L / (p1 * p2)),
+                    ns > 1 ? (unsigned)(((1ull << 32) + ns - 1) / ns) : 0u};
     ++pl.n;
     ns *= p1 * p2;
   };
@@ -263,7 +214,7 @@ static int r_plan(int L, RPlan& pl, bool single = false) {
   for (int i = a; i < b; ++i) add(f[i], 1);
   if (lp) add(f[nf - 2], f[nf - 1]);
   else add(b < nf ? f[b] : 1, 1);
-  if (pl.n > RP_MAX) return set_error(MLG_ESIZE, "fft: length too large");
+  if (pl.n > RP_MAX || L > 65535) return set_error(MLG_ESIZE, "fft: length too large");
   return 0;
 }
 // lines per CTA: 32, fewer where shared memory (`bytes` a line) would pass 96 KiB

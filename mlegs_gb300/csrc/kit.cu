@@ -263,9 +263,10 @@ static bool factors235(int n) {
   return n == 1;
 }
 
-// exp(-2 pi i k / L), k < count, for L a power of two, in units of 2^-61: (re, im) upper parts and (re, im) lower 31 bits of
-// the nearest integers.  The roots exp(2 pi i / 2^j) come from the half-angle formulas in double-double arithmetic and
-// every k is the product of the roots of its bits, so the entries do not depend on the machine's sin and cos.
+// exp(-2 pi i k / L), k < count <= L, in units of 2^-61: (re, im) upper parts and (re, im) lower 31 bits of the nearest
+// integers.  Every k is the product of the roots of its bits in double-double arithmetic, so the entries do not depend on
+// the machine's sin and cos: for L a power of two the roots are exp(2 pi i / 2^j), from the half-angle formulas; otherwise
+// the squares of exp(2 pi i / L), from its Taylor series.
 static std::vector<int4> twid_q(int L, int count) {
   struct D2 { double h, l; };
   auto two_s = [](double a, double b) { const double s = a + b, v = s - a; return D2{s, (a - (s - v)) + (b - v)}; };
@@ -283,20 +284,47 @@ static std::vector<int4> twid_q(int L, int count) {
     return quick(x, r.h / (2.0 * x));
   };
   std::vector<D2> c{{1.0, 0.0}, {-1.0, 0.0}, {0.0, 0.0}}, sn{{0.0, 0.0}, {0.0, 0.0}, {1.0, 0.0}};   // angles 2 pi, pi, pi / 2
-  while ((1 << (c.size() - 1)) < L) {
+  const bool pow2 = (L & (L - 1)) == 0;
+  while (pow2 && (1 << (c.size() - 1)) < L) {
     const D2 q = c.back();
     c.push_back(root(mul(add({1.0, 0.0}, q), {0.5, 0.0})));
     sn.push_back(root(mul(add({1.0, 0.0}, neg(q)), {0.5, 0.0})));
+  }
+  if (!pow2) {   // c[j], sn[j]: the angle 2 pi 2^j / L
+    const D2 th = mul({2.0 * PI, 2.0 * 1.2246467991473532e-16}, [&] {   // 2 pi times 1 / L
+      const double q = 1.0 / L;
+      return quick(q, std::fma(-q, (double)L, 1.0) / L);
+    }());
+    const D2 t2 = mul(th, th);
+    D2 x{1.0, 0.0}, y = th, tx{1.0, 0.0}, ty = th;
+    auto over = [&](D2 a, double d) { const double q = a.h / d; return quick(q, (std::fma(-q, d, a.h) + a.l) / d); };
+    for (int i = 1; i <= 20; ++i) {
+      tx = neg(over(mul(tx, t2), (2.0 * i - 1.0) * (2.0 * i)));
+      ty = neg(over(mul(ty, t2), (2.0 * i) * (2.0 * i + 1.0)));
+      x = add(x, tx);
+      y = add(y, ty);
+    }
+    c = {x};
+    sn = {y};
+    for (int j = 1; (1 << j) < L; ++j) {
+      const D2 nx = add(mul(x, x), neg(mul(y, y))), ny = mul({2.0, 0.0}, mul(x, y));
+      x = nx; y = ny;
+      c.push_back(x);
+      sn.push_back(y);
+    }
   }
   auto fixed = [](D2 v) { return (long long)std::ldexp(v.h, 61) + std::llrint(std::ldexp(v.l, 61)); };
   std::vector<int4> t(std::max(count, 1));
   for (int k = 0; k < count; ++k) {
     D2 x{1.0, 0.0}, y{0.0, 0.0};
-    for (int j = 1, bit = L / 2; bit >= 1; ++j, bit /= 2)   // bit: an angle of 2 pi / 2^j
-      if (k & bit) {
+    for (size_t i = 1; i <= c.size(); ++i) {
+      // root j is the angle 2 pi / 2^j, for bit L / 2^j of k (powers of two), or 2 pi 2^j / L, for bit 2^j
+      const size_t j = pow2 ? i : i - 1;
+      if (j < c.size() && (k & (pow2 ? L >> j : 1 << j))) {
         const D2 nx = add(mul(x, c[j]), neg(mul(y, sn[j]))), ny = add(mul(x, sn[j]), mul(y, c[j]));
         x = nx; y = ny;
       }
+    }
     const long long re = fixed(x), im = fixed(neg(y));
     t[k] = make_int4((int)(re >> 31), (int)(im >> 31), (int)(re & 0x7FFFFFFF), (int)(im & 0x7FFFFFFF));
   }
@@ -444,11 +472,27 @@ int kit_build(const mlg_params* P) {
   MLG_TRY(upload(&G.tw_prdf, todf(tpr)));
   MLG_TRY(upload(&G.tw_zdf, todf(tz)));
 
-  // fixed-point twiddles of the plain form's power-of-two transforms
-  if (fftq_length(nz)) MLG_TRY(upload(&G.tw_zq, twid_q(nz, nz)));
-  if (fftq_length(G.nph)) {
-    MLG_TRY(upload(&G.tw_pq, twid_q(G.nph, G.nph)));
-    MLG_TRY(upload(&G.tw_prq, twid_q(np, G.nph + 1)));
+  // fixed-point twiddles of the plain form's transforms; for lengths that are no power of two also rounded to FP64 (the table
+  // above has the angle's rounding error in it)
+  auto rounded = [](const std::vector<int4>& t) {
+    std::vector<double2> d(t.size());
+    auto val = [](int h, int l) { return std::ldexp((double)((long long)h * (1ll << 31) + l), -61); };
+    for (size_t i = 0; i < t.size(); ++i) d[i] = make_double2(val(t[i].x, t[i].z), val(t[i].y, t[i].w));
+    return d;
+  };
+  if (fftq_length(nz) || fftqr_length(nz)) {
+    const std::vector<int4> t = twid_q(nz, nz);
+    MLG_TRY(upload(&G.tw_zq, t));
+    if (fftqr_length(nz)) MLG_TRY(upload(&G.tw_zqd, rounded(t)));
+  }
+  if (fftq_length(G.nph) || fftqr_length(G.nph)) {
+    const std::vector<int4> t = twid_q(G.nph, G.nph), tr = twid_q(np, G.nph + 1);
+    MLG_TRY(upload(&G.tw_pq, t));
+    MLG_TRY(upload(&G.tw_prq, tr));
+    if (fftqr_length(G.nph)) {
+      MLG_TRY(upload(&G.tw_pqd, rounded(t)));
+      MLG_TRY(upload(&G.tw_prqd, rounded(tr)));
+    }
   }
 
   MLG_CUDA(cudaStreamSynchronize(G.stream));

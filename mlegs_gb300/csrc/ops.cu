@@ -1309,7 +1309,7 @@ int mlg_finalize(void) {
   xv_free();
   for (cd* b : G.all_bufs) cudaFree(b);
   void* arrs[] = {G.x, G.w, G.w32, G.r, G.rinv, G.lnx, G.ak, G.lognorm, G.pf, G.at0, G.at1, G.bd2, G.bxx, G.bd2f, G.bxxf, G.ak2f, G.tV, G.tD, G.tT,
-                  G.tV32, G.tD32, G.tT32, G.tw_p, G.tw_z, G.tw_pr, G.tw_p32, G.tw_z32, G.tw_pr32, G.tw_pdf, G.tw_zdf, G.tw_prdf, G.tw_zq, G.tw_pq, G.tw_prq, G.ln_slots, G.dscal, G.band_ws};
+                  G.tV32, G.tD32, G.tT32, G.tw_p, G.tw_z, G.tw_pr, G.tw_p32, G.tw_z32, G.tw_pr32, G.tw_pdf, G.tw_zdf, G.tw_prdf, G.tw_zq, G.tw_pq, G.tw_prq, G.tw_zqd, G.tw_pqd, G.tw_prqd, G.ln_slots, G.dscal, G.band_ws};
   for (void* a : arrs) if (a) cudaFree(a);
   cudaStream_t st = G.stream;
   cudaEvent_t e0 = G.ev0, e1 = G.ev1, ef = G.ev_fork, ej = G.ev_join;
