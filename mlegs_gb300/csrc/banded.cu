@@ -6,9 +6,8 @@
 //           applies the band in place.
 //   solve:  ihelm, idel2 (pre/pro ln), ihelmp (:575-1000) through lsolve -> zgbtrf + zgbtrs
 //           (mlegs_bndmat_ops.f90:369-457): LU with partial pivoting over kl rows, multipliers by the
-//           reciprocal pivot, U of bandwidth kl+ku, one right-hand side.  One thread per system;
-//           the factor lives in a scratch band laid out [row][diagonal][system] so that a warp's
-//           32 systems touch consecutive addresses.
+//           reciprocal pivot, U of bandwidth kl+ku, one right-hand side.  The factors are kept per (kind, alpha,
+//           chop window); a solve is a substitution, one thread per real system.
 // Every per-(m,k) loop of the reference visits k = 1..nzc and then k = nzcu..nzdim; when nzc == nzcu
 // (nzchop = nz/2+1) the shared slot is processed twice, and so it is here.
 #include "common.cuh"
@@ -535,7 +534,7 @@ int launch_band_apply(Scalar& s, int op, const ChopIdx& c) {
 }
 
 // ------------------------------------------------------------------------------------------------
-// banded LU solve, one thread per (m, k) system.
+// banded LU solves, one thread per (m, k) system.
 // mode 0: ihelm / idel2 generic:  A = D0(m) - ak^2 I + alpha I             (kl = ku = 2)
 // mode 1: idel2_proln on (0,0):   A = D0(0) with the column-1 log-term additions (:705-711)
 // mode 2: idel2_preln on (0,0):   rows shifted down, bordered by the ln unknown (:609-625), kl = 3
@@ -594,136 +593,6 @@ __device__ __forceinline__ double dmat(const SolveArgs& a, int m, double akv, in
   double v = a.bd2[c + 5 * ((size_t)i + (size_t)a.ne * m)];
   if (c == 2) v = v - akv * akv;
   return v;
-}
-
-__global__ void k_band_solve(SolveArgs a) {
-  int sys = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sys >= a.nsys) return;
-  int m = sys / a.nzdim, k = sys % a.nzdim;
-  int cnt = k_count(k, a.nzc, a.nzcu, a.nzdim);
-  int nn = max(min(a.nrc, a.nrc - m), 0);
-  bool root = (m == 0 && k == 0);
-  double e2 = pow(a.ell, 2.0);
-  // ln handling before the solves (ihelm :818-824, ihelmp :937-951 is done separately)
-  if (root && a.kind == 0) {
-    double lnin = *a.lnp;
-    double lno = lnin / a.alpha;
-    *a.lnp = lno;
-    double2* g = a.e;
-    g[0].x -= 4.0 / 3.0 / e2 / exp(a.lognorm[0]) * lno;
-    g[1].x += 2.0 / 1.0 / e2 / exp(a.lognorm[1]) * lno;
-    g[2].x -= 2.0 / 3.0 / e2 / exp(a.lognorm[2]) * lno;
-  }
-  if (m >= a.npc || nn < 1 || cnt == 0) return;
-  bool special = root && (a.kind == 1 || a.kind == 2);
-  int kl = 2, ku = 2;
-  if (special && a.kind == 2) { kl = 3; ku = 2; }
-  if (a.kind == 3) { kl = a.power; ku = a.power; }
-  int W = 2 * kl + ku + 1;
-  double akv = a.ak[k];
-  double2* x = a.e + (size_t)a.nrdim * (m + (size_t)a.npdim * k);
-  double alpha = (a.kind == 0 || a.kind == 3) ? a.alpha : 0.0;
-  size_t ns = a.nsys;
-#define U(i, j) a.ws[((size_t)(i) * W + ((j) - (i) + kl)) * ns + sys]
-  for (int rep = 0; rep < cnt; ++rep) {
-    // build the band rows (columns i-kl .. i+ku) into the work band
-    for (int i = 0; i < nn; ++i) {
-      for (int c = 0; c < W; ++c) a.ws[((size_t)i * W + c) * ns + sys] = 0.0;
-      if (a.kind == 3) {
-        // row i of the truncated power D^q, q = power/2 (the band products of mulrbrb,
-        // mlegs_bndmat_ops.f90:251-318, on nn x nn matrices), window i-8 .. i+8
-        int q = a.power / 2;
-        double rv[17], nv[17];
-        int w0 = i - 8;
-        for (int u = 0; u < 17; ++u) rv[u] = 0.0;
-        for (int jj = max(0, i - 2); jj <= min(nn - 1, i + 2); ++jj) rv[jj - w0] = dmat(a, m, akv, nn, i, jj);
-        for (int t = 2; t <= q; ++t) {
-          for (int u = 0; u < 17; ++u) nv[u] = 0.0;
-          for (int u = 0; u < 17; ++u) {
-            int col = w0 + u;
-            if (col < 0 || col >= nn) continue;
-            for (int jj = max(0, col - 2); jj <= min(nn - 1, col + 2); ++jj) {
-              int uu = jj - w0;
-              if (uu >= 0 && uu < 17) nv[uu] += rv[u] * dmat(a, m, akv, nn, col, jj);
-            }
-          }
-          for (int u = 0; u < 17; ++u) rv[u] = nv[u];
-        }
-        for (int j = max(0, i - kl); j <= min(nn - 1, i + ku); ++j) {
-          double v = rv[j - w0] + a.beta * dmat(a, m, akv, nn, i, j);
-          if (i == j) v += alpha;
-          U(i, j) = v;
-        }
-        continue;
-      }
-      for (int j = max(0, i - kl); j <= min(nn - 1, i + ku); ++j) {
-        double v;
-        if (special && a.kind == 1) {
-          v = dmat(a, 0, akv, nn, i, j);
-          if (j == 0) {
-            if (i == 0) v += 4.0 / 3.0 / e2;
-            if (i == 1) v -= 2.0 / 1.0 / e2 * exp(a.lognorm[0] - a.lognorm[1]);
-            if (i == 2) v += 2.0 / 3.0 / e2 * exp(a.lognorm[0] - a.lognorm[2]);
-          }
-        } else if (special && a.kind == 2) {
-          // del2_pre(2:nn,:) = del2_pre(1:nn-1,:); row 1 = e_1; column-1 additions (:609-617)
-          if (i == 0) v = (j == 0) ? 1.0 : 0.0;
-          else {
-            v = dmat(a, 0, akv, nn, i - 1, j);
-            if (j == 0) {
-              if (i == 1) v += 4.0 / 3.0 / e2;
-              if (i == 2) v -= 2.0 / 1.0 / e2 * exp(a.lognorm[0] - a.lognorm[1]);
-              if (i == 3) v += 2.0 / 3.0 / e2 * exp(a.lognorm[0] - a.lognorm[2]);
-            }
-          }
-        } else {
-          v = dmat(a, m, akv, nn, i, j);
-          if (i == j) v += alpha;
-        }
-        U(i, j) = v;
-      }
-    }
-    if (special && a.kind == 2 && rep == 0) {
-      for (int i = nn - 1; i >= 1; --i) x[i] = x[i - 1];
-      x[0] = make_double2(a.preln / exp(a.lognorm[0]), 0.0);
-    }
-    // factor + forward substitution (gbtrf/gbtrs 'N')
-    for (int j = 0; j < nn; ++j) {
-      int km = min(kl, nn - 1 - j), p = j;
-      double best = fabs(U(j, j));
-      for (int i = j + 1; i <= j + km; ++i) {
-        double t = fabs(U(i, j));
-        if (t > best) { best = t; p = i; }
-      }
-      if (U(p, j) == 0.0) { atomicExch(a.status, 1); return; }
-      int ju = min(nn - 1, j + kl + ku);
-      if (p != j) {
-        for (int c = j; c <= ju; ++c) { double t = U(p, c); U(p, c) = U(j, c); U(j, c) = t; }
-        double2 t = x[p]; x[p] = x[j]; x[j] = t;
-      }
-      double rp = 1.0 / U(j, j);
-      double2 xj = x[j];
-      for (int i = j + 1; i <= j + km; ++i) {
-        double l = U(i, j) * rp;
-        U(i, j) = l;
-        for (int c = j + 1; c <= ju; ++c) U(i, c) -= l * U(j, c);
-        x[i].x -= l * xj.x;
-        x[i].y -= l * xj.y;
-      }
-    }
-    for (int j = nn - 1; j >= 0; --j) {
-      double d = U(j, j);
-      double2 xj = make_double2(x[j].x / d, x[j].y / d);
-      x[j] = xj;
-      for (int i = j - 1; i >= max(0, j - kl - ku); --i) {
-        double u = U(i, j);
-        x[i].x -= xj.x * u;
-        x[i].y -= xj.y * u;
-      }
-    }
-  }
-#undef U
-  if (special) *a.lnp = x[0].x * exp(a.lognorm[0]);
 }
 
 // Entry (i, j) of the system matrix of (m, k) for kinds 0..2 (0-based, n x n truncation).
@@ -852,12 +721,17 @@ __device__ void window_solve(const SolveArgs& a, int sys, int kind, bool special
 //   slot KL          pivot row offset p in 0..KL (gbtrf's ipiv(j) - j)
 //   slot KL+1        1 / U(j, j)
 //   slot KL+2 ..     U(j, j+1 .. j+KL+KU)
+// The powered Helmholtz systems (kind 3; kl = ku = power), factored anew by one thread each on every call until they came
+// here (two diffusion steps with hyperviscosity of power 4: 200 x 100 x 50 19.4 -> 0.97 ms, 512 x 128 x 64 56 -> 2.7 ms), keep, per row, the multipliers, the pivot offset, 1 / U(j,j),
+// U(j,j) and U(j, j+1 ..) as they are: 3 power + 3 slots.
 constexpr int FKL = 2, FKU = 2, FSL = 2 * FKL + FKU + 2, FPAD = 16;
-// the doubles of one row (its slots are 16 apart), and of 16 systems with n rows each
-constexpr int FROW = FSL * 16;
-__host__ __device__ __forceinline__ size_t fac_group(int n) { return (size_t)(n + 2 * FPAD) * FROW; }
+__host__ __device__ constexpr int fac_slots(int power) { return power ? 3 * power + 3 : FSL; }   // power 0: kinds 0 and 1
+// the doubles of 16 systems with n rows each (a row's slots are 16 apart)
+__host__ __device__ __forceinline__ size_t fac_group(int n, int power) { return (size_t)(n + 2 * FPAD) * fac_slots(power) * 16; }
 // row 0 of the system at position sys
-__device__ __forceinline__ size_t fac_at(int sys, int n) { return (size_t)(sys >> 4) * fac_group(n) + (size_t)FPAD * FROW + (sys & 15); }
+__device__ __forceinline__ size_t fac_at(int sys, int n, int power) {
+  return (size_t)(sys >> 4) * fac_group(n, power) + (size_t)FPAD * fac_slots(power) * 16 + (sys & 15);
+}
 
 __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restrict__ fac) {
   int sys = blockIdx.x * blockDim.x + threadIdx.x;   // position in the system order (sys_mk)
@@ -871,7 +745,7 @@ __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restr
   double alpha = (a.kind == 0) ? a.alpha : 0.0;
   double e2 = a.ell * a.ell;
   constexpr int WC = FKL + FKU + 1, ns = 16;
-  double* const f0 = fac + fac_at(sys, a.frows);
+  double* const f0 = fac + fac_at(sys, a.frows, 0);
   double W[FKL + 1][WC];
 #pragma unroll
   for (int t = 0; t <= FKL; ++t)
@@ -893,7 +767,7 @@ __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restr
         for (int c = 0; c < WC; ++c) { double q = W[0][c]; W[0][c] = W[t][c]; W[t][c] = q; }
       }
     double rp = 1.0 / W[0][0];
-    double* f = f0 + (size_t)j * FROW;
+    double* f = f0 + (size_t)j * FSL * ns;
 #pragma unroll
     for (int t = 1; t <= FKL; ++t) {
       double l = 0.0;
@@ -921,9 +795,82 @@ __global__ void __launch_bounds__(32) k_band_factor(SolveArgs a, double* __restr
   }
 }
 
+// Row i of the powered Helmholtz matrix: the truncated power D^q, q = power/2 (the band products of mulrbrb,
+// mlegs_bndmat_ops.f90:251-318, on nn x nn matrices), plus beta D + alpha I; out[c] is column i - power + c
+template <int K> __device__ void hyper_row(const SolveArgs& a, int m, double akv, int nn, int i, double* out) {
+  double rv[17], nv[17];
+  const int w0 = i - 8;
+  for (int u = 0; u < 17; ++u) rv[u] = 0.0;
+  for (int jj = max(0, i - 2); jj <= min(nn - 1, i + 2); ++jj) rv[jj - w0] = dmat(a, m, akv, nn, i, jj);
+  for (int t = 2; t <= K / 2; ++t) {
+    for (int u = 0; u < 17; ++u) nv[u] = 0.0;
+    for (int u = 0; u < 17; ++u) {
+      int col = w0 + u;
+      if (col < 0 || col >= nn) continue;
+      for (int jj = max(0, col - 2); jj <= min(nn - 1, col + 2); ++jj) {
+        int uu = jj - w0;
+        if (uu >= 0 && uu < 17) nv[uu] += rv[u] * dmat(a, m, akv, nn, col, jj);
+      }
+    }
+    for (int u = 0; u < 17; ++u) rv[u] = nv[u];
+  }
+  for (int c = 0; c <= 2 * K; ++c) {
+    const int j = i - K + c;
+    out[c] = 0.0;
+    if (i >= nn || j < 0 || j >= nn) continue;
+    double v = rv[j - w0] + a.beta * dmat(a, m, akv, nn, i, j);
+    if (i == j) v += a.alpha;
+    out[c] = v;
+  }
+}
+// the factors of the powered Helmholtz systems (gbtrf semantics on a sliding window, as k_band_factor)
+template <int K>
+__global__ void __launch_bounds__(32) k_hyper_factor(SolveArgs a, double* __restrict__ fac) {
+  const int sys = blockIdx.x * blockDim.x + threadIdx.x;   // position in the system order (sys_mk)
+  if (sys >= a.nsys) return;
+  int m, k;
+  if (!sys_mk(a, sys, m, k)) return;
+  const int nn = max(min(a.nrc, a.nrc - m), 0);
+  if (m >= a.npc || nn < 1 || k_count(k, a.nzc, a.nzcu, a.nzdim) == 0) return;
+  const double akv = a.ak[k];
+  constexpr int WC = 2 * K + 1, ns = 16, NSL = fac_slots(K);
+  double* const f0 = fac + fac_at(sys, a.frows, K);
+  double W[K + 1][WC], row[WC];
+  for (int t = 0; t <= K; ++t) {
+    hyper_row<K>(a, m, akv, nn, t, row);
+    for (int c = 0; c < WC; ++c) W[t][c] = c - t + K < WC ? row[c - t + K] : 0.0;   // column c is row[c - (t - K)]
+  }
+  for (int j = 0; j < nn; ++j) {
+    const int km = min(K, nn - 1 - j);
+    int p = 0;
+    double best = fabs(W[0][0]);
+    for (int t = 1; t <= km; ++t)
+      if (fabs(W[t][0]) > best) { best = fabs(W[t][0]); p = t; }
+    if (W[p][0] == 0.0) { atomicExch(a.status, 1); atomicOr(&a.pivflag[sys >> 5], 2); return; }
+    if (p != 0) {
+      atomicOr(&a.pivflag[sys >> 5], 1);
+      for (int c = 0; c < WC; ++c) { double q = W[0][c]; W[0][c] = W[p][c]; W[p][c] = q; }
+    }
+    const double rp = 1.0 / W[0][0];
+    double* f = f0 + (size_t)j * NSL * ns;
+    for (int t = 1; t <= km; ++t) {
+      const double l = W[t][0] * rp;
+      for (int c = 1; c < WC; ++c) W[t][c] -= l * W[0][c];
+      f[(t - 1) * ns] = l;
+    }
+    f[K * ns] = (double)p;
+    f[(K + 1) * ns] = rp;
+    for (int c = 0; c < WC; ++c) f[(K + 2 + c) * ns] = W[0][c];
+    for (int t = 0; t < K; ++t) {
+      for (int c = 0; c < WC - 1; ++c) W[t][c] = W[t + 1][c + 1];
+      W[t][WC - 1] = 0.0;
+    }
+    hyper_row<K>(a, m, akv, nn, j + 1 + K, row);
+    for (int c = 0; c < WC; ++c) W[K][c] = row[c];
+  }
+}
+
 // forward and back substitution with the cached factors (gbtrs 'N', one or two right-hand sides), in place on the column
-constexpr int SNU = FKL + FKU;
-static_assert(FKL == 2, "the substitution compares the pivot index by the high words of 1.0 and 2.0");
 
 // ihelm's pre-solve log-term handling of one field (:818-824): so%ln = s%ln/alpha, the log terms on
 // e(1..3, 1, 1)
@@ -953,31 +900,45 @@ __device__ __forceinline__ void st_here(double* p, double v, bool in) {
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(p)); }
 
+// the high word of t = 0..8 in FP64: the pivot index of a row is compared by it, off the FP64 pipe
+__host__ __device__ constexpr int hi_of(int t) {
+  return t == 0 ? 0 : t == 1 ? 0x3FF00000 : t < 4 ? 0x40000000 + ((t - 2) << 19) : t < 8 ? 0x40100000 + ((t - 4) << 18) : 0x40200000;
+}
+// y / d, correctly rounded, from r = 1 / d correctly rounded (P. Markstein, Computation of elementary functions on the IBM
+// RISC System/6000 processor, 1990: the quotient's remainder is exact, and one correction rounds it): three FP64 operations
+__device__ __forceinline__ double div_by(double y, double d, double r) {
+  const double q = y * r, e = fma(-q, d, y);
+  const double x = fma(e, r, q);
+  return (__double2hiint(e) & 0x7FF00000) == 0x7FF00000 ? q : x;   // an infinite quotient stays one
+}
+
 // A pass of the substitution over the rows of a thread's real system (factors f0, row 0; right-hand side x, stride 2): step
 // i = 0, 1, ... works on row j = i (forward) or nnw - 1 - i (backward).  Two batches of SB rows alternate: one is read while
-// the other is computed.
-template <bool BWD, bool NX>
+// the other is computed.  P: 0 (kinds 0 and 1) or the power of the powered Helmholtz systems.
+template <int P, bool BWD, bool NX>
 __device__ __forceinline__ void subst_pass(const double* __restrict__ f0, double* x, int nn, int nnw, int nrdim, bool act,
-                                           double (&r)[FKL + 1]) {
-  // without row exchanges: the multipliers, or 1 / U(j,j) and the FKU entries of U's own band only
-  constexpr int NF = BWD ? (NX ? FKU + 1 : SNU + 1) : (NX ? FKL : FKL + 1), S0 = BWD ? FKL + 1 : 0, SB = NX ? 8 : 4, AHEAD = 32;
-  constexpr int D = BWD ? -1 : 1, J0 = BWD ? 0 : 1 + FKL;   // direction; the row entering at a step is J0 further
-  static_assert(2 * SB <= FPAD && SB * NF <= 32, "whole batches of factor rows; one prefetch per batch");
+                                           double (&r)[(P ? P : FKL) + 1]) {
+  constexpr int K = P ? P : FKL, SNU = 2 * K, NU = NX ? K : SNU, ROW = fac_slots(P) * 16;
+  // without row exchanges: the multipliers, or 1 / U(j,j) (and U(j,j)) and the K entries of U's own band only
+  constexpr int U1 = P ? 2 : 1, NF = BWD ? NU + U1 : (NX ? K : K + 1), S0 = BWD ? K + 1 : 0;
+  constexpr int SB = P == 0 ? (NX ? 8 : 4) : P < 8 ? (NX ? 4 : 2) : 2, AHEAD = 32;
+  constexpr int D = BWD ? -1 : 1, J0 = BWD ? 0 : 1 + K;   // direction; the row entering at a step is J0 further
+  static_assert(2 * SB <= FPAD, "whole batches of factor rows");
   const int rows = act ? nn : 0, jb = BWD ? nnw - 1 : 0, lane = threadIdx.x & 31;
-  const double* const fb = f0 + (ptrdiff_t)jb * FROW + S0 * 16;
+  const double* const fb = f0 + (ptrdiff_t)jb * ROW + S0 * 16;
   double* const xb = x + 2 * jb;
-  // this lane's share of a batch's factor rows, a 128-byte line each
-  const ptrdiff_t pf = D * (min(lane, SB * NF - 1) / NF) * FROW + min(lane, SB * NF - 1) % NF * 16 + (ptrdiff_t)D * AHEAD * FROW;
+  // this lane's share of a batch's factor rows, a 128-byte line each (of the widest rows, the first 32 lines)
+  const ptrdiff_t pf = D * (min(lane, SB * NF - 1) / NF) * ROW + min(lane, SB * NF - 1) % NF * 16 + (ptrdiff_t)D * AHEAD * ROW;
   double xs[SNU], late = 0.0;
 #pragma unroll
   for (int c = 0; c < SNU; ++c) xs[c] = 0.0;
   auto take = [&](double (&v)[SB][NF + 1], int i0) {
-    const double* f = fb + (ptrdiff_t)D * i0 * FROW;
+    const double* f = fb + (ptrdiff_t)D * i0 * ROW;
     const double* xv = xb + 2 * D * i0;
 #pragma unroll
     for (int u = 0; u < SB; ++u)
 #pragma unroll
-      for (int t = 0; t < NF; ++t) v[u][t] = ld_here(f + D * u * FROW + t * 16);
+      for (int t = 0; t < NF; ++t) v[u][t] = ld_here(f + D * u * ROW + t * 16);
     // (rows past a system's own count reach no row of its own: a whole batch inside the column is read as it stands)
     const int jn = BWD ? jb - (i0 + SB - 1) : i0 + J0 + SB - 1;   // the batch's last row
     if (BWD ? jn >= 0 : jn < nrdim) {
@@ -998,25 +959,31 @@ __device__ __forceinline__ void subst_pass(const double* __restrict__ f0, double
     for (int u = 0; u < SB; ++u) {
       if constexpr (!BWD) {
         if constexpr (!NX) {
-          // the pivot row index p (0..FKL), stored as a double: compared by its high word, off the FP64 pipe
-          const int ph = __double2hiint(v[u][FKL]);
+          const int ph = __double2hiint(v[u][K]);   // the pivot row index, stored as a double
 #pragma unroll
-          for (int t = 1; t <= FKL; ++t)
-            if (ph == (t == 1 ? 0x3FF00000 : 0x40000000)) { double w = r[0]; r[0] = r[t]; r[t] = w; }
+          for (int t = 1; t <= K; ++t)
+            if (ph == hi_of(t)) { double w = r[0]; r[0] = r[t]; r[t] = w; }
         }
         st_here(xo + 2 * u, r[0], rows - i0 > u);
 #pragma unroll
-        for (int t = 1; t <= FKL; ++t) r[t] = fma(-v[u][t - 1], r[0], r[t]);
+        for (int t = 1; t <= K; ++t) r[t] = fma(-v[u][t - 1], r[0], r[t]);
 #pragma unroll
-        for (int t = 0; t < FKL; ++t) r[t] = r[t + 1];
-        r[FKL] = v[u][NF];
+        for (int t = 0; t < K; ++t) r[t] = r[t + 1];
+        r[K] = v[u][NF];
       } else {
-        constexpr int NU = NX ? FKU : SNU;
-        // x(j) = y(j)/U(j,j) - sum_c (U(j,j+c)/U(j,j)) x(j+c): only the last FMA waits on x(j+1)
-        double t = v[u][NF] * v[u][0];
+        double xj;
+        if constexpr (P == 0) {
+          // x(j) = y(j)/U(j,j) - sum_c (U(j,j+c)/U(j,j)) x(j+c): only the last FMA waits on x(j+1)
+          double t = v[u][NF] * v[u][0];
 #pragma unroll
-        for (int c = 2; c <= NU; ++c) t = fma(-v[u][c], xs[c - 1], t);
-        double xj = fma(-v[u][1], xs[0], t);
+          for (int c = 2; c <= NU; ++c) t = fma(-v[u][c], xs[c - 1], t);
+          xj = fma(-v[u][1], xs[0], t);
+        } else {
+          double t = v[u][NF];
+#pragma unroll
+          for (int c = NU; c >= 1; --c) t = fma(-v[u][1 + c], xs[c - 1], t);
+          xj = div_by(t, v[u][1], v[u][0]);
+        }
         if (jb - i0 - u >= nn) xj = 0.0;
         // the row before is stored behind this one's operations, which would wait behind a store waiting for its own
         st_here(xo - 2 * (u - 1), late, (unsigned)(nnw - i0 - u) < (unsigned)rows);
@@ -1055,7 +1022,7 @@ __device__ __forceinline__ void subst_pass(const double* __restrict__ f0, double
 // with staging warps beside the computing ones and mbarriers, 270 to 330 (each wait cost 200).  Per call at 192 x 128 x
 // 128, one and two fields' mean: 157 -> 106 us; two fields at 512 x 512 x 256: 1.24 -> 0.84 ms; the FP64 instructions alone,
 // spread evenly, 27 and 46 us at 192.
-template <int NR>
+template <int NR, int P>
 __global__ void __launch_bounds__(128, 2) k_band_subst(SolveArgs a, const double* __restrict__ fac) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q = NR == 2 ? warp >> 1 : 0, comp = lane & 1;
   // The systems that are solved twice (the first positions) make the longest chains.  Where two CTAs per SM hold the whole
@@ -1084,24 +1051,27 @@ __global__ void __launch_bounds__(128, 2) k_band_subst(SolveArgs a, const double
     cntw = max(cntw, __shfl_xor_sync(0xffffffffu, cntw, o));
   }
   if (cntw == 0) return;
-  const double* fc = fac + fac_at(sys, a.frows);
+  const double* fc = fac + fac_at(sys, a.frows, P);
   // the factorisation records, per 32 systems, whether any of them exchanges rows; where none does the forward pass runs
   // without the pivot slot and the exchanges, and U keeps the matrix's own FKU superdiagonals (its fill-in entries are exact
   // zeros), so that the backward pass reads and applies only those, with the same result bit for bit, since
   // fma(-0, x, t) = t for finite x
-  const bool nopiv = a.pivflag != nullptr && __ldcg(&a.pivflag[sys >> 5]) == 0;
+  const int flag = __ldcg(&a.pivflag[sys >> 5]);
+  const bool nopiv = flag == 0;
+  if (flag & 2) atomicExch(a.status, 1);   // a zero pivot (kind 3)
   for (int rep = 0; rep < cntw; ++rep) {
     const bool act = rep < cnt;
-    double r[FKL + 1];
+    constexpr int K = P ? P : FKL;
+    double r[K + 1];
 #pragma unroll
-    for (int t = 0; t <= FKL; ++t) r[t] = ld_here(x + 2 * t, act && t < nn);
+    for (int t = 0; t <= K; ++t) r[t] = ld_here(x + 2 * t, act && t < nn);
     // L y = P b, y(j) into the field's slot of row j; then U x = y from row nnw-1 down, a system joining at its own last row
     if (nopiv) {
-      subst_pass<false, true>(fc, x, nn, nnw, a.nrdim, act, r);
-      subst_pass<true, true>(fc, x, nn, nnw, a.nrdim, act, r);
+      subst_pass<P, false, true>(fc, x, nn, nnw, a.nrdim, act, r);
+      subst_pass<P, true, true>(fc, x, nn, nnw, a.nrdim, act, r);
     } else {
-      subst_pass<false, false>(fc, x, nn, nnw, a.nrdim, act, r);
-      subst_pass<true, false>(fc, x, nn, nnw, a.nrdim, act, r);
+      subst_pass<P, false, false>(fc, x, nn, nnw, a.nrdim, act, r);
+      subst_pass<P, true, false>(fc, x, nn, nnw, a.nrdim, act, r);
     }
   }
   if (root && comp == 0 && a.kind == 1 && !a.skip_root && !a.no_ln && cnt > 0) *lv = x[0] * exp(a.lognorm[0]);
@@ -1260,9 +1230,9 @@ static size_t set_positions(SolveArgs& a) {
   return n;
 }
 
-// LRU cache of factor sets, keyed by (kind, alpha, chop window)
+// LRU cache of factor sets, keyed by (kind, alpha, chop window) and, for kind 3, beta and power
 struct LUEntry {
-  int kind; double alpha; int nrc, npc, nzc, nzcu; double* buf; size_t bytes; unsigned long long used;
+  int kind, power; double alpha, beta; int nrc, npc, nzc, nzcu; double* buf; size_t bytes; unsigned long long used;
 };
 static std::vector<LUEntry> g_lu;
 static unsigned long long g_lu_clock = 0;
@@ -1274,27 +1244,31 @@ void lu_cache_clear() {
 }
 
 // the factors' per-32-system row-exchange flags follow the factor rows in the cache entry
-static size_t lu_flag_offset(int nrc, size_t nsp) { return nsp / 16 * fac_group(lu_rows(nrc)); }
-static int* lu_flags(double* buf, int nrc, size_t nsp) { return (int*)(buf + lu_flag_offset(nrc, nsp)); }
+static size_t lu_flag_offset(int nrc, size_t nsp, int power) { return nsp / 16 * fac_group(lu_rows(nrc), power); }
+static int* lu_flags(double* buf, int nrc, size_t nsp, int power = 0) { return (int*)(buf + lu_flag_offset(nrc, nsp, power)); }
 
 // the cached factors of (kind, alpha, chop window) for nsp positions, then nsp/32 row-exchange flags; made by factor() on a
 // miss
 template <class F>
-static int lu_cache_get(int kind, double alpha, const ChopIdx& c, size_t nsp, double** out, F factor) {
+static int lu_cache_get(int kind, double alpha, const ChopIdx& c, size_t nsp, double** out, F factor, double beta = 0.0, int power = 0) {
   for (auto& e : g_lu)
-    if (e.kind == kind && e.alpha == alpha && e.nrc == c.nrc && e.npc == c.npc && e.nzc == c.nzc && e.nzcu == c.nzcu) {
+    if (e.kind == kind && e.alpha == alpha && e.beta == beta && e.power == power && e.nrc == c.nrc && e.npc == c.npc && e.nzc == c.nzc && e.nzcu == c.nzcu) {
       e.used = ++g_lu_clock;
       *out = e.buf;
       return 0;
     }
-  size_t bytes = lu_flag_offset(c.nrc, nsp) * sizeof(double) + (nsp / 32) * sizeof(int);
-  if (g_lu.size() >= LU_MAX_ENTRIES) {
+  size_t bytes = lu_flag_offset(c.nrc, nsp, power) * sizeof(double) + (nsp / 32) * sizeof(int);
+  auto evict = [] {
     auto it = std::min_element(g_lu.begin(), g_lu.end(), [](const LUEntry& x, const LUEntry& y) { return x.used < y.used; });
     dfree(it->buf, it->bytes);
     g_lu.erase(it);
+  };
+  if (g_lu.size() >= LU_MAX_ENTRIES) evict();
+  LUEntry e{kind, power, alpha, beta, c.nrc, c.npc, c.nzc, c.nzcu, nullptr, bytes, ++g_lu_clock};
+  while (int rc = dmalloc((void**)&e.buf, bytes)) {   // out of memory: older sets make room
+    if (g_lu.empty()) return rc;
+    evict();
   }
-  LUEntry e{kind, alpha, c.nrc, c.npc, c.nzc, c.nzcu, nullptr, bytes, ++g_lu_clock};
-  MLG_TRY(dmalloc((void**)&e.buf, bytes));
   // rows past a system's own count (and systems outside the chop) stay zero: pivot offset 0, so a
   // block's substitution can take its no-exchange paths; the flags start at zero
   MLG_CUDA(cudaMemsetAsync(e.buf, 0, bytes, G.stream));
@@ -1305,32 +1279,28 @@ static int lu_cache_get(int kind, double alpha, const ChopIdx& c, size_t nsp, do
 }
 
 // the substitution launch: 32 systems of two fields or 64 of one per CTA
-template <int NR>
+template <int NR, int P = 0>
 static int launch_subst(const SolveArgs& a, const double* fac, size_t nsys) {
-  k_band_subst<NR><<<cdiv(nsys, NR == 2 ? 32 : 64), 128, 0, G.stream>>>(a, fac);
+  k_band_subst<NR, P><<<cdiv(nsys, NR == 2 ? 32 : 64), 128, 0, G.stream>>>(a, fac);
   MLG_LAUNCH();
   return 0;
 }
-// kind as in SolveArgs; the band scratch grows to fit (kl, ku)
 // algorithmic bytes of one substitution pass over nrhs fields: each field read and written once, the
-// cached factors (FSL doubles per row and system) read once
-static double solve_bytes(int nrhs, const ChopIdx& c) {
+// cached factors read once
+static double solve_bytes(int nrhs, const ChopIdx& c, int power = 0) {
   double nsys = (double)std::max(c.npc, 1) * G.nzdim;
   double rows = std::max(std::min(c.nrc, G.nrdim), 1);
-  return 2.0 * nrhs * G.fsize * 16 + rows * FSL * nsys * 8;
+  return 2.0 * nrhs * G.fsize * 16 + rows * fac_slots(power) * nsys * 8;
 }
 
 int launch_band_solve(Scalar& s, int kind, const ChopIdx& c, double alpha, double beta, double preln, int power) {
   if (c.npc > G.npchop) return set_error(MLG_ECHOP, "chop_index: chopping in p beyond the kit's azimuthal modes");
-  int kl = 2, ku = 2;
-  if (kind == 2) kl = 3;
-  if (kind == 3) { kl = power; ku = power; }
-  int W = std::max(2 * kl + ku + 1, kl + ku + 3);
+  const int kl = kind == 2 ? 3 : 2, ku = 2, W = std::max(2 * kl + ku + 1, kl + ku + 3);
   int npc = std::max(c.npc, 1);
   size_t nsys = (size_t)npc * G.nzdim;
   int nnmax = std::max(std::min(c.nrc, G.nrdim), 1);
   size_t need = (size_t)nnmax * W * nsys * sizeof(double);
-  if (need > G.band_ws_bytes) {
+  if (kind != 3 && need > G.band_ws_bytes) {
     if (G.band_ws) dfree(G.band_ws, G.band_ws_bytes);
     G.band_ws = nullptr;
     G.band_ws_bytes = 0;
@@ -1345,8 +1315,23 @@ int launch_band_solve(Scalar& s, int kind, const ChopIdx& c, double alpha, doubl
   a.kind = kind; a.power = power; a.skip_root = 0; a.transpose = 0; a.no_ln = 0;
   kt_begin(KT_SOLVE);
   if (kind == 3) {
-    k_band_solve<<<cdiv(nsys, 64), 64, 0, G.stream>>>(a);
-    MLG_LAUNCH();
+    const size_t npos = set_positions(a);
+    double* fac = nullptr;
+    auto solve = [&](auto pc) -> int {
+      constexpr int P = decltype(pc)::value;
+      MLG_TRY(lu_cache_get(3, alpha, c, (size_t)a.nsp, &fac, [&](double* buf) -> int {
+        SolveArgs fa = a;
+        fa.pivflag = lu_flags(buf, a.nrc, (size_t)a.nsp, P);
+        k_hyper_factor<P><<<cdiv(npos, 32), 32, 0, G.stream>>>(fa, buf);
+        MLG_LAUNCH();
+        return 0;
+      }, beta, P));
+      a.pivflag = lu_flags(fac, a.nrc, (size_t)a.nsp, P);
+      return launch_subst<1, P>(a, fac, npos);
+    };
+    if (power == 4) MLG_TRY(solve(std::integral_constant<int, 4>()));
+    else if (power == 6) MLG_TRY(solve(std::integral_constant<int, 6>()));
+    else MLG_TRY(solve(std::integral_constant<int, 8>()));
   } else {
     // kinds 0 and 1 (and the batch of kind 2): cached factors, substitution only; the bordered
     // (0,0) system of kind 2 is skipped by the batch and solved on its own afterwards
@@ -1370,7 +1355,7 @@ int launch_band_solve(Scalar& s, int kind, const ChopIdx& c, double alpha, doubl
       MLG_LAUNCH();
     }
   }
-  kt_end(KT_SOLVE, solve_bytes(1, c));
+  kt_end(KT_SOLVE, solve_bytes(1, c, kind == 3 ? power : 0));
   return 0;
 }
 
