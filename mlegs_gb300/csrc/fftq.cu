@@ -117,7 +117,7 @@ template <int L, int TRL, bool HALF> __device__ __forceinline__ bool q_scale(con
 
 // z FFT (lines as k_zfft2), scaled by 2^sexp
 template <int L, int SGN, int TRL>
-__global__ void __launch_bounds__(TRL * Split<L>::R2) k_zfft_q(FSet fs, int nrdim, int npdim, const int4* __restrict__ tw,
+__global__ void __launch_bounds__(TRL * Split<L>::R2, TRL * Split<L>::R2 == 256 ? 2 : 0) k_zfft_q(FSet fs, int nrdim, int npdim, const int4* __restrict__ tw,
                                                                const double2* __restrict__ tw64, int sexp, double scale,
                                                                int nlines) {
   constexpr int R1 = Split<L>::R1, R2 = Split<L>::R2, Q = R1 / R2, NB = 61;
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(TRL * Split<L>::R2) k_zfft_q(FSet fs, int nrdi
 // X_(L-k) come from the same sums: with e = Z_k + conj Z_(L-k), t = -i w_k (Z_k - conj Z_(L-k)), X_k = (e + t) / 2 and
 // X_(L-k) = conj(e - t) / 2
 template <int L, int TRL>
-__global__ void __launch_bounds__(TRL * Split<L>::R2) k_pfft_fwd_q(FSet fs, int nrdim, int npdim, int nzdim,
+__global__ void __launch_bounds__(TRL * Split<L>::R2, TRL * Split<L>::R2 == 256 ? 2 : 0) k_pfft_fwd_q(FSet fs, int nrdim, int npdim, int nzdim,
                                                                    const int4* __restrict__ tw, const int4* __restrict__ twr,
                                                                    const double2* __restrict__ tw64,
                                                                    const double2* __restrict__ twr64, int sexp, double scale,
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(TRL * Split<L>::R2) k_pfft_fwd_q(FSet fs, int 
 
 // φ backward: X_0..X_L -> packed reals (unnormalised; rows times rs[r] last, in FP64), slot L <- np X_L, in place
 template <int L, int TRL>
-__global__ void __launch_bounds__(TRL * Split<L>::R2) k_pfft_bwd_q(FSet fs, int nrdim, int npdim, int nzdim,
+__global__ void __launch_bounds__(TRL * Split<L>::R2, TRL * Split<L>::R2 == 256 ? 2 : 0) k_pfft_bwd_q(FSet fs, int nrdim, int npdim, int nzdim,
                                                                    const int4* __restrict__ tw, const int4* __restrict__ twr,
                                                                    const double2* __restrict__ tw64,
                                                                    const double2* __restrict__ twr64, double np_d, int nrs) {
@@ -305,8 +305,9 @@ template <class K> static int q_smem(K k, size_t bytes) {
 }
 
 template <int L, int SGN> static int zfft_q(const FSet& fs, int sexp) {
-  // 256 points: 16 lines of 16 threads, so that two CTAs share an SM
-  constexpr int TRL = L == 256 ? 16 : 32, R2 = Split<L>::R2;
+  // 16 lines from 64 points on, so that several CTAs share an SM (two of the 256 threads of 256 points, held to 128 registers:
+  // four transforms of three fields at 512 x 512 x 256 7.3 -> 6.0 ms)
+  constexpr int TRL = L >= 64 ? 16 : 32, R2 = Split<L>::R2;
   const size_t sm = (size_t)L * TRL * sizeof(qc) + (size_t)R2 * TRL * sizeof(QStat);
   MLG_TRY(q_smem(k_zfft_q<L, SGN, TRL>, sm));
   const int nlines = G.nrdim * G.npdim;
@@ -325,7 +326,7 @@ int launch_zfft_q(const FSet& fs, int dir, int sexp) {
 }
 
 template <int L> static int pfft_q(const FSet& fs, int dir, int sexp) {
-  constexpr int TRL = L == 256 ? 16 : 32, R2 = Split<L>::R2;
+  constexpr int TRL = L >= 64 ? 16 : 32, R2 = Split<L>::R2;
   const size_t sm = (size_t)(L + 1) * TRL * sizeof(qc) + (size_t)R2 * TRL * sizeof(QStat);
   const int grid = cdiv((long long)G.nrdim * G.nzdim * fs.n, TRL);
   if (dir < 0) {
