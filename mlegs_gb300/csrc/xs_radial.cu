@@ -703,8 +703,10 @@ constexpr size_t XS_SMEM_MAX = 227 * 1024;
 // (up to 256 points), so that an item's columns land and are scanned while the one before is cut; then digit stages, at
 // most four (six measured the same), and table entries in what is left.
 struct XsPlan { int nz, aent, bst, nraw; };
-static bool xs_plan(int ns, int rawk, XsPlan& p) {
-  for (int nz = G.nzdim > 8 ? 16 : 8; nz >= 8; nz /= 2)
+// `few`: no more items than half the SMs; halved, they take less time each (24 x 20 x 12, plain: 17.1 and 21.1 us forward and
+// backward with 16 columns, 14.9 and 17.2 with 8).
+static bool xs_plan(int ns, int rawk, XsPlan& p, bool few = false) {
+  for (int nz = G.nzdim > 8 && !few ? 16 : 8; nz >= 8; nz /= 2)
     for (int nraw = 2; nraw >= 1; --nraw)
       for (int sb = XS_SBMAX; sb >= 2; --sb)
         for (int ae = XS_AEMAX; ae >= 2; --ae)
@@ -738,7 +740,8 @@ int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int n
   const int kmax = mode == 0 ? G.nrh : (nrc + 1) / 2;
   const int ns = xs_cfg(kmax, nrc, plain);
   XsPlan plan;
-  if (!ns || !xs_plan(ns, xs_rawk(nrc), plan)) return set_error(MLG_ESIZE, "radial contraction: too many radial points for exact slices");
+  const bool few = (long long)(npc - m0) * cdiv(G.nzdim, 16) * nf <= 76;
+  if (!ns || !xs_plan(ns, xs_rawk(nrc), plan, few)) return set_error(MLG_ESIZE, "radial contraction: too many radial points for exact slices");
   const int nmt = cdiv(nrows, 128), nkc = cdiv(kmax, XS_KC), nrp = nmt * 128;
   XsImg& im = g_xs[mode][plain ? 0 : 1];
   if (im.nrc != nrc || im.npc != npc || !im.p || im.ns != ns) {
