@@ -134,10 +134,11 @@ __global__ void k_band_apply(double2* __restrict__ e, BandTabs tb, double* __res
 //   svis = s; svis = del2(svis) (band rows, with the log terms of (0,0)); svis = visc*svis;
 //   s = a*(s + 1.5 dt nl - 0.5 dt nl_p + dt/2 svis)   (e and ln; svis%ln = 0 after del2)
 // One CTA per (m, k) column of the whole array, the same operations and order as the copy, band
-// apply, scale and four-term combination it replaces.  The mixed form runs the m >= 1 stencils in FP32.
-template <typename T>
-__global__ void k_abcn_rhs(double2* __restrict__ e, const double2* __restrict__ nl, const double2* __restrict__ nlp,
-                           double* __restrict__ lnp, const double* __restrict__ lnnl, const double* __restrict__ lnnlp,
+// apply, scale and four-term combination it replaces.  The mixed form runs the m >= 1 stencils in FP32 and, in a vortex
+// step, sums the increment in FP32 too (SUM64 false).  next: nl_p takes nl's values, each where it has just been read.
+template <typename T, bool SUM64>
+__global__ void k_abcn_rhs(double2* __restrict__ e, const double2* __restrict__ nl, double2* nlp,
+                           double* __restrict__ lnp, const double* __restrict__ lnnl, double* lnnlp, int next,
                            BandTabs tb, const double* __restrict__ lognorm,
                            int nrdim, int npdim, int ne, int nrc, int npc, int nzc, int nzcu, int nzdim, double ell,
                            double visc, double c1, double c2, double c3, double post) {
@@ -149,8 +150,19 @@ __global__ void k_abcn_rhs(double2* __restrict__ e, const double2* __restrict__ 
   size_t off = (size_t)nrdim * (m + (size_t)npdim * k);
   double2* g = e + off;
   const double2* n0 = nl + off;
-  const double2* n1 = nlp + off;
+  double2* n1 = nlp + off;
   const bool act = m < npc && nn > 0 && cnt > 0;
+  auto sum = [&](int i, double2 s3) {
+    double2 x = g[i], a1 = n0[i], a2 = n1[i];
+    s3 = make_double2(0.0 + visc * s3.x, 0.0 + visc * s3.y);   // svis = visc*svis
+    double2 acc = make_double2(0, 0);
+    acc.x += 1.0 * x.x; acc.y += 1.0 * x.y;
+    acc.x += c1 * a1.x; acc.y += c1 * a1.y;
+    acc.x += c2 * a2.x; acc.y += c2 * a2.y;
+    acc.x += c3 * s3.x; acc.y += c3 * s3.y;
+    g[i] = make_double2(post * acc.x, post * acc.y);
+    if (next) n1[i] = a1;
+  };
   if (m > 0 && sizeof(T) == sizeof(float)) {
     // the mixed form's m >= 1 columns: the increment 1.5 dt nl - 0.5 dt nl_p + dt/2 visc del2(s) summed
     // in FP32 (its terms carry the FP32 contractions' rounding already), added to the FP64 state
@@ -180,6 +192,14 @@ __global__ void k_abcn_rhs(double2* __restrict__ e, const double2* __restrict__ 
         for (int i = threadIdx.x; i < nn; i += blockDim.x) c0[i] = c1b[i];
         __syncthreads();
       }
+    }
+    if constexpr (SUM64) {
+      for (int i = threadIdx.x; i < nrdim; i += blockDim.x) {
+        double2 s3 = g[i];
+        if (act && i < nn) s3 = make_double2(f2d_fast(c0[i].x), f2d_fast(c0[i].y));
+        sum(i, s3);
+      }
+      return;
     }
     const float f1 = d2f_fast(c1), f2 = d2f_fast(c2), f3 = d2f_fast(c3 * visc);
     for (int i = threadIdx.x; i < nrdim; i += blockDim.x) {
@@ -228,16 +248,7 @@ __global__ void k_abcn_rhs(double2* __restrict__ e, const double2* __restrict__ 
     sv[2].x += 2.0 / 3.0 / e2 / exp(lognorm[2]) * lnin;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < nrdim; i += blockDim.x) {
-    double2 x = g[i], a1 = n0[i], a2 = n1[i], s3 = sv[i];
-    s3 = make_double2(0.0 + visc * s3.x, 0.0 + visc * s3.y);   // svis = visc*svis
-    double2 acc = make_double2(0, 0);
-    acc.x += 1.0 * x.x; acc.y += 1.0 * x.y;
-    acc.x += c1 * a1.x; acc.y += c1 * a1.y;
-    acc.x += c2 * a2.x; acc.y += c2 * a2.y;
-    acc.x += c3 * s3.x; acc.y += c3 * s3.y;
-    g[i] = make_double2(post * acc.x, post * acc.y);
-  }
+  for (int i = threadIdx.x; i < nrdim; i += blockDim.x) sum(i, sv[i]);
   if (lnblk && threadIdx.x == 0) {
     double l = 0.0;
     l += 1.0 * lnin;
@@ -245,29 +256,24 @@ __global__ void k_abcn_rhs(double2* __restrict__ e, const double2* __restrict__ 
     l += c2 * *lnnlp;
     l += c3 * 0.0;
     *lnp = post * l;
+    if (next) *lnnlp = *lnnl;
   }
 }
 
 static BandTabs band_tabs() { return BandTabs{G.bd2, G.bxx, G.ak, G.bd2f, G.bxxf, G.ak2f}; }
 
-int launch_abcn_rhs(Scalar& s, const Scalar& nl, const Scalar& nl_p, double dt, double a) {
+// sum64: the mixed form's increment in FP64; next: nl_p takes nl's values
+int launch_abcn_rhs(Scalar& s, const Scalar& nl, Scalar& nl_p, double dt, double a, bool sum64, bool next) {
   ChopIdx c;
   MLG_TRY(chop_index(s, c));
   if (c.npc > G.npchop) return set_error(MLG_ECHOP, "chop_index: chopping in p beyond the kit's azimuthal modes");
   dim3 grid(G.nzdim, G.npdim);
   size_t sm = 2ull * G.nrdim * sizeof(double2);
   kt_begin(2);
-  if (G.precision == MLG_MIXED) {
-    if (sm > 48 * 1024) MLG_CUDA(cudaFuncSetAttribute(k_abcn_rhs<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_abcn_rhs<float><<<grid, 128, sm, G.stream>>>(s.e, nl.e, nl_p.e, s.ln, nl.ln, nl_p.ln, band_tabs(), G.lognorm, G.nrdim,
-                                                   G.npdim, G.ne, c.nrc, c.npc, c.nzc, c.nzcu, G.nzdim, G.ell, G.P.visc,
-                                                   1.5 * dt, -.5 * dt, dt / 2.0, a);
-  } else {
-    if (sm > 48 * 1024) MLG_CUDA(cudaFuncSetAttribute(k_abcn_rhs<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_abcn_rhs<double><<<grid, 128, sm, G.stream>>>(s.e, nl.e, nl_p.e, s.ln, nl.ln, nl_p.ln, band_tabs(), G.lognorm, G.nrdim,
-                                                    G.npdim, G.ne, c.nrc, c.npc, c.nzc, c.nzcu, G.nzdim, G.ell, G.P.visc,
-                                                    1.5 * dt, -.5 * dt, dt / 2.0, a);
-  }
+  auto kern = G.precision != MLG_MIXED ? k_abcn_rhs<double, true> : sum64 ? k_abcn_rhs<float, true> : k_abcn_rhs<float, false>;
+  if (sm > 48 * 1024) MLG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  kern<<<grid, 128, sm, G.stream>>>(s.e, nl.e, nl_p.e, s.ln, nl.ln, nl_p.ln, next ? 1 : 0, band_tabs(), G.lognorm, G.nrdim, G.npdim,
+                                    G.ne, c.nrc, c.npc, c.nzc, c.nzcu, G.nzdim, G.ell, G.P.visc, 1.5 * dt, -.5 * dt, dt / 2.0, a);
   MLG_LAUNCH();
   kt_end(2, 5.0 * G.fsize * 16);
   return 0;

@@ -264,7 +264,7 @@ int launch_band_solve(Scalar& s, int kind, const ChopIdx& c, double alpha, doubl
 int launch_band_solve_T(Scalar& s, int kind, const ChopIdx& c, double alpha);
 int launch_band_solve_T_pair(Scalar& s1, Scalar& s2, const ChopIdx& c, double alpha);
 int launch_ihelm_pair(Scalar& s1, Scalar& s2, const ChopIdx& c, double alpha);
-int launch_abcn_rhs(Scalar& s, const Scalar& nl, const Scalar& nl_p, double dt, double a);
+int launch_abcn_rhs(Scalar& s, const Scalar& nl, Scalar& nl_p, double dt, double a, bool sum64, bool next);
 
 }  // namespace mlg
 

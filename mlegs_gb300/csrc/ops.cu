@@ -978,17 +978,27 @@ int op_abcn(Scalar& s, Scalar& s_p, Scalar& nl, Scalar& nl_p, double dt) {
   if (!fff4(s, nl) || !fff4(s_p, nl_p)) return set_error(MLG_ESPACE, "fefe: all input scalars must be in FFF for time stepping");
   if (G.P.hyperpow == 0 && G.P.visc < 5.0e-14)
     return set_error(MLG_EINVISCID, "abcn: inviscid case and no linear term in rhs. semi-implicit time adv is impossible");
+  if (G.P.hyperpow == 0) {
+    // the right-hand side and nl_p = nl in one pass, the solve, s_p = s: three launches for the seven of the operations one
+    // by one (four steps at 32^3: 188 -> 124 us)
+    const double al = -2.0 / (dt * G.P.visc);
+    const bool next = nl.e != s.e && nl_p.e != s.e;
+    MLG_TRY(launch_abcn_rhs(s, nl, nl_p, dt, al, true, next));
+    MLG_TRY(op_ihelm(s, al));
+    MLG_TRY(assign(s_p, s));
+    if (!next) return assign(nl_p, nl);
+    std::memcpy(nl_p.space, nl.space, 4);
+    for (int i = 0; i < 3; ++i) nl_p.off[i] = nl.off[i];
+    return 0;
+  }
   TMP(svis);
   MLG_TRY(assign(svis, s));
   MLG_TRY(lterm(svis));
-  double a;
-  if (G.P.hyperpow == 0) a = -2.0 / (dt * G.P.visc);
-  else a = -2.0 / (dt * (G.P.hypervisc * hsign()));
+  const double a = -2.0 / (dt * (G.P.hypervisc * hsign()));
   // sh = s + dt*(1.5 nl - .5 nl_p); sh = a*(sh + dt/2*svis)
   MLG_TRY(lincomb(s, {{&s, 1.0}, {&nl, 1.5 * dt}, {&nl_p, -.5 * dt}, {&svis, dt / 2.0}},
                   {{&s, 1.0}, {&nl, 1.5 * dt}, {&nl_p, -.5 * dt}, {&svis, dt / 2.0}}, a));
-  if (G.P.hyperpow == 0) MLG_TRY(op_ihelm(s, a));
-  else MLG_TRY(op_ihelmp(s, G.P.hyperpow, a, G.P.visc / (G.P.hypervisc * hsign())));
+  MLG_TRY(op_ihelmp(s, G.P.hyperpow, a, G.P.visc / (G.P.hypervisc * hsign())));
   MLG_TRY(assign(s_p, s));
   MLG_TRY(assign(nl_p, nl));
   return 0;
@@ -1019,8 +1029,8 @@ static int op_abcn_pair(Scalar& s, Scalar& s_p, Scalar& nl, Scalar& nl_p, Scalar
     return set_error(MLG_EINVISCID, "abcn: inviscid case and no linear term in rhs. semi-implicit time adv is impossible");
   double a = -2.0 / (dt * G.P.visc);
   if (std::fabs(a) < 5.0e-14) return set_error(MLG_EALPHA, "ihelm: alpha equals to zero. Inversion of 0*identity is impossible");
-  MLG_TRY(launch_abcn_rhs(s, nl, nl_p, dt, a));
-  MLG_TRY(launch_abcn_rhs(t, ml, ml_p, dt, a));
+  MLG_TRY(launch_abcn_rhs(s, nl, nl_p, dt, a, false, false));
+  MLG_TRY(launch_abcn_rhs(t, ml, ml_p, dt, a, false, false));
   ChopIdx c1, c2;
   MLG_TRY(chop_index(s, c1));
   MLG_TRY(chop_index(t, c2));
