@@ -11,19 +11,20 @@ __device__ __forceinline__ qc q_conj(qc a) { return {a.x, -a.y}; }
 __device__ __forceinline__ qc q_muli(qc a, int sgn) { return sgn > 0 ? qc{-a.y, a.x} : qc{a.y, -a.x}; }   // a (sgn i)
 
 // x w for |x| <= 2^62 and a real constant w = (WH 2^31 + WL) 2^-61 below 1: with x = xh 2^31 + xl the products xh WH, xh WL
-// and xl WH are summed in their places and xl WL, less than one unit, is replaced by its mean WL / 2 (it spreads by 0.29
+// and xl WH are summed in their places and xl WL, less than two units, is replaced by its mean WL / 2 (it spreads by 0.58
 // units at most); the middle terms are rounded at the unit
-template <int WH, int WL> __device__ __forceinline__ long long q_mulc(long long x) {
+template <int WH, int WL> __host__ __device__ __forceinline__ long long q_mulc(long long x) {
   const int xh = (int)(x >> 31), xl = (int)((unsigned)x & 0x7FFFFFFFu);
   const long long m = (long long)xh * WL + (long long)xl * WH + ((1ll << 29) + (WL >> 1));
   return (((long long)xh * WH) << 1) + (m >> 30);
 }
 // v w for a twiddle w = ((wx + i wy) 2^31 + (wz + i ww)) 2^-61 (low parts in [0, 2^31), or both parts of a component
 // negated); |v| <= 2^61.5, so that the four middle products stay below 2^63
-__device__ __forceinline__ qc q_mul(qc v, int4 w) {
+__host__ __device__ __forceinline__ qc q_mul(qc v, int4 w) {
   const int xh = (int)(v.x >> 31), xl = (int)((unsigned)v.x & 0x7FFFFFFFu);
   const int yh = (int)(v.y >> 31), yl = (int)((unsigned)v.y & 0x7FFFFFFFu);
-  long long a = (long long)((w.z - w.w) >> 1) + (1ll << 29), b = (long long)((w.z >> 1) + (w.w >> 1)) + (1ll << 29);
+  // (halves first: the low parts' difference can pass 32 bits where one is negated)
+  long long a = (long long)((w.z >> 1) - (w.w >> 1)) + (1ll << 29), b = (long long)((w.z >> 1) + (w.w >> 1)) + (1ll << 29);
   a += (long long)xh * w.z; a += (long long)xl * w.x; a -= (long long)yh * w.w; a -= (long long)yl * w.y;
   b += (long long)xh * w.w; b += (long long)xl * w.y; b += (long long)yh * w.z; b += (long long)yl * w.x;
   return {(((long long)xh * w.x - (long long)yh * w.y) << 1) + (a >> 30),
