@@ -982,7 +982,9 @@ int op_abcn(Scalar& s, Scalar& s_p, Scalar& nl, Scalar& nl_p, double dt) {
     // the right-hand side and nl_p = nl in one pass, the solve, s_p = s: three launches for the seven of the operations one
     // by one (four steps at 32^3: 188 -> 124 us)
     const double al = -2.0 / (dt * G.P.visc);
-    const bool next = nl.e != s.e && nl_p.e != s.e;
+    // nl_p takes nl early only where no field is in two of the places that the assignments at the end, s_p = s and then
+    // nl_p = nl, read and write, and where the solve will not refuse alpha
+    const bool next = nl.e != s.e && nl_p.e != s.e && nl.e != nl_p.e && s_p.e != nl.e && s_p.e != nl_p.e && std::fabs(al) >= 5.0e-14;
     MLG_TRY(launch_abcn_rhs(s, nl, nl_p, dt, al, true, next));
     MLG_TRY(op_ihelm(s, al));
     MLG_TRY(assign(s_p, s));
