@@ -13,8 +13,10 @@
 // integer T = sum_d G_d 2^(w (NO-1-d)) in 64 bits (its lowest bits shifted out where it would not fit) and rounds
 // T 2^(EA + EB + const) once to FP64, on the integer pipe.
 // The result differs from the exact product of the FP64 operands by what the dropped orders hold, about 2^-(nb - 2) of
-// max|A(row,:)| max|B(:,n)|: 63 bits, in eight or nine balanced digits, is an FP64-grade product (the plain form), 42
-// bits the mixed form's.  No floating-point rounding happens anywhere else: the forward fold f(i) +- f(nr-1-i) is an exact
+// max|A(row,:)| max|B(:,n)|: 63 bits, in eight or nine balanced digits, for the plain form, 42 bits for the mixed form.  Where
+// FP64 sums were the plain form's alternative (nine digits), the outputs whose terms are all small beside those maxima, points
+// near the axis for one, are found by a contraction of the magnitudes and summed again in FP64 (xs_least_sum, k_xs_again): each
+// output is as near to the exact sum of its terms as an FP64 sum.  No floating-point rounding happens anywhere else: the forward fold f(i) +- f(nr-1-i) is an exact
 // integer sum of the two rounded samples, and the quadrature weights are folded into the table (A = pf w, one FP64
 // rounding at kit init).
 //
@@ -90,8 +92,11 @@ __global__ void k_xs_aexp(const double* __restrict__ pf, const double* __restric
 template <int NS> __host__ __device__ constexpr int xs_w() { return NS == 8 ? 8 : NS == 7 || NS == 10 ? 6 : 7; }
 template <int NS> __host__ __device__ constexpr bool xs_bal() { return NS == 8 || NS == 9; }
 template <int NS> __host__ __device__ constexpr int xs_nb() { return xs_bal<NS>() ? 63 : xs_w<NS>() * NS; }
+// nine digits carry a magnitude tile beside them (xs_least_sum); it costs 7 % (velocity and vorticity at 512 x 512 x 256:
+// 17.0 -> 18.2 ms, where FP64 sums took 159)
+template <int NS> __host__ __device__ constexpr int xs_mag() { return NS == 9 ? 1 : 0; }
 
-// digit tiles of 128 rows x 16 K: [m][row tile mt][par][chunk kc][digit t]
+// digit tiles of 128 rows x 16 K: [m][row tile mt][par][chunk kc][digit t, then the magnitudes]
 template <int NS>
 __global__ void k_xs_table(const double* __restrict__ pf, const double* __restrict__ w, const int* __restrict__ aexp,
                            uint16_t* __restrict__ img, int mode, int nrh, int ne, int nrc, int nmt, int nkc, int nrp) {
@@ -99,8 +104,9 @@ __global__ void k_xs_table(const double* __restrict__ pf, const double* __restri
   const size_t blk = blockIdx.x;   // (m * nmt + mt) * nkc + kc
   const int kc = (int)(blk % nkc), mt = (int)((blk / nkc) % nmt), m = (int)(blk / ((size_t)nkc * nmt));
   const int nn = max(min(nrc, nrc - m), 0);
-  uint8_t* base = (uint8_t*)img + ((blk / nkc) * 2 * nkc + kc) * (size_t)(NS * XS_ATILE);
-  const size_t pstep = (size_t)nkc * NS * XS_ATILE;   // from the even to the odd parity
+  constexpr int TILES = NS + xs_mag<NS>();
+  uint8_t* base = (uint8_t*)img + ((blk / nkc) * 2 * nkc + kc) * (size_t)(TILES * XS_ATILE);
+  const size_t pstep = (size_t)nkc * TILES * XS_ATILE;   // from the even to the odd parity
   for (int idx = threadIdx.x; idx < 2 * 128 * XS_KC; idx += blockDim.x) {
     const int k = idx % XS_KC, r = (idx / XS_KC) % 128, par = idx / (XS_KC * 128);
     const int row = mt * 128 + r, kk = kc * XS_KC + k;
@@ -110,11 +116,13 @@ __global__ void k_xs_table(const double* __restrict__ pf, const double* __restri
       E = aexp[(size_t)(mode == 0 ? m * 2 + par : m) * nrp + row];
       a = xs_a(pf, w, mode, row, kk, par, m, nn, nrh, ne);
     }
-    const unsigned long long X = (unsigned long long)xs_fix(a, E, xs_nb<NS>()) + (xs_bal<NS>() ? xs_bias<NS, W>() : 0ull);
+    const long long A = xs_fix(a, E, xs_nb<NS>());
+    const unsigned long long X = (unsigned long long)A + (xs_bal<NS>() ? xs_bias<NS, W>() : 0ull);
     xs_static_for<NS>([&](auto tc) {
       constexpr int t = decltype(tc)::value;
       *(uint16_t*)(base + par * pstep + t * XS_ATILE + xs_off(r, k)) = (uint16_t)xs_digit2<NS, W, xs_bal<NS>(), t>(X, X);
     });
+    if (xs_mag<NS>()) *(uint16_t*)(base + par * pstep + NS * XS_ATILE + xs_off(r, k)) = (uint16_t)xs_mag2(A, A);
   }
 }
 
@@ -131,7 +139,15 @@ struct XsArgs {
   int* status;
   int add_ln, nf, nr, nrh, nrdim, npdim, nzdim, nrc, m0, npc, nmt, nkc, nrp, rawk;
   int aent, bst, nraw;   // ring sizes: table entries and field-digit stages (one parity of a chunk), field-column buffers
+  int sent;              // and magnitude tiles
+  unsigned* again;       // nine digits: the outputs to be summed again, a word of 32 rows (xs_word)
+  int ngrp;
+  float least;           // xs_least_sum
 };
+// the word of the rows 32 g .. 32 g + 31 (of parity par, forward) of column (m, z) of field f
+__device__ __forceinline__ size_t xs_word(const XsArgs& a, int mode, int f, int m, int par, int g, int z) {
+  return ((((size_t)f * a.npc + m) * (mode == 0 ? 2 : 1) + par) * a.ngrp + g) * a.nzdim + z;
+}
 // field f's pointer without an indexed access to the kernel parameters (which would copy them to local
 // memory)
 template <class P> __device__ __forceinline__ P xs_sel(const P (&p)[XS_NF], int f) {
@@ -154,8 +170,8 @@ __device__ __forceinline__ bool xs_wait(uint64_t* bar, uint32_t phase, bool& ok)
 //   warps 12..27  epilogue: tensor memory -> 64-bit order sums -> FP64 results
 // A work unit is one parity of a row tile of an item: its accumulators are NO N columns, so that two sets fit tensor
 // memory (one with nine digits and 32 columns) and the MMAs of a unit run while the epilogue reads the one before.
-// Every hand-off is an mbarrier: the table entries and the field-digit stages (one parity of a chunk each) are rings,
-// the field columns are one buffer (the next item's columns land while the MMAs and the epilogue of this one run).  The
+// Every hand-off is an mbarrier: the table entries, their magnitude tiles and the field-digit stages (one parity of a chunk
+// each) are rings, the field columns are one buffer (the next item's columns land while the MMAs and the epilogue of this one run).  The
 // epilogue keeps the even parity's sums in registers and writes both parities' results after the odd unit.
 // What bounds it (clock64 traces, 192 points, six digits, about 13 000 cycles an item): the integer pipe, on which the
 // digits, the order sums and the conversions take about 8 000 of them; the MMAs need 4 000 (7 400 while one lane issued
@@ -171,12 +187,12 @@ __device__ __forceinline__ bool xs_wait_w(uint64_t* bar, uint32_t phase, bool& o
   return ok;
 }
 
-constexpr int XS_SBMAX = 4, XS_AEMAX = 8;   // ring sizes (at most)
+constexpr int XS_SBMAX = 4, XS_AEMAX = 8, XS_MEMAX = 2;   // ring sizes (at most)
 constexpr int XS_CXS = 4;                   // column-scale slots (items)
 constexpr int XS_NSW = 2, XS_NDW = 8, XS_NEW = 16;   // scale warps (2, 3), digit warps (4..11), epilogue warps (12..27)
 constexpr int XS_NG = 2;                    // groups of digit warps (at most the digit stages: a group waits at most one phase ahead)
 constexpr int XS_NEPI = XS_NEW * 32;
-constexpr int XS_NBAR = 4 + 2 * XS_AEMAX + 2 * XS_SBMAX + 4 + 2 * XS_CXS;
+constexpr int XS_NBAR = 4 + 2 * XS_AEMAX + 2 * XS_MEMAX + 2 * XS_SBMAX + 4 + 2 * XS_CXS;
 static_assert(2 + XS_NSW + XS_NDW + XS_NEW == XS_THREADS / 32, "warp roles");
 
 // MODE 0 forward, 1 backward; NS digits (and orders), NZ complex z columns per item
@@ -225,8 +241,10 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   constexpr int N = 2 * NZ;                       // real columns (MMA N per digit)
   constexpr int BT = N * XS_KC * 2;               // B digit tile bytes
   constexpr int AENT = NS * XS_ATILE;             // a table entry: the digits of one parity of a chunk
-  constexpr int BSTAGE = NS * BT;
-  constexpr int ACC = NO * N;                     // accumulator columns of a unit
+  constexpr bool MAG = xs_mag<NS>() != 0;         // with magnitude sums
+  constexpr int TILES = NS + xs_mag<NS>();        // tiles of a table entry's image and of a digit stage
+  constexpr int BSTAGE = TILES * BT;
+  constexpr int ACC = (NO + xs_mag<NS>()) * N;    // accumulator columns of a unit
   constexpr int TB = 2 * ACC <= 512 ? 2 : 1;      // sets of them
   constexpr int TUSE = TB * ACC;
   constexpr int TCOLS = TUSE <= 128 ? 128 : TUSE <= 256 ? 256 : 512;
@@ -238,10 +256,11 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   static_assert(NBLK % GW == 0, "digit blocks per warp");
   extern __shared__ __align__(1024) uint8_t xs_smem_raw[];
   uint8_t* sbase = (uint8_t*)(((uintptr_t)xs_smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t AE = (uint32_t)a.aent, SB = (uint32_t)a.bst;
+  const uint32_t AE = (uint32_t)a.aent, SB = (uint32_t)a.bst, ME = MAG ? (uint32_t)a.sent : 0u;
   const int RB = a.nraw;
   uint8_t* sA = sbase;                                   // [AE][AENT]
-  uint8_t* sB = sA + AE * AENT;                          // [SB][BSTAGE]
+  uint8_t* sM = sA + AE * AENT;                          // [ME][XS_ATILE]
+  uint8_t* sB = sM + ME * XS_ATILE;                      // [SB][BSTAGE]
   double* raw0 = (double*)(sB + SB * BSTAGE);            // [RB][NZ][rawk] complex (re, im)
   const size_t rawsz = (size_t)2 * NZ * a.rawk;
   int* colexp = (int*)(raw0 + RB * rawsz);               // [XS_CXS][N], by item
@@ -250,7 +269,9 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   uint64_t* bar_re = bars + 2;             // [RB] field columns consumed (digit threads)
   uint64_t* bar_af = bars + 4;             // [AE] table entry landed
   uint64_t* bar_ae = bar_af + XS_AEMAX;    // [AE] table entry consumed (MMA commit)
-  uint64_t* bar_bf = bar_ae + XS_AEMAX;    // [SB] digit stage written (the group's digit threads)
+  uint64_t* bar_mf = bar_ae + XS_AEMAX;    // [ME] magnitude tile landed
+  uint64_t* bar_me = bar_mf + XS_MEMAX;    // [ME] magnitude tile consumed (MMA commit)
+  uint64_t* bar_bf = bar_me + XS_MEMAX;    // [SB] digit stage written (the group's digit threads)
   uint64_t* bar_be = bar_bf + XS_SBMAX;    // [SB] digit stage consumed (MMA commit)
   uint64_t* bar_tf = bar_be + XS_SBMAX;    // [TB] accumulators complete (MMA commit)
   uint64_t* bar_te = bar_tf + 2;           // [TB] accumulators read (epilogue threads)
@@ -305,19 +326,27 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   if (warp == 0) {
     // ---- producer
     if (lane == 0) {
-      uint32_t c = 0, s = 0, ph = 0;   // table entries issued, ring slot and phase
+      uint32_t c = 0, s = 0, ph = 0, cm = 0, sm = 0, pm = 0;   // table entries and magnitude tiles issued, ring slots and phases
       for (int item = first; item < nitems && ok; item = next_item(item)) {
         const int m = item_m(item);
         int nkc_m, nrows, nmt_m;
         geom(item_nn(item), nkc_m, nrows, nmt_m);
         for (int mt = 0; mt < nmt_m && ok; ++mt)
           for (int par = 0; par < 2 && ok; ++par) {
-            const uint8_t* img_u = (const uint8_t*)a.img + (((size_t)m * a.nmt + mt) * 2 + par) * a.nkc * (size_t)AENT;
+            const uint8_t* img_u = (const uint8_t*)a.img + (((size_t)m * a.nmt + mt) * 2 + par) * a.nkc * (size_t)(TILES * XS_ATILE);
             for (int kc = 0; kc < nkc_m; ++kc, ++c) {
               if (c >= AE && !xs_wait(&bar_ae[s], ph ^ 1u, ok)) break;
               mbar_expect_tx(&bar_af[s], AENT);
-              bulk_g2s(sA + s * AENT, img_u + (size_t)kc * AENT, AENT, &bar_af[s]);
+              const uint8_t* ent = img_u + (size_t)kc * (TILES * XS_ATILE);
+              bulk_g2s(sA + s * AENT, ent, AENT, &bar_af[s]);
               if (++s == AE) { s = 0; ph ^= 1u; }
+              if constexpr (MAG) {
+                if (cm >= ME && !xs_wait(&bar_me[sm], pm ^ 1u, ok)) { ++c; break; }
+                mbar_expect_tx(&bar_mf[sm], XS_ATILE);
+                bulk_g2s(sM + sm * XS_ATILE, ent + AENT, XS_ATILE, &bar_mf[sm]);
+                ++cm;
+                if (++sm == ME) { sm = 0; pm ^= 1u; }
+              }
             }
           }
       }
@@ -327,12 +356,18 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
         bool ok2 = true;
         xs_wait(&bar_af[j % AE], (j / AE) & 1, ok2);
       }
+      if constexpr (MAG) {
+        for (uint32_t j = cm > ME ? cm - ME : 0; j < cm; ++j) {
+          bool ok2 = true;
+          xs_wait(&bar_mf[j % ME], (j / ME) & 1, ok2);
+        }
+      }
     }
   } else if (warp == 1) {
     // ---- MMA issue (the whole warp, one elected lane issuing)
     const uint32_t el = elect_lane();
-    uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
-    bool any = false;
+    uint32_t sa = 0, pa = 0, sm = 0, pm = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0, mlast = 0, pmlast = 0;
+    bool any = false, many = false;
     for (int item = first; item < nitems && ok; item = next_item(item)) {
       int nkc_m, nrows, nmt_m;
       geom(item_nn(item), nkc_m, nrows, nmt_m);
@@ -361,9 +396,18 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
                         idesc_bf16(128, (NO - t - NB1) * N), (kc > 0 || t > 0) ? 1u : 0u, el);
           }
           umma_commit(&bar_ae[sa], el);
-          umma_commit(&bar_be[sb], el);
           last = sa; plast = pa; any = true;
           if (++sa == AE) { sa = 0; pa ^= 1u; }
+          if constexpr (MAG) {   // the magnitudes' product, after the orders
+            if (!xs_wait_w(&bar_mf[sm], pm, ok)) break;
+            tc_fence_after();
+            umma_bf16(tacc + (uint32_t)(NO * N), sdesc(smem_u32(sM) + sm * XS_ATILE, XS_LBO, XS_SBO), sdesc(b0 + NS * BT, XS_LBO, XS_SBO),
+                      idesc_bf16(128, N), kc > 0 ? 1u : 0u, el);
+            umma_commit(&bar_me[sm], el);
+            mlast = sm; pmlast = pm; many = true;
+            if (++sm == ME) { sm = 0; pm ^= 1u; }
+          }
+          umma_commit(&bar_be[sb], el);
           if (++sb == SB) { sb = 0; pb ^= 1u; }
         }
         if (ok) umma_commit(&bar_tf[tb], el);
@@ -372,6 +416,10 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
     if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
       bool ok2 = true;
       xs_wait_w(&bar_ae[last], plast, ok2);
+    }
+    if (MAG && many) {
+      bool ok2 = true;
+      xs_wait_w(&bar_me[mlast], pmlast, ok2);
     }
   } else if (warp < 2 + XS_NSW) {
     // ---- column scales from the largest magnitudes' high words of the re and im parts: |x| < 2^(exponent field - 1022),
@@ -476,6 +524,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
               const double* col = raw + (size_t)2 * zz * a.rawk + (n & 1);
               const int off = xs_off(n, 2 * kp);
               unsigned long long x[2];
+              long long xm[2];
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 const int k = kc * XS_KC + 2 * kp + h;
@@ -491,8 +540,10 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
                   const int j = 2 * k + par;
                   if (j < nn) X = xs_fixs(col[2 * j], base[bi]);
                 }
+                xm[h] = X;
                 x[h] = (unsigned long long)X + (BAL ? xs_bias<NS, W>() : 0ull);
               }
+              if constexpr (MAG) *(uint32_t*)(bst + NS * BT + off) = xs_mag2(xm[0], xm[1]);
               xs_static_for<NS>([&](auto tc) {
                 constexpr int t = decltype(tc)::value;
                 *(uint32_t*)(bst + t * BT + off) = xs_digit2<NS, W, BAL, t>(x[0], x[1]);
@@ -518,6 +569,9 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
       double2* fout = xs_sel(a.out, item_f(item));
       int nkc_m, nrows, nmt_m;
       geom(nn, nkc_m, nrows, nmt_m);
+      // the item's column scales: written before its digits were cut, and so before its accumulators were complete
+      if (!xs_wait_w(&bar_cx[ii % XS_CXS], (ii / XS_CXS) & 1, ok)) break;
+      const int* cx = colexp + (ii % XS_CXS) * N + cg * CW;
       for (int mt = 0; mt < nmt_m && ok; ++mt) {
         const int row = mt * 128 + lq * 32 + lane;
         const bool live = mt * 128 + lq * 32 < nrows;   // a warp of rows past the tile's rows reads nothing
@@ -533,10 +587,15 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
         }
         // T 2^(row exp + column exp + eo + esh): the products carry 2^(-2 nb), the orders' unit is
         // 2^(2 w (NS-1) - w (NO-1)).  The mixed form's sums fit 64 bits with a fixed shift; the plain form's take the
-        // shift esh that the unit's own sums allow (xs_order_shift), one for the warp's columns
+        // shift esh that each sum itself allows (xs_order_shift): a column's small sums would lose bits to a neighbour's
+        // large ones in a common shift
         constexpr int eo = (BAL ? xs_low<NS>() : ESH) + W * (2 * (NS - 1) - (NO - 1)) - 2 * nb;
-        long long T[2][CW];
-        int esh[2] = {0, 0};
+        auto value = [&](long long t, int E, int ea, int e) {   // E: the column's scale
+          return ea > -2000 && E > -2000 ? xs_i64_to_double(t, ea + E + e) : 0.0;
+        };
+        long long T[2][CW];            // order sums (forward, balanced: the results' bits)
+        uint32_t esh = 0;              // backward, balanced: the columns' shifts, four bits each
+        uint32_t small[2] = {0, 0};    // magnitude sums below the least, a bit a column
 #pragma unroll
         for (int par = 0; par < 2; ++par, ++u) {
           const uint32_t tb = u % TB;
@@ -565,36 +624,50 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
               xs_tmem_ld<CW>(tcol, g);
               xs_tmem_ld<CW>(tcol + (uint32_t)N, h);
               tmem_wait_ld();
-              int mx = 0;
 #pragma unroll
               for (int c = 0; c < CW; ++c) {
                 const int C = xs_f2i(__uint_as_float(g[c])) * (1 << W) + xs_f2i(__uint_as_float(h[c]));
-                mx = max(mx, abs(C));
-                g[c] = (uint32_t)C;
+                int es = xs_order_shift<NS>(abs(C));
+                if (MODE == 1 && par == 1) {   // the two parities are added: the same shift for both
+                  const int e0 = (int)(esh >> (4 * c)) & 15;
+                  es = max(es, e0);
+                  T[0][c] >>= es - e0;
+                  esh = (esh & ~(15u << (4 * c))) | ((uint32_t)es << (4 * c));
+                } else if (MODE == 1) {
+                  esh |= (uint32_t)es << (4 * c);
+                }
+                const long long t = ((long long)C << (xs_cb<NS>() - es)) + (T[par][c] >> es);
+                T[par][c] = MODE == 0 ? __double_as_longlong(value(t, cx[c], EA[par], es + eo)) : t;
               }
-              const int es = xs_order_shift<NS>(mx);
-              esh[par] = es;
+              if constexpr (MAG) {
+                xs_tmem_ld<CW>(tcol + (uint32_t)(NO * N), g);
+                tmem_wait_ld();
 #pragma unroll
-              for (int c = 0; c < CW; ++c) T[par][c] = ((long long)(int)g[c] << (xs_cb<NS>() - es)) + (T[par][c] >> es);
+                for (int c = 0; c < CW; ++c) small[par] |= __uint_as_float(g[c]) < a.least ? 1u << c : 0u;
+              }
             }
           }
           tc_fence_before();
           mbar_arrive(&bar_te[tb]);
         }
         if (!ok) break;
-        // the item's column scales: written before its digits were cut, and so before its accumulators were complete
-        const int* cx = colexp + (ii % XS_CXS) * N + cg * CW;
-        if (!xs_wait_w(&bar_cx[ii % XS_CXS], (ii / XS_CXS) & 1, ok)) break;
-        if (MODE == 0 ? row < nrows : row < a.nrh) {
-          if (MODE == 1 && BAL) {   // the two parities are added: the same shift for both
-            const int es = max(esh[0], esh[1]);
+        if (MAG && live) {
+          // the outputs whose terms are all small beside their row's and column's largest entries, for k_xs_again
 #pragma unroll
-            for (int c = 0; c < CW; ++c) {
-              T[0][c] >>= es - esh[0];
-              T[1][c] >>= es - esh[1];
+          for (int par = 0; par < (MODE == 0 ? 2 : 1); ++par) {
+            const uint32_t sm = MODE == 0 ? small[par] : small[0] & small[1];
+            const bool rok = MODE == 0 ? 2 * row + par < nn : row < a.nrh;
+#pragma unroll
+            for (int c = 0; c < CW; c += 2) {
+              const int zo = z0 + ((cg * CW + c) >> 1);
+              if (zo >= a.nzdim) continue;
+              const bool few = EA[par] > -2000 && (((sm >> c) & 1 && cx[c] > -2000) || ((sm >> (c + 1)) & 1 && cx[c + 1] > -2000));
+              const unsigned word = __ballot_sync(0xFFFFFFFFu, rok && few);
+              if (lane == 0) a.again[xs_word(a, MODE, item_f(item), m, par, mt * 4 + lq, zo)] = word;
             }
-            esh[0] = es;
           }
+        }
+        if (MODE == 0 ? row < nrows : row < a.nrh) {
           // the log term is added at m = 0 only: an integer test per item, so that the other items
           // issue no FP64 compares or (predicated) FP64 additions on GB300's narrow FP64 pipe
           const bool ln_here = MODE == 1 && a.add_ln && m == 0;
@@ -602,27 +675,22 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
           for (int c = 0; c < CW; c += 2) {
             const int zo = z0 + ((cg * CW + c) >> 1);
             if (zo >= a.nzdim) continue;
-            const int E0 = cx[c], E1 = cx[c + 1];
             double2* o = fout + (size_t)a.nrdim * (m + (size_t)a.npdim * zo);
             if (MODE == 0) {
 #pragma unroll
               for (int par = 0; par < 2; ++par) {
                 if (2 * row + par >= nn) continue;
-                const int e = EA[par] + esh[par] + eo;
-                const double re = EA[par] > -2000 && E0 > -2000 ? xs_i64_to_double(T[par][c], e + E0) : 0.0;
-                const double im = EA[par] > -2000 && E1 > -2000 ? xs_i64_to_double(T[par][c + 1], e + E1) : 0.0;
-                o[2 * row + par] = make_double2(re, im);
+                o[2 * row + par] = BAL ? make_double2(__longlong_as_double(T[par][c]), __longlong_as_double(T[par][c + 1]))
+                                       : make_double2(value(T[par][c], cx[c], EA[par], eo), value(T[par][c + 1], cx[c + 1], EA[par], eo));
               }
             } else {
-              double v[4] = {0.0, 0.0, 0.0, 0.0};   // f(i) re, im; f(nr-1-i) re, im
+              double v[4];   // f(i) re, im; f(nr-1-i) re, im
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
-                const int E = h ? E1 : E0;
-                if (EA[0] > -2000 && E > -2000) {
-                  // f(i) = D_0 + D_1, f(nr-1-i) = D_0 - D_1: both parities share the scales
-                  v[h] = xs_i64_to_double(T[0][c + h] + T[1][c + h], EA[0] + E + esh[0] + eo);
-                  v[2 + h] = xs_i64_to_double(T[0][c + h] - T[1][c + h], EA[0] + E + esh[0] + eo);
-                }
+                // f(i) = D_0 + D_1, f(nr-1-i) = D_0 - D_1: both parities share the scales
+                const int e = eo + ((int)(esh >> (4 * (c + h))) & 15);
+                v[h] = value(T[0][c + h] + T[1][c + h], cx[c + h], EA[0], e);
+                v[2 + h] = value(T[0][c + h] - T[1][c + h], cx[c + h], EA[0], e);
               }
               if (ln_here) {
                 const double lnv = *xs_sel(a.lnp, item_f(item));
@@ -645,21 +713,101 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
 }
 
 // ------------------------------------------------------------------------------------------------
+// The marked outputs of the nine-digit form, summed in FP64 (as the FP64 kernels of radial.cu sum, term after term, backward).
+// Few and scattered, or whole regions (the points near the axis where the functions of high m vanish), so each warp takes words
+// from all over the grid.  Backward: a lane per row of the word, the table read along the rows.  Forward: a marked row after the
+// other, the lanes over the radial points.  Nothing marked: 4 us.
+template <int MODE>
+__global__ void __launch_bounds__(256) k_xs_again(XsArgs a, const double* __restrict__ pf, const double* __restrict__ w, int ne,
+                                                  size_t nwords) {
+  const int lane = threadIdx.x & 31;
+  const size_t nw = (size_t)gridDim.x * (blockDim.x >> 5), wid = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  int f, m, par, g, z;
+  auto place = [&](size_t idx) {
+    z = (int)(idx % a.nzdim); idx /= a.nzdim;
+    g = (int)(idx % a.ngrp); idx /= a.ngrp;
+    if (MODE == 0) { par = (int)(idx & 1); idx >>= 1; } else par = 0;
+    m = (int)(idx % a.npc);
+    f = (int)(idx / a.npc);
+  };
+  for (size_t base = wid; base < nwords; base += 32 * nw) {
+    const size_t mine = base + nw * lane;
+    unsigned word = 0;
+    if (mine < nwords) {
+      place(mine);
+      const int nn = max(min(a.nrc, a.nrc - m), 0);
+      if (m >= a.m0 && nn > 0 && g * 32 < (MODE == 0 ? (nn + 1) / 2 : a.nrh)) word = a.again[mine];   // (others are not written)
+    }
+    for (unsigned todo = __ballot_sync(0xFFFFFFFFu, word != 0); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const unsigned rows = __shfl_sync(0xFFFFFFFFu, word, src);
+      place(base + nw * src);
+      const int nn = max(min(a.nrc, a.nrc - m), 0);
+      const size_t off = (size_t)a.nrdim * (m + (size_t)a.npdim * z);
+      const double2* in = xs_sel(a.in, f) + off;
+      double2* out = xs_sel(a.out, f) + off;
+      const double* tab = pf + (size_t)a.nrh * ne * m;
+      if (MODE == 1) {
+        const int i = min(g * 32 + lane, a.nrh - 1);
+        double er = 0.0, ei = 0.0, dr = 0.0, di = 0.0;
+#pragma unroll 4
+        for (int j = 0; j + 1 < nn; j += 2) {
+          const double ve = __ldg(tab + i + (size_t)a.nrh * j), vo = __ldg(tab + i + (size_t)a.nrh * (j + 1));
+          const double2 ce = __ldg(in + j), co = __ldg(in + j + 1);
+          er = fma(ve, ce.x, er); ei = fma(ve, ce.y, ei);
+          dr = fma(vo, co.x, dr); di = fma(vo, co.y, di);
+        }
+        if (nn & 1) {
+          const double ve = __ldg(tab + i + (size_t)a.nrh * (nn - 1));
+          const double2 ce = __ldg(in + nn - 1);
+          er = fma(ve, ce.x, er); ei = fma(ve, ce.y, ei);
+        }
+        if ((rows >> lane) & 1) {
+          out[i] = make_double2(er + dr, ei + di);
+          out[a.nr - 1 - i] = make_double2(er - dr, ei - di);
+        }
+      } else {
+        const double sgn = par ? -1.0 : 1.0;
+        for (unsigned left = rows; left; left &= left - 1) {
+          const int j = 2 * (g * 32 + __ffs(left) - 1) + par;
+          double re = 0.0, im = 0.0;
+          for (int i = lane; i < a.nrh; i += 32) {
+            const double v = __ldg(tab + i + (size_t)a.nrh * j), wi = __ldg(w + i);
+            const double2 p = __ldg(in + i), q = __ldg(in + a.nr - 1 - i);
+            re = fma(v, (p.x + sgn * q.x) * wi, re);
+            im = fma(v, (p.y + sgn * q.y) * wi, im);
+          }
+#pragma unroll
+          for (int o = 16; o; o >>= 1) {
+            re += __shfl_xor_sync(0xFFFFFFFFu, re, o);
+            im += __shfl_xor_sync(0xFFFFFFFFu, im, o);
+          }
+          if (lane == 0) out[j] = make_double2(re, im);
+        }
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
 struct XsImg {
   uint16_t* p = nullptr;
   int* aexp = nullptr;
-  size_t bytes = 0, abytes = 0;
+  unsigned* again = nullptr;
+  size_t bytes = 0, abytes = 0, gbytes = 0;
   int nrc = -1, npc = -1, ns = 0, nmt = 0, nkc = 0, nrp = 0;
 };
 static XsImg g_xs[2][2];   // [mode][plain/mixed]
+static void xs_drop(XsImg& t) {
+  if (t.p) dfree(t.p, t.bytes);
+  if (t.aexp) dfree(t.aexp, t.abytes);
+  if (t.again) dfree(t.again, t.gbytes);
+  t = XsImg();
+}
 
 void xs_free() {
   for (auto& r : g_xs)
-    for (auto& t : r) {
-      if (t.p) dfree(t.p, t.bytes);
-      if (t.aexp) dfree(t.aexp, t.abytes);
-      t = XsImg();
-    }
+    for (auto& t : r) xs_drop(t);
 }
 
 // the digit configuration: FP64-grade (plain: 63 bits) or the mixed form's 42 bits, with the widest digits whose
@@ -671,17 +819,14 @@ void xs_free() {
 // needs more than 53 bits: the rounding is relative to the column maximum, and the nonlinear term's
 // curl cancellation magnifies what that loses on small entries (at 192 x 128 x 128 the vortex step's
 // nonlinear term differed from the FP64 reference by 5e-10 with 49-bit and 2.4e-11 with 56-bit digits).
-// The plain form takes balanced digits, eight (K <= 113) or nine.  Between 114 and 142 terms on grids of up to 284 points
-// it keeps ten unsigned digits of 6 bits with a fixed 64-bit shift, as it always had there: its sums are cut at 2^-52 of
-// max|A| max|B|, and the inverse Laplacian of the projection's (0, 0) column magnifies that cut to 4e-8 of single
-// coefficients of the nonlinear term, so that other digits would visibly move the results of a kit of 256 points.
+// On grids of up to 284 points it takes eight balanced digits up to 113 terms and ten unsigned ones of 6 bits, with a fixed
+// 64-bit shift that cuts the sums at 2^-52 of max|A| max|B|, beyond; on larger grids nine balanced digits with magnitude sums.
 // returns the digit count (its width is xs_w's), 0 where no configuration is exact
 static int xs_rawk(int nrc) { return std::max(G.nr, nrc) | 1; }   // odd: the staged columns start in different banks
 static int xs_cfg(int kmax, int nrc, bool plain) {
   const double lim = 16777216.0;
   if (plain) {
-    if (kmax <= 113) return 8;                         // 8 128 128 K <= 2^24 up to 128
-    if (kmax <= 142 && xs_rawk(nrc) <= 285) return 10;
+    if (xs_rawk(nrc) <= 285) return kmax <= 113 ? 8 : 10;   // 8 128 128 K <= 2^24 up to 128
     if (11.0 * kmax * 64 * 64 <= lim) return 9;        // order 8: seven pairs of 64 x 64 and two of 64 x 128
   } else {
     if (6.0 * kmax * 128 * 128 < lim) return 6;
@@ -690,9 +835,9 @@ static int xs_cfg(int kmax, int nrc, bool plain) {
   return 0;
 }
 
-static size_t xs_smem(int ns, int nz, int rawk, int aent, int bst, int nraw) {
+static size_t xs_smem(int ns, int nz, int rawk, int aent, int bst, int nraw, int sent) {
   const int n = 2 * nz;
-  return 1024 + aent * (size_t)(ns * XS_ATILE) + bst * (size_t)(ns * n * XS_KC * 2) +
+  return 1024 + aent * (size_t)(ns * XS_ATILE) + sent * (size_t)XS_ATILE + bst * (size_t)((ns + (sent > 0)) * n * XS_KC * 2) +
          nraw * (size_t)2 * nz * rawk * sizeof(double) + XS_CXS * n * sizeof(int) + 512;
 }
 constexpr size_t XS_SMEM_MAX = 227 * 1024;
@@ -702,15 +847,16 @@ constexpr size_t XS_SMEM_MAX = 227 * 1024;
 // digits: 19.1 ms for two steps' backward transforms with 8 columns, 13.8 ms with 16).  Two column buffers where they fit
 // (up to 256 points), so that an item's columns land and are scanned while the one before is cut; then digit stages, at
 // most four (six measured the same), and table entries in what is left.
-struct XsPlan { int nz, aent, bst, nraw; };
+struct XsPlan { int nz, aent, bst, nraw, sent; };
 // `few`: no more items than half the SMs; halved, they take less time each (24 x 20 x 12, plain: 17.1 and 21.1 us forward and
 // backward with 16 columns, 14.9 and 17.2 with 8).
 static bool xs_plan(int ns, int rawk, XsPlan& p, bool few = false) {
   for (int nz = G.nzdim > 8 && !few ? 16 : 8; nz >= 8; nz /= 2)
     for (int nraw = 2; nraw >= 1; --nraw)
       for (int sb = XS_SBMAX; sb >= 2; --sb)
-        for (int ae = XS_AEMAX; ae >= 2; --ae)
-          if (xs_smem(ns, nz, rawk, ae, sb, nraw) <= XS_SMEM_MAX) { p = {nz, ae, sb, nraw}; return true; }
+        for (int me = ns == 9 ? XS_MEMAX : 0; me >= (ns == 9 ? 1 : 0); --me)
+          for (int ae = XS_AEMAX; ae >= 2; --ae)
+            if (xs_smem(ns, nz, rawk, ae, sb, nraw, me) <= XS_SMEM_MAX) { p = {nz, ae, sb, nraw, me}; return true; }
   return false;
 }
 // whether the exact-slice contraction covers this kit: the orders stay exact and the rings fit
@@ -720,14 +866,19 @@ bool xs_supported(int mode, int nrc, bool plain) {
   return ns > 0 && xs_plan(ns, xs_rawk(nrc), p);
 }
 
+static size_t xs_words(int mode, int nf, int npc, int ngrp) { return (size_t)nf * npc * (mode == 0 ? 2 : 1) * ngrp * G.nzdim; }
 template <int MODE, int NS, int NZ>
 static int xs_launch(const XsArgs& args, int nitems) {
-  const size_t sm = xs_smem(NS, NZ, args.rawk, args.aent, args.bst, args.nraw);
+  const size_t sm = xs_smem(NS, NZ, args.rawk, args.aent, args.bst, args.nraw, args.sent);
   if (sm > XS_SMEM_MAX) return set_error(MLG_ESIZE, "radial contraction: shared-memory stage too large");
   auto kern = k_xs_rtrans<MODE, NS, NZ>;
   MLG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   kern<<<std::min(nitems, 152), XS_THREADS, sm, G.stream>>>(args);
   MLG_LAUNCH();
+  if constexpr (xs_mag<NS>() != 0) {
+    k_xs_again<MODE><<<152 * 4, 256, 0, G.stream>>>(args, G.pf, G.w, G.ne, xs_words(MODE, args.nf, args.npc, args.ngrp));
+    MLG_LAUNCH();
+  }
   return 0;
 }
 
@@ -745,13 +896,15 @@ int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int n
   const int nmt = cdiv(nrows, 128), nkc = cdiv(kmax, XS_KC), nrp = nmt * 128;
   XsImg& im = g_xs[mode][plain ? 0 : 1];
   if (im.nrc != nrc || im.npc != npc || !im.p || im.ns != ns) {
-    if (im.p) dfree(im.p, im.bytes);
-    if (im.aexp) dfree(im.aexp, im.abytes);
-    im = XsImg();
-    im.bytes = (size_t)npc * nmt * nkc * 2 * ns * XS_ATILE;
+    xs_drop(im);
+    im.bytes = (size_t)npc * nmt * nkc * 2 * (ns + (ns == 9)) * XS_ATILE;
     im.abytes = (size_t)npc * (mode == 0 ? 2 : 1) * nrp * sizeof(int);
     MLG_TRY(dmalloc((void**)&im.p, im.bytes));
     MLG_TRY(dmalloc((void**)&im.aexp, im.abytes));
+    if (ns == 9) {
+      im.gbytes = xs_words(mode, XS_NF, npc, cdiv(nrows, 32)) * sizeof(unsigned);
+      MLG_TRY(dmalloc((void**)&im.again, im.gbytes));
+    }
     k_xs_aexp<<<dim3(cdiv(nrp, 128), npc), 128, 0, G.stream>>>(G.pf, G.w, im.aexp, mode, G.nrh, G.ne, nrc, nrp, kmax,
                                                                    ns == 8 || ns == 9 ? 1 : 0);
     MLG_LAUNCH();
@@ -780,6 +933,8 @@ int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int n
   args.aent = plan.aent;
   args.bst = plan.bst;
   args.nraw = plan.nraw;
+  args.sent = plan.sent;
+  args.again = im.again; args.ngrp = cdiv(nrows, 32); args.least = xs_least_sum(kmax);
   const bool nz16 = plan.nz == 16;
   const int nitems = (npc - m0) * cdiv(G.nzdim, plan.nz) * nf;
 #define XS_CASE(NSV)                                                                                   \
