@@ -99,8 +99,12 @@ __global__ void k_xv_rexp(const double* __restrict__ tV, const double* __restric
 // digit configurations: the plain form's nine balanced digits, else two's complement
 template <int NS> __host__ __device__ constexpr bool xv_bal() { return NS == 9; }
 template <int NS, int W> __host__ __device__ constexpr int xv_nb(int n) { return xv_bal<NS>() ? 63 : W * n; }
+// the plain form's digits carry a magnitude tile beside them (xs_least_sum)
+template <int NS> __host__ __device__ constexpr int xv_mag() { return xv_bal<NS>() ? 1 : 0; }
+// tiles of a chunk's three table entries
+template <int NS, int NT> __host__ __device__ constexpr int xv_tiles() { return 2 * NS + NT + 3 * xv_mag<NS>(); }
 
-// tiles per (m, par, row tile mt, chunk kc): [m V digits NS | D digits NS | T digits NT]
+// tiles per (m, par, row tile mt, chunk kc): [m V digits NS | D digits NS | T digits NT], each with its magnitude tile behind it
 template <int NS, int NT, int W>
 __global__ void k_xv_table(const double* __restrict__ tV, const double* __restrict__ tD, const double* __restrict__ tT,
                            const int* __restrict__ rexp, const int* __restrict__ texp, uint16_t* __restrict__ img,
@@ -110,7 +114,8 @@ __global__ void k_xv_table(const double* __restrict__ tV, const double* __restri
   const int kc = (int)(blk % nkc), mt = (int)((blk / nkc) % nmt), mp = (int)(blk / ((size_t)nkc * nmt));
   const int m = mp >> 1, par = mp & 1;
   const int nn = max(min(nrc, nrc - m), 0);
-  uint8_t* base = (uint8_t*)img + blk * (size_t)((2 * NS + NT) * XV_ATILE);
+  constexpr int MG = xv_mag<NS>();
+  uint8_t* base = (uint8_t*)img + blk * (size_t)(xv_tiles<NS, NT>() * XV_ATILE);
   for (int idx = threadIdx.x; idx < 128 * XV_KC; idx += blockDim.x) {
     const int k = idx % XV_KC, r = idx / XV_KC;
     const int t = mt * 128 + r, j = 2 * t + par, i = kc * XV_KC + k;
@@ -123,18 +128,22 @@ __global__ void k_xv_table(const double* __restrict__ tV, const double* __restri
     }
     const int off = xv_off(r, k);
     constexpr unsigned long long bs = BAL ? xs_bias<NS, W>() : 0ull, bt = BAL ? xs_bias<NT, W>() : 0ull;
-    const unsigned long long xv = (unsigned long long)xs_fix(v, er, xv_nb<NS, W>(NS)) + bs;
-    const unsigned long long xd = (unsigned long long)xs_fix(d, er, xv_nb<NS, W>(NS)) + bs;
-    const unsigned long long xt = (unsigned long long)xs_fix(tt, et, xv_nb<NS, W>(NT)) + bt;
+    const long long iv = xs_fix(v, er, xv_nb<NS, W>(NS)), id = xs_fix(d, er, xv_nb<NS, W>(NS)), it = xs_fix(tt, et, xv_nb<NS, W>(NT));
+    const unsigned long long xv = (unsigned long long)iv + bs, xd = (unsigned long long)id + bs, xt = (unsigned long long)it + bt;
     xs_static_for<NS>([&](auto sc) {
       constexpr int q = decltype(sc)::value;
       *(uint16_t*)(base + q * XV_ATILE + off) = (uint16_t)xs_digit2<NS, W, BAL, q>(xv, xv);
-      *(uint16_t*)(base + (NS + q) * XV_ATILE + off) = (uint16_t)xs_digit2<NS, W, BAL, q>(xd, xd);
+      *(uint16_t*)(base + (NS + MG + q) * XV_ATILE + off) = (uint16_t)xs_digit2<NS, W, BAL, q>(xd, xd);
     });
     xs_static_for<NT>([&](auto sc) {
       constexpr int q = decltype(sc)::value;
-      *(uint16_t*)(base + (2 * NS + q) * XV_ATILE + off) = (uint16_t)xs_digit2<NT, W, BAL, q>(xt, xt);
+      *(uint16_t*)(base + (2 * (NS + MG) + q) * XV_ATILE + off) = (uint16_t)xs_digit2<NT, W, BAL, q>(xt, xt);
     });
+    if (MG) {
+      *(uint16_t*)(base + NS * XV_ATILE + off) = (uint16_t)xs_mag2(iv, iv);
+      *(uint16_t*)(base + (2 * NS + 1) * XV_ATILE + off) = (uint16_t)xs_mag2(id, id);
+      *(uint16_t*)(base + (2 * (NS + 1) + NT) * XV_ATILE + off) = (uint16_t)xs_mag2(it, it);
+    }
   }
 }
 
@@ -148,8 +157,16 @@ struct XvArgs {
   int* status;
   int nr, nrh, nrdim, npdim, nzdim, nrc, nzc, nzcu, nmt, nkc, ntr, m0, npc;
   int aent;           // table entries of the ring
+  unsigned* again;    // plain form: the outputs to be summed again, a word of 32 rows (xv_word)
+  int ngrp;
+  float least;        // xs_least_sum
   int esh_s, esh_t;   // two's complement digits: right shifts that keep the 64-bit order sums of psi / X and of Y below 2^62
 };
+
+// the word of the rows t = 32 g .. 32 g + 31 of parity par of column (m, z)
+__device__ __forceinline__ size_t xv_word(const XvArgs& a, int m, int par, int g, int z) {
+  return (((size_t)m * 2 + par) * a.ngrp + g) * a.nzdim + z;
+}
 
 constexpr int XV_NZ = 8, XV_N = 2 * XV_NZ;   // complex z columns per item, real columns
 constexpr int XV_NSW = 2, XV_GW = 6, XV_NEW = 8;   // scale warps, warps of a digit group (two groups), epilogue warps
@@ -157,69 +174,70 @@ constexpr int XV_THREADS = (2 + XV_NSW + 2 * XV_GW + XV_NEW) * 32;
 constexpr int XV_CXS = 4, XV_AEMAX = 6, XV_SB = 2;   // column-scale slots, table entries (at most), digit stages
 constexpr int XV_BTILE = XV_N * XV_KC * 2;
 static_assert(3 * XV_NZ * 8 == XV_GW * 32, "one staging item per digit thread");
-__host__ __device__ constexpr int xv_aent_bytes(int ns, int nt) { return (ns > nt ? ns : nt) * XV_ATILE; }
-__host__ __device__ constexpr int xv_bstage_bytes(int ns, int nt) { return (4 * ns + nt) * XV_BTILE; }
+template <int NS, int NT> __host__ __device__ constexpr int xv_aent_bytes() { return ((NS > NT ? NS : NT) + xv_mag<NS>()) * XV_ATILE; }
+template <int NS, int NT> __host__ __device__ constexpr int xv_bstage_bytes() { return (4 * NS + NT + 5 * xv_mag<NS>()) * XV_BTILE; }
 
-// order sums of eight columns: T[c] = sum_d G_d 2^(w (n-1-d)) (shifted; see xs_radial.cu), order d at tcol + d step;
-// returns the shift of a balanced sum
-template <int NO, int W, bool BAL> __device__ __forceinline__ int xv_sums(uint32_t tcol, uint32_t step, int esh, long long* T) {
-  if constexpr (!BAL) {
+// order sums of eight columns, two's complement digits: T[c] = sum_d G_d 2^(w (n-1-d) - esh), order d at tcol + d step
+template <int NO, int W> __device__ __forceinline__ void xv_sums(uint32_t tcol, uint32_t step, int esh, long long* T) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) T[c] = 0;
-    xs_static_for<(NO + 1) / 2>([&](auto dc) {
-      constexpr int D = 2 * decltype(dc)::value, D2 = D + 1 < NO ? D + 1 : D;
-      uint32_t g[8], h[8];
-      tmem_ld8_nw(tcol + D * step, g);
-      if constexpr (D2 != D) tmem_ld8_nw(tcol + D2 * step, h);
-      tmem_wait_ld();
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        T[c] += xs_shl((long long)xs_f2i(__uint_as_float(g[c])), W * (NO - 1 - D) - esh);
-        if constexpr (D2 != D) T[c] += xs_shl((long long)xs_f2i(__uint_as_float(h[c])), W * (NO - 1 - D2) - esh);
-      }
-    });
-    return esh;
-  } else {
-    // L = sum_{d>=2} G_d 2^(w (NO-1-d) - 3): |G_2| <= 2 K (2^(2w-2) + 2 2^(w+6)) with K <= 372, so |L| < 2^62.9 and
-    // |L| 2^-cb < 2^17; then C = G_0 2^w + G_1 (|C| < 2^31) and T = C 2^(cb - es) + (L >> es) below 2^62
-    constexpr int LOW = 3, CB = W * (NO - 2) - LOW;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) T[c] = 0;
-    auto acc = [&](auto dc, uint32_t g, int c) {
-      constexpr int SH = W * (NO - 1 - decltype(dc)::value) - LOW;
-      const int v = xs_f2i(__uint_as_float(g));
-      if constexpr (SH > 30) T[c] += (long long)v << SH;
-      else if constexpr (SH >= 0) T[c] += (long long)v * (long long)(1 << SH);
-      else T[c] += (long long)(v >> -SH);
-    };
-    xs_static_for<(NO - 1) / 2>([&](auto dc) {
-      constexpr int D = 2 * decltype(dc)::value + 2, D2 = D + 1 < NO ? D + 1 : D;
-      uint32_t g[8], h[8];
-      tmem_ld8_nw(tcol + D * step, g);
-      if constexpr (D2 != D) tmem_ld8_nw(tcol + D2 * step, h);
-      tmem_wait_ld();
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        acc(std::integral_constant<int, D>(), g[c], c);
-        if constexpr (D2 != D) acc(std::integral_constant<int, D2>(), h[c], c);
-      }
-    });
+  for (int c = 0; c < 8; ++c) T[c] = 0;
+  xs_static_for<(NO + 1) / 2>([&](auto dc) {
+    constexpr int D = 2 * decltype(dc)::value, D2 = D + 1 < NO ? D + 1 : D;
     uint32_t g[8], h[8];
-    tmem_ld8_nw(tcol, g);
-    tmem_ld8_nw(tcol + step, h);
+    tmem_ld8_nw(tcol + D * step, g);
+    if constexpr (D2 != D) tmem_ld8_nw(tcol + D2 * step, h);
     tmem_wait_ld();
-    int mx = 0;
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const int C = xs_f2i(__uint_as_float(g[c])) * (1 << W) + xs_f2i(__uint_as_float(h[c]));
-      mx = max(mx, abs(C));
-      g[c] = (uint32_t)C;
+      T[c] += xs_shl((long long)xs_f2i(__uint_as_float(g[c])), W * (NO - 1 - D) - esh);
+      if constexpr (D2 != D) T[c] += xs_shl((long long)xs_f2i(__uint_as_float(h[c])), W * (NO - 1 - D2) - esh);
     }
-    const int es = max(32 - __clz(mx + 131072) + CB - 62, 0);
+  });
+}
+// Balanced digits (xs_radial.cu): L = sum_{d>=2} G_d 2^(w (NO-1-d) - 3) and C = G_0 2^w + G_1; with K <= 372 and two products
+// |G_2| <= 2 K (2^(2w-2) + 2 2^(w+6)), so |L| < 2^62.9, |L| 2^-cb < 2^17 and |C| < 2^31.  mag: the magnitude sums' columns.
+constexpr int XV_LOW = 3;
+template <int NO, int W> constexpr int xv_cb() { return W * (NO - 2) - XV_LOW; }
+struct XvSum { long long L[8]; int C[8]; float S[8]; };
+template <int NO, int W> __device__ __forceinline__ void xv_drain(uint32_t tcol, uint32_t step, uint32_t mag, XvSum& q, bool first) {
+  if (first) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) T[c] = ((long long)(int)g[c] << (CB - es)) + (T[c] >> es);
-    return es + LOW;
+    for (int c = 0; c < 8; ++c) { q.L[c] = 0; q.C[c] = 0; q.S[c] = 0.f; }
   }
+  auto acc = [&](auto dc, uint32_t g, int c) {
+    constexpr int SH = W * (NO - 1 - decltype(dc)::value) - XV_LOW;
+    const int v = xs_f2i(__uint_as_float(g));
+    if constexpr (SH > 30) q.L[c] += (long long)v << SH;
+    else if constexpr (SH >= 0) q.L[c] += (long long)v * (long long)(1 << SH);
+    else q.L[c] += (long long)(v >> -SH);
+  };
+  xs_static_for<(NO - 1) / 2>([&](auto dc) {
+    constexpr int D = 2 * decltype(dc)::value + 2, D2 = D + 1 < NO ? D + 1 : D;
+    uint32_t g[8], h[8];
+    tmem_ld8_nw(tcol + D * step, g);
+    if constexpr (D2 != D) tmem_ld8_nw(tcol + D2 * step, h);
+    tmem_wait_ld();
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      acc(std::integral_constant<int, D>(), g[c], c);
+      if constexpr (D2 != D) acc(std::integral_constant<int, D2>(), h[c], c);
+    }
+  });
+  uint32_t g[8], h[8];
+  tmem_ld8_nw(tcol, g);
+  tmem_ld8_nw(tcol + step, h);
+  tmem_wait_ld();
+#pragma unroll
+  for (int c = 0; c < 8; ++c) q.C[c] += xs_f2i(__uint_as_float(g[c])) * (1 << W) + xs_f2i(__uint_as_float(h[c]));
+  tmem_ld8_nw(mag, g);
+  tmem_wait_ld();
+#pragma unroll
+  for (int c = 0; c < 8; ++c) q.S[c] += __uint_as_float(g[c]);
+}
+// column c's sum in FP64, times 2^e: T = C 2^(cb - es) + (L >> es) below 2^62, es the shift that this sum needs
+template <int NO, int W> __device__ __forceinline__ double xv_value(const XvSum& q, int c, int e) {
+  const int es = max(32 - __clz(abs(q.C[c]) + 131072) + xv_cb<NO, W>() - 62, 0);
+  return xs_i64_to_double(((long long)q.C[c] << (xv_cb<NO, W>() - es)) + (q.L[c] >> es), e + es + XV_LOW);
 }
 
 template <int NS, int NT, int W>
@@ -227,10 +245,12 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
   constexpr bool BAL = xv_bal<NS>();
   constexpr int NZ = XV_NZ, N = XV_N;
   constexpr int nbs = xv_nb<NS, W>(NS), nbt = xv_nb<NS, W>(NT);
-  constexpr int AENT = xv_aent_bytes(NS, NT), BSTAGE = xv_bstage_bytes(NS, NT);
-  constexpr int COLS = (2 * NS + NT) * N;
+  constexpr int MG = xv_mag<NS>();
+  constexpr int AENT = xv_aent_bytes<NS, NT>(), BSTAGE = xv_bstage_bytes<NS, NT>();
+  constexpr int COLS = xv_tiles<NS, NT>() * N;
   constexpr int TCOLS = COLS <= 256 ? 256 : 512;
   constexpr uint32_t TY = 2 * NS * N;             // Y's accumulators, after psi's and X's
+  constexpr uint32_t TM = TY + NT * N;            // the magnitude sums of psi, X and Y
   static_assert(COLS <= 512, "accumulators exceed tensor memory");
   extern __shared__ __align__(1024) uint8_t xv_smem_raw[];
   uint8_t* sbase = (uint8_t*)(((uintptr_t)xv_smem_raw + 1023) & ~(uintptr_t)1023);
@@ -303,11 +323,11 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       uint32_t c = 0, s = 0, ph = 0;
       for (int it = first; it < nitems && ok; it = next_item(it)) {
         const uint8_t* img = (const uint8_t*)a.img +
-                             (((size_t)(item_m(it) * 2 + item_par(it)) * a.nmt + item_mt(it)) * nkc) * (size_t)((2 * NS + NT) * XV_ATILE);
+                             (((size_t)(item_m(it) * 2 + item_par(it)) * a.nmt + item_mt(it)) * nkc) * (size_t)(xv_tiles<NS, NT>() * XV_ATILE);
         for (int kc = 0; kc < nkc && ok; ++kc)
           for (int q = 0; q < 3; ++q, ++c) {
             if (c >= AE && !xs_wait(&bar_ae[s], ph ^ 1u, ok)) break;
-            const uint32_t bytes = (uint32_t)(q < 2 ? NS : NT) * XV_ATILE;
+            const uint32_t bytes = (uint32_t)((q < 2 ? NS : NT) + MG) * XV_ATILE;
             mbar_expect_tx(&bar_af[s], bytes);
             bulk_g2s(sA + s * AENT, img, bytes, &bar_af[s]);
             img += bytes;
@@ -327,8 +347,8 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
     uint32_t sa = 0, pa = 0, sb = 0, pb = 0, u = 0, last = 0, plast = 0;
     bool any = false;
     // the MMAs of one table entry: digit t against the B tiles [b, b + (n - t) cols), cols tiles per digit, onto the
-    // accumulators from tc on
-    auto entry = [&](auto nc, auto colsc, uint32_t b, uint32_t tc, bool add) {
+    // accumulators from tc on; then the magnitudes, against the tiles at bm onto tm
+    auto entry = [&](auto nc, auto colsc, uint32_t b, uint32_t tc, uint32_t bm, uint32_t tm, bool add) {
       constexpr int n = decltype(nc)::value, cols = decltype(colsc)::value;
       if (!xs_wait_w(&bar_af[sa], pa, ok)) return;
       tc_fence_after();
@@ -343,6 +363,8 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
           umma_bf16(tmem + tc + (uint32_t)((t * cols + t1) * N), ad, sdesc(b + t1 * XV_BTILE, XV_LBO, XV_SBO),
                     idesc_bf16(128, (tiles - t1) * N), (add || t > 0) ? 1u : 0u, el);
       }
+      if constexpr (MG != 0)
+        umma_bf16(tmem + tm, sdesc(a0 + n * XV_ATILE, XV_LBO, XV_SBO), sdesc(bm, XV_LBO, XV_SBO), idesc_bf16(128, cols * N), add ? 1u : 0u, el);
       umma_commit(&bar_ae[sa], el);
       last = sa; plast = pa; any = true;
       if (++sa == AE) { sa = 0; pa ^= 1u; }
@@ -352,13 +374,13 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       if (u > 0 && !xs_wait_w(&bar_te[0], (u - 1) & 1, ok)) break;
       for (int kc = 0; kc < nkc && ok; ++kc) {
         if (!xs_wait_w(&bar_bf[sb], pb, ok)) break;
-        const uint32_t b0 = smem_u32(sB) + sb * BSTAGE;
+        const uint32_t b0 = smem_u32(sB) + sb * BSTAGE, bm = b0 + (4 * NS + NT) * XV_BTILE;
         // psi and X alternate by order (psi_d at 2d N, X_d at (2d+1) N) and their field digits alternate the same way
         // ([psi_ur_s, X_up_s] against m V, [psi_up_s, X_ur_s] against D), so one MMA covers both sums
-        entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, kc > 0);
-        if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, true);
+        entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, bm, TM, kc > 0);
+        if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, bm + 2 * XV_BTILE, TM, true);
         if (kc == 0 && u > 0) xs_wait_w(&bar_te[1], (u - 1) & 1, ok);
-        if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, kc > 0);
+        if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, bm + 4 * XV_BTILE, TM + 2 * N, kc > 0);
         if (!ok) break;
         umma_commit(&bar_be[sb], el);
         if (++sb == XV_SB) { sb = 0; pb ^= 1u; }
@@ -465,20 +487,22 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       if (f < 2) {
         // f = 0: psi_ur = -i F_s(ur) = (Im, -Re), X_ur = i F_o(ur) = (-Im, Re)
         // f = 1: psi_up = -F_o(up) = (-Re, -Im),  X_up = F_s(up) = (Re, Im)
-        // B tiles: [psi_ur_s, X_up_s] at 2s, 2s+1; [psi_up_s, X_ur_s] at 2 NS + 2s, 2 NS + 2s + 1
+        // B tiles: [psi_ur_s, X_up_s] at 2s, 2s+1; [psi_up_s, X_ur_s] at 2 NS + 2s, 2 NS + 2s + 1; their magnitudes in the same
+        // order behind all digits
         constexpr unsigned long long bias = BAL ? xs_bias<NS, W>() : 0ull;
-        const int tp = f == 0 ? 0 : 2 * NS, tx = f == 0 ? 2 * NS + 1 : 1;
-        auto put = [&](int tile, int o, long long p, long long q) {
+        const int tp = f == 0 ? 0 : 2 * NS, tx = f == 0 ? 2 * NS + 1 : 1, mp = f == 0 ? 0 : 2, mx = f == 0 ? 3 : 1;
+        auto put = [&](int tile, int mag, int o, long long p, long long q) {
+          if constexpr (MG != 0) *(uint32_t*)(bst + (4 * NS + NT + mag) * XV_BTILE + o) = xs_mag2(p, q);
           const unsigned long long x0 = (unsigned long long)p + bias, x1 = (unsigned long long)q + bias;
           xs_static_for<NS>([&](auto sc) {
             constexpr int g = decltype(sc)::value;
             *(uint32_t*)(bst + (tile + 2 * g) * XV_BTILE + o) = xs_digit2<NS, W, BAL, g>(x0, x1);
           });
         };
-        put(tp, off, f == 0 ? sim[0] : -ore[0], f == 0 ? sim[1] : -ore[1]);
-        put(tp, off1, f == 0 ? -sre[0] : -oim[0], f == 0 ? -sre[1] : -oim[1]);
-        put(tx, off, f == 0 ? -oim[0] : sre[0], f == 0 ? -oim[1] : sre[1]);
-        put(tx, off1, f == 0 ? ore[0] : sim[0], f == 0 ? ore[1] : sim[1]);
+        put(tp, mp, off, f == 0 ? sim[0] : -ore[0], f == 0 ? sim[1] : -ore[1]);
+        put(tp, mp, off1, f == 0 ? -sre[0] : -oim[0], f == 0 ? -sre[1] : -oim[1]);
+        put(tx, mx, off, f == 0 ? -oim[0] : sre[0], f == 0 ? -oim[1] : sre[1]);
+        put(tx, mx, off1, f == 0 ? ore[0] : sim[0], f == 0 ? ore[1] : sim[1]);
       } else {
         // Y: F_s(uz) with the uz column scales
         constexpr unsigned long long bias = BAL ? xs_bias<NT, W>() : 0ull;
@@ -489,6 +513,10 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
           *(uint32_t*)(bst + (4 * NS + g) * XV_BTILE + off1) =
               xs_digit2<NT, W, BAL, g>((unsigned long long)sim[0] + bias, (unsigned long long)sim[1] + bias);
         });
+        if constexpr (MG != 0) {
+          *(uint32_t*)(bst + (4 * NS + NT + 4) * XV_BTILE + off) = xs_mag2(sre[0], sre[1]);
+          *(uint32_t*)(bst + (4 * NS + NT + 4) * XV_BTILE + off1) = xs_mag2(sim[0], sim[1]);
+        }
       }
       fence_async_smem();
       mbar_arrive(&bar_bf[s]);
@@ -511,40 +539,97 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       const int et = rok ? a.texp[(size_t)(m * 2 + par) * a.ntr + t] : -2000;
       if (!xs_wait_w(bar_tf, u & 1, ok)) break;
       tc_fence_after();
-      long long tp[8], tx[8], ty[8];
-      int ep = 0, ex = 0, ey = 0;
-      if (wlive) {
-        ep = xv_sums<NS, W, BAL>(tcol, 2 * N, a.esh_s, tp);
-        ex = xv_sums<NS, W, BAL>(tcol + N, 2 * N, a.esh_s, tx);
-      }
-      tc_fence_before();
-      mbar_arrive(&bar_te[0]);
-      if (wlive) ey = xv_sums<NT, W, BAL>(tcol + TY, N, a.esh_t, ty);
-      tc_fence_before();
-      mbar_arrive(&bar_te[1]);
       const uint32_t slot = u % XV_CXS;
-      if (!xs_wait_w(&bar_cx[slot], (u / XV_CXS) & 1, ok)) break;   // long since complete
-      const int* cx = cxs + slot * 2 * N + cb * 8;
-      if (rok && wlive) {
-        // the products carry 2^(-2 nb), the orders' unit is 2^(w (n-1))
-        constexpr int os = W * (NS - 1) - 2 * nbs, ot = W * (NT - 1) - 2 * nbt;
+      const int* cx = cxs + slot * 2 * N + cb * 8;   // written before the item's digits were cut, and so before its accumulators
+      // the products carry 2^(-2 nb), the orders' unit is 2^(w (n-1))
+      constexpr int os = W * (NS - 1) - 2 * nbs, ot = W * (NT - 1) - 2 * nbt;
+      auto kept = [&](int c) {   // column c's z
+        const int zc = z0 + (cb * 8 + c) / 2, kk = zc + 1;
+        return zc < a.nzdim && (kk <= a.nzc || kk >= a.nzcu);
+      };
+      auto put = [&](int c, const double* pv, const double* xv, const double* yv) {
+        const int zc = z0 + (cb * 8 + c) / 2;
+        const double kz = a.ak[zc];
+        const size_t o = j + (size_t)a.nrdim * (m + (size_t)a.npdim * zc);
+        a.psi[o] = make_double2(pv[0], pv[1]);
+        a.chi[o] = make_double2(fma(kz, xv[0], -yv[0]), fma(kz, xv[1], -yv[1]));
+      };
+      if constexpr (!BAL) {
+        long long tp[8], tx[8], ty[8];
+        if (wlive) {
+          xv_sums<NS, W>(tcol, 2 * N, a.esh_s, tp);
+          xv_sums<NS, W>(tcol + N, 2 * N, a.esh_s, tx);
+        }
+        tc_fence_before();
+        mbar_arrive(&bar_te[0]);
+        if (wlive) xv_sums<NT, W>(tcol + TY, N, a.esh_t, ty);
+        tc_fence_before();
+        mbar_arrive(&bar_te[1]);
+        if (!xs_wait_w(&bar_cx[slot], (u / XV_CXS) & 1, ok)) break;   // long since complete
+        if (rok && wlive) {
 #pragma unroll
-        for (int c = 0; c < 8; c += 2) {
-          const int zc = z0 + (cb * 8 + c) / 2, kk = zc + 1;
-          if (zc >= a.nzdim || !(kk <= a.nzc || kk >= a.nzcu)) continue;
-          double pv[2], xv[2], yv[2];
+          for (int c = 0; c < 8; c += 2) {
+            if (!kept(c)) continue;
+            double pv[2], xv[2], yv[2];
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int E = cx[c + h], F = cx[N + c + h];
-            const bool ox = er > -2000 && E > -2000, oy = et > -2000 && F > -2000;
-            pv[h] = ox ? xs_i64_to_double(tp[c + h], er + E + ep + os) : 0.0;
-            xv[h] = ox ? xs_i64_to_double(tx[c + h], er + E + ex + os) : 0.0;
-            yv[h] = oy ? xs_i64_to_double(ty[c + h], et + F + ey + ot) : 0.0;
+            for (int h = 0; h < 2; ++h) {
+              const int E = cx[c + h], F = cx[N + c + h];
+              const bool ox = er > -2000 && E > -2000, oy = et > -2000 && F > -2000;
+              pv[h] = ox ? xs_i64_to_double(tp[c + h], er + E + a.esh_s + os) : 0.0;
+              xv[h] = ox ? xs_i64_to_double(tx[c + h], er + E + a.esh_s + os) : 0.0;
+              yv[h] = oy ? xs_i64_to_double(ty[c + h], et + F + a.esh_t + ot) : 0.0;
+            }
+            put(c, pv, xv, yv);
           }
-          const double kz = a.ak[zc];
-          const size_t o = j + (size_t)a.nrdim * (m + (size_t)a.npdim * zc);
-          a.psi[o] = make_double2(pv[0], pv[1]);
-          a.chi[o] = make_double2(fma(kz, xv[0], -yv[0]), fma(kz, xv[1], -yv[1]));
+        }
+      } else {
+        if (!xs_wait_w(&bar_cx[slot], (u / XV_CXS) & 1, ok)) break;   // long since complete
+        XvSum q;
+        double pv[8], xv[8];
+        float sx[8];
+        uint32_t few = 0;   // columns whose psi has only small terms
+        if (wlive) {
+          xv_drain<NS, W>(tcol, 2 * N, tcol + TM, q, true);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const bool on = er > -2000 && cx[c] > -2000;
+            pv[c] = on ? xv_value<NS, W>(q, c, er + cx[c] + os) : 0.0;
+            few |= on && q.S[c] < a.least ? 1u << c : 0u;
+          }
+          xv_drain<NS, W>(tcol + N, 2 * N, tcol + TM + N, q, true);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            xv[c] = er > -2000 && cx[c] > -2000 ? xv_value<NS, W>(q, c, er + cx[c] + os) : 0.0;
+            sx[c] = q.S[c];
+          }
+        }
+        tc_fence_before();
+        mbar_arrive(&bar_te[0]);
+        if (wlive) xv_drain<NT, W>(tcol + TY, N, tcol + TM + 2 * N, q, true);
+        tc_fence_before();
+        mbar_arrive(&bar_te[1]);
+        if (wlive) {
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) {
+            if (!kept(c)) continue;
+            const int zc = z0 + (cb * 8 + c) / 2;
+            const float kz = fabsf((float)a.ak[zc]);
+            double yv[2];
+            bool again = (few >> c) & 3u;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int E = cx[c + h], F = cx[N + c + h];
+              const bool ox = er > -2000 && E > -2000 && kz > 0.f, oy = et > -2000 && F > -2000;
+              yv[h] = oy ? xv_value<NT, W>(q, c + h, et + F + ot) : 0.0;
+              // chi = k X - Y: the terms of both against the unit of the larger; k X's in units of Y's
+              const float one = oy ? 1.f : 0.f;
+              const float rel = !ox ? 0.f : oy ? kz * __int_as_float((127 + min(max(er + E - et - F, -100), 100)) << 23) : 1.f;
+              again = again || (ox || oy) && rel * sx[c + h] + one * q.S[c + h] < a.least * (rel + one);
+            }
+            if (rok) put(c, pv + c, xv + c, yv);
+            const unsigned word = __ballot_sync(0xFFFFFFFFu, rok && again);
+            if (lane == 0) a.again[xv_word(a, m, par, mt * 4 + lq, zc)] = word;
+          }
         }
       }
       mbar_arrive(&bar_ce[slot]);
@@ -556,22 +641,85 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
   if (warp == 1) tmem_dealloc(tmem, TCOLS);
 }
 
+// The marked outputs (k_xs_again), summed in FP64: a marked row after the other, the lanes over the radial points, each lane's
+// shares of the five sums combined before they are added over the warp.
+__global__ void __launch_bounds__(256) k_xv_again(XvArgs a, const double* __restrict__ tV, const double* __restrict__ tD,
+                                                  const double* __restrict__ tT, int ne, size_t nwords) {
+  const int lane = threadIdx.x & 31;
+  const size_t nw = (size_t)gridDim.x * (blockDim.x >> 5), wid = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  int m, par, g, z;
+  auto place = [&](size_t idx) {
+    z = (int)(idx % a.nzdim); idx /= a.nzdim;
+    g = (int)(idx % a.ngrp); idx /= a.ngrp;
+    par = (int)(idx & 1);
+    m = (int)(idx >> 1);
+  };
+  for (size_t base = wid; base < nwords; base += 32 * nw) {
+    const size_t mine = base + nw * lane;
+    unsigned word = 0;
+    if (mine < nwords) {
+      place(mine);
+      const int nn = max(min(a.nrc, a.nrc - m), 0);
+      // (words of other rows and columns are not written)
+      if (m >= a.m0 && 2 * (g * 32) + par < nn && (z + 1 <= a.nzc || z + 1 >= a.nzcu)) word = a.again[mine];
+    }
+    for (unsigned todo = __ballot_sync(0xFFFFFFFFu, word != 0); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const unsigned rows = __shfl_sync(0xFFFFFFFFu, word, src);
+      place(base + nw * src);
+      const size_t off = (size_t)a.nrdim * (m + (size_t)a.npdim * z);
+      const double2 *ur = a.ur + off, *up = a.up + off, *uz = a.uz + off;
+      const double ss = par ? -1.0 : 1.0, mv = (double)m, kv = a.ak[z];
+      for (unsigned left = rows; left; left &= left - 1) {
+        const int j = 2 * (g * 32 + __ffs(left) - 1) + par;
+        const size_t row = (size_t)a.nrh * (j + (size_t)ne * m);
+        double v[10];   // V.F_s(ur), D.F_o(up), D.F_o(ur), V.F_s(up), T.F_s(uz)
+#pragma unroll
+        for (int q = 0; q < 10; ++q) v[q] = 0.0;
+        for (int i = lane; i < a.nrh; i += 32) {
+          const double V = __ldg(tV + row + i), D = __ldg(tD + row + i), T = __ldg(tT + row + i);
+          double2 p = __ldg(ur + i), q = __ldg(ur + a.nr - 1 - i);
+          v[0] = fma(V, p.x + ss * q.x, v[0]); v[1] = fma(V, p.y + ss * q.y, v[1]);
+          v[4] = fma(D, p.x - ss * q.x, v[4]); v[5] = fma(D, p.y - ss * q.y, v[5]);
+          p = __ldg(up + i); q = __ldg(up + a.nr - 1 - i);
+          v[6] = fma(V, p.x + ss * q.x, v[6]); v[7] = fma(V, p.y + ss * q.y, v[7]);
+          v[2] = fma(D, p.x - ss * q.x, v[2]); v[3] = fma(D, p.y - ss * q.y, v[3]);
+          p = __ldg(uz + i); q = __ldg(uz + a.nr - 1 - i);
+          v[8] = fma(T, p.x + ss * q.x, v[8]); v[9] = fma(T, p.y + ss * q.y, v[9]);
+        }
+        double o[4] = {mv * v[1] - v[2], -mv * v[0] - v[3], -kv * v[5] + mv * kv * v[6] - v[8], kv * v[4] + mv * kv * v[7] - v[9]};
+#pragma unroll
+        for (int d = 16; d; d >>= 1)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) o[q] += __shfl_xor_sync(0xFFFFFFFFu, o[q], d);
+        if (lane == 0) {
+          a.psi[off + j] = make_double2(o[0], o[1]);
+          a.chi[off + j] = make_double2(o[2], o[3]);
+        }
+      }
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
 struct XvImg {
   uint16_t* p = nullptr;
   int *rexp = nullptr, *texp = nullptr;
-  size_t bytes = 0, ebytes = 0;
+  unsigned* again = nullptr;
+  size_t bytes = 0, ebytes = 0, gbytes = 0;
   int nrc = -1, npc = -1, ns = 0;
 };
 static XvImg g_xvs[2];   // plain, mixed
 
+static void xv_drop(XvImg& im) {
+  if (im.p) dfree(im.p, im.bytes);
+  if (im.rexp) dfree(im.rexp, im.ebytes);
+  if (im.texp) dfree(im.texp, im.ebytes);
+  if (im.again) dfree(im.again, im.gbytes);
+  im = XvImg();
+}
 void xv_free() {
-  for (XvImg& im : g_xvs) {
-    if (im.p) dfree(im.p, im.bytes);
-    if (im.rexp) dfree(im.rexp, im.ebytes);
-    if (im.texp) dfree(im.texp, im.ebytes);
-    im = XvImg();
-  }
+  for (XvImg& im : g_xvs) xv_drop(im);
 }
 
 // digit counts of psi / X and of Y and their width; ns = 0 where no configuration is exact
@@ -593,15 +741,16 @@ bool xv_supported(bool plain) { return xv_cfg(G.nrh, plain).ns > 0; }
 template <int NS, int NT, int W>
 static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
   if (im.nrc != args.nrc || im.npc != npc || !im.p || im.ns != NS) {
-    if (im.p) dfree(im.p, im.bytes);
-    if (im.rexp) dfree(im.rexp, im.ebytes);
-    if (im.texp) dfree(im.texp, im.ebytes);
-    im = XvImg();
-    im.bytes = (size_t)npc * 2 * args.nmt * args.nkc * (2 * NS + NT) * XV_ATILE;
+    xv_drop(im);
+    im.bytes = (size_t)npc * 2 * args.nmt * args.nkc * xv_tiles<NS, NT>() * XV_ATILE;
     im.ebytes = (size_t)npc * 2 * args.ntr * sizeof(int);
     MLG_TRY(dmalloc((void**)&im.p, im.bytes));
     MLG_TRY(dmalloc((void**)&im.rexp, im.ebytes));
     MLG_TRY(dmalloc((void**)&im.texp, im.ebytes));
+    if (xv_mag<NS>()) {
+      im.gbytes = (size_t)npc * 2 * cdiv(args.ntr, 32) * G.nzdim * sizeof(unsigned);
+      MLG_TRY(dmalloc((void**)&im.again, im.gbytes));
+    }
     k_xv_rexp<<<dim3(cdiv(args.ntr, 128), npc * 2), 128, 0, G.stream>>>(G.tV, G.tD, G.tT, im.rexp, im.texp, G.nrh, G.ne, args.nrc,
                                                                         args.ntr, plain ? 1 : 0);
     MLG_LAUNCH();
@@ -611,14 +760,19 @@ static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
     im.nrc = args.nrc; im.npc = npc; im.ns = NS;
   }
   args.img = im.p; args.rexp = im.rexp; args.texp = im.texp;
-  const size_t fixed = 1024 + XV_SB * (size_t)xv_bstage_bytes(NS, NT) + XV_CXS * 2 * XV_N * sizeof(int) + 512;
-  args.aent = (int)std::min<size_t>(XV_AEMAX, (227 * 1024 - fixed) / xv_aent_bytes(NS, NT));
-  const size_t sm = fixed + (size_t)args.aent * xv_aent_bytes(NS, NT);
+  args.again = im.again; args.ngrp = cdiv(args.ntr, 32); args.least = xs_least_sum(2 * G.nrh);   // psi's and X's sums of two products
+  const size_t fixed = 1024 + XV_SB * (size_t)xv_bstage_bytes<NS, NT>() + XV_CXS * 2 * XV_N * sizeof(int) + 512;
+  args.aent = (int)std::min<size_t>(XV_AEMAX, (227 * 1024 - fixed) / xv_aent_bytes<NS, NT>());
+  const size_t sm = fixed + (size_t)args.aent * xv_aent_bytes<NS, NT>();
   auto kern = k_xv_contract<NS, NT, W>;
   MLG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int nitems = (npc - args.m0) * 2 * args.nmt * cdiv(G.nzdim, XV_NZ);
   kern<<<std::min(nitems, 152), XV_THREADS, sm, G.stream>>>(args);
   MLG_LAUNCH();
+  if (xv_mag<NS>()) {
+    k_xv_again<<<152 * 4, 256, 0, G.stream>>>(args, G.tV, G.tD, G.tT, G.ne, (size_t)npc * 2 * args.ngrp * G.nzdim);
+    MLG_LAUNCH();
+  }
   return 0;
 }
 
