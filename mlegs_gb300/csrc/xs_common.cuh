@@ -44,6 +44,19 @@ __device__ __forceinline__ long long xs_fix(double x, int E, int nb) {
   return (b >> 63) ? -(long long)X : (long long)X;
 }
 
+// What FP32 accumulates exactly, and the largest magnitude that an order of ns balanced digits of w bits can reach with `products`
+// products per digit pair over K terms: order d has d + 1 pairs, two of them (one, for d = 0) with a first digit
+constexpr double XS_EXACT = 16777216.0;
+__host__ __device__ constexpr double xs_order_bound(int ns, int w, int products, int K) {
+  const double first = 128.0, other = (double)(1 << (w - 1));
+  double most = first * first;
+  for (int d = 1; d < ns; ++d) {
+    const double v = 2.0 * first * other + (d - 1) * other * other;
+    most = v > most ? v : most;
+  }
+  return most * products * K;
+}
+
 // exponent bound for balanced digits from a magnitude's high word: |v| < 2^E (1 - 2^-7)
 __device__ __forceinline__ int xs_ebound_bal(unsigned abshi) { return (int)((abshi + 0x4000u) >> 20) - 1022; }
 

@@ -827,7 +827,7 @@ static int xs_cfg(int kmax, int nrc, bool plain) {
   const double lim = 16777216.0;
   if (plain) {
     if (xs_rawk(nrc) <= 285) return kmax <= 113 ? 8 : 10;   // 8 128 128 K <= 2^24 up to 128
-    if (11.0 * kmax * 64 * 64 <= lim) return 9;        // order 8: seven pairs of 64 x 64 and two of 64 x 128
+    if (xs_order_bound(9, 7, 1, kmax) <= XS_EXACT) return 9;   // up to 372
   } else {
     if (6.0 * kmax * 128 * 128 < lim) return 6;
     if (7.0 * kmax * 64 * 64 < lim) return 7;

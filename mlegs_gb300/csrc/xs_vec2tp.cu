@@ -23,9 +23,9 @@
 // Laplacian that ends the projection magnifies its error in the weak low modes; with 42-bit Y the
 // (m = 1, k = 0) column left the step's nonlinear term chi 9e-6 from FP64 at 192 x 128 x 128, with
 // 49 bits 2e-7.
-// Plain form: nine balanced digits of 7 bits (63 bits) for all three, up to 744 radial points.  With up to 372 points
-// every order is exact; beyond, the orders from 6 on could pass 2^24 if all their digits were extreme and would then
-// lose units of 2^-56 of max|A| max|B|.  The order sums are shifted by what they need (xs_radial.cu): cut at a fixed
+// Plain form: nine balanced digits of 7 bits (63 bits) for all three, up to 744 radial points.  An order of psi or X holds two
+// products per digit pair and is exact up to 186 terms (xs_order_bound); beyond 372 radial points the accumulators are drained
+// every 176 and the parts added in 64-bit integers.  The order sums are shifted by what they need (xs_radial.cu): cut at a fixed
 // 2^-52, as 54-bit slices once were, chi = k X - Y is left 7e-9 from FP64.
 //
 // Engine: a persistent grid of one CTA per SM over work items (m, 8 complex z columns, 128-row tile, parity).
@@ -168,6 +168,8 @@ __device__ __forceinline__ size_t xv_word(const XvArgs& a, int m, int par, int g
   return (((size_t)m * 2 + par) * a.ngrp + g) * a.nzdim + z;
 }
 
+constexpr int XV_PART = 11;   // chunks between drains where one set of accumulators does not take all radial points
+static_assert(xs_order_bound(9, 7, 2, XV_PART * XV_KC) <= XS_EXACT, "the orders of a part stay exact");
 constexpr int XV_NZ = 8, XV_N = 2 * XV_NZ;   // complex z columns per item, real columns
 constexpr int XV_NSW = 2, XV_GW = 6, XV_NEW = 8;   // scale warps, warps of a digit group (two groups), epilogue warps
 constexpr int XV_THREADS = (2 + XV_NSW + 2 * XV_GW + XV_NEW) * 32;
@@ -240,7 +242,8 @@ template <int NO, int W> __device__ __forceinline__ double xv_value(const XvSum&
   return xs_i64_to_double(((long long)q.C[c] << (xv_cb<NO, W>() - es)) + (q.L[c] >> es), e + es + XV_LOW);
 }
 
-template <int NS, int NT, int W>
+// PARTS: more radial points than one set of accumulators takes exactly (xv_exact), drained every XV_PART chunks
+template <int NS, int NT, int W, bool PARTS>
 __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
   constexpr bool BAL = xv_bal<NS>();
   constexpr int NZ = XV_NZ, N = XV_N;
@@ -315,7 +318,7 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
   };
   int first = blockIdx.x;
   if (first < nitems && !live(first)) first = next_item(first);
-  const int nkc = a.nkc;
+  const int nkc = a.nkc, npart = PARTS ? XV_PART : nkc;   // chunks between drains
 
   if (warp == 0) {
     // ---- the table entries
@@ -369,24 +372,25 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       last = sa; plast = pa; any = true;
       if (++sa == AE) { sa = 0; pa ^= 1u; }
     };
-    for (int it = first; it < nitems && ok; it = next_item(it), ++u) {
-      // psi's and X's accumulators, once the epilogue has read the item before
-      if (u > 0 && !xs_wait_w(&bar_te[0], (u - 1) & 1, ok)) break;
-      for (int kc = 0; kc < nkc && ok; ++kc) {
-        if (!xs_wait_w(&bar_bf[sb], pb, ok)) break;
-        const uint32_t b0 = smem_u32(sB) + sb * BSTAGE, bm = b0 + (4 * NS + NT) * XV_BTILE;
-        // psi and X alternate by order (psi_d at 2d N, X_d at (2d+1) N) and their field digits alternate the same way
-        // ([psi_ur_s, X_up_s] against m V, [psi_up_s, X_ur_s] against D), so one MMA covers both sums
-        entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, bm, TM, kc > 0);
-        if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, bm + 2 * XV_BTILE, TM, true);
-        if (kc == 0 && u > 0) xs_wait_w(&bar_te[1], (u - 1) & 1, ok);
-        if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, bm + 4 * XV_BTILE, TM + 2 * N, kc > 0);
-        if (!ok) break;
-        umma_commit(&bar_be[sb], el);
-        if (++sb == XV_SB) { sb = 0; pb ^= 1u; }
+    for (int it = first; it < nitems && ok; it = next_item(it))
+      for (int k0 = 0; k0 < nkc && ok; k0 += npart, ++u) {
+        // psi's and X's accumulators, once the epilogue has read what they held before
+        if (u > 0 && !xs_wait_w(&bar_te[0], (u - 1) & 1, ok)) break;
+        for (int kc = k0; kc < min(k0 + npart, nkc) && ok; ++kc) {
+          if (!xs_wait_w(&bar_bf[sb], pb, ok)) break;
+          const uint32_t b0 = smem_u32(sB) + sb * BSTAGE, bm = b0 + (4 * NS + NT) * XV_BTILE;
+          // psi and X alternate by order (psi_d at 2d N, X_d at (2d+1) N) and their field digits alternate the same way
+          // ([psi_ur_s, X_up_s] against m V, [psi_up_s, X_ur_s] against D), so one MMA covers both sums
+          entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, bm, TM, kc > k0);
+          if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, bm + 2 * XV_BTILE, TM, true);
+          if (kc == k0 && u > 0) xs_wait_w(&bar_te[1], (u - 1) & 1, ok);
+          if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, bm + 4 * XV_BTILE, TM + 2 * N, kc > k0);
+          if (!ok) break;
+          umma_commit(&bar_be[sb], el);
+          if (++sb == XV_SB) { sb = 0; pb ^= 1u; }
+        }
+        if (ok) umma_commit(bar_tf, el);
       }
-      if (ok) umma_commit(bar_tf, el);
-    }
     if (any) {   // the MMAs issued have finished (bounded) before tensor memory is freed
       bool ok2 = true;
       xs_wait_w(&bar_ae[last], plast, ok2);
@@ -528,8 +532,8 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
     // ---- epilogue: warp e reads TMEM lanes 32 (e % 4) .. (rows t) and the 8-column block e / 4
     const int lq = warp & 3, cb = (warp - 2 - XV_NSW - 2 * XV_GW) >> 2;
     const uint32_t tcol = tmem + ((uint32_t)(lq * 32) << 16) + (uint32_t)(cb * 8);
-    uint32_t u = 0;
-    for (int it = first; it < nitems; it = next_item(it), ++u) {
+    uint32_t u = 0, ii = 0;   // drains, items
+    for (int it = first; it < nitems; it = next_item(it), ++u, ++ii) {
       const int m = item_m(it), mt = item_mt(it), par = item_par(it), z0 = item_z0(it);
       const int nn = max(min(a.nrc, a.nrc - m), 0);
       const int t = mt * 128 + lq * 32 + lane, j = 2 * t + par;
@@ -539,7 +543,7 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       const int et = rok ? a.texp[(size_t)(m * 2 + par) * a.ntr + t] : -2000;
       if (!xs_wait_w(bar_tf, u & 1, ok)) break;
       tc_fence_after();
-      const uint32_t slot = u % XV_CXS;
+      const uint32_t slot = ii % XV_CXS;
       const int* cx = cxs + slot * 2 * N + cb * 8;   // written before the item's digits were cut, and so before its accumulators
       // the products carry 2^(-2 nb), the orders' unit is 2^(w (n-1))
       constexpr int os = W * (NS - 1) - 2 * nbs, ot = W * (NT - 1) - 2 * nbt;
@@ -565,7 +569,7 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
         if (wlive) xv_sums<NT, W>(tcol + TY, N, a.esh_t, ty);
         tc_fence_before();
         mbar_arrive(&bar_te[1]);
-        if (!xs_wait_w(&bar_cx[slot], (u / XV_CXS) & 1, ok)) break;   // long since complete
+        if (!xs_wait_w(&bar_cx[slot], (ii / XV_CXS) & 1, ok)) break;   // long since complete
         if (rok && wlive) {
 #pragma unroll
           for (int c = 0; c < 8; c += 2) {
@@ -583,31 +587,62 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
           }
         }
       } else {
-        if (!xs_wait_w(&bar_cx[slot], (u / XV_CXS) & 1, ok)) break;   // long since complete
-        XvSum q;
+        if (!xs_wait_w(&bar_cx[slot], (ii / XV_CXS) & 1, ok)) break;   // long since complete
+        XvSum q;   // Y's sums in the end
         double pv[8], xv[8];
         float sx[8];
         uint32_t few = 0;   // columns whose psi has only small terms
-        if (wlive) {
-          xv_drain<NS, W>(tcol, 2 * N, tcol + TM, q, true);
+        auto take_psi = [&](const XvSum& v) {
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
             const bool on = er > -2000 && cx[c] > -2000;
-            pv[c] = on ? xv_value<NS, W>(q, c, er + cx[c] + os) : 0.0;
-            few |= on && q.S[c] < a.least ? 1u << c : 0u;
+            pv[c] = on ? xv_value<NS, W>(v, c, er + cx[c] + os) : 0.0;
+            few |= on && v.S[c] < a.least ? 1u << c : 0u;
           }
-          xv_drain<NS, W>(tcol + N, 2 * N, tcol + TM + N, q, true);
+        };
+        auto take_x = [&](const XvSum& v) {
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            xv[c] = er > -2000 && cx[c] > -2000 ? xv_value<NS, W>(q, c, er + cx[c] + os) : 0.0;
-            sx[c] = q.S[c];
+            xv[c] = er > -2000 && cx[c] > -2000 ? xv_value<NS, W>(v, c, er + cx[c] + os) : 0.0;
+            sx[c] = v.S[c];
+          }
+        };
+        auto release = [&](int which) {
+          tc_fence_before();
+          mbar_arrive(&bar_te[which]);
+        };
+        if constexpr (!PARTS) {
+          if (wlive) {
+            xv_drain<NS, W>(tcol, 2 * N, tcol + TM, q, true);
+            take_psi(q);
+            xv_drain<NS, W>(tcol + N, 2 * N, tcol + TM + N, q, true);
+            take_x(q);
+          }
+          release(0);
+          if (wlive) xv_drain<NT, W>(tcol + TY, N, tcol + TM + 2 * N, q, true);
+          release(1);
+        } else {
+          XvSum qp, qx;
+          for (int k0 = 0; k0 < nkc; k0 += npart) {
+            if (k0 > 0) {
+              ++u;
+              if (!xs_wait_w(bar_tf, u & 1, ok)) break;
+              tc_fence_after();
+            }
+            if (wlive) {
+              xv_drain<NS, W>(tcol, 2 * N, tcol + TM, qp, k0 == 0);
+              xv_drain<NS, W>(tcol + N, 2 * N, tcol + TM + N, qx, k0 == 0);
+            }
+            release(0);
+            if (wlive) xv_drain<NT, W>(tcol + TY, N, tcol + TM + 2 * N, q, k0 == 0);
+            release(1);
+          }
+          if (!ok) break;
+          if (wlive) {
+            take_psi(qp);
+            take_x(qx);
           }
         }
-        tc_fence_before();
-        mbar_arrive(&bar_te[0]);
-        if (wlive) xv_drain<NT, W>(tcol + TY, N, tcol + TM + 2 * N, q, true);
-        tc_fence_before();
-        mbar_arrive(&bar_te[1]);
         if (wlive) {
 #pragma unroll
           for (int c = 0; c < 8; c += 2) {
@@ -738,7 +773,7 @@ static XvCfg xv_cfg(int k, bool plain) {
 
 bool xv_supported(bool plain) { return xv_cfg(G.nrh, plain).ns > 0; }
 
-template <int NS, int NT, int W>
+template <int NS, int NT, int W, bool PARTS = false>
 static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
   if (im.nrc != args.nrc || im.npc != npc || !im.p || im.ns != NS) {
     xv_drop(im);
@@ -764,7 +799,7 @@ static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
   const size_t fixed = 1024 + XV_SB * (size_t)xv_bstage_bytes<NS, NT>() + XV_CXS * 2 * XV_N * sizeof(int) + 512;
   args.aent = (int)std::min<size_t>(XV_AEMAX, (227 * 1024 - fixed) / xv_aent_bytes<NS, NT>());
   const size_t sm = fixed + (size_t)args.aent * xv_aent_bytes<NS, NT>();
-  auto kern = k_xv_contract<NS, NT, W>;
+  auto kern = k_xv_contract<NS, NT, W, PARTS>;
   MLG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   const int nitems = (npc - args.m0) * 2 * args.nmt * cdiv(G.nzdim, XV_NZ);
   kern<<<std::min(nitems, 152), XV_THREADS, sm, G.stream>>>(args);
@@ -799,7 +834,7 @@ int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int 
     args.esh_t = esh(cfg.nt, cfg.nt);
   }
   XvImg& im = g_xvs[plain ? 0 : 1];
-  if (cfg.ns == 9) return xv_run<9, 9, 7>(args, im, npc, plain);
+  if (cfg.ns == 9) return xs_order_bound(9, 7, 2, G.nrh) <= XS_EXACT ? xv_run<9, 9, 7>(args, im, npc, plain) : xv_run<9, 9, 7, true>(args, im, npc, plain);
   if (cfg.ns == 5) return xv_run<5, 7, 7>(args, im, npc, plain);
   return xv_run<6, 8, 6>(args, im, npc, plain);
 }
