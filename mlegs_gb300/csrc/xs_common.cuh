@@ -112,18 +112,20 @@ template <int NS, int W, bool BAL, int S> __device__ __forceinline__ uint32_t xs
   }
 }
 
-// |X0| and |X1| (|X| < 2^63) in units of 2^40, truncated to 8 significant bits, as a packed BF16 pair: the operands of a
-// contraction's magnitude sum
+// |X0| and |X1| (|X| < 2^63) in units of 2^32 as a packed BF16 pair: the operands of a contraction's magnitude sum
 __device__ __forceinline__ uint32_t xs_mag2(long long X0, long long X1) {
-  const uint32_t a = (uint32_t)abs((int)(X0 >> 32)) >> 8, b = (uint32_t)abs((int)(X1 >> 32)) >> 8;
-  return xs_sub2_pack(a | 0x4B000000u, b | 0x4B000000u, 8388608.0f);
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"((float)(int)(X1 >> 32)), "f"((float)(int)(X0 >> 32)));
+  return r & 0x7FFF7FFFu;
 }
 // Where the digits of a plain contraction of K terms are too few.  Their error, the dropped orders and the rounding of the
 // operands, is 2^-61.9 sqrt(K / 96) of 2^(row scale + column scale) in the root mean square (measured over K = 96..372); an FP64
-// sum's is 2^-54 of S = sum |terms|, give or take a factor of three.  The magnitude sum S is contracted beside the digits as one
-// more digit product (xs_mag2), and outputs with S below this times 2^(row scale + column scale) are summed again in FP64
-// (k_xs_again, k_xv_again).  In units of 2^-46, those of the products of xs_mag2.
-inline float xs_least_sum(int K) { return (float)(std::exp2(46.0 - 7.9) * std::sqrt(K / 96.0)); }
+// sum rounds K times by up to 2^-53 of S = sum |terms|.  The magnitude sum S is contracted beside the digits as one more digit
+// product (xs_mag2), and outputs whose S is so small that the digits' error would pass one such rounding, 2^-53 S, are summed
+// again in FP64 (k_xs_again, k_xv_again).  The least S in units of 2^-62 2^(row scale + column scale), those of the products of
+// xs_mag2.
+constexpr int XS_AGAIN = 4861, XS_AGAIN_T = 256;   // their warps (about 32 an SM) and threads per CTA
+inline float xs_least_sum(int K) { return (float)(std::exp2(62.0 - 8.9) * std::sqrt(K / 96.0)); }
 
 // the FP32 value of a small integer (|d| < 2^22), exactly, on the FP32 pipe
 __device__ __forceinline__ float xs_i2f(int d) { return __int_as_float(0x4B400000 + d) - 12582912.0f; }

@@ -593,8 +593,8 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
         auto value = [&](long long t, int E, int ea, int e) {   // E: the column's scale
           return ea > -2000 && E > -2000 ? xs_i64_to_double(t, ea + E + e) : 0.0;
         };
-        long long T[2][CW];            // order sums (forward, balanced: the results' bits)
-        uint32_t esh = 0;              // backward, balanced: the columns' shifts, four bits each
+        long long T[2][CW];            // order sums
+        uint32_t esh[2] = {0, 0};      // balanced: the columns' shifts, four bits each (backward: esh[0] for both parities)
         uint32_t small[2] = {0, 0};    // magnitude sums below the least, a bit a column
 #pragma unroll
         for (int par = 0; par < 2; ++par, ++u) {
@@ -629,15 +629,14 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
                 const int C = xs_f2i(__uint_as_float(g[c])) * (1 << W) + xs_f2i(__uint_as_float(h[c]));
                 int es = xs_order_shift<NS>(abs(C));
                 if (MODE == 1 && par == 1) {   // the two parities are added: the same shift for both
-                  const int e0 = (int)(esh >> (4 * c)) & 15;
+                  const int e0 = (int)(esh[0] >> (4 * c)) & 15;
                   es = max(es, e0);
                   T[0][c] >>= es - e0;
-                  esh = (esh & ~(15u << (4 * c))) | ((uint32_t)es << (4 * c));
-                } else if (MODE == 1) {
-                  esh |= (uint32_t)es << (4 * c);
+                  esh[0] = (esh[0] & ~(15u << (4 * c))) | ((uint32_t)es << (4 * c));
+                } else {
+                  esh[par] |= (uint32_t)es << (4 * c);
                 }
-                const long long t = ((long long)C << (xs_cb<NS>() - es)) + (T[par][c] >> es);
-                T[par][c] = MODE == 0 ? __double_as_longlong(value(t, cx[c], EA[par], es + eo)) : t;
+                T[par][c] = ((long long)C << (xs_cb<NS>() - es)) + (T[par][c] >> es);
               }
               if constexpr (MAG) {
                 xs_tmem_ld<CW>(tcol + (uint32_t)(NO * N), g);
@@ -680,15 +679,18 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
 #pragma unroll
               for (int par = 0; par < 2; ++par) {
                 if (2 * row + par >= nn) continue;
-                o[2 * row + par] = BAL ? make_double2(__longlong_as_double(T[par][c]), __longlong_as_double(T[par][c + 1]))
-                                       : make_double2(value(T[par][c], cx[c], EA[par], eo), value(T[par][c + 1], cx[c + 1], EA[par], eo));
+                double v[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                  v[h] = value(T[par][c + h], cx[c + h], EA[par], eo + ((int)(esh[par] >> (4 * (c + h))) & 15));
+                o[2 * row + par] = make_double2(v[0], v[1]);
               }
             } else {
               double v[4];   // f(i) re, im; f(nr-1-i) re, im
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 // f(i) = D_0 + D_1, f(nr-1-i) = D_0 - D_1: both parities share the scales
-                const int e = eo + ((int)(esh >> (4 * (c + h))) & 15);
+                const int e = eo + ((int)(esh[0] >> (4 * (c + h))) & 15);
                 v[h] = value(T[0][c + h] + T[1][c + h], cx[c + h], EA[0], e);
                 v[2 + h] = value(T[0][c + h] - T[1][c + h], cx[c + h], EA[0], e);
               }
@@ -715,13 +717,14 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
 // ------------------------------------------------------------------------------------------------
 // The marked outputs of the nine-digit form, summed in FP64 (as the FP64 kernels of radial.cu sum, term after term, backward).
 // Few and scattered, or whole regions (the points near the axis where the functions of high m vanish), so each warp takes words
-// from all over the grid.  Backward: a lane per row of the word, the table read along the rows.  Forward: a marked row after the
+// from all over the grid, XS_AGAIN (a prime) apart.  Backward: a lane per row of the word, the table read along the rows.  Forward: a marked row after the
 // other, the lanes over the radial points.  Nothing marked: 4 us.
 template <int MODE>
-__global__ void __launch_bounds__(256) k_xs_again(XsArgs a, const double* __restrict__ pf, const double* __restrict__ w, int ne,
+__global__ void __launch_bounds__(XS_AGAIN_T) k_xs_again(XsArgs a, const double* __restrict__ pf, const double* __restrict__ w, int ne,
                                                   size_t nwords) {
   const int lane = threadIdx.x & 31;
-  const size_t nw = (size_t)gridDim.x * (blockDim.x >> 5), wid = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const size_t nw = XS_AGAIN, wid = (size_t)blockIdx.x * (XS_AGAIN_T / 32) + (threadIdx.x >> 5);
+  if (wid >= nw) return;
   int f, m, par, g, z;
   auto place = [&](size_t idx) {
     z = (int)(idx % a.nzdim); idx /= a.nzdim;
@@ -876,7 +879,7 @@ static int xs_launch(const XsArgs& args, int nitems) {
   kern<<<std::min(nitems, 152), XS_THREADS, sm, G.stream>>>(args);
   MLG_LAUNCH();
   if constexpr (xs_mag<NS>() != 0) {
-    k_xs_again<MODE><<<152 * 4, 256, 0, G.stream>>>(args, G.pf, G.w, G.ne, xs_words(MODE, args.nf, args.npc, args.ngrp));
+    k_xs_again<MODE><<<cdiv(XS_AGAIN, XS_AGAIN_T / 32), XS_AGAIN_T, 0, G.stream>>>(args, G.pf, G.w, G.ne, xs_words(MODE, args.nf, args.npc, args.ngrp));
     MLG_LAUNCH();
   }
   return 0;

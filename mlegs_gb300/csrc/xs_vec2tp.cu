@@ -678,10 +678,11 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
 
 // The marked outputs (k_xs_again), summed in FP64: a marked row after the other, the lanes over the radial points, each lane's
 // shares of the five sums combined before they are added over the warp.
-__global__ void __launch_bounds__(256) k_xv_again(XvArgs a, const double* __restrict__ tV, const double* __restrict__ tD,
+__global__ void __launch_bounds__(XS_AGAIN_T) k_xv_again(XvArgs a, const double* __restrict__ tV, const double* __restrict__ tD,
                                                   const double* __restrict__ tT, int ne, size_t nwords) {
   const int lane = threadIdx.x & 31;
-  const size_t nw = (size_t)gridDim.x * (blockDim.x >> 5), wid = (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const size_t nw = XS_AGAIN, wid = (size_t)blockIdx.x * (XS_AGAIN_T / 32) + (threadIdx.x >> 5);
+  if (wid >= nw) return;
   int m, par, g, z;
   auto place = [&](size_t idx) {
     z = (int)(idx % a.nzdim); idx /= a.nzdim;
@@ -805,7 +806,7 @@ static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
   kern<<<std::min(nitems, 152), XV_THREADS, sm, G.stream>>>(args);
   MLG_LAUNCH();
   if (xv_mag<NS>()) {
-    k_xv_again<<<152 * 4, 256, 0, G.stream>>>(args, G.tV, G.tD, G.tT, G.ne, (size_t)npc * 2 * args.ngrp * G.nzdim);
+    k_xv_again<<<cdiv(XS_AGAIN, XS_AGAIN_T / 32), XS_AGAIN_T, 0, G.stream>>>(args, G.tV, G.tD, G.tT, G.ne, (size_t)npc * 2 * args.ngrp * G.nzdim);
     MLG_LAUNCH();
   }
   return 0;
