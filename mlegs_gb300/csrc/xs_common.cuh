@@ -60,6 +60,11 @@ __host__ __device__ constexpr double xs_order_bound(int ns, int w, int products,
 // exponent bound for balanced digits from a magnitude's high word: |v| < 2^E (1 - 2^-7)
 __device__ __forceinline__ int xs_ebound_bal(unsigned abshi) { return (int)((abshi + 0x4000u) >> 20) - 1022; }
 
+// the scale of a plain-form column that holds a non-finite sample: every value of it gives 0 (xs_fix_base), and its outputs come
+// from elsewhere
+constexpr int XS_NONFIN = 4096;
+__device__ __forceinline__ bool xs_nonfin(unsigned abshi) { return abshi >= 0x7FF00000u; }   // a largest magnitude's high word
+
 // the shift base of xs_fixs for a scale E; `ok` false (no column, or an all-zero one): every value gives 0
 __device__ __forceinline__ int xs_fix_base(int E, int nb, bool ok) { return ok && E > -2000 ? 1085 - nb + E : (1 << 20); }
 // xs_fix with the shift base worked out once per column.  The significand starts at bit 63 and is shifted right only

@@ -16,7 +16,8 @@
 // max|A(row,:)| max|B(:,n)|: 63 bits, in eight or nine balanced digits, for the plain form, 42 bits for the mixed form.  Where
 // FP64 sums were the plain form's alternative (nine digits), the outputs whose terms are all small beside those maxima, points
 // near the axis for one, are found by a contraction of the magnitudes and summed again in FP64 (xs_least_sum, k_xs_again): each
-// output is as near to the exact sum of its terms as an FP64 sum.  No floating-point rounding happens anywhere else: the forward fold f(i) +- f(nr-1-i) is an exact
+// output is as near to the exact sum of its terms as an FP64 sum.  A column of the plain form with a NaN or an infinity gives
+// NaN, or what an FP64 sum gives (nine digits).  No floating-point rounding happens anywhere else: the forward fold f(i) +- f(nr-1-i) is an exact
 // integer sum of the two rounded samples, and the quadrature weights are folded into the table (A = pf w, one FP64
 // rounding at kit init).
 //
@@ -238,6 +239,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
   constexpr int NO = NS;
   constexpr int W = xs_w<NS>(), ESH = xs_esh<NS>(), nb = xs_nb<NS>();
   constexpr bool BAL = xs_bal<NS>();
+  constexpr bool PLAIN = NS >= 8;                 // else the mixed form's digits
   constexpr int N = 2 * NZ;                       // real columns (MMA N per digit)
   constexpr int BT = N * XS_KC * 2;               // B digit tile bytes
   constexpr int AENT = NS * XS_ATILE;             // a table entry: the digits of one parity of a chunk
@@ -476,8 +478,12 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
       if ((lane & 3) == 0 && zz < NZ) {
         constexpr int fold = MODE == 0 ? 1 : 0;
         // an all-subnormal column counts as zero
-        cxw[2 * zz] = (mr >> 20) ? (BAL ? xs_ebound_bal(mr) : (int)(mr >> 20) - 1022) + fold : -2000;
-        cxw[2 * zz + 1] = (mi >> 20) ? (BAL ? xs_ebound_bal(mi) : (int)(mi >> 20) - 1022) + fold : -2000;
+        auto scale = [](unsigned h) {
+          if (PLAIN && xs_nonfin(h)) return XS_NONFIN;
+          return (h >> 20) ? (BAL ? xs_ebound_bal(h) : (int)(h >> 20) - 1022) + fold : -2000;
+        };
+        cxw[2 * zz] = scale(mr);
+        cxw[2 * zz + 1] = scale(mi);
       }
       mbar_arrive(&bar_cx[slot]);
       if (RB > 1) copy_columns(next_item(item), ii + 1);
@@ -591,6 +597,7 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
         // large ones in a common shift
         constexpr int eo = (BAL ? xs_low<NS>() : ESH) + W * (2 * (NS - 1) - (NO - 1)) - 2 * nb;
         auto value = [&](long long t, int E, int ea, int e) {   // E: the column's scale
+          if (PLAIN && E == XS_NONFIN) return __longlong_as_double(0x7FF8000000000000ll);
           return ea > -2000 && E > -2000 ? xs_i64_to_double(t, ea + E + e) : 0.0;
         };
         long long T[2][CW];            // order sums
@@ -651,7 +658,8 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
         }
         if (!ok) break;
         if (MAG && live) {
-          // the outputs whose terms are all small beside their row's and column's largest entries, for k_xs_again
+          // the outputs whose terms are all small beside their row's and column's largest entries, and those of columns with
+        // non-finite samples, for k_xs_again
 #pragma unroll
           for (int par = 0; par < (MODE == 0 ? 2 : 1); ++par) {
             const uint32_t sm = MODE == 0 ? small[par] : small[0] & small[1];
@@ -660,7 +668,8 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
             for (int c = 0; c < CW; c += 2) {
               const int zo = z0 + ((cg * CW + c) >> 1);
               if (zo >= a.nzdim) continue;
-              const bool few = EA[par] > -2000 && (((sm >> c) & 1 && cx[c] > -2000) || ((sm >> (c + 1)) & 1 && cx[c + 1] > -2000));
+              const bool few = (EA[par] > -2000 && (((sm >> c) & 1 && cx[c] > -2000) || ((sm >> (c + 1)) & 1 && cx[c + 1] > -2000))) ||
+                               cx[c] == XS_NONFIN || cx[c + 1] == XS_NONFIN;
               const unsigned word = __ballot_sync(0xFFFFFFFFu, rok && few);
               if (lane == 0) a.again[xs_word(a, MODE, item_f(item), m, par, mt * 4 + lq, zo)] = word;
             }

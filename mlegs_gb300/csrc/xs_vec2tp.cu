@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       }
       if ((lane & 7) == 0) {
         // an all-subnormal column counts as zero
-        auto bound = [](unsigned h) { return !(h >> 20) ? -2000 : (BAL ? xs_ebound_bal(h) : (int)(h >> 20) - 1022) + 1; };
+        auto bound = [](unsigned h) { return BAL && xs_nonfin(h) ? XS_NONFIN : !(h >> 20) ? -2000 : (BAL ? xs_ebound_bal(h) : (int)(h >> 20) - 1022) + 1; };
         int* cx = cxs + slot * 2 * N;
         cx[2 * zz] = bound(e0);
         cx[2 * zz + 1] = bound(e1);
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
               // chi = k X - Y: the terms of both against the unit of the larger; k X's in units of Y's
               const float one = oy ? 1.f : 0.f;
               const float rel = !ox ? 0.f : oy ? kz * __int_as_float((127 + min(max(er + E - et - F, -100), 100)) << 23) : 1.f;
-              again = again || (ox || oy) && rel * sx[c + h] + one * q.S[c + h] < a.least * (rel + one);
+              again = again || E == XS_NONFIN || F == XS_NONFIN || (ox || oy) && rel * sx[c + h] + one * q.S[c + h] < a.least * (rel + one);
             }
             if (rok) put(c, pv + c, xv + c, yv);
             const unsigned word = __ballot_sync(0xFFFFFFFFu, rok && again);
