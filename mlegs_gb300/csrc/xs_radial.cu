@@ -841,8 +841,9 @@ static int xs_cfg(int kmax, int nrc, bool plain) {
     if (xs_rawk(nrc) <= 285) return kmax <= 113 ? 8 : 10;   // 8 128 128 K <= 2^24 up to 128
     if (xs_order_bound(9, 7, 1, kmax) <= XS_EXACT) return 9;   // up to 372
   } else {
-    if (6.0 * kmax * 128 * 128 < lim) return 6;
-    if (7.0 * kmax * 64 * 64 < lim) return 7;
+    // (larger grids' sums are FP64 in this form too: 740 points with seven digits, 892 with six)
+    if (6.0 * kmax * 128 * 128 < lim) return xs_rawk(nrc) <= 893 ? 6 : 0;
+    if (7.0 * kmax * 64 * 64 < lim) return xs_rawk(nrc) <= 741 ? 7 : 0;
   }
   return 0;
 }
