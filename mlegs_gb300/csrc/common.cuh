@@ -117,6 +117,8 @@ enum { DS_SUM0 = 0, DS_SUM1 = 1, DS_GAIN0 = 4, DS_GAIN1 = 5, DS_FLAG = 8, DS_CAL
 
 // device memory accounting
 int dmalloc(void** p, size_t bytes);
+// several arrays, all or none (those of 0 bytes stay null)
+int dmalloc_all(std::initializer_list<std::pair<void**, size_t>> arrays);
 void dfree(void* p, size_t bytes);
 cd* get_buf();
 void put_buf(cd* b);
@@ -167,11 +169,13 @@ bool xs_supported(int mode, int nrc, bool plain);
 int xs_rtrans(int mode, const cd* in, cd* out, int nrc, int npc, int m0, const double* lnp, bool add_ln, bool plain);
 int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int nrc, int npc, int m0,
                     const double* const* lnp, bool add_ln, bool plain);
+int xs_prepare(int mode, int nrc, int npc, bool plain);   // its tables: MLG_EALLOC where there is no room for them
 void xs_free();
 // the projection contraction as exact slices (xs_vec2tp.cu): psi, chi rows of m0 <= m < npc written; plain: FP64-grade
 // digits, else the mixed form's
 bool xv_supported(bool plain);
 int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain);
+int xv_prepare(int nrc, int npc, bool plain);
 void xv_free();
 int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc_off);
 // zeros to the rows of a mixed-form contraction's output that its kernels leave unwritten (radial.cu)

@@ -28,6 +28,20 @@ int dmalloc(void** p, size_t bytes) {
   G.mem_high = std::max(G.mem_high, G.mem_bytes);
   return 0;
 }
+int dmalloc_all(std::initializer_list<std::pair<void**, size_t>> arrays) {
+  for (auto& a : arrays) *a.first = nullptr;
+  for (auto& a : arrays) {
+    const int rc = a.second ? dmalloc(a.first, a.second) : 0;
+    if (!rc) continue;
+    for (auto& b : arrays)
+      if (*b.first) {
+        dfree(*b.first, b.second);
+        *b.first = nullptr;
+      }
+    return rc;
+  }
+  return 0;
+}
 void dfree(void* p, size_t bytes) {
   if (p) cudaFree(p);
   G.mem_bytes -= (long long)bytes;

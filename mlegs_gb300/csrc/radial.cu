@@ -637,13 +637,28 @@ static int dfma_rtrans_bwd(const cd* in, cd* out, int nrc, int mcount, const dou
   return 0;
 }
 
+// whether the slices take a contraction (mode 0, 1: the radial transforms; 2: the projection): where they cover the grid, and in
+// the plain form where there is room for their tables, since the FP64 kernels cover every grid
+static int use_slices(int mode, int nrc, int npc, bool plain, bool& use) {
+  use = mode == 2 ? xv_supported(plain) : xs_supported(mode, nrc, plain);
+  if (!use || npc < 2) return 0;   // (m = 0 has kernels of its own)
+  const int rc = mode == 2 ? xv_prepare(nrc, npc, plain) : xs_prepare(mode, nrc, npc, plain);
+  if (rc != MLG_EALLOC || !plain) return rc;
+  use = false;
+  return 0;
+}
+
 int launch_rtrans_fwd(Scalar& s) {
   int nrc, npc;
   MLG_TRY(rtrans_check(s, nrc, npc, "rtrans_forward"));
   cd* out = get_buf();
   if (!out) return set_error(MLG_EALLOC, "rtrans_forward: out of device memory");
   const bool mixed = G.precision == MLG_MIXED;
-  const bool xs = xs_supported(0, nrc, !mixed);   // exact-slice tensor-core contraction (xs_radial.cu)
+  bool xs;   // exact-slice tensor-core contraction (xs_radial.cu)
+  if (int rc = use_slices(0, nrc, npc, !mixed, xs)) {
+    put_buf(out);
+    return rc;
+  }
   // the tensor-core contractions write rows < nn(m) of every column m < npc: only the rest needs zeros
   // (beside them, below)
   if (xs && npc < 1) {
@@ -681,7 +696,11 @@ int launch_rtrans_bwd(Scalar& s, bool add_ln) {
   cd* out = get_buf();
   if (!out) return set_error(MLG_EALLOC, "rtrans_backward: out of device memory");
   const bool mixed = G.precision == MLG_MIXED;
-  const bool xs = xs_supported(1, nrc, !mixed);
+  bool xs;
+  if (int rc = use_slices(1, nrc, npc, !mixed, xs)) {
+    put_buf(out);
+    return rc;
+  }
   // the tensor-core contractions write rows < nr of every column m < npc with nn(m) > 0 (the m = 0
   // plane included): only the rest needs zeros (beside them, below)
   if (xs && npc < 1) {
@@ -726,7 +745,8 @@ int launch_rtrans_fwd_multi(Scalar* const* f, int n) {
     }
   }
   const bool mixed = G.precision == MLG_MIXED;
-  const bool xs = xs_supported(0, nrc, !mixed);
+  bool xs;
+  MLG_TRY(use_slices(0, nrc, npc, !mixed, xs));
   if (!xs || npc < 1) {
     for (int k = 0; k < n; ++k) MLG_TRY(launch_rtrans_fwd(*f[k]));
     return 0;
@@ -771,7 +791,8 @@ int launch_rtrans_bwd_multi(Scalar* const* f, int n, bool add_ln) {
     }
   }
   const bool mixed = G.precision == MLG_MIXED;
-  const bool xs = xs_supported(1, nrc, !mixed);
+  bool xs;
+  MLG_TRY(use_slices(1, nrc, npc, !mixed, xs));
   if (!xs || npc < 1) {
     for (int k = 0; k < n; ++k) MLG_TRY(launch_rtrans_bwd(*f[k], add_ln));
     return 0;
@@ -810,7 +831,8 @@ int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd
   int nzc = G.chopzl, nzcu = G.chopzu;
   if (nrc > G.ne || nrc > G.nrdim) return set_error(MLG_ECHOP, "vec2tp: chopping in r too large");
   const bool mixed = G.precision == MLG_MIXED;
-  const bool xv = xv_supported(!mixed);   // the exact-slice tensor-core contraction (xs_vec2tp.cu)
+  bool xv;   // the exact-slice tensor-core contraction (xs_vec2tp.cu)
+  MLG_TRY(use_slices(2, nrc, npc, !mixed, xv));
   // the tensor-core contractions write rows < nn(m) of the kept columns: only the rest needs zeros
   // (beside them, below)
   if (!xv) {

@@ -895,6 +895,33 @@ static int xs_launch(const XsArgs& args, int nitems) {
   return 0;
 }
 
+// the table images of a chop: made on its first transform; MLG_EALLOC where there is no room for them
+int xs_prepare(int mode, int nrc, int npc, bool plain) {
+  const int nrows = mode == 0 ? (nrc + 1) / 2 : G.nrh, kmax = mode == 0 ? G.nrh : (nrc + 1) / 2, ns = xs_cfg(kmax, nrc, plain);
+  const int nmt = cdiv(nrows, 128), nkc = cdiv(kmax, XS_KC), nrp = nmt * 128;
+  XsImg& im = g_xs[mode][plain ? 0 : 1];
+  if (im.nrc == nrc && im.npc == npc && im.p && im.ns == ns) return 0;
+  xs_drop(im);
+  im.bytes = (size_t)npc * nmt * nkc * 2 * (ns + (ns == 9)) * XS_ATILE;
+  im.abytes = (size_t)npc * (mode == 0 ? 2 : 1) * nrp * sizeof(int);
+  im.gbytes = ns == 9 ? xs_words(mode, XS_NF, npc, cdiv(nrows, 32)) * sizeof(unsigned) : 0;
+  if (int rc = dmalloc_all({{(void**)&im.p, im.bytes}, {(void**)&im.aexp, im.abytes}, {(void**)&im.again, im.gbytes}})) return rc;
+  k_xs_aexp<<<dim3(cdiv(nrp, 128), npc), 128, 0, G.stream>>>(G.pf, G.w, im.aexp, mode, G.nrh, G.ne, nrc, nrp, kmax,
+                                                                 ns == 8 || ns == 9 ? 1 : 0);
+  MLG_LAUNCH();
+  const int nblk_t = npc * nmt * nkc;
+  switch (ns) {
+    case 6: k_xs_table<6><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+    case 7: k_xs_table<7><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+    case 8: k_xs_table<8><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+    case 10: k_xs_table<10><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+    default: k_xs_table<9><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
+  }
+  MLG_LAUNCH();
+  im.nrc = nrc; im.npc = npc; im.ns = ns; im.nmt = nmt; im.nkc = nkc; im.nrp = nrp;
+  return 0;
+}
+
 // mode 0 forward, 1 backward, for m0 <= m < npc; out's rows that it writes are overwritten, the rest left
 int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int nrc, int npc, int m0,
                     const double* const* lnp, bool add_ln, bool plain) {
@@ -907,31 +934,8 @@ int xs_rtrans_multi(int mode, const cd* const* in, cd* const* out, int nf, int n
   const bool few = (long long)(npc - m0) * cdiv(G.nzdim, 16) * nf <= 76;
   if (!ns || !xs_plan(ns, xs_rawk(nrc), plan, few)) return set_error(MLG_ESIZE, "radial contraction: too many radial points for exact slices");
   const int nmt = cdiv(nrows, 128), nkc = cdiv(kmax, XS_KC), nrp = nmt * 128;
-  XsImg& im = g_xs[mode][plain ? 0 : 1];
-  if (im.nrc != nrc || im.npc != npc || !im.p || im.ns != ns) {
-    xs_drop(im);
-    im.bytes = (size_t)npc * nmt * nkc * 2 * (ns + (ns == 9)) * XS_ATILE;
-    im.abytes = (size_t)npc * (mode == 0 ? 2 : 1) * nrp * sizeof(int);
-    MLG_TRY(dmalloc((void**)&im.p, im.bytes));
-    MLG_TRY(dmalloc((void**)&im.aexp, im.abytes));
-    if (ns == 9) {
-      im.gbytes = xs_words(mode, XS_NF, npc, cdiv(nrows, 32)) * sizeof(unsigned);
-      MLG_TRY(dmalloc((void**)&im.again, im.gbytes));
-    }
-    k_xs_aexp<<<dim3(cdiv(nrp, 128), npc), 128, 0, G.stream>>>(G.pf, G.w, im.aexp, mode, G.nrh, G.ne, nrc, nrp, kmax,
-                                                                   ns == 8 || ns == 9 ? 1 : 0);
-    MLG_LAUNCH();
-    const int nblk_t = npc * nmt * nkc;
-    switch (ns) {
-      case 6: k_xs_table<6><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
-      case 7: k_xs_table<7><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
-      case 8: k_xs_table<8><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
-      case 10: k_xs_table<10><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
-      default: k_xs_table<9><<<nblk_t, 256, 0, G.stream>>>(G.pf, G.w, im.aexp, im.p, mode, G.nrh, G.ne, nrc, nmt, nkc, nrp); break;
-    }
-    MLG_LAUNCH();
-    im.nrc = nrc; im.npc = npc; im.ns = ns; im.nmt = nmt; im.nkc = nkc; im.nrp = nrp;
-  }
+  MLG_TRY(xs_prepare(mode, nrc, npc, plain));
+  const XsImg& im = g_xs[mode][plain ? 0 : 1];
   XsArgs args;
   for (int f = 0; f < XS_NF; ++f) {
     const int g = f < nf ? f : 0;

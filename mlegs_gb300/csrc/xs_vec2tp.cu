@@ -774,19 +774,16 @@ static XvCfg xv_cfg(int k, bool plain) {
 
 bool xv_supported(bool plain) { return xv_cfg(G.nrh, plain).ns > 0; }
 
-template <int NS, int NT, int W, bool PARTS = false>
-static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
+template <int NS, int NT, int W>
+static int xv_image(const XvArgs& args, XvImg& im, int npc, bool plain) {
   if (im.nrc != args.nrc || im.npc != npc || !im.p || im.ns != NS) {
     xv_drop(im);
     im.bytes = (size_t)npc * 2 * args.nmt * args.nkc * xv_tiles<NS, NT>() * XV_ATILE;
     im.ebytes = (size_t)npc * 2 * args.ntr * sizeof(int);
-    MLG_TRY(dmalloc((void**)&im.p, im.bytes));
-    MLG_TRY(dmalloc((void**)&im.rexp, im.ebytes));
-    MLG_TRY(dmalloc((void**)&im.texp, im.ebytes));
-    if (xv_mag<NS>()) {
-      im.gbytes = (size_t)npc * 2 * cdiv(args.ntr, 32) * G.nzdim * sizeof(unsigned);
-      MLG_TRY(dmalloc((void**)&im.again, im.gbytes));
-    }
+    im.gbytes = xv_mag<NS>() ? (size_t)npc * 2 * cdiv(args.ntr, 32) * G.nzdim * sizeof(unsigned) : 0;
+    if (int rc = dmalloc_all({{(void**)&im.p, im.bytes}, {(void**)&im.rexp, im.ebytes}, {(void**)&im.texp, im.ebytes},
+                              {(void**)&im.again, im.gbytes}}))
+      return rc;
     k_xv_rexp<<<dim3(cdiv(args.ntr, 128), npc * 2), 128, 0, G.stream>>>(G.tV, G.tD, G.tT, im.rexp, im.texp, G.nrh, G.ne, args.nrc,
                                                                         args.ntr, plain ? 1 : 0);
     MLG_LAUNCH();
@@ -795,6 +792,10 @@ static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
     MLG_LAUNCH();
     im.nrc = args.nrc; im.npc = npc; im.ns = NS;
   }
+  return 0;
+}
+template <int NS, int NT, int W, bool PARTS = false>
+static int xv_run(XvArgs args, const XvImg& im, int npc) {
   args.img = im.p; args.rexp = im.rexp; args.texp = im.texp;
   args.again = im.again; args.ngrp = cdiv(args.ntr, 32); args.least = xs_least_sum(2 * G.nrh);   // psi's and X's sums of two products
   const size_t fixed = 1024 + XV_SB * (size_t)xv_bstage_bytes<NS, NT>() + XV_CXS * 2 * XV_N * sizeof(int) + 512;
@@ -812,6 +813,23 @@ static int xv_run(XvArgs args, XvImg& im, int npc, bool plain) {
   return 0;
 }
 
+// the table images, as xs_prepare
+static void xv_extent(XvArgs& args, int nrc) {
+  args.nrc = nrc;
+  args.ntr = (nrc + 1) / 2;
+  args.nmt = cdiv(args.ntr, 128); args.nkc = cdiv(G.nrh, XV_KC);
+}
+int xv_prepare(int nrc, int npc, bool plain) {
+  XvArgs args{};
+  xv_extent(args, nrc);
+  XvImg& im = g_xvs[plain ? 0 : 1];
+  switch (xv_cfg(G.nrh, plain).ns) {
+    case 9: return xv_image<9, 9, 7>(args, im, npc, plain);
+    case 5: return xv_image<5, 7, 7>(args, im, npc, plain);
+    default: return xv_image<6, 8, 6>(args, im, npc, plain);
+  }
+}
+
 // psi, chi: the rows of m0 <= m < npc written (zeroed elsewhere by the caller)
 int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain) {
   if (npc <= m0) return 0;
@@ -820,10 +838,9 @@ int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int 
   XvArgs args{};
   args.ur = ur; args.up = up; args.uz = uz; args.psi = psi; args.chi = chi;
   args.ak = G.ak; args.status = (int*)(G.dscal + DS_FLAG + 1) + 1;
-  args.nr = G.nr; args.nrh = G.nrh; args.nrdim = G.nrdim; args.npdim = G.npdim; args.nzdim = G.nzdim; args.nrc = nrc;
+  args.nr = G.nr; args.nrh = G.nrh; args.nrdim = G.nrdim; args.npdim = G.npdim; args.nzdim = G.nzdim;
   args.nzc = G.chopzl; args.nzcu = G.chopzu; args.m0 = m0; args.npc = npc;
-  args.ntr = (nrc + 1) / 2;
-  args.nmt = cdiv(args.ntr, 128); args.nkc = cdiv(G.nrh, XV_KC);
+  xv_extent(args, nrc);
   {
     // the 64-bit order sums stay below 2^62: |G_d| <= K (pairs of order d) 2^(2w), with two products
     // per digit pair for psi and X
@@ -834,10 +851,11 @@ int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int 
     args.esh_s = esh(cfg.ns, 2 * cfg.ns);
     args.esh_t = esh(cfg.nt, cfg.nt);
   }
-  XvImg& im = g_xvs[plain ? 0 : 1];
-  if (cfg.ns == 9) return xs_order_bound(9, 7, 2, G.nrh) <= XS_EXACT ? xv_run<9, 9, 7>(args, im, npc, plain) : xv_run<9, 9, 7, true>(args, im, npc, plain);
-  if (cfg.ns == 5) return xv_run<5, 7, 7>(args, im, npc, plain);
-  return xv_run<6, 8, 6>(args, im, npc, plain);
+  MLG_TRY(xv_prepare(nrc, npc, plain));
+  const XvImg& im = g_xvs[plain ? 0 : 1];
+  if (cfg.ns == 9) return xs_order_bound(9, 7, 2, G.nrh) <= XS_EXACT ? xv_run<9, 9, 7>(args, im, npc) : xv_run<9, 9, 7, true>(args, im, npc);
+  if (cfg.ns == 5) return xv_run<5, 7, 7>(args, im, npc);
+  return xv_run<6, 8, 6>(args, im, npc);
 }
 
 }  // namespace mlg
