@@ -782,6 +782,7 @@ __global__ void __launch_bounds__(XS_AGAIN_T) k_xs_again(XsArgs a, const double*
         const double sgn = par ? -1.0 : 1.0;
         for (unsigned left = rows; left; left &= left - 1) {
           const int j = 2 * (g * 32 + __ffs(left) - 1) + par;
+          if (j >= nn) break;   // (words that a contraction which ran out of time left unwritten)
           double re = 0.0, im = 0.0;
           for (int i = lane; i < a.nrh; i += 32) {
             const double v = __ldg(tab + i + (size_t)a.nrh * j), wi = __ldg(w + i);

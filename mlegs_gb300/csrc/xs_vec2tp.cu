@@ -708,6 +708,7 @@ __global__ void __launch_bounds__(XS_AGAIN_T) k_xv_again(XvArgs a, const double*
       const double ss = par ? -1.0 : 1.0, mv = (double)m, kv = a.ak[z];
       for (unsigned left = rows; left; left &= left - 1) {
         const int j = 2 * (g * 32 + __ffs(left) - 1) + par;
+        if (j >= min(a.nrc, a.nrc - m)) break;   // (words that a contraction which ran out of time left unwritten)
         const size_t row = (size_t)a.nrh * (j + (size_t)ne * m);
         double v[10];   // V.F_s(ur), D.F_o(up), D.F_o(ur), V.F_s(up), T.F_s(uz)
 #pragma unroll
