@@ -18,7 +18,7 @@
 // Layout: a field is (nrdim, npdim, nzdim) with r fastest.  Both transforms run along a strided
 // dimension; a CTA takes TRL consecutive lines (the contiguous batch, so every global access is a run of
 // TRL*16 bytes) and several threads per line, which exchange through shared memory as [point][TRL].
-// Lengths: powers of two from 16 to 256 here (FP32 and FP64) and, for the plain form, in fftq.cu; others in fftr.cu and, for the
+// Lengths: powers of two from 16 to 256 here (the mixed form) and in fftq.cu (the plain one); others in fftr.cu and, for the
 // plain form where they split into two passes, in fftqr.cu.
 #include "common.cuh"
 #include "fft_common.cuh"
@@ -138,16 +138,17 @@ static int zfft2_any(const FSet& fs, int dir, double scale, int m0, int nm, cuda
 static bool pow2_fast(int L) { return L == 16 || L == 32 || L == 64 || L == 128 || L == 256; }
 
 template <typename T>
-static int vfft_t(const FSet& fs, int dir, double scale, int m0, int nm, int tr_max, cudaStream_t stream) {
+static int vfft_t(const FSet& fs, int dir, double scale, int m0, int nm, cudaStream_t stream) {
   int L = G.nz;
   if (L <= 1 || nm <= 0) return 0;
   if (pow2_fast(L)) {
-    if (tr_max >= 32) return zfft2_any<T, 32>(fs, dir, scale, m0, nm, stream);
-    // a single plane (m = 0): four lines per CTA, so that its few hundred lines spread over most SMs
-    return tr_max >= 8 ? zfft2_any<T, 8>(fs, dir, scale, m0, nm, stream) : zfft2_any<T, 4>(fs, dir, scale, m0, nm, stream);
+    // FP64: the mixed form's m = 0 plane alone, four lines per CTA, so that its few hundred lines spread over most SMs (a plain
+    // field's lines are in fixed point, but for a scale that is no power of two)
+    if constexpr (!std::is_same<T, double>::value) return zfft2_any<T, 32>(fs, dir, scale, m0, nm, stream);
+    else if (nm == 1) return zfft2_any<T, 4>(fs, dir, scale, m0, nm, stream);
   }
   if constexpr (std::is_same<T, dfl>::value) {
-    return vfft_t<double>(fs, dir, scale, m0, nm, tr_max, stream);   // other lengths: FP64
+    return vfft_t<double>(fs, dir, scale, m0, nm, stream);   // other lengths: FP64
   } else {
     return launch_zfft_r<T>(fs, TwTab<T>::rz(), dir, scale, m0, nm, stream);
   }
@@ -159,14 +160,14 @@ static int vfft_any(const FSet& fs, int dir, double scale) {
   kt_begin(1);
   if (G.precision == MLG_MIXED) {
     MLG_TRY(side_fork());
-    MLG_TRY(vfft_t<double>(fs, dir, scale, 0, 1, 2, G.side));
-    MLG_TRY(vfft_t<MixFT>(fs, dir, scale, 1, G.npdim - 1, 32, G.stream));
+    MLG_TRY(vfft_t<double>(fs, dir, scale, 0, 1, G.side));
+    MLG_TRY(vfft_t<MixFT>(fs, dir, scale, 1, G.npdim - 1, G.stream));
     MLG_TRY(side_join());
   } else {
     int sexp;
     if (fftq_length(G.nz) && std::frexp(scale, &sexp) == 0.5) MLG_TRY(launch_zfft_q(fs, dir, sexp - 1));
     else if (fftqr_pays(G.nz, (long long)G.nrdim * G.npdim * fs.n)) MLG_TRY(launch_zfft_qr(fs, dir, scale));
-    else MLG_TRY(vfft_t<double>(fs, dir, scale, 0, G.npdim, 32, G.stream));
+    else MLG_TRY(vfft_t<double>(fs, dir, scale, 0, G.npdim, G.stream));
   }
   kt_end(1, 2.0 * fs.n * G.fsize * 16);
   return 0;
@@ -222,16 +223,18 @@ static int hfft_t(const FSet& fs, int dir, double scale) {
       return 0;
     }
   }
-  if (pow2_fast(L)) {
-    switch (L) {
-      case 16: MLG_TRY((pfft2_launch<T, 16>(fs, dir, scale))); break;
-      case 32: MLG_TRY((pfft2_launch<T, 32>(fs, dir, scale))); break;
-      case 64: MLG_TRY((pfft2_launch<T, 64>(fs, dir, scale))); break;
-      case 128: MLG_TRY((pfft2_launch<T, 128>(fs, dir, scale))); break;
-      case 256: MLG_TRY((pfft2_launch<T, 256>(fs, dir, scale))); break;
+  if constexpr (!std::is_same<T, double>::value) {
+    if (pow2_fast(L)) {
+      switch (L) {
+        case 16: MLG_TRY((pfft2_launch<T, 16>(fs, dir, scale))); break;
+        case 32: MLG_TRY((pfft2_launch<T, 32>(fs, dir, scale))); break;
+        case 64: MLG_TRY((pfft2_launch<T, 64>(fs, dir, scale))); break;
+        case 128: MLG_TRY((pfft2_launch<T, 128>(fs, dir, scale))); break;
+        case 256: MLG_TRY((pfft2_launch<T, 256>(fs, dir, scale))); break;
+      }
+      kt_end(1, 2.0 * fs.n * G.fsize * 16);
+      return 0;
     }
-    kt_end(1, 2.0 * fs.n * G.fsize * 16);
-    return 0;
   }
   if constexpr (std::is_same<T, dfl>::value) {
     kt_end(1, 0.0);

@@ -132,20 +132,6 @@ __device__ __forceinline__ uint32_t xs_mag2(long long X0, long long X1) {
 constexpr int XS_AGAIN = 4861, XS_AGAIN_T = 256;   // their warps (about 32 an SM) and threads per CTA
 inline float xs_least_sum(int K) { return (float)(std::exp2(62.0 - 8.9) * std::sqrt(K / 96.0)); }
 
-// the FP32 value of a small integer (|d| < 2^22), exactly, on the FP32 pipe
-__device__ __forceinline__ float xs_i2f(int d) { return __int_as_float(0x4B400000 + d) - 12582912.0f; }
-
-// the NS digits of X as FP32 values (each exact, so its BF16 pattern is the top half of its bits)
-template <int NS>
-__device__ __forceinline__ void xs_digits_f(long long X, int w, float* f) {
-  const unsigned mask = (1u << w) - 1u;
-  f[0] = xs_i2f((int)(X >> (w * (NS - 1))));
-#pragma unroll
-  for (int s = 1; s < NS; ++s) f[s] = xs_i2f((int)((unsigned)(X >> (w * (NS - 1 - s))) & mask));
-}
-// two FP32 digit values as one packed BF16 pair (a low, b high)
-__device__ __forceinline__ uint32_t xs_pack(float a, float b) { return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632); }
-
 // the exact integer value of an FP32 accumulator entry (integral, |x| < 2^24)
 __device__ __forceinline__ int xs_f2i(float x) { return __float2int_rn(x); }
 
@@ -178,40 +164,6 @@ __device__ __forceinline__ double xs_i64_to_double(long long T, int e2) {
   if (a == 0ull || ex <= 0) return __longlong_as_double((long long)sign);
   if (ex >= 2047) return __longlong_as_double((long long)(sign | 0x7FF0000000000000ull));
   return __longlong_as_double((long long)(sign | bits));
-}
-
-// y 2^e2 as FP64, exactly (FP32 subnormals and results below the normal range give zero)
-__device__ __forceinline__ double xs_f2d_scaled(float y, int e2) {
-  const unsigned f = __float_as_uint(y);
-  const unsigned e = (f >> 23) & 0xFFu;
-  if (e == 0u) return 0.0;
-  const int ex = (int)e + 896 + e2;   // FP64 exponent field
-  if (ex <= 0) return 0.0;
-  const unsigned sign = f & 0x80000000u, m = f & 0x7FFFFFu;
-  const unsigned hi = sign | ((unsigned)min(ex, 2047) << 20) | (m >> 3);
-  return __hiloint2double((int)hi, (int)(m << 29));
-}
-
-// double-float accumulation of exact FP32 terms: (hi, lo) += x (Knuth's two-sum; lo collects the
-// rounding errors, which are exact)
-__device__ __forceinline__ void xs_df_add(float& hi, float& lo, float x) {
-  const float s = __fadd_rn(hi, x), v = __fsub_rn(s, hi);
-  const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, v)), __fsub_rn(x, v));
-  hi = s;
-  lo = __fadd_rn(lo, e);
-}
-
-// sum_d G_d 2^(-w d) of NO exact accumulator orders in double-float, then times 2^e2 as FP64 (about 46
-// bits: enough for the mixed form's 35-bit digits; the plain form combines in 64-bit integers)
-template <int NO>
-__device__ __forceinline__ void xs_orders_df(const float* g, int w, float& hi, float& lo) {
-  hi = g[0];
-  lo = 0.f;
-#pragma unroll
-  for (int d = 1; d < NO; ++d) xs_df_add(hi, lo, g[d] * __int_as_float((127 - w * d) << 23));
-}
-__device__ __forceinline__ double xs_df_to_double(float hi, float lo, int e2) {
-  return xs_f2d_scaled(hi, e2) + xs_f2d_scaled(lo, e2);
 }
 
 }  // namespace mlg
