@@ -9,8 +9,8 @@
 // a K-term sum of the products of one digit order stays exact while K (pairs of the order) 2^(2w) < 2^24.
 // Balanced digits (nb = 63): the digits after the first lie in [-2^(w-1), 2^(w-1)) and the first, of
 // eight bits, in [-128, 128), so a digit product is at most 2^(2w-2) (2^(w+6) with one first digit, 2^14 with two) and
-// the order sums stay exact for 8 digits of 8 bits up to K = 128 and for 9 of 7 bits up to K = 372 (unsigned digits
-// need 9 of 7 bits up to K = 113 and 10 of 6, 60 bits, beyond).
+// the order sums stay exact for 8 digits of 8 bits up to K = 128 and for 9 of 7 bits up to K = 372, half of that where an
+// order holds two products (xs_order_bound; unsigned digits need 9 of 7 bits up to K = 113 and 10 of 6, 60 bits, beyond).
 // The first digit needs |X| < 2^63 - 2^56, so that the carry of the digits below it does not leave its eight bits: the
 // scale E of a row or column whose largest magnitude has its upper six fraction bits set is one larger
 // (xs_ebound_bal).

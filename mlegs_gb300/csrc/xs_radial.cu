@@ -160,11 +160,16 @@ __device__ __forceinline__ bool xs_wait(uint64_t* bar, uint32_t phase, bool& ok)
   ok = mbar_wait(bar, phase);
   return ok;
 }
-
-
+// a bounded wait whose outcome every lane of the warp shares (the warp-collective operations that
+// follow need the whole warp)
+__device__ __forceinline__ bool xs_wait_w(uint64_t* bar, uint32_t phase, bool& ok) {
+  xs_wait(bar, phase, ok);
+  ok = __all_sync(0xFFFFFFFFu, ok);
+  return ok;
+}
 
 // Warp roles of the contraction kernel (896 threads, one CTA per SM):
-//   warp 0        the table entries, by bulk copy (one thread)
+//   warp 0        the table entries and magnitude tiles, by bulk copy (one thread)
 //   warp 1        MMA issue and the tensor-memory allocation
 //   warps 2, 3    the items' field columns, by bulk copy (one thread), and their scales
 //   warps 4..11   field digits, in two groups that take the stages in turn
@@ -180,14 +185,6 @@ __device__ __forceinline__ bool xs_wait(uint64_t* bar, uint32_t phase, bool& ok)
 // Ten steps' radial transforms at 192 x 128 x 128, mixed: 4.27 -> 3.49 ms against eight-warp epilogues that released both
 // parities together and reduced the scales themselves (20 700 cycles an item); 512 x 512 x 256, two mixed steps:
 // 22.4 -> 15.1 ms; plain: 2.48 -> 1.70 ms for four steps.
-// a bounded wait whose outcome every lane of the warp shares (the warp-collective operations that
-// follow need the whole warp)
-__device__ __forceinline__ bool xs_wait_w(uint64_t* bar, uint32_t phase, bool& ok) {
-  xs_wait(bar, phase, ok);
-  ok = __all_sync(0xFFFFFFFFu, ok);
-  return ok;
-}
-
 constexpr int XS_SBMAX = 4, XS_AEMAX = 8, XS_MEMAX = 2;   // ring sizes (at most)
 constexpr int XS_CXS = 4;                   // column-scale slots (items)
 constexpr int XS_NSW = 2, XS_NDW = 8, XS_NEW = 16;   // scale warps (2, 3), digit warps (4..11), epilogue warps (12..27)
@@ -212,8 +209,8 @@ template <int NS> __host__ __device__ constexpr int xs_esh() {
 // 372 and nine digits, 2^22.9 2^(42 - 3)
 template <int NS> __host__ __device__ constexpr int xs_low() { return NS == 9 ? 3 : 0; }
 template <int NS> __host__ __device__ constexpr int xs_cb() { return xs_w<NS>() * (NS - 2) - xs_low<NS>(); }
-// the shift for sums with |C| <= mx: |T| <= (mx + 2^16) 2^(cb - esh) < 2^62 (|L| 2^-cb <= 2^16), so that the sum of two
-// fits 64 bits too
+// the shift for a sum with |C| = mx: |T| <= (mx + 2^16) 2^(cb - esh) < 2^62 (|L| 2^-cb <= 2^16), so that the sum of two
+// fits 64 bits too; at most 15, since |C| < 2^30 (nine digits, K <= 372) or 2^29 (eight, K <= 113)
 template <int NS> __device__ __forceinline__ int xs_order_shift(int mx) {
   return max(32 - __clz(mx + 65536) + xs_cb<NS>() - 62, 0);
 }

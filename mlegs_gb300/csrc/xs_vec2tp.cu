@@ -26,10 +26,13 @@
 // Plain form: nine balanced digits of 7 bits (63 bits) for all three, up to 744 radial points.  An order of psi or X holds two
 // products per digit pair and is exact up to 186 terms (xs_order_bound); beyond 372 radial points the accumulators are drained
 // every 176 and the parts added in 64-bit integers.  The order sums are shifted by what they need (xs_radial.cu): cut at a fixed
-// 2^-52, as 54-bit slices once were, chi = k X - Y is left 7e-9 from FP64.
+// 2^-52, as 54-bit slices once were, chi = k X - Y is left 7e-9 from FP64.  Beside the digits the magnitudes are contracted
+// (xs_least_sum): psi and chi of outputs whose terms are all small beside their row's and column's largest entries, and of
+// columns with non-finite samples, are summed again in FP64 (k_xv_again).
 //
 // Engine: a persistent grid of one CTA per SM over work items (m, 8 complex z columns, 128-row tile, parity).
-//   warp 0        the table entries (the digits of m V, D or T for a chunk of 16 radial points), by bulk copy
+//   warp 0        the table entries (the digits, and in the plain form the magnitudes, of m V, D or T for a chunk of 16
+//                 radial points), by bulk copy
 //   warp 1        MMA issue: a table digit t meets every field digit s <= n-1-t of its operands in
 //                 one MMA (M = 128, K = 16; the field digits side by side in shared memory, the orders side by
 //                 side in tensor memory, psi's and X's alternating), two where that passes 256 columns
