@@ -174,10 +174,13 @@ void xs_free();
 // the projection contraction as exact slices (xs_vec2tp.cu): psi, chi rows of m0 <= m < npc written; plain: FP64-grade
 // digits, else the mixed form's
 bool xv_supported(bool plain);
-int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain);
+int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain, bool dealias_next);
 int xv_prepare(int nrc, int npc, bool plain);
 void xv_free();
-int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc_off);
+int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc_off, bool dealias_next);
+// the dealias mask keeps m < pcut and, of k = z + 1, k <= zcut and k >= nz - zcut + 2
+inline int dealias_pcut() { return std::max(G.np / 3 + 1, 1); }
+inline int dealias_zcut() { return std::max(G.nz / 3 + 1, 1); }
 // zeros to the rows of a mixed-form contraction's output that its kernels leave unwritten (radial.cu)
 int launch_zero_tails(cd* out, int mode, int nrc, int npc, int nzc, int nzcu);
 int launch_zero_tails_n(cd* const* out, int n, int mode, int nrc, int npc, int nzc, int nzcu, cudaStream_t st = nullptr);

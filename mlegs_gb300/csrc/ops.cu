@@ -668,7 +668,7 @@ static int mask_launch(Scalar* const* f, int n, bool chop, bool dealias, const C
   fs.lnz[0] = lnz0;
   fs.lnz[1] = lnz1;
   const Scalar& s = *f[0];
-  int pcut = std::max(G.np / 3 + 1, 1), zcut = std::max(G.nz / 3 + 1, 1), zupper = G.nz - zcut + 2;
+  const int pcut = dealias_pcut(), zcut = dealias_zcut(), zupper = G.nz - zcut + 2;
   k_mask<<<cdiv((long long)n * G.npdim * G.nzdim, 8), 256, 0, G.stream>>>(
       fs, G.nrdim, G.npdim, G.nzdim, chop ? 1 : 0, dealias ? 1 : 0, s.space[0] == 'F', s.space[1] == 'F', s.space[2] == 'F',
       c.nrc, c.npc, c.nzc, c.nzcu, pcut, zcut, zupper, G.np > 1, G.nz > 1);
@@ -1096,7 +1096,8 @@ int scale_r(Scalar& s, int mode) {
 
 // vector_projection on (ur, up, uz) PPP fields that it may overwrite (the caller's copies or its own
 // temporaries): r*ur, r*up enter the φ transforms (scale_r folded into them)
-static int vec2tp_core(Scalar& ur, Scalar& up, Scalar& uz, Scalar& psi, Scalar& chi) {
+// dealias_next: the caller's next operation on psi and chi is the dealias mask
+static int vec2tp_core(Scalar& ur, Scalar& up, Scalar& uz, Scalar& psi, Scalar& chi, bool dealias_next = false) {
   // the three components stage by stage, each stage one launch over the three: phi forward (ur and up
   // times r first), then up's radial forward (op_trans's PFP -> FFP step), then z forward
   Scalar* u3[3] = {&ur, &uz, &up};   // up last: its radial transform follows while it is in L2
@@ -1124,7 +1125,7 @@ static int vec2tp_core(Scalar& ur, Scalar& up, Scalar& uz, Scalar& psi, Scalar& 
   // and chi%e = 0 (:1330-1331) are the zeros written by the contraction below
   k_proj_ln<<<1, 256, 0, G.stream>>>(up.e, (const double2*)(G.dscal + DS_CALC), -1.0 / 2.0, psi.ln, chi.ln, G.x, G.nr);
   MLG_LAUNCH();
-  MLG_TRY(launch_vec2tp_contract(ur.e, up.e, uz.e, psi.e, chi.e, 3));
+  MLG_TRY(launch_vec2tp_contract(ur.e, up.e, uz.e, psi.e, chi.e, 3, dealias_next));
   MLG_TRY(op_idel2(chi, false, 0.0));
   psi.off[0] = psi.off[1] = psi.off[2] = 0;
   chi.off[0] = chi.off[1] = chi.off[2] = 0;
@@ -1250,7 +1251,7 @@ int op_advection_rhs(Scalar& psi, Scalar& chi, Scalar& nlpsi, Scalar& nlchi, con
   // (vz + uz) with the background flow; in place, or into the temporaries when v and w are kept
   Scalar* prod[3] = {&vr_t, &vp_t, &vz_t};
   MLG_TRY(vecprod_bg(vr, vp, vz, wr, wp, wz, &uz, keep ? prod : nullptr));
-  MLG_TRY(vec2tp_core(vr_t, vp_t, vz_t, nlpsi, nlchi));
+  MLG_TRY(vec2tp_core(vr_t, vp_t, vz_t, nlpsi, nlchi, true));
   MLG_TRY(op_zero_ln_dealias2(nlpsi, nlchi));   // ln = 0, then dealias
   return 0;
 }

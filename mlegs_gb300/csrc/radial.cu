@@ -826,7 +826,7 @@ int launch_rtrans_bwd_multi(Scalar* const* f, int n, bool add_ln) {
 }
 
 // ur, up, uz in (r physical, m, k) space; psi and chi written in full
-int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc_off) {
+int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc_off, bool dealias_next) {
   int nrc = G.nrchop + nrc_off, npc = G.npchop;
   int nzc = G.chopzl, nzcu = G.chopzu;
   if (nrc > G.ne || nrc > G.nrdim) return set_error(MLG_ECHOP, "vec2tp: chopping in r too large");
@@ -850,7 +850,7 @@ int launch_vec2tp_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd
     MLG_TRY(launch_zero_tails_n(pc, 2, 0, nrc, npc, nzc, nzcu, G.side));
     MLG_TRY(mixed ? plane_vec2tp<dfl>(ur, up, uz, psi, chi, nrc, nzc, nzcu, G.side)
                   : plane_vec2tp<double>(ur, up, uz, psi, chi, nrc, nzc, nzcu, G.side));
-    MLG_TRY(xv_contract(ur, up, uz, psi, chi, nrc, npc, 1, !mixed));
+    MLG_TRY(xv_contract(ur, up, uz, psi, chi, nrc, npc, 1, !mixed, dealias_next));
     MLG_TRY(side_join());
     kt_end(KT_V2TP, 5.0 * fwd_flops(nrc, npc));
     return 0;

@@ -161,6 +161,7 @@ struct XvArgs {
   int nr, nrh, nrdim, npdim, nzdim, nrc, nzc, nzcu, nmt, nkc, ntr, m0, npc;
   int aent;           // table entries of the ring
   unsigned* again;    // plain form: the outputs to be summed again, a word of 32 rows (xv_word)
+  int again_m, again_zl, again_zu;   // of them those of m < again_m and of z + 1 <= again_zl or >= again_zu
   int ngrp;
   float least;        // xs_least_sum
   int esh_s, esh_t;   // two's complement digits: right shifts that keep the 64-bit order sums of psi / X and of Y below 2^62
@@ -700,7 +701,9 @@ __global__ void __launch_bounds__(XS_AGAIN_T) k_xv_again(XvArgs a, const double*
       place(mine);
       const int nn = max(min(a.nrc, a.nrc - m), 0);
       // (words of other rows and columns are not written)
-      if (m >= a.m0 && 2 * (g * 32) + par < nn && (z + 1 <= a.nzc || z + 1 >= a.nzcu)) word = a.again[mine];
+      if (m >= a.m0 && m < a.again_m && 2 * (g * 32) + par < nn && (z + 1 <= a.nzc || z + 1 >= a.nzcu) &&
+          (z + 1 <= a.again_zl || z + 1 >= a.again_zu))
+        word = a.again[mine];
     }
     for (unsigned todo = __ballot_sync(0xFFFFFFFFu, word != 0); todo; todo &= todo - 1) {
       const int src = __ffs(todo) - 1;
@@ -834,8 +837,9 @@ int xv_prepare(int nrc, int npc, bool plain) {
   }
 }
 
-// psi, chi: the rows of m0 <= m < npc written (zeroed elsewhere by the caller)
-int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain) {
+// psi, chi: the rows of m0 <= m < npc written (zeroed elsewhere by the caller).  dealias_next: outputs that the caller's dealias
+// mask zeroes are not summed again (many of the marked ones are high modes: 41 -> 19 us in the nonlinear term at 256 x 128 x 128)
+int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int nrc, int npc, int m0, bool plain, bool dealias_next) {
   if (npc <= m0) return 0;
   const XvCfg cfg = xv_cfg(G.nrh, plain);
   if (!cfg.ns) return set_error(MLG_ESIZE, "vec2tp: too many radial points for exact slices");
@@ -843,6 +847,10 @@ int xv_contract(const cd* ur, const cd* up, const cd* uz, cd* psi, cd* chi, int 
   args.ur = ur; args.up = up; args.uz = uz; args.psi = psi; args.chi = chi;
   args.ak = G.ak; args.status = (int*)(G.dscal + DS_FLAG + 1) + 1;
   args.nr = G.nr; args.nrh = G.nrh; args.nrdim = G.nrdim; args.npdim = G.npdim; args.nzdim = G.nzdim;
+  const bool dp = dealias_next && G.np > 1, dz = dealias_next && G.nz > 1;
+  args.again_m = dp ? std::min(npc, dealias_pcut()) : npc;
+  args.again_zl = dz ? dealias_zcut() : G.nzdim;
+  args.again_zu = dz ? G.nz - dealias_zcut() + 2 : 1;
   args.nzc = G.chopzl; args.nzcu = G.chopzu; args.m0 = m0; args.npc = npc;
   xv_extent(args, nrc);
   {
