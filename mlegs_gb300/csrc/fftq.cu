@@ -4,7 +4,7 @@
 // Why: GB300 issues about 2 FP64 operations per clock per SM and 64 32-bit integer ones; a 64-bit addition takes two of the
 // latter, a multiplication by a constant seven.  The FP64 transforms stood at that pipe: 218 us for the z transform of
 // three fields at 192 x 128 x 128 (about 23 FP64 operations a sample), 275 and 307 us for the phi transforms, where the
-// fields' way through HBM takes 23.  Now 75 us (z), 72 us (phi forward) and 83 us (phi backward).
+// fields' way through HBM takes 23.  Now 80 us (z), 68 us (phi forward) and 79 us (phi backward).
 //
 // Scaling: every line has its own power of two.  With S >= sum_n (|re x_n| + |im x_n|), 2^es > S, the samples are rounded to
 // integers X_n = x_n 2^(NB - es); no partial sum of a DFT exceeds sum |X_n| < 2^NB in modulus, so nothing overflows at any

@@ -45,8 +45,8 @@
 // What bounds it (clock64 traces, 192 points): plain, the MMAs, 1 200 cycles an entry, three entries a chunk, and 4 000
 // cycles more a unit while the epilogue drains tensor memory (its three sets of order sums fill it, so that units do
 // not overlap there).  Mixed: the MMAs (600 an entry) and the digits (2 300 a chunk for each of two groups) alike.
-// Per launch at 192 x 128 x 128: plain 259 us (FP64 DFMA 2 602; 302 while one lane issued the MMAs from a branch), mixed
-// 199 us (234; 264 when one CTA of 256 threads walked scales, chunks and epilogue in turn); 512 x 512 x 256 mixed 5.4 ms
+// Per launch at 192 x 128 x 128 (ncu): plain 263 us and 36 for k_xv_again (221 without the magnitudes; FP64 DFMA 2 602), mixed
+// 176 us (events: 199; 234 while one lane issued the MMAs from a branch; 264 when one CTA of 256 threads walked scales, chunks and epilogue in turn); 512 x 512 x 256 mixed 5.4 ms
 // (6.7; 7.3).
 #include "common.cuh"
 #include "tc_common.cuh"
