@@ -11,8 +11,8 @@
 // stage.  Sums are exact; a multiplication by a twiddle of 61 bits rounds to about the nearest integer; a result is
 // rounded once to FP64.  From 128 points on the first pass has a finer unit of its own (q_scale).  The rounding is
 // below the FP64 transforms' at every length: against extended precision, in units of 2^-53 of a line's root mean square
-// (white, decaying and one-mode lines; FP64 beside it), z: 0.2-0.5 (0.9-1.7) at 64 points, 0.3-0.5 (1.1-2.0) at 256; phi:
-// 0.3-0.8 (1.2-2.1) at np = 128, 0.5-0.7 (1.1-2.3) at 512.
+// (white, decaying and one-mode lines; FP64 beside it), z: 0.4-0.5 (0.9-1.7) at 64 points, 0.4-0.5 (1.1-2.0) at 256; phi:
+// 0.5-0.6 (1.2-2.1) at np = 128, 0.5-0.6 (1.1-2.3) at 512.
 // A block one of whose lines holds a non-finite or a huge sample (2^1007 and up) or none above 2^-922 (but not all zero)
 // takes the FP64 transform.
 //
@@ -86,7 +86,7 @@ __device__ __forceinline__ void q_fft2pass(qc* a, qc (*b)[Split<L>::R2], qc* S, 
 // the line's scale from its R2 threads' shares: sum |x| < 2^e over the line, and < 2^e1 over any one thread's samples
 // (HALF: over those of threads w and R2 - w together), sh = e - e1; false where the line needs FP64.  A thread's samples
 // are what the first pass sums: its own, finer unit keeps the rounding of the first pass' twiddles, which all later
-// stages add up, below that of the second's (np = 512, white: 2.6 -> 0.65 units of 2^-53; it costs 2 % of the time)
+// stages add up, below that of the second's (np = 512, white: 2.6 -> 0.6 units of 2^-53; it costs 2 % of the time)
 template <int L, int TRL, bool HALF> __device__ __forceinline__ bool q_scale(const QStat* red, int lane, QScale& sc) {
   constexpr int R2 = Split<L>::R2;
   unsigned mx = 0;

@@ -4,7 +4,7 @@
 // Scaling, rounding and the lines that take the FP64 transform are as in fftq.cu; lines of 80 points and more have the finer
 // unit of their own in the first pass, up to and with the twiddles between the passes.  The rounding is a quarter of the FP64
 // transforms' (whose twiddle angles are rounded besides): in units of 2^-53 of a line's root mean square, FP64 beside it, z:
-// 0.4-0.8 (0.9-2.8) at 48 points, 0.4-0.6 (1.1-3.1) at 240; phi: 0.4-0.9 (1.1-4.0) at np = 96, 0.5-0.7 (1.1-3.8) at 480.
+// 0.4-0.8 (0.9-2.8) at 48 points, 0.4-0.7 (1.1-3.1) at 240; phi: 0.5-0.8 (1.1-4.0) at np = 96, 0.5-0.7 (1.1-3.8) at 480.
 //
 // Shape: n = n2 + R2 n1, k = k1 + R1 k2, two register passes through shared memory.  A thread of the first pass takes the R1
 // points of one n2, one of the second the R2 values of one k1; a transform of R points is done as P1 P2 points, P1 of 2..5,
