@@ -723,8 +723,8 @@ __global__ void __launch_bounds__(XS_THREADS, 1) k_xs_rtrans(XsArgs a) {
 // ------------------------------------------------------------------------------------------------
 // The marked outputs of the nine-digit form, summed in FP64 (as the FP64 kernels of radial.cu sum, term after term, backward).
 // Few and scattered, or whole regions (the points near the axis where the functions of high m vanish), so each warp takes words
-// from all over the grid, XS_AGAIN (a prime) apart.  Backward: a lane per row of the word, the table read along the rows.  Forward: a marked row after the
-// other, the lanes over the radial points.  Nothing marked: 4 us.
+// from all over the grid, XS_AGAIN (a prime) apart.  Backward: a lane per row of the word, the table read along the rows.
+// Forward: a marked row after the other, the lanes over the radial points.  Nothing marked: 4 us.
 template <int MODE>
 __global__ void __launch_bounds__(XS_AGAIN_T) k_xs_again(XsArgs a, const double* __restrict__ pf, const double* __restrict__ w, int ne,
                                                   size_t nwords) {
@@ -887,7 +887,8 @@ static int xs_launch(const XsArgs& args, int nitems) {
   kern<<<std::min(nitems, 152), XS_THREADS, sm, G.stream>>>(args);
   MLG_LAUNCH();
   if constexpr (xs_mag<NS>() != 0) {
-    k_xs_again<MODE><<<cdiv(XS_AGAIN, XS_AGAIN_T / 32), XS_AGAIN_T, 0, G.stream>>>(args, G.pf, G.w, G.ne, xs_words(MODE, args.nf, args.npc, args.ngrp));
+    k_xs_again<MODE><<<cdiv(XS_AGAIN, XS_AGAIN_T / 32), XS_AGAIN_T, 0, G.stream>>>(args, G.pf, G.w, G.ne,
+                                                                                 xs_words(MODE, args.nf, args.npc, args.ngrp));
     MLG_LAUNCH();
   }
   return 0;

@@ -46,8 +46,8 @@
 // cycles more a unit while the epilogue drains tensor memory (its three sets of order sums fill it, so that units do
 // not overlap there).  Mixed: the MMAs (600 an entry) and the digits (2 300 a chunk for each of two groups) alike.
 // Per launch at 192 x 128 x 128 (ncu): plain 263 us and 36 for k_xv_again (221 without the magnitudes; FP64 DFMA 2 602), mixed
-// 176 us (events: 199; 234 while one lane issued the MMAs from a branch; 264 when one CTA of 256 threads walked scales, chunks and epilogue in turn); 512 x 512 x 256 mixed 5.4 ms
-// (6.7; 7.3).
+// 176 us (events: 199; 234 while one lane issued the MMAs from a branch; 264 when one CTA of 256 threads walked scales, chunks and
+// epilogue in turn); 512 x 512 x 256 mixed 5.4 ms (6.7; 7.3).
 #include "common.cuh"
 #include "tc_common.cuh"
 #include "xs_common.cuh"
@@ -388,7 +388,9 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
           entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0, 0, bm, TM, kc > k0);
           if (ok) entry(std::integral_constant<int, NS>(), std::integral_constant<int, 2>(), b0 + 2 * NS * XV_BTILE, 0, bm + 2 * XV_BTILE, TM, true);
           if (kc == k0 && u > 0) xs_wait_w(&bar_te[1], (u - 1) & 1, ok);
-          if (ok) entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, bm + 4 * XV_BTILE, TM + 2 * N, kc > k0);
+          if (ok)
+            entry(std::integral_constant<int, NT>(), std::integral_constant<int, 1>(), b0 + 4 * NS * XV_BTILE, TY, bm + 4 * XV_BTILE,
+                  TM + 2 * N, kc > k0);
           if (!ok) break;
           umma_commit(&bar_be[sb], el);
           if (++sb == XV_SB) { sb = 0; pb ^= 1u; }
@@ -433,7 +435,10 @@ __global__ void __launch_bounds__(XV_THREADS, 1) k_xv_contract(XvArgs a) {
       }
       if ((lane & 7) == 0) {
         // an all-subnormal column counts as zero
-        auto bound = [](unsigned h) { return BAL && xs_nonfin(h) ? XS_NONFIN : !(h >> 20) ? -2000 : (BAL ? xs_ebound_bal(h) : (int)(h >> 20) - 1022) + 1; };
+        auto bound = [](unsigned h) {
+          if (BAL && xs_nonfin(h)) return XS_NONFIN;
+          return !(h >> 20) ? -2000 : (BAL ? xs_ebound_bal(h) : (int)(h >> 20) - 1022) + 1;
+        };
         int* cx = cxs + slot * 2 * N;
         cx[2 * zz] = bound(e0);
         cx[2 * zz + 1] = bound(e1);
